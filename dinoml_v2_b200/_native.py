@@ -18,6 +18,7 @@ ACTIVATIONS = {"silu": 1, "fast_gelu": 2}
 DEQUANT_DTYPE = {"float32": 0, "float16": 1, "bfloat16": 2}
 
 _lib = None
+_binding = None
 
 
 def variant_code(variant) -> int:
@@ -81,6 +82,20 @@ def lib() -> ctypes.CDLL:
     L.dinoml_b200_peer_enable_access.restype = ci
     _lib = L
     return L
+
+
+def binding():
+    """The CPython module over the library (csrc/torch_binding.cpp): tensors in, tensors out, one native call."""
+    global _binding
+    if _binding is None:
+        lib()                                   # a missing library is reported by its own message
+        import torch  # noqa: F401              (the module links torch's libraries, which this import loads)
+        try:
+            from . import _torch_binding
+        except ImportError as exc:
+            raise NativeLibraryMissing(f"_torch_binding.so is missing or does not load ({exc}): build it with `python -m dinoml_v2_b200.build`") from exc
+        _binding = _torch_binding
+    return _binding
 
 
 def last_error() -> str:

@@ -23,9 +23,25 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
         raise ValueError(f"{name} must be contiguous")
 
 
+_binding = None
+
+
+def _native_call(name: str):
+    """A function of the native binding.  The binding is loaded on the first call."""
+    global _binding
+    if _binding is None:
+        _binding = _native.binding()
+    return getattr(_binding, name)
+
+
 def dequantize_rows(blocks: torch.Tensor, qtype, n_per_row: int, dtype: str = "float32", out: torch.Tensor | None = None,
                     stream=None) -> torch.Tensor:
     """uint8 [rows, row_bytes] GGUF blocks -> dense [rows, n_per_row] (bit-exact dequantization)."""
+    done = _native_call("dequantize")(blocks, qtype, n_per_row, dtype, out, stream)      # None: not the plain case, checked below
+    if done is not None:
+        if type(done) is int:
+            _native.check(done, "libgguf_cuda_dequantize_rows_on_stream")
+        return done
     q = qtype_of(qtype)
     _require_cuda(blocks, "blocks")
     if blocks.dtype != torch.uint8 or blocks.dim() != 2 or blocks.shape[1] != row_bytes(q, n_per_row):
@@ -43,6 +59,11 @@ def dequantize_rows(blocks: torch.Tensor, qtype, n_per_row: int, dtype: str = "f
 def gemm_rcr(a: torch.Tensor, b_quant: torch.Tensor, qtype, bias: torch.Tensor | None = None, *, variant: str = "auto",
              out: torch.Tensor | None = None, stream=None) -> torch.Tensor:
     """a [..., K] x GGUF-encoded weight (uint8 [N, row_bytes]) -> [..., N], same dtype as `a`."""
+    done = _native_call("linear")(a, b_quant, qtype, bias, variant, out, stream)          # None: not the plain case, checked below
+    if done is not None:
+        if type(done) is int:
+            _native.check(done, "dinoml_b200_gguf_gemm_rcr")
+        return done
     q = qtype_of(qtype)
     _require_cuda(a, "a")
     _require_cuda(b_quant, "b_quant")
@@ -93,6 +114,11 @@ def dual_gemm_rcr(a: torch.Tensor, b01_interleaved: torch.Tensor, qtype, activat
     interleave_rows8(B0, B1), `bias01_interleaved` = interleave_bias8(bias0, bias1) in the activation dtype.
     a [..., K] -> [..., N] with N = rows of each matrix.  Mirrors dml.ops.dual_gemm_rcr_silu / _fast_gelu and their
     _bias_ forms of the reference (src/dinoml/ops/gemm.py:63-121) for GGUF weights."""
+    done = _native_call("gated")(a, b01_interleaved, qtype, bias01_interleaved, variant, out, stream, activation)
+    if done is not None:
+        if type(done) is int:
+            _native.check(done, "dinoml_b200_gguf_dual_gemm_rcr")
+        return done
     q = qtype_of(qtype)
     _require_cuda(a, "a")
     _require_cuda(b01_interleaved, "b01_interleaved")

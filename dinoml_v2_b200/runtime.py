@@ -204,12 +204,14 @@ class Session:
         module._check(self._lib.dino_session_create(module._handle, ctypes.byref(self._handle)))
         self._pinned: dict[str, Any] = {}
         self._numpy_plans: dict[Any, dict[str, Any]] = {}
+        self._runner: Any = None              # native form of run_torch, made on its first call
         self._user_stream = 0
         self._graph_replay = False
         self.numpy_graph_replay = True        # run_numpy keeps its arenas, so its launch sequences are replayed as CUDA graphs
         self.numpy_zero_copy_bytes = 65536    # run_numpy: results up to this size are stored by the kernels into pinned host memory
 
     def close(self) -> None:
+        self._runner = None
         if self._handle:
             self._lib.dino_session_destroy(self._handle)
             self._handle = None
@@ -258,7 +260,35 @@ class Session:
         ins, outs, keep = self._pack(inputs, outputs)
         self.module._check(self._lib.dino_session_run(self._handle, ins, len(ins), outs, len(outs)))
 
+    def _make_runner(self):
+        """What the native run_torch needs of the graph: ports by name and tensor number, and how shapes follow from the nodes."""
+        if not hasattr(self, "_graph"):
+            self._graph = json.loads((self.module.path / "graph.dinoir.json").read_text())
+        graph = self._graph
+        consts = {c["name"]: c for c in graph["constants"]}
+        number: dict[str, int] = {}
+        for name in [i["name"] for i in graph["inputs"]] + [n["outputs"][0] for n in graph["nodes"]]:
+            number.setdefault(name, len(number))
+        nodes = []
+        for node in graph["nodes"]:
+            rows = consts[node["inputs"][1]]["shape"][0]
+            nodes.append((number[node["inputs"][0]], number[node["outputs"][0]], rows // 2 if node["op"].startswith("dual_gemm_rcr_") else rows))
+        ports = lambda entries: [(e["name"], number[e["name"]], e["dtype"]) for e in entries]
+        from . import _native
+        run = ctypes.cast(self._lib.dino_session_run, ctypes.c_void_p).value
+        return _native.binding().make_runner(run, self._handle.value, len(number), ports(self.module.metadata["inputs"]),
+                                             ports(self.module.metadata["outputs"]), nodes)
+
     def run_torch(self, inputs: Mapping[str, Any], outputs: Mapping[str, Any] | None = None) -> dict[str, Any]:
+        if self._handle:
+            if self._runner is None:
+                from . import _native
+                self._runner, self._run_native = self._make_runner(), _native.binding().run_torch
+            done = self._run_native(self._runner, inputs, outputs)        # None: not the plain case, taken apart below
+            if done is not None:
+                if type(done) is int:
+                    self.module._check(done)
+                return done
         import torch
         meta = self.module.metadata
         out_shapes = self._output_shapes({k: tuple(v.shape) for k, v in inputs.items()})
