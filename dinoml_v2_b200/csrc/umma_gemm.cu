@@ -49,6 +49,9 @@ static Plan make_plan(int m, int n, int k) {
   Plan pl;
   pl.bm = m <= 64 ? 64 : m <= 128 ? 128 : 256;
   pl.m_tiles = (m + pl.bm - 1) / pl.bm;
+  // The M rows in equal tiles of a multiple of 16: M = 333 is two tiles of 176 rows, not 256 + 77 padded to 512 (the MMA time and
+  // the activation bytes go with the rows of a tile).
+  pl.bn = ((m + pl.m_tiles - 1) / pl.m_tiles + 15) / 16 * 16;
   const long long tiles = static_cast<long long>(pl.m_tiles) * ((n + kRowsW - 1) / kRowsW);
   const int nsb = k / 256;
   pl.units = tiles * nsb;

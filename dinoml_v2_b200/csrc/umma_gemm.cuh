@@ -45,6 +45,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "gemv_mma_common.cuh"
 
 namespace b200gguf {
@@ -380,6 +382,7 @@ struct Params {
   int* status;            // device status word
   int m, n, k;
   int m_tiles;            // activation tiles per weight panel
+  int bn;                 // activation rows of a tile: a multiple of 16, at most BM (the UMMA N of this launch)
   long long units;        // output tiles x super-blocks
   PeerOut peers;          // extra destinations of the output (SCATTER kernels only)
 };
@@ -429,8 +432,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
   constexpr int kPitch = RawGeom<QT>::kPitch;
   constexpr int kRawBytes = raw_slot_bytes<QT>();
   constexpr int kBlockBytes = RawGeom<QT>::kSuper;
-  constexpr uint32_t kIdesc = (1u << 4) | (P::kFormat << 7) | (P::kFormat << 10) | (uint32_t(BM >> 3) << 17) |
-                              (uint32_t(kRowsW >> 4) << 24);
+  const uint32_t idesc = (1u << 4) | (P::kFormat << 7) | (P::kFormat << 10) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kRowsW >> 4) << 24);
+  const uint32_t x_bytes = uint32_t(p.bn) * (kBK * 2);        // bytes of one activation stage (its shared-memory slot holds BM rows)
   constexpr uint32_t kWarpArrivals = kGroupThreads / 32;     // one elected arrive per producer warp of a group
 
   extern __shared__ uint8_t smem_raw[];
@@ -526,7 +529,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         if (!ok) return false;
       }
       tcgen05_fence_after();
-      const int n0 = (t / p.m_tiles) * kRowsW, m0 = (t % p.m_tiles) * BM;
+      const int n0 = (t / p.m_tiles) * kRowsW, m0 = (t % p.m_tiles) * p.bn;
       const int n_row = n0 + row;
       const bool whole = sb_b == 0 && sb_e == nsb;
       const bool finishes = sb_e == nsb;            // this CTA stores the tile (after adding the others' partial sums)
@@ -544,11 +547,13 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         if (!producer_sync()) return false;
       }
       const float bias_v = (finishes && p.bias != nullptr && n_row < p.n) ? P::up(static_cast<const T*>(p.bias)[n_row]) : 0.f;
-      constexpr int kColsPerWarp = BM / 4;
-      constexpr int CH = kColsPerWarp >= 32 ? 32 : 16;   // columns per round: enough independent loads / stores in flight
-#pragma unroll
-      for (int c0 = 0; c0 < kColsPerWarp; c0 += CH) {
-        const int col = (warp >> 2) * kColsPerWarp + c0;
+      // The four warps that share a lane quarter split the tile's bn columns: up to 64 columns evenly (bn / 4 each), above that in
+      // rounds of 16 taken in turn (32 per round, or uneven splits, spill registers that the unpack loop needs).
+      constexpr int CH = 16;
+      constexpr bool kEven = BM <= 64;
+      for (int r0 = 0; r0 < (kEven ? 1 : p.bn); r0 += 4 * CH) {
+        const int col = (warp >> 2) * (kEven ? p.bn >> 2 : CH) + r0, lim = kEven ? p.bn >> 2 : CH;
+        if (!kEven && col >= p.bn) break;
         uint32_t r[CH];
 #pragma unroll
         for (int q = 0; q < CH / 16; ++q)
@@ -557,41 +562,51 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         if (!finishes) {
           float* dst = p.partial + (static_cast<size_t>(cta) * BM + col) * kRowsW + row;     // tile-local [BM][128]
 #pragma unroll
-          for (int j = 0; j < CH; ++j) dst[j * kRowsW] = __uint_as_float(r[j]);
+          for (int j = 0; j < CH; ++j)
+            if (j < lim) dst[j * kRowsW] = __uint_as_float(r[j]);
         } else {
           for (int peer = peer0; peer < cta; ++peer) {
             const float* src = p.partial + (static_cast<size_t>(peer) * BM + col) * kRowsW + row;
             float v[CH];
 #pragma unroll
-            for (int j = 0; j < CH; ++j) v[j] = __ldcg(src + j * kRowsW);
+            for (int j = 0; j < CH; ++j) v[j] = j < lim ? __ldcg(src + j * kRowsW) : 0.f;
 #pragma unroll
             for (int j = 0; j < CH; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + v[j]);
           }
           if (p.peers.act != ACT_NONE) {
             // gated pair: within every 16 weight rows the first 8 belong to the first matrix, the next 8 to the second;
             // lane l and lane l ^ 8 hold the two halves, the output has n / 2 columns
+            // Of every two columns the gate lane finishes the even one and its partner the odd one: one exchange and one
+            // activation per lane and pair (the activations were a third of an M = 512 launch with half of the lanes idle).
             const int out_row = ((n_row >> 4) << 3) + (n_row & 7);
             const int64_t n_out = p.n >> 1;
+            const int odd = (lane >> 3) & 1;
+            auto gated_columns = [&](auto act) {
 #pragma unroll
-            for (int j = 0; j < CH; ++j) {
-              const float mine = __uint_as_float(r[j]) + bias_v;       // bias interleaved like the rows (0 without one)
-              const float other = __shfl_xor_sync(0xffffffffu, mine, 8);
-              if ((lane & 8) == 0 && n_row < p.n && m0 + col + j < p.m) {
-                const T v = P::cvt(gate_activation(mine, p.peers.act) * other);
-                const int64_t at = int64_t(m0 + col + j) * n_out + out_row;
-                static_cast<T*>(p.out)[at] = v;
-                if (SCATTER) {
+              for (int j = 0; j < CH; j += 2) {
+                const float even_v = __uint_as_float(r[j]) + bias_v, odd_v = __uint_as_float(r[j + 1]) + bias_v;   // bias interleaved like the rows (0 without one)
+                const float got = __shfl_xor_sync(0xffffffffu, odd ? even_v : odd_v, 8);
+                const float gate = odd ? got : even_v, up = odd ? odd_v : got;
+                const int mcol = m0 + col + j + odd;
+                if (n_row < p.n && mcol < p.m && j < lim) {
+                  const T v = P::cvt(gate_activation(gate, decltype(act)::value) * up);
+                  const int64_t at = int64_t(mcol) * n_out + out_row;
+                  static_cast<T*>(p.out)[at] = v;
+                  if (SCATTER) {
 #pragma unroll
-                  for (int pi = 0; pi < 8; ++pi)
-                    if (pi < p.peers.count) static_cast<T*>(p.peers.ptr[pi])[at] = v;
+                    for (int pi = 0; pi < 8; ++pi)
+                      if (pi < p.peers.count) static_cast<T*>(p.peers.ptr[pi])[at] = v;
+                  }
                 }
               }
-            }
+            };
+            if (p.peers.act == ACT_SILU) gated_columns(std::integral_constant<int, ACT_SILU>{});
+            else gated_columns(std::integral_constant<int, ACT_FAST_GELU>{});
           } else if (n_row < p.n) {
             T* dst = static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row;
 #pragma unroll
             for (int j = 0; j < CH; ++j)
-              if (m0 + col + j < p.m) {
+              if (j < lim && m0 + col + j < p.m) {
                 const T v = P::cvt(__uint_as_float(r[j]) + bias_v);
                 dst[int64_t(j) * p.n] = v;
                 if (SCATTER) {
@@ -941,13 +956,13 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     for (int t = tile_hi; t >= tile_lo && ok; --t) {
       int sb_b, sb_e;
       walk.segment(t, sb_b, sb_e);
-      const int m0 = (t % p.m_tiles) * BM;
+      const int m0 = (t % p.m_tiles) * p.bn;
       for (int sb = sb_b; sb < sb_e && ok; ++sb, ++it) {
         if constexpr (COARSE) {
           const int ub = it % U, trip = it / U;
           if (trip > 0 && !warp_wait(empty(ub), uint32_t(trip - 1) & 1u, abort_flag, p.status, ST_EMPTY_TIMEOUT)) { ok = false; break; }
           if (elect_one()) {
-            mbar_arrive_expect_tx(full(ub), uint32_t(kStagesPerSb * kXTile));
+            mbar_arrive_expect_tx(full(ub), uint32_t(kStagesPerSb) * x_bytes);
 #pragma unroll
             for (int st = 0; st < kStagesPerSb; ++st)
               tma_load_2d(smem_u32(xtiles + (ub * kStagesPerSb + st) * kXTile), &x_map, full(ub), sb * 256 + st * kBK, m0);
@@ -958,7 +973,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
           for (int slot = 0; slot < NS; ++slot) {
             if (it > 0 && !warp_wait(empty(slot), uint32_t(it - 1) & 1u, abort_flag, p.status, ST_EMPTY_TIMEOUT)) { ok = false; break; }
             if (elect_one()) {
-              mbar_arrive_expect_tx(full(slot), uint32_t(kXTile));
+              mbar_arrive_expect_tx(full(slot), x_bytes);
               tma_load_2d(smem_u32(xtiles + slot * kXTile), &x_map, full(slot), sb * 256 + slot * kBK, m0);
             }
             __syncwarp();
@@ -1022,7 +1037,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
 #pragma unroll
               for (int kk = 0; kk < kBK / 16; ++kk)
                 umma_f16_ts(tmem_base, tmem_base + uint32_t(BM + slot * kWSlotCols + 8 * kk), db0 + uint64_t((slot * kXTile) >> 4) + uint64_t(2 * kk),
-                            kIdesc, (sb > sb_b || st > 0 || kk > 0) ? 1u : 0u);
+                            idesc, (sb > sb_b || st > 0 || kk > 0) ? 1u : 0u);
             }
             umma_commit(empty(ub));
           }
@@ -1038,7 +1053,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
 #pragma unroll
               for (int kk = 0; kk < kBK / 16; ++kk)      // 16 K values = 8 TMEM columns of A, 32 bytes of each B row
                 umma_f16_ts(tmem_base, tmem_base + uint32_t(BM + slot * kWSlotCols + 8 * kk), db0 + uint64_t((slot * kXTile) >> 4) + uint64_t(2 * kk),
-                            kIdesc, (sb > sb_b || slot > 0 || kk > 0) ? 1u : 0u);
+                            idesc, (sb > sb_b || slot > 0 || kk > 0) ? 1u : 0u);
               umma_commit(empty(slot));
             }
             __syncwarp();
@@ -1082,7 +1097,7 @@ constexpr int kMaxCtas = 1024;      // flag words per device; the grid never exc
 
 // Tile shape and stream-K grid of one problem.
 struct Plan {
-  int bm, m_tiles, ctas;
+  int bm, bn, m_tiles, ctas;      // bm: the kernel instantiation (slot sizes), bn: activation rows of a tile
   long long units;
   size_t workspace_bytes;     // fp32 partial tiles, one per CTA; 0 when every CTA range ends on a tile boundary
 };
@@ -1097,10 +1112,10 @@ int launch(const void* a, const void* b, const void* bias, void* c, int m, int n
   if (enc == nullptr) return RC_LAUNCH;
   const cuuint32_t estr[2] = {1, 1};
   CUtensorMap x_map, w_map;
-  {   // activations [m, k], 16-bit: box = one K stage x BM rows, 128-byte swizzle (the MMA's B operand layout)
+  {   // activations [m, k], 16-bit: box = one K stage x bn rows, 128-byte swizzle (the MMA's B operand layout)
     const cuuint64_t dims[2] = {cuuint64_t(k), cuuint64_t(m)};
     const cuuint64_t strides[1] = {cuuint64_t(k) * 2};
-    const cuuint32_t box[2] = {cuuint32_t(kBK), cuuint32_t(BM)};
+    const cuuint32_t box[2] = {cuuint32_t(kBK), cuuint32_t(pl.bn)};
     if (enc(&x_map, Pair<T>::kTmaType, 2, const_cast<void*>(a), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return RC_LAUNCH;
@@ -1129,6 +1144,7 @@ int launch(const void* a, const void* b, const void* bias, void* c, int m, int n
   p.status = sc.status;
   p.m = m; p.n = n; p.k = k;
   p.m_tiles = pl.m_tiles;
+  p.bn = pl.bn;
   p.units = pl.units;
   p.peers = peers;
   // programmatic stream serialization: see the griddepcontrol notes in the kernel
