@@ -78,25 +78,22 @@ int select_variant(int qtype, int dtype, int m, int n, int k) {
   //   ([8192 x 14336] Q4_K: 27.6 us against 33.9 persistent / 58.2 tile; [4096 x 4096]: 10.4 against 8.9 persistent).
   if (m == 8 && weights >= (int64_t(32) << 20) && (qtype == QTYPE_Q4_K || qtype == QTYPE_Q6_K) && gemm_umma_supports(qtype, dtype, 9, n, k))
     return DINOML_B200_GGUF_VARIANT_UMMA;
-  // M <= 8 on Q4_K / Q6_K: the persistent bulk-copy GEMV, except where the tile kernel measured faster:
-  //   Q4_K, M = 1, when the tile kernel's grid (three CTAs of 16 rows per SM) fills at least three quarters of its last wave
-  //   ([11008 x 4096]: 9.4 us against 10.5 us; with emptier waves or less than one wave the persistent kernel wins);
-  //   Q4_K, M >= 2, with fewer row tiles than half the SMs: the tile kernel cuts K across a cluster and so uses more SMs
-  //   ([256 x 14336], M = 8: 4.9 us against 9.3 us; [2048 x 4096], M = 8: 6.3 against 5.9);
+  // M <= 8: the persistent bulk-copy GEMV (M <= 2 with byte operands), except where the tile kernel measured faster:
+  //   Q4_K, M = 1 / 2, with fewer row tiles than SMs / half the SMs on K < 8192, where making the digit planes is a large part of the
+  //   launch ([1024 x 4096]: 3.2 us against 3.9, M = 2: 3.8 against 4.7), and M = 1 on the shapes whose waves fill the tile kernel's
+  //   grid (named mma; the family runs them on the persistent kernel since that takes byte operands);
+  //   Q4_K, M >= 3, with fewer row tiles than half the SMs on a long K: the tile kernel cuts K across a cluster and so uses more SMs
+  //   ([256 x 14336], M = 8: 4.9 us against 9.3 us);
   //   Q6_K, M >= 3, on weights below 32 M elements ([4096 x 4096], M = 4: 6.3 us against 6.8 us), where the launch is too short
-  //   for the ring to pay off (at M <= 2 and on larger weights it is 7 - 30 % faster: [4096 x 14336], M = 1: 15.0 us against 21.1 us).
+  //   for the ring to pay off.
   if (gemv_stream_supports(qtype, dtype, m, n, k)) {
     bool tile_kernel = false;
     if (qtype == QTYPE_Q4_K && m == 1) {
-      const int slots = 3 * sms;
-      const int waves = (tiles + slots - 1) / slots;
-      // fewer tiles than SMs: the tile kernel on a short K ([1024 x 4096]: 3.1 us against 3.5), the persistent one on a long K,
-      // where its ring keeps more bytes in flight per SM ([1024 x 14336]: 7.2 us against 8.9; [256 x 14336]: 7.0 against 8.5)
+      const int slots = 3 * sms, waves = (tiles + slots - 1) / slots;
+      // the mma family: it keeps the shapes with fewer tiles than SMs and hands the others to the persistent kernel itself
       tile_kernel = (tiles <= sms && k < 8192) || (tiles >= slots && double(tiles) / (double(waves) * slots) >= 0.75);
     } else if (qtype == QTYPE_Q4_K) {
-      // ... on a long K; on K = 4096 the persistent kernel (16 consumer warps per CTA) is ahead from M = 4 since both kernels take
-      // their activation sums from the tensor cores ([1024 x 4096], M = 8: 4.6 us against 5.5; [1024 x 14336]: 9.6 against 7.6)
-      tile_kernel = 2 * tiles <= sms && (m < 4 || k >= 8192);
+      tile_kernel = 2 * tiles <= sms && (m == 2 ? k < 8192 : m < 4 || k >= 8192);
     } else if (qtype == QTYPE_Q6_K && m >= 3) {
       tile_kernel = weights < (int64_t(32) << 20);
     }

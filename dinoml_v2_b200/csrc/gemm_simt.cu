@@ -7,9 +7,11 @@
 // kernels/rocm/src/ck_gguf_q8_gemm.hip:1168-1207) and the only variant that keeps fp32 activations
 // un-rounded.  It reads W once per group of MT activation rows, so it is bandwidth-efficient only
 // for M <= MT; the tensor-core variants take over elsewhere.
-#include "gguf_common.cuh"
+#include "gemv_mma_common.cuh"
 
 namespace b200gguf {
+
+int gemv_planes(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, const PeerOut& peers, cudaStream_t s);
 
 template <typename T> __device__ __forceinline__ void load8(const T* p, float (&x)[8]);
 template <> __device__ __forceinline__ void load8<float>(const float* p, float (&x)[8]) {
@@ -128,6 +130,12 @@ int check_gemm_args(const void* a, const void* b, const void* c, int qtype, int 
 int gemm_rcr_simt(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k,
                   cudaStream_t s) {
   if (int rc = check_gemm_args(a, b, c, qtype, dtype, m, n, k)) return rc;
+  // One or two rows: exact byte operands on the tensor cores where the type has them, for every dtype and row alignment
+  // (float32 activations, weight rows that are not 16-byte multiples).
+  if (m <= 2) {
+    const int rc = gemv_planes(a, b, bias, c, qtype, dtype, m, n, k, no_peers(), s);
+    if (rc != RC_RANGE) return rc;
+  }
   switch (qtype) {
     case QTYPE_Q8_0: return launch_simt_q<QTYPE_Q8_0>(a, b, bias, c, dtype, m, n, k, s);
     case QTYPE_Q4_K: return launch_simt_q<QTYPE_Q4_K>(a, b, bias, c, dtype, m, n, k, s);

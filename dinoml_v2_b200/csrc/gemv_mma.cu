@@ -34,6 +34,10 @@
 namespace b200gguf {
 
 int check_gemm_args(const void* a, const void* b, const void* c, int qtype, int dtype, int m, int n, int k);
+int gemv_planes(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, const PeerOut& peers, cudaStream_t s);
+int gemm_rcr_stream_peers(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, int config,
+                          const PeerOut* peer_out, cudaStream_t s);
+namespace stream { int sm_count(); }
 bool gemv_q6k_mma_supports(int dtype, int m, int k);
 bool gemv_q8_0_mma_supports(int dtype, int m, int k);
 int gemv_q8_0_mma(const void* a, const void* b, const void* bias, void* c, int dtype, int m, int n, int k, cudaStream_t s);
@@ -348,6 +352,15 @@ int gemm_rcr_mma_peers(const void* a, const void* b, const void* bias, void* c, 
   if (qtype != QTYPE_Q4_K && qtype != QTYPE_Q6_K && qtype != QTYPE_Q8_0) return RC_QTYPE;
   if (!gemv_mma_supports(qtype, dtype, m, n, k)) return RC_ALIGN;   // Q8_0 with K % 256 != 0
   if ((reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(a)) & 15) return RC_ALIGN;  // 16-byte cp.async sources, vector loads
+  // One or two rows of Q8_0, and of Q6_K with rows that are not 16-byte multiples: byte operands on the persistent kernel (the tile
+  // kernels below stay for a K whose digit planes do not fit).
+  if (m <= 2 && (qtype == QTYPE_Q8_0 || (qtype == QTYPE_Q6_K && k % 2048 != 0)) && !(qtype == QTYPE_Q8_0 && (peers.count > 0 || peers.act != ACT_NONE))) {
+    const int rc = gemv_planes(a, b, bias, c, qtype, dtype, m, n, k, peers, s);
+    if (rc != RC_RANGE) return rc;
+  }
+  // Q4_K, one row and more tiles than SMs: [11008 x 4096] 7.9 us on the persistent kernel with byte operands, 9.3 us here.
+  if (qtype == QTYPE_Q4_K && m == 1 && (n + kGemvRows - 1) / kGemvRows > stream::sm_count())
+    return gemm_rcr_stream_peers(a, b, bias, c, qtype, dtype, m, n, k, 0, &peers, s);
   if (qtype == QTYPE_Q6_K) return gemv_q6k_mma(a, b, bias, c, dtype, m, n, k, peers, s);
   if (qtype == QTYPE_Q8_0) {
     if (peers.count > 0 || peers.act != ACT_NONE) return RC_RANGE;   // no scatter / gated epilogue for Q8_0

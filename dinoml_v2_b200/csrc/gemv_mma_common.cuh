@@ -70,6 +70,11 @@ template <> struct MmaType<__half> {
   }
 };
 
+template <> struct MmaType<float> {                      // outputs of the integer path with float32 activations
+  static __device__ __forceinline__ float to_float(float v) { return v; }
+  static __device__ __forceinline__ float from_float(float v) { return v; }
+};
+
 // Four registers holding 0.f whose contents the compiler cannot see through: a stable zero C tuple for mma_c.
 __device__ __forceinline__ void opaque_zero4(float (&z)[4]) {
 #pragma unroll

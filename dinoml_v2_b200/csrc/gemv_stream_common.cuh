@@ -46,7 +46,7 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 // Bounded wait.  Returns false - after recording `code` in the status word and raising the CTA's abort flag - if the
 // phase does not complete within the limit, or as soon as another role has raised the abort flag.
 // The slow path is kept out of line: the loops that call it stay small in the instruction cache.
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+static __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
   const uint64_t start = globaltimer_ns();
   for (uint32_t i = 1; i < kSpinLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -82,12 +82,12 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
                "r"(bytes), "r"(bar)
                : "memory");
 }
-__device__ __forceinline__ int ld_acquire_gpu(const int* p) {
-  int v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];\n" : "=r"(v) : "l"(p) : "memory");
+__device__ __forceinline__ uint64_t ld_relaxed_gpu(const uint64_t* p) {
+  uint64_t v;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];\n" : "=l"(v) : "l"(p) : "memory");
   return v;
 }
-__device__ __forceinline__ void st_release_gpu(int* p, int v) { asm volatile("st.release.gpu.global.s32 [%0], %1;\n" ::"l"(p), "r"(v) : "memory"); }
+__device__ __forceinline__ void st_relaxed_gpu(uint64_t* p, uint64_t v) { asm volatile("st.relaxed.gpu.global.b64 [%0], %1;\n" ::"l"(p), "l"(v) : "memory"); }
 __device__ __forceinline__ void named_barrier(int id, int threads) {
   asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }

@@ -48,6 +48,8 @@ int dual_gemm_rcr(const void* a, const void* b01, const void* bias01, void* c, i
                   int variant, cudaStream_t s);
 int gemm_rcr(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k,
              int variant, cudaStream_t s);
+void stream_release_scratch(cudaStream_t s);      // workspaces the kernels keep for a stream
+void umma_release_scratch(cudaStream_t s);
 }  // namespace b200gguf
 
 using b200gguf::set_error_message;
@@ -825,6 +827,8 @@ int dino_session_destroy(DinoSession* session) {
   if (session == nullptr) return 0;
   if (session->owned_stream != nullptr) {
     cudaStreamSynchronize(session->owned_stream);
+    b200gguf::stream_release_scratch(session->owned_stream);
+    b200gguf::umma_release_scratch(session->owned_stream);
     cudaStreamDestroy(session->owned_stream);
   }
   for (auto& entry : session->graphs)

@@ -2,6 +2,7 @@
 // entry that checks a problem and hands it to the weight type's translation unit.  The kernel is in umma_gemm.cuh.
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 
 #include "umma_gemm.cuh"
 
@@ -26,15 +27,23 @@ struct StateKeyHash {
   size_t operator()(const StateKey& k) const { return std::hash<void*>()(static_cast<void*>(k.stream)) * 31u + size_t(k.dev); }
 };
 static std::unordered_map<StateKey, DeviceState, StateKeyHash> g_state;
+// Sets of streams that are gone (see release), for the next new stream of their device.
+constexpr size_t kMaxSpare = 4;
+static std::unordered_map<int, std::vector<DeviceState>> g_spare;
 
 static DeviceState* device_state(size_t need_workspace, cudaStream_t stream) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
   std::lock_guard<std::mutex> lock(g_mutex);
   DeviceState& st = g_state[StateKey{dev, stream}];
+  std::vector<DeviceState>& spare = g_spare[dev];
+  if (st.status == nullptr && !spare.empty()) {
+    st = spare.back();                          // flags are down: every flag raised was lowered by its reader
+    spare.pop_back();
+  }
   if (st.status == nullptr) {
     if (cudaMalloc(&st.status, sizeof(int) * (1 + kMaxCtas)) != cudaSuccess) return nullptr;
-    cudaMemset(st.status, 0, sizeof(int) * (1 + kMaxCtas));
+    cudaMemsetAsync(st.status, 0, sizeof(int) * (1 + kMaxCtas), stream);
   }
   if (need_workspace > st.workspace_bytes) {
     // Grown outside of stream capture only: callers warm a shape up once before capturing a graph.
@@ -43,6 +52,24 @@ static DeviceState* device_state(size_t need_workspace, cudaStream_t stream) {
     st.workspace_bytes = need_workspace;
   }
   return &st;
+}
+
+// `stream` is about to be destroyed and has no work left: its set is kept for a later stream (a bounded number) or freed.
+static void release(cudaStream_t stream) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  for (auto it = g_state.begin(); it != g_state.end();) {
+    if (it->first.stream != stream) { ++it; continue; }
+    std::vector<DeviceState>& spare = g_spare[it->first.dev];
+    if (it->second.status != nullptr) {
+      if (spare.size() < kMaxSpare) {
+        spare.push_back(it->second);
+      } else {
+        cudaFree(it->second.status);
+        if (it->second.workspace != nullptr) cudaFree(it->second.workspace);
+      }
+    }
+    it = g_state.erase(it);
+  }
 }
 
 static Plan make_plan(int m, int n, int k) {
@@ -128,6 +155,8 @@ static int launch_bm(int qtype, int dtype, const void* a, const void* b, const v
 }
 
 }  // namespace umma
+
+void umma_release_scratch(cudaStream_t s) { umma::release(s); }
 
 // Packed bytes per 256 weights of a row, 0 for a qtype this kernel does not unpack.
 static int super_block_bytes(int qtype) {

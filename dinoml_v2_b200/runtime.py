@@ -216,6 +216,12 @@ class Session:
             self._lib.dino_session_destroy(self._handle)
             self._handle = None
 
+    def __del__(self):           # a dropped session gives its stream and the kernels' workspaces for it back
+        try:
+            self.close()
+        except Exception:
+            pass
+
     def set_stream(self, stream_ptr: int | None) -> None:
         self._user_stream = stream_ptr or 0
         self._set_stream_raw(self._user_stream)

@@ -1,0 +1,50 @@
+"""The decode GEMV with byte operands (one and two activation rows) at the sizes where it can go wrong: fewer rows than a tile, a
+tile cut between two CTAs, K from one super-block to the lengths that are cut into slices, weight rows that are not 16-byte
+multiples, a last super-block that is not full, activations of very different size.  Against the float64 product of the dequantized weights."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from dinoml_v2_b200 import kernels, synthetic as S
+
+pytestmark = pytest.mark.gpu
+TDT = {"float16": torch.float16, "bfloat16": torch.bfloat16, "float32": torch.float32}
+BOUND = {"float16": 6e-4, "bfloat16": 4e-3, "float32": 2e-6}          # output rounding; float32: the sums
+KS = {"Q4_K": (256, 4096, 20480), "Q5_K": (2304, 14336), "Q6_K": (256, 768, 11008, 20480), "Q8_0": (32, 288, 2048, 14336),
+      "Q4_0": (96, 2880, 4096), "Q2_K": (256, 1280, 4096), "Q3_K": (256, 2560, 4096)}
+
+
+def _check(x, blocks, qtype, k, dtype, dev):
+    y = kernels.gemm_rcr(x, torch.from_numpy(blocks).to(dev), qtype)
+    assert kernels.device_status() == 0
+    ref = x.double().cpu().numpy() @ oracle.dequantize(blocks, qtype, k).astype(np.float64).T
+    _, _, norm = oracle.max_errors(ref, y.float().cpu().numpy())
+    assert norm <= BOUND[dtype], norm
+
+
+@pytest.mark.parametrize("m", [1, 2])
+@pytest.mark.parametrize("dtype", sorted(TDT))
+@pytest.mark.parametrize("qtype", sorted(KS))
+def test_edges(qtype, dtype, m):
+    dev = torch.device("cuda:0")
+    for k in KS[qtype]:
+        for n in (1, 17, 4800 if k <= 4096 else 400):         # 4800: a few tiles more than CTAs
+            x = torch.from_numpy(S.random_activations(m, k, 11, "float32")).to(dev).to(TDT[dtype])
+            _check(x, S.random_blocks(qtype, n, k, seed=n + k), qtype, k, dtype, dev)
+
+
+@pytest.mark.parametrize("qtype", ["Q4_K", "Q6_K", "Q8_0"])
+def test_range_of_the_activations(qtype):
+    """Zeros, tiny and huge values in one row: the digits are relative to the largest of a super-block, results to the largest result."""
+    dev = torch.device("cuda:0")
+    k, n = 1024, 64
+    x = torch.zeros(2, k, device=dev)
+    x[0, ::7] = 1e-30
+    x[0, 300] = 3.0
+    x[1, 256:512] = torch.randn(256, device=dev) * 1e20
+    x[1, 600:700] = 1e-3
+    _check(x, S.random_blocks(qtype, n, k, seed=5), qtype, k, "float32", dev)
+    x[1, 5] = float("inf")
+    y = kernels.gemm_rcr(x, torch.from_numpy(S.random_blocks(qtype, n, k, seed=5)).to(dev), qtype)
+    assert torch.isfinite(y[0]).all() and not torch.isfinite(y[1]).any()
