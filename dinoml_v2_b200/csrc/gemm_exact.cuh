@@ -1,0 +1,424 @@
+// Fused GGUF gemm_rcr that rounds neither weights nor activations, from three rows on ("simt" family): C[M,N] = A[M,K] * dequant(W[N,K])^T
+// (+ bias) for float32 activations and for weight rows that are not multiples of 16 bytes, on mma.sync tensor cores.
+//
+// The quants are small integers (FP4 codes small binary fractions), exact as 16-bit MMA operands.  A float32 activation is the exact
+// sum of three bfloat16 numbers, one MMA each; a 16-bit activation is its own operand.  The MMA of a group of 16 weights (one K
+// step) yields the exact products summed in fp32, and the group's scale and min are applied to that sum in fp32: no operand is rounded,
+// as in the CUDA-core kernel this replaces (which reads the whole weight again for every four activation rows: Q6_K [4096 x 11008],
+// M = 333: 2626 us).
+//
+// A CTA of 8 warps owns ROWS weight rows x BT activation rows and walks K in super-blocks of 256:
+//   * packed bytes: every row's 16-byte aligned window around its super-block, 16-byte cp.async (rows have phases of their own);
+//   * per half super-block each thread decodes 64 weights (four groups) of one row into the operand tile and its scales; the next
+//     super-block's bytes are requested as soon as the second half is decoded;
+//   * warps 4 x 2 take ROWS/4 x BT/2 of the tile with ldmatrix operands;
+//   * with few tiles K is cut across a cluster of up to 8 CTAs whose sums meet through distributed shared memory.
+// Two CTAs share an SM (< 113 KB each), so that one decodes while the other keeps the tensor pipe busy.
+#pragma once
+#include <type_traits>
+
+#include "gemv_mma_common.cuh"
+
+namespace b200gguf {
+namespace exact {
+
+constexpr int kThreads = 256;
+constexpr int kHalfK = 128;                      // K per operand tile
+constexpr int kPitchB = (kHalfK + 8) * 2;        // bytes of an operand row: 272, ldmatrix rows on distinct banks
+
+template <int QT> constexpr int sb_bytes() { return 256 / QTraits<QT>::kBlock * QTraits<QT>::kBytes; }
+template <int QT> constexpr int raw_pitch() { return (sb_bytes<QT>() + 15 + 15) / 16 * 16 + (((sb_bytes<QT>() + 30) / 16) % 2 == 0 ? 16 : 0); }   // an odd number of 16-byte chunks
+template <int QT> constexpr bool has_mins() { return QT == QTYPE_Q4_K || QT == QTYPE_Q5_K || QT == QTYPE_Q2_K; }
+template <typename T> using Operand = typename std::conditional<std::is_same<T, __half>::value, __half, __nv_bfloat16>::type;
+template <typename T> constexpr int x_planes() { return std::is_same<T, float>::value ? 3 : 1; }
+
+template <int QT, typename T, int ROWS, int BT> constexpr size_t smem_bytes() {
+  return size_t(ROWS) * raw_pitch<QT>() + size_t(ROWS) * kPitchB + size_t(x_planes<T>()) * BT * kPitchB + size_t(8) * ROWS * sizeof(float) * (has_mins<QT>() ? 2 : 1) +
+         (has_mins<QT>() ? size_t(8) * BT * sizeof(float) : 0);
+}
+
+// 16 consecutive bytes from any shared-memory address.
+__device__ __forceinline__ void lds16(const uint8_t* p, uint32_t (&w)[4]) {
+  const uint32_t off = uint32_t(__cvta_generic_to_shared(p)) & 3u;
+  const uint32_t* q = reinterpret_cast<const uint32_t*>(p - off);
+  uint32_t v[5];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) v[i] = q[i];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(v[i], v[i + 1], 8u * off);
+}
+
+// Four unsigned bytes less an offset -> two operand pairs, exact (bytes below 128 for bfloat16, any for float16).
+template <typename O>
+__device__ __forceinline__ void bytes_minus(uint32_t w, int off, uint32_t& p01, uint32_t& p23) {
+  const uint32_t a = __byte_perm(w, MmaType<O>::kMagicBytes, 0x4140), b = __byte_perm(w, MmaType<O>::kMagicBytes, 0x4342);
+  if constexpr (std::is_same<O, __half>::value) {
+    const __half2 o = __float2half2_rn(1024.f + float(off));
+    const __half2 x = __hsub2(*reinterpret_cast<const __half2*>(&a), o), y = __hsub2(*reinterpret_cast<const __half2*>(&b), o);
+    p01 = *reinterpret_cast<const uint32_t*>(&x);
+    p23 = *reinterpret_cast<const uint32_t*>(&y);
+  } else {
+    const __nv_bfloat162 o = __float2bfloat162_rn(128.f + float(off));
+    const __nv_bfloat162 x = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&a), o), y = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&b), o);
+    p01 = *reinterpret_cast<const uint32_t*>(&x);
+    p23 = *reinterpret_cast<const uint32_t*>(&y);
+  }
+}
+template <typename O> __device__ __forceinline__ uint32_t pack(float lo, float hi) {
+  if constexpr (std::is_same<O, __half>::value) {
+    const __half2 v = __floats2half2_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  } else {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+  }
+}
+// Four FP4 codes (low nibbles of the bytes of w, high nibbles zero) -> their e2m1 values as two operand pairs: byte look-ups of the
+// magnitudes (0, .5, 1, 1.5, 2, 3, 4, 6) with the codes as selector, then the sign bits.
+template <typename O>
+__device__ __forceinline__ void fp4_pairs(uint32_t w, uint32_t& p01, uint32_t& p23) {
+  const uint32_t mag = w & 0x07070707u, sign = (w & 0x08080808u) << 4;
+  const uint32_t sel = __byte_perm(mag | (mag >> 4), 0u, 0x4420);
+  if constexpr (std::is_same<O, __half>::value) {
+    const uint32_t hi = __byte_perm(0x3E3C3800u, 0x46444240u, sel) | sign;
+    p01 = __byte_perm(hi, 0u, 0x1404);
+    p23 = __byte_perm(hi, 0u, 0x3424);
+  } else {
+    const uint32_t hi = __byte_perm(0x3F3F3F00u, 0x40404040u, sel) | sign, lo = __byte_perm(0xC0800000u, 0xC0804000u, sel);
+    p01 = __byte_perm(lo, hi, 0x5140);
+    p23 = __byte_perm(lo, hi, 0x7362);
+  }
+}
+
+// Group gi (16 weights) of the super-block at p: operand pairs in K order, scale, min (w = scale * operand - min).
+template <int QT, typename O>
+__device__ __forceinline__ void group16(const uint8_t* p, int gi, uint32_t (&o)[8], float& scale, float& mn) {
+  uint32_t w[4];
+  mn = 0.f;
+  if constexpr (QT == QTYPE_Q8_0) {
+    const uint8_t* b = p + 34 * (gi >> 1);
+    scale = half_at(b);
+    lds16(b + 2 + 16 * (gi & 1), w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      o[2 * i] = pack<O>(float(int(int8_t(w[i]))), float(int(int8_t(w[i] >> 8))));
+      o[2 * i + 1] = pack<O>(float(int(int8_t(w[i] >> 16))), float(int(int8_t(w[i] >> 24))));
+    }
+  } else if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4) {
+    constexpr int BB = QT == QTYPE_Q4_0 ? 18 : 17;
+    const uint8_t* b = p + BB * (gi >> 1);
+    scale = QT == QTYPE_Q4_0 ? half_at(b) : 2.f * e8m0_half(b[0]);
+    lds16(b + BB - 16, w);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t n = (w[i] >> (4 * (gi & 1))) & 0x0f0f0f0fu;
+      if constexpr (QT == QTYPE_Q4_0) bytes_minus<O>(n, 8, o[2 * i], o[2 * i + 1]);
+      else fp4_pairs<O>(n, o[2 * i], o[2 * i + 1]);
+    }
+  } else if constexpr (QT == QTYPE_NVFP4) {
+    const uint8_t* b = p + 36 * (gi >> 2);
+    scale = 2.f * ue4m3_half(b[gi & 3]);
+    lds16(b + 4 + 8 * (gi & 3), w);              // 8 bytes of this sub-block (and 8 of the next)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      fp4_pairs<O>(w[i] & 0x0f0f0f0fu, o[2 * i], o[2 * i + 1]);
+      fp4_pairs<O>((w[i] >> 4) & 0x0f0f0f0fu, o[4 + 2 * i], o[4 + 2 * i + 1]);
+    }
+  } else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) {
+    const int j = gi >> 1;
+    int sc, m;
+    k4_scale_min(j, p + 4, sc, m);
+    scale = half_at(p) * float(sc);
+    mn = half_at(p + 2) * float(m);
+    lds16(p + (QT == QTYPE_Q4_K ? 16 : 48) + 32 * (j >> 1) + 16 * (gi & 1), w);
+    uint32_t h[4] = {0u, 0u, 0u, 0u};
+    if constexpr (QT == QTYPE_Q5_K) lds16(p + 16 + 16 * (gi & 1), h);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bytes_minus<O>(((w[i] >> (4 * (j & 1))) & 0x0f0f0f0fu) | (((h[i] >> j) & 0x01010101u) << 4), 0, o[2 * i], o[2 * i + 1]);
+  } else {
+    const int hb = gi >> 3, quad = (gi >> 1) & 3, u = gi & 1;
+    if constexpr (QT == QTYPE_Q6_K) {
+      scale = half_at(p + 208) * float(int(int8_t(p[192 + gi])));
+      uint32_t h[4];
+      lds16(p + 64 * hb + 32 * (quad & 1) + 16 * u, w);
+      lds16(p + 128 + 32 * hb + 16 * u, h);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        bytes_minus<O>(((w[i] >> (quad & 2 ? 4 : 0)) & 0x0f0f0f0fu) | (((h[i] >> (2 * quad)) & 0x03030303u) << 4), 32, o[2 * i], o[2 * i + 1]);
+    } else if constexpr (QT == QTYPE_Q2_K) {
+      const uint32_t s = p[gi];
+      scale = half_at(p + 80) * float(s & 0x0fu);
+      mn = half_at(p + 82) * float(s >> 4);
+      lds16(p + 16 + 32 * hb + 16 * u, w);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) bytes_minus<O>((w[i] >> (2 * quad)) & 0x03030303u, 0, o[2 * i], o[2 * i + 1]);
+    } else {
+      scale = half_at(p + 108) * float(q3k_scale(p + 96, gi) - 32);
+      uint32_t h[4];
+      lds16(p + 32 + 32 * hb + 16 * u, w);
+      lds16(p + 16 * u, h);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        bytes_minus<O>(((w[i] >> (2 * quad)) & 0x03030303u) | (((h[i] >> (4 * hb + quad)) & 0x01010101u) << 2), 4, o[2 * i], o[2 * i + 1]);
+    }
+  }
+}
+
+__device__ __forceinline__ void ldmatrix4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+
+template <int QT, typename T, int ROWS, int BT>
+__global__ void __launch_bounds__(kThreads, 2)
+gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y, int m, int n, int k) {
+  using O = Operand<T>;
+  constexpr int PL = x_planes<T>(), MI = ROWS / 64, NI = BT / 16, kRawPitch = raw_pitch<QT>();
+  constexpr bool kMins = has_mins<QT>();
+  constexpr int kPer = (QT == QTYPE_Q6_K || QT == QTYPE_Q2_K || QT == QTYPE_Q3_K || QT == QTYPE_NVFP4) ? 1 : 2;    // K steps that share a scale
+  extern __shared__ __align__(16) uint8_t smem[];
+  uint8_t* raw = smem;                                            // [ROWS][kRawPitch]
+  uint8_t* sA = raw + ROWS * kRawPitch;                           // [ROWS][kPitchB]
+  uint8_t* sB = sA + ROWS * kPitchB;                              // [PL][BT][kPitchB]
+  float* sS = reinterpret_cast<float*>(sB + PL * BT * kPitchB);   // [8 groups][ROWS] scales, then mins
+  float* sM = sS + 8 * ROWS;
+  float* sX = sM + 8 * ROWS;                                      // [8 groups][BT] activation sums (types with mins)
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int n0 = blockIdx.x * ROWS, m0 = blockIdx.y * BT;
+  const int64_t row_bytes = int64_t(k / QTraits<QT>::kBlock) * QTraits<QT>::kBytes;
+  // this CTA's super-blocks: one of gridDim.z (= cluster size) slices of K
+  const int nsb = (k + 255) >> 8, per_slice = (nsb + int(gridDim.z) - 1) / int(gridDim.z);
+  const int h_begin = 2 * int(blockIdx.z) * per_slice, halves = min((k + kHalfK - 1) / kHalfK, h_begin + 2 * per_slice);
+
+  // packed bytes of super-block c: TPR threads per row, 16-byte chunks of the row's window in turn
+  constexpr int TPR = kThreads / ROWS;
+  const int crow = tid / TPR;
+  const uint8_t* wrow = w + int64_t(min(n0 + crow, n - 1)) * row_bytes;
+  auto issue_raw = [&](int c) {
+    const uint8_t* src = wrow + int64_t(c) * sb_bytes<QT>();
+    const int phase = int(reinterpret_cast<uintptr_t>(src) & 15);
+    const int piece = int(min(int64_t(sb_bytes<QT>()), row_bytes - int64_t(c) * sb_bytes<QT>()));
+    const int chunks = (phase + piece + 15) >> 4;
+    const uint32_t dst = uint32_t(__cvta_generic_to_shared(raw + crow * kRawPitch));
+    for (int i = tid % TPR; i < chunks; i += TPR) cp_async16(dst + 16 * i, src - phase + 16 * i);
+  };
+  // activations of half h: units of 8 values
+  constexpr int kUnits = BT * (kHalfK / 8) / kThreads;
+  float4 xf[PL == 3 ? kUnits : 1][2];
+  auto fetch_x = [&](int h) {
+#pragma unroll
+    for (int i = 0; i < kUnits; ++i) {
+      const int unit = tid + i * kThreads, row = unit >> 4, k8 = unit & 15;
+      const int kk = h * kHalfK + 8 * k8;
+      const bool in = m0 + row < m && kk < k;
+      if constexpr (PL == 3) {
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(x) + int64_t(m0 + row) * k + kk);
+        xf[i][0] = in ? __ldg(p) : z;
+        xf[i][1] = in ? __ldg(p + 1) : z;
+      } else {
+        uint8_t* dst = sB + row * kPitchB + 16 * k8;
+        if (in) cp_async16(uint32_t(__cvta_generic_to_shared(dst)), x + int64_t(m0 + row) * k + kk);
+        else *reinterpret_cast<uint4*>(dst) = make_uint4(0u, 0u, 0u, 0u);
+      }
+    }
+  };
+  auto store_x = [&]() {                       // float32: three bfloat16 numbers whose sum is the value
+    if constexpr (PL == 3) {
+#pragma unroll
+      for (int i = 0; i < kUnits; ++i) {
+        const int unit = tid + i * kThreads, row = unit >> 4, k8 = unit & 15;
+        float v[8] = {xf[i][0].x, xf[i][0].y, xf[i][0].z, xf[i][0].w, xf[i][1].x, xf[i][1].y, xf[i][1].z, xf[i][1].w};
+#pragma unroll
+        for (int pl = 0; pl < 3; ++pl) {
+          uint32_t o[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            o[j] = pack<O>(v[2 * j], v[2 * j + 1]);
+            v[2 * j] -= __uint_as_float(o[j] << 16);
+            v[2 * j + 1] -= __uint_as_float(o[j] & 0xffff0000u);
+          }
+          *reinterpret_cast<uint4*>(sB + (pl * BT + row) * kPitchB + 16 * k8) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+      }
+    }
+  };
+
+  float res[MI][NI][4];
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) res[i][j][q] = 0.f;
+
+  float zero4[4];
+  opaque_zero4(zero4);
+  const int wm = warp & 3, wn = warp >> 2, g = lane >> 2, t = lane & 3;
+  const uint32_t a_addr = uint32_t(__cvta_generic_to_shared(sA + (wm * (ROWS / 4) + (lane & 15)) * kPitchB + (lane >> 4) * 16));
+  const uint32_t b_addr = uint32_t(__cvta_generic_to_shared(sB + (wn * (BT / 2) + (lane & 7) + ((lane >> 4) << 3)) * kPitchB + ((lane >> 3) & 1) * 16));
+
+  if (h_begin < halves) {
+    issue_raw(h_begin >> 1);
+    fetch_x(h_begin);
+  }
+  cp_async_commit();
+  for (int h = h_begin; h < halves; ++h) {
+    store_x();
+    cp_async_wait<0>();
+    __syncthreads();                             // bytes and activations of this half are here
+    {
+      // decode: ROWS * 8 groups of 16 weights
+      const int c = h >> 1;
+      for (int u = tid; u < ROWS * 8; u += kThreads) {
+        const int row = u >> 3, grp = u & 7;                     // eight threads per row
+        const uint8_t* src = w + int64_t(min(n0 + row, n - 1)) * row_bytes + int64_t(c) * sb_bytes<QT>();
+        uint32_t o[8];
+        float scale, mn;
+        group16<QT, O>(raw + row * kRawPitch + (reinterpret_cast<uintptr_t>(src) & 15), 8 * (h & 1) + grp, o, scale, mn);
+        if (h * kHalfK + 16 * grp >= k) scale = mn = 0.f;        // past the end of the row: whatever the buffer holds
+        uint4* dst = reinterpret_cast<uint4*>(sA + row * kPitchB + 32 * grp);
+        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        sS[grp * ROWS + row] = scale;
+        if constexpr (kMins) sM[grp * ROWS + row] = mn;
+      }
+      if constexpr (kMins) {
+        for (int u = tid; u < BT * 8; u += kThreads) {
+          const int row = u >> 3, grp = u & 7;
+          float sum = 0.f;
+#pragma unroll
+          for (int pl = PL - 1; pl >= 0; --pl) {
+            const uint4* p = reinterpret_cast<const uint4*>(sB + (pl * BT + row) * kPitchB + 32 * grp);
+            sum += MmaType<O>::sum8(p[0]) + MmaType<O>::sum8(p[1]);
+          }
+          sX[grp * BT + row] = sum;
+        }
+      }
+    }
+    __syncthreads();
+    if ((h & 1) && h + 1 < halves) issue_raw((h + 1) >> 1);      // both halves of the super-block are decoded
+    if (PL == 3 && h + 1 < halves) fetch_x(h + 1);
+#pragma unroll
+    for (int gg = 0; gg < 8; gg += kPer) {
+      uint32_t a[kPer][MI][4], b[kPer][NI / 2][4];
+      float acc[MI][NI][4];
+#pragma unroll
+      for (int s = 0; s < kPer; ++s) {
+#pragma unroll
+        for (int i = 0; i < MI; ++i) ldmatrix4(a_addr + i * 16 * kPitchB + (gg + s) * 32, a[s][i]);
+#pragma unroll
+        for (int pl = PL - 1; pl >= 0; --pl) {                   // the small parts first
+#pragma unroll
+          for (int j = 0; j < NI / 2; ++j) ldmatrix4(b_addr + (pl * BT + j * 16) * kPitchB + (gg + s) * 32, b[s][j]);
+#pragma unroll
+          for (int i = 0; i < MI; ++i)
+#pragma unroll
+            for (int j = 0; j < NI; ++j) {
+              const uint32_t b0 = b[s][j >> 1][2 * (j & 1)], b1 = b[s][j >> 1][2 * (j & 1) + 1];
+              if (s == 0 && pl == PL - 1) MmaType<O>::mma_c(acc[i][j], a[s][i], b0, b1, zero4);
+              else MmaType<O>::mma(acc[i][j], a[s][i], b0, b1);
+            }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < MI; ++i) {
+        const int r = wm * (ROWS / 4) + i * 16 + g;
+        const float s0 = sS[gg * ROWS + r], s1 = sS[gg * ROWS + r + 8];
+#pragma unroll
+        for (int j = 0; j < NI; ++j) {
+          res[i][j][0] = fmaf(s0, acc[i][j][0], res[i][j][0]);
+          res[i][j][1] = fmaf(s0, acc[i][j][1], res[i][j][1]);
+          res[i][j][2] = fmaf(s1, acc[i][j][2], res[i][j][2]);
+          res[i][j][3] = fmaf(s1, acc[i][j][3], res[i][j][3]);
+        }
+        if constexpr (kMins) {
+#pragma unroll
+          for (int s = 0; s < kPer; ++s) {
+            const float m0v = sM[(gg + s) * ROWS + r], m1v = sM[(gg + s) * ROWS + r + 8];
+#pragma unroll
+            for (int j = 0; j < NI; ++j) {
+              const float2 X = *reinterpret_cast<const float2*>(&sX[(gg + s) * BT + wn * (BT / 2) + j * 8 + 2 * t]);
+              res[i][j][0] = fmaf(-m0v, X.x, res[i][j][0]);
+              res[i][j][1] = fmaf(-m0v, X.y, res[i][j][1]);
+              res[i][j][2] = fmaf(-m1v, X.x, res[i][j][2]);
+              res[i][j][3] = fmaf(-m1v, X.y, res[i][j][3]);
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();                             // the operand tiles may be overwritten
+    if (PL == 1 && h + 1 < halves) fetch_x(h + 1);
+    cp_async_commit();
+  }
+
+  // The sums go through shared memory (row pitch ROWS + 4: the two token rows of a lane pair on distinct banks), where the CTAs of a
+  // cluster add their slices, each a part of the tile in slice order, and rows of the output are stored whole.
+  cp_async_wait<0>();
+  __syncthreads();
+  constexpr int kSumPitch = ROWS + 4;
+  float* sums = reinterpret_cast<float*>(smem);                   // [BT][kSumPitch]
+  static_assert(size_t(BT) * kSumPitch * sizeof(float) <= smem_bytes<QT, T, ROWS, BT>(), "sums");
+#pragma unroll
+  for (int i = 0; i < MI; ++i)
+#pragma unroll
+    for (int j = 0; j < NI; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        sums[(wn * (BT / 2) + j * 8 + 2 * t + (q & 1)) * kSumPitch + wm * (ROWS / 4) + i * 16 + g + 8 * (q >> 1)] = res[i][j][q];
+  const int slices = int(gridDim.z);
+  if (slices > 1) cluster_barrier(); else __syncthreads();
+  for (int idx = int(blockIdx.z) * kThreads + tid; idx < ROWS * BT; idx += slices * kThreads) {
+    const int r = idx % ROWS, col = idx / ROWS;
+    if (n0 + r >= n || m0 + col >= m) continue;
+    float* at = &sums[col * kSumPitch + r];
+    float v = 0.f;
+    if (slices > 1)
+      for (int z = 0; z < slices; ++z) v += ld_cluster_f32(at, uint32_t(z));
+    else
+      v = *at;
+    if (bias != nullptr) v += MmaType<T>::to_float(bias[n0 + r]);
+    y[int64_t(m0 + col) * n + n0 + r] = MmaType<T>::from_float(v);
+  }
+  if (slices > 1) cluster_barrier();           // nobody leaves while its sums may still be read
+}
+
+template <int QT, typename T, int ROWS, int BT>
+int launch_tile(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
+  constexpr size_t smem = smem_bytes<QT, T, ROWS, BT>();
+  static_assert(smem <= 113 * 1024, "two CTAs per SM");
+  auto kern = gemm_exact_kernel<QT, T, ROWS, BT>;
+  static SmemOptIn granted;
+  if (!smem_opt_in(kern, smem, granted)) return RC_LAUNCH;
+  const int tiles = (n + ROWS - 1) / ROWS, m_tiles = (m + BT - 1) / BT, nsb = (k + 255) / 256;
+  if (m_tiles > 65535) return RC_RANGE;
+  // slices of K until two CTAs per SM have work
+  int slices = 1;
+  while (slices < 8 && int64_t(tiles) * m_tiles * (slices + 1) <= 2 * 148 && slices + 1 <= nsb) ++slices;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(tiles), unsigned(m_tiles), unsigned(slices));
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 1;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = unsigned(slices);
+  cfg.attrs = attr;
+  cfg.numAttrs = slices > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<const T*>(a), static_cast<const uint8_t*>(b), static_cast<const T*>(bias), static_cast<T*>(c), m, n,
+                            k) == cudaSuccess ? RC_OK : RC_LAUNCH;
+}
+
+// 128 x 64 tiles (float32: 128 x 32, for its three operand planes) where they give every SM one, else 64 x 32.
+template <int QT, typename T>
+int launch(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
+  constexpr int BT = x_planes<T>() == 3 ? 32 : 64;
+  if (int64_t((n + 127) / 128) * ((m + BT - 1) / BT) >= 148) return launch_tile<QT, T, 128, BT>(a, b, bias, c, m, n, k, s);
+  return launch_tile<QT, T, 64, 32>(a, b, bias, c, m, n, k, s);
+}
+
+}  // namespace exact
+}  // namespace b200gguf

@@ -1,0 +1,30 @@
+"""The exact tensor-core GEMM behind the simt family, from three activation rows on: tiles that are not full in either direction, K of one
+block up to several super-blocks with a remainder, rows at every 16-byte phase, K cut across a cluster.  Against the float64 product."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from dinoml_v2_b200 import kernels, synthetic as S
+from dinoml_v2_b200.gguf_blocks import QTYPES
+
+pytestmark = pytest.mark.gpu
+TDT = {"float16": torch.float16, "bfloat16": torch.bfloat16, "float32": torch.float32}
+BOUND = {"float16": 6e-4, "bfloat16": 4e-3, "float32": 2e-6}          # output rounding; float32: the sums
+
+
+@pytest.mark.parametrize("dtype", sorted(TDT))
+@pytest.mark.parametrize("qtype", sorted(QTYPES))
+def test_edges(qtype, dtype):
+    dev = torch.device("cuda:0")
+    block = QTYPES[qtype].block_size
+    for k in (block, 768, 1280 + (block if block < 256 else 0)):
+        for n, m in ((1, 3), (65, 33), (300, 70), (4097, 130)):
+            blocks = S.random_blocks(qtype, n, k, seed=n + k)
+            x = torch.from_numpy(S.random_activations(m, k, 7, "float32")).to(dev).to(TDT[dtype])
+            bias = torch.randn(n, device=dev).to(TDT[dtype])
+            ref = x.double().cpu().numpy() @ oracle.dequantize(blocks, qtype, k).astype(np.float64).T + bias.double().cpu().numpy()
+            y = kernels.gemm_rcr(x, torch.from_numpy(blocks).to(dev), qtype, bias, variant="simt")
+            assert kernels.device_status() == 0
+            _, _, norm = oracle.max_errors(ref, y.float().cpu().numpy())
+            assert norm <= BOUND[dtype], (k, n, m, norm)
