@@ -15,6 +15,7 @@
 //   * with few tiles K is cut across a cluster of up to 8 CTAs whose sums meet through distributed shared memory.
 // Two CTAs share an SM (< 113 KB each), so that one decodes while the other keeps the tensor pipe busy.
 #pragma once
+#include <cstdint>
 #include <type_traits>
 
 #include "gemv_mma_common.cuh"
@@ -270,6 +271,7 @@ gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const 
     {
       // decode: ROWS * 8 groups of 16 weights
       const int c = h >> 1;
+#pragma unroll 1
       for (int u = tid; u < ROWS * 8; u += kThreads) {
         const int row = u >> 3, grp = u & 7;                     // eight threads per row
         const uint8_t* src = w + int64_t(min(n0 + row, n - 1)) * row_bytes + int64_t(c) * sb_bytes<QT>();
@@ -299,52 +301,65 @@ gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const 
     __syncthreads();
     if ((h & 1) && h + 1 < halves) issue_raw((h + 1) >> 1);      // both halves of the super-block are decoded
     if (PL == 3 && h + 1 < halves) fetch_x(h + 1);
+#pragma unroll 1
+    for (int gg = 0; gg < 8; gg += kPer) {        // not unrolled: hoisted operand loads spill
+      uint32_t a[kPer][MI][4];
 #pragma unroll
-    for (int gg = 0; gg < 8; gg += kPer) {
-      uint32_t a[kPer][MI][4], b[kPer][NI / 2][4];
-      float acc[MI][NI][4];
-#pragma unroll
-      for (int s = 0; s < kPer; ++s) {
+      for (int s = 0; s < kPer; ++s)
 #pragma unroll
         for (int i = 0; i < MI; ++i) ldmatrix4(a_addr + i * 16 * kPitchB + (gg + s) * 32, a[s][i]);
-#pragma unroll
-        for (int pl = PL - 1; pl >= 0; --pl) {                   // the small parts first
-#pragma unroll
-          for (int j = 0; j < NI / 2; ++j) ldmatrix4(b_addr + (pl * BT + j * 16) * kPitchB + (gg + s) * 32, b[s][j]);
-#pragma unroll
-          for (int i = 0; i < MI; ++i)
-#pragma unroll
-            for (int j = 0; j < NI; ++j) {
-              const uint32_t b0 = b[s][j >> 1][2 * (j & 1)], b1 = b[s][j >> 1][2 * (j & 1) + 1];
-              if (s == 0 && pl == PL - 1) MmaType<O>::mma_c(acc[i][j], a[s][i], b0, b1, zero4);
-              else MmaType<O>::mma(acc[i][j], a[s][i], b0, b1);
-            }
-        }
-      }
+      float sc[MI][2];
 #pragma unroll
       for (int i = 0; i < MI; ++i) {
         const int r = wm * (ROWS / 4) + i * 16 + g;
-        const float s0 = sS[gg * ROWS + r], s1 = sS[gg * ROWS + r + 8];
+        sc[i][0] = sS[gg * ROWS + r];
+        sc[i][1] = sS[gg * ROWS + r + 8];
+      }
+      // 16 activation rows at a time: few live accumulators, so that 64 of them per warp fit beside the results
 #pragma unroll
-        for (int j = 0; j < NI; ++j) {
-          res[i][j][0] = fmaf(s0, acc[i][j][0], res[i][j][0]);
-          res[i][j][1] = fmaf(s0, acc[i][j][1], res[i][j][1]);
-          res[i][j][2] = fmaf(s1, acc[i][j][2], res[i][j][2]);
-          res[i][j][3] = fmaf(s1, acc[i][j][3], res[i][j][3]);
-        }
+      for (int jj = 0; jj < NI / 2; ++jj) {
+        float acc[MI][2][4];
+#pragma unroll
+        for (int s = 0; s < kPer; ++s)
+#pragma unroll
+          for (int pl = PL - 1; pl >= 0; --pl) {                 // the small parts first
+            uint32_t b[4];
+            ldmatrix4(b_addr + (pl * BT + jj * 16) * kPitchB + (gg + s) * 32, b);
+#pragma unroll
+            for (int i = 0; i < MI; ++i)
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                if (s == 0 && pl == PL - 1) MmaType<O>::mma_c(acc[i][j], a[s][i], b[2 * j], b[2 * j + 1], zero4);
+                else MmaType<O>::mma(acc[i][j], a[s][i], b[2 * j], b[2 * j + 1]);
+              }
+          }
+#pragma unroll
+        for (int i = 0; i < MI; ++i)
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            float (&r)[4] = res[i][2 * jj + j];
+            r[0] = fmaf(sc[i][0], acc[i][j][0], r[0]);
+            r[1] = fmaf(sc[i][0], acc[i][j][1], r[1]);
+            r[2] = fmaf(sc[i][1], acc[i][j][2], r[2]);
+            r[3] = fmaf(sc[i][1], acc[i][j][3], r[3]);
+          }
         if constexpr (kMins) {
 #pragma unroll
-          for (int s = 0; s < kPer; ++s) {
-            const float m0v = sM[(gg + s) * ROWS + r], m1v = sM[(gg + s) * ROWS + r + 8];
+          for (int s = 0; s < kPer; ++s)
 #pragma unroll
-            for (int j = 0; j < NI; ++j) {
-              const float2 X = *reinterpret_cast<const float2*>(&sX[(gg + s) * BT + wn * (BT / 2) + j * 8 + 2 * t]);
-              res[i][j][0] = fmaf(-m0v, X.x, res[i][j][0]);
-              res[i][j][1] = fmaf(-m0v, X.y, res[i][j][1]);
-              res[i][j][2] = fmaf(-m1v, X.x, res[i][j][2]);
-              res[i][j][3] = fmaf(-m1v, X.y, res[i][j][3]);
+            for (int i = 0; i < MI; ++i) {
+              const int row = wm * (ROWS / 4) + i * 16 + g;
+              const float m0v = sM[(gg + s) * ROWS + row], m1v = sM[(gg + s) * ROWS + row + 8];
+#pragma unroll
+              for (int j = 0; j < 2; ++j) {
+                const float2 X = *reinterpret_cast<const float2*>(&sX[(gg + s) * BT + wn * (BT / 2) + (2 * jj + j) * 8 + 2 * t]);
+                float (&r)[4] = res[i][2 * jj + j];
+                r[0] = fmaf(-m0v, X.x, r[0]);
+                r[1] = fmaf(-m0v, X.y, r[1]);
+                r[2] = fmaf(-m1v, X.x, r[2]);
+                r[3] = fmaf(-m1v, X.y, r[3]);
+              }
             }
-          }
         }
       }
     }
@@ -393,9 +408,14 @@ int launch_tile(const void* a, const void* b, const void* bias, void* c, int m, 
   if (!smem_opt_in(kern, smem, granted)) return RC_LAUNCH;
   const int tiles = (n + ROWS - 1) / ROWS, m_tiles = (m + BT - 1) / BT, nsb = (k + 255) / 256;
   if (m_tiles > 65535) return RC_RANGE;
-  // slices of K until two CTAs per SM have work
+  // The number of K slices with the shortest walk: rounds of two CTAs per SM times super-blocks per slice (a slice costs about two
+  // super-blocks more for its start and the exchange of sums).
   int slices = 1;
-  while (slices < 8 && int64_t(tiles) * m_tiles * (slices + 1) <= 2 * 148 && slices + 1 <= nsb) ++slices;
+  int64_t best = INT64_MAX;
+  for (int z = 1; z <= 8 && z <= nsb; ++z) {
+    const int64_t walk = ((int64_t(tiles) * m_tiles * z + 2 * 148 - 1) / (2 * 148)) * ((nsb + z - 1) / z + 2);
+    if (walk < best) { best = walk; slices = z; }
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(unsigned(tiles), unsigned(m_tiles), unsigned(slices));
   cfg.blockDim = dim3(kThreads);
@@ -412,11 +432,18 @@ int launch_tile(const void* a, const void* b, const void* bias, void* c, int m, 
                             k) == cudaSuccess ? RC_OK : RC_LAUNCH;
 }
 
-// 128 x 64 tiles (float32: 128 x 32, for its three operand planes) where they give every SM one, else 64 x 32.
+// 128 x 128 tiles above 64 activation rows, 128 x 64 above 32 (float32: 128 x 32, for its three operand planes) where that gives a
+// quarter of the SMs a tile, else 64 x 32.
 template <int QT, typename T>
 int launch(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
-  constexpr int BT = x_planes<T>() == 3 ? 32 : 64;
-  if (int64_t((n + 127) / 128) * ((m + BT - 1) / BT) >= 148) return launch_tile<QT, T, 128, BT>(a, b, bias, c, m, n, k, s);
+  constexpr bool kPlanes = x_planes<T>() == 3;
+  const int64_t row_tiles = (n + 127) / 128;
+  if constexpr (!kPlanes) {
+    if (m > 64 && row_tiles * ((m + 127) / 128) >= 37) return launch_tile<QT, T, 128, 128>(a, b, bias, c, m, n, k, s);
+    if (m > 32 && row_tiles * ((m + 63) / 64) >= 37) return launch_tile<QT, T, 128, 64>(a, b, bias, c, m, n, k, s);
+  } else {
+    if (row_tiles * ((m + 31) / 32) >= 37) return launch_tile<QT, T, 128, 32>(a, b, bias, c, m, n, k, s);
+  }
   return launch_tile<QT, T, 64, 32>(a, b, bias, c, m, n, k, s);
 }
 
