@@ -9,7 +9,7 @@
 //
 // A CTA of 8 warps owns ROWS weight rows x BT activation rows and walks K in super-blocks of 256:
 //   * packed bytes: every row's 16-byte aligned window around its super-block, 16-byte cp.async (rows have phases of their own);
-//   * per half super-block each thread decodes 64 weights (four groups) of one row into the operand tile and its scales; the next
+//   * per half super-block each thread decodes 64 (or 32) weights of one row into the operand tile and its scales; the next
 //     super-block's bytes are requested as soon as the second half is decoded;
 //   * warps 4 x 2 take ROWS/4 x BT/2 of the tile with ldmatrix operands;
 //   * with few tiles K is cut across a cluster of up to 8 CTAs whose sums meet through distributed shared memory.
@@ -74,94 +74,113 @@ template <typename O> __device__ __forceinline__ uint32_t pack(float lo, float h
     return *reinterpret_cast<const uint32_t*>(&v);
   }
 }
-// Four FP4 codes (low nibbles of the bytes of w, high nibbles zero) -> their e2m1 values as two operand pairs: byte look-ups of the
-// magnitudes (0, .5, 1, 1.5, 2, 3, 4, 6) with the codes as selector, then the sign bits.
-template <typename O>
-__device__ __forceinline__ void fp4_pairs(uint32_t w, uint32_t& p01, uint32_t& p23) {
-  const uint32_t mag = w & 0x07070707u, sign = (w & 0x08080808u) << 4;
+// Offset of a type's quants as unsigned bytes: weight = scale * (byte - offset) - min.  FP4 codes become 12 + 2 * e2m1.
+template <int QT> constexpr int byte_offset() {
+  return QT == QTYPE_Q8_0 ? 128 : QT == QTYPE_Q6_K ? 32 : QT == QTYPE_Q4_0 ? 8 : QT == QTYPE_Q3_K ? 4 : (QT == QTYPE_MXFP4 || QT == QTYPE_NVFP4) ? 12 : 0;
+}
+// Four FP4 codes (low nibbles of the bytes, high nibbles zero) -> bytes 12 + 2 * e2m1: look-ups of the eight magnitudes, both signs.
+__device__ __forceinline__ uint32_t fp4_bytes(uint32_t w) {
+  const uint32_t mag = w & 0x07070707u;
   const uint32_t sel = __byte_perm(mag | (mag >> 4), 0u, 0x4420);
-  if constexpr (std::is_same<O, __half>::value) {
-    const uint32_t hi = __byte_perm(0x3E3C3800u, 0x46444240u, sel) | sign;
-    p01 = __byte_perm(hi, 0u, 0x1404);
-    p23 = __byte_perm(hi, 0u, 0x3424);
-  } else {
-    const uint32_t hi = __byte_perm(0x3F3F3F00u, 0x40404040u, sel) | sign, lo = __byte_perm(0xC0800000u, 0xC0804000u, sel);
-    p01 = __byte_perm(lo, hi, 0x5140);
-    p23 = __byte_perm(lo, hi, 0x7362);
-  }
+  const uint32_t pos = __byte_perm(0x0F0E0D0Cu, 0x18141210u, sel), neg = __byte_perm(0x090A0B0Cu, 0x00040608u, sel);
+  const uint32_t sign = ((w >> 3) & 0x01010101u) * 0xffu;
+  return (pos & ~sign) | (neg & sign);
 }
 
-// Group gi (16 weights) of the super-block at p: operand pairs in K order, scale, min (w = scale * operand - min).
-template <int QT, typename O>
-__device__ __forceinline__ void group16(const uint8_t* p, int gi, uint32_t (&o)[8], float& scale, float& mn) {
-  uint32_t w[4];
-  mn = 0.f;
-  if constexpr (QT == QTYPE_Q8_0) {
-    const uint8_t* b = p + 34 * (gi >> 1);
-    scale = half_at(b);
-    lds16(b + 2 + 16 * (gi & 1), w);
+// NJ groups of 16 weights of the super-block at p that lie 32 apart: weights 128 hb + 32 j + 16 u + 0..15, j = j0 .. j0 + NJ - 1 (NJ = 2 or 4,
+// j0 = 0 or 2).  Each packed word is read once for all groups that it serves.
+template <int QT, int NJ> struct Unit {
+  static constexpr bool kHigh = QT == QTYPE_Q5_K || QT == QTYPE_Q6_K || QT == QTYPE_Q3_K;
+  static constexpr int kWords = (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) ? NJ / 2 : QT == QTYPE_Q6_K ? 2 : (QT == QTYPE_Q2_K || QT == QTYPE_Q3_K) ? 1 : NJ;
+  uint32_t w[kWords][4], h[kHigh ? 4 : 1];
+  float scale[NJ], mn[NJ];
+  int hb, j0, u;
+
+  __device__ __forceinline__ void load(const uint8_t* p, int hb_, int j0_, int u_) {
+    hb = hb_; j0 = j0_; u = u_;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      o[2 * i] = pack<O>(float(int(int8_t(w[i]))), float(int(int8_t(w[i] >> 8))));
-      o[2 * i + 1] = pack<O>(float(int(int8_t(w[i] >> 16))), float(int(int8_t(w[i] >> 24))));
-    }
-  } else if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4) {
-    constexpr int BB = QT == QTYPE_Q4_0 ? 18 : 17;
-    const uint8_t* b = p + BB * (gi >> 1);
-    scale = QT == QTYPE_Q4_0 ? half_at(b) : 2.f * e8m0_half(b[0]);
-    lds16(b + BB - 16, w);
+    for (int i = 0; i < NJ; ++i) mn[i] = 0.f;
+    if constexpr (QT == QTYPE_Q8_0) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t n = (w[i] >> (4 * (gi & 1))) & 0x0f0f0f0fu;
-      if constexpr (QT == QTYPE_Q4_0) bytes_minus<O>(n, 8, o[2 * i], o[2 * i + 1]);
-      else fp4_pairs<O>(n, o[2 * i], o[2 * i + 1]);
-    }
-  } else if constexpr (QT == QTYPE_NVFP4) {
-    const uint8_t* b = p + 36 * (gi >> 2);
-    scale = 2.f * ue4m3_half(b[gi & 3]);
-    lds16(b + 4 + 8 * (gi & 3), w);              // 8 bytes of this sub-block (and 8 of the next)
+      for (int i = 0; i < NJ; ++i) {
+        const uint8_t* b = p + 34 * (4 * hb + j0 + i);
+        scale[i] = half_at(b);
+        lds16(b + 2 + 16 * u, w[i]);
+      }
+    } else if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4) {
+      constexpr int BB = QT == QTYPE_Q4_0 ? 18 : 17;
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      fp4_pairs<O>(w[i] & 0x0f0f0f0fu, o[2 * i], o[2 * i + 1]);
-      fp4_pairs<O>((w[i] >> 4) & 0x0f0f0f0fu, o[4 + 2 * i], o[4 + 2 * i + 1]);
-    }
-  } else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) {
-    const int j = gi >> 1;
-    int sc, m;
-    k4_scale_min(j, p + 4, sc, m);
-    scale = half_at(p) * float(sc);
-    mn = half_at(p + 2) * float(m);
-    lds16(p + (QT == QTYPE_Q4_K ? 16 : 48) + 32 * (j >> 1) + 16 * (gi & 1), w);
-    uint32_t h[4] = {0u, 0u, 0u, 0u};
-    if constexpr (QT == QTYPE_Q5_K) lds16(p + 16 + 16 * (gi & 1), h);
+      for (int i = 0; i < NJ; ++i) {
+        const uint8_t* b = p + BB * (4 * hb + j0 + i);
+        scale[i] = QT == QTYPE_Q4_0 ? half_at(b) : e8m0_half(b[0]);
+        lds16(b + BB - 16, w[i]);
+      }
+    } else if constexpr (QT == QTYPE_NVFP4) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) bytes_minus<O>(((w[i] >> (4 * (j & 1))) & 0x0f0f0f0fu) | (((h[i] >> j) & 0x01010101u) << 4), 0, o[2 * i], o[2 * i + 1]);
-  } else {
-    const int hb = gi >> 3, quad = (gi >> 1) & 3, u = gi & 1;
-    if constexpr (QT == QTYPE_Q6_K) {
-      scale = half_at(p + 208) * float(int(int8_t(p[192 + gi])));
-      uint32_t h[4];
-      lds16(p + 64 * hb + 32 * (quad & 1) + 16 * u, w);
+      for (int i = 0; i < NJ; ++i) {
+        const uint8_t* b = p + 36 * (2 * hb + ((j0 + i) >> 1));
+        const int sub = 2 * ((j0 + i) & 1) + u;
+        scale[i] = ue4m3_half(b[sub]);
+        lds16(b + 4 + 8 * sub, w[i]);            // 8 bytes of this sub-block (and 8 of the next)
+      }
+    } else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) {
+      const float d = half_at(p), dmin = half_at(p + 2);
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) {
+        int sc, m;
+        k4_scale_min(4 * hb + j0 + i, p + 4, sc, m);
+        scale[i] = d * float(sc);
+        mn[i] = dmin * float(m);
+      }
+#pragma unroll
+      for (int i = 0; i < NJ / 2; ++i) lds16(p + (QT == QTYPE_Q4_K ? 16 : 48) + 32 * (2 * hb + (j0 >> 1) + i) + 16 * u, w[i]);
+      if constexpr (QT == QTYPE_Q5_K) lds16(p + 16 + 16 * u, h);
+    } else if constexpr (QT == QTYPE_Q6_K) {
+      const float d = half_at(p + 208);
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) scale[i] = d * float(int(int8_t(p[192 + 8 * hb + 2 * (j0 + i) + u])));
+      lds16(p + 64 * hb + 16 * u, w[0]);
+      lds16(p + 64 * hb + 32 + 16 * u, w[1]);
       lds16(p + 128 + 32 * hb + 16 * u, h);
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        bytes_minus<O>(((w[i] >> (quad & 2 ? 4 : 0)) & 0x0f0f0f0fu) | (((h[i] >> (2 * quad)) & 0x03030303u) << 4), 32, o[2 * i], o[2 * i + 1]);
     } else if constexpr (QT == QTYPE_Q2_K) {
-      const uint32_t s = p[gi];
-      scale = half_at(p + 80) * float(s & 0x0fu);
-      mn = half_at(p + 82) * float(s >> 4);
-      lds16(p + 16 + 32 * hb + 16 * u, w);
+      const float d = half_at(p + 80), dmin = half_at(p + 82);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) bytes_minus<O>((w[i] >> (2 * quad)) & 0x03030303u, 0, o[2 * i], o[2 * i + 1]);
+      for (int i = 0; i < NJ; ++i) {
+        const uint32_t s = p[8 * hb + 2 * (j0 + i) + u];
+        scale[i] = d * float(s & 0x0fu);
+        mn[i] = dmin * float(s >> 4);
+      }
+      lds16(p + 16 + 32 * hb + 16 * u, w[0]);
     } else {
-      scale = half_at(p + 108) * float(q3k_scale(p + 96, gi) - 32);
-      uint32_t h[4];
-      lds16(p + 32 + 32 * hb + 16 * u, w);
-      lds16(p + 16 * u, h);
+      const float d = half_at(p + 108);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        bytes_minus<O>(((w[i] >> (2 * quad)) & 0x03030303u) | (((h[i] >> (4 * hb + quad)) & 0x01010101u) << 2), 4, o[2 * i], o[2 * i + 1]);
+      for (int i = 0; i < NJ; ++i) scale[i] = d * float(q3k_scale(p + 96, 8 * hb + 2 * (j0 + i) + u) - 32);
+      lds16(p + 32 + 32 * hb + 16 * u, w[0]);
+      lds16(p + 16 * u, h);
     }
+  }
+  // Word k (weights 4k .. 4k+3) of group i as unsigned bytes.
+  __device__ __forceinline__ uint32_t bytes(int i, int k) const {
+    const int j = j0 + i;
+    if constexpr (QT == QTYPE_Q8_0) return w[i][k] ^ 0x80808080u;
+    else if constexpr (QT == QTYPE_Q4_0) return (w[i][k] >> (4 * u)) & 0x0f0f0f0fu;
+    else if constexpr (QT == QTYPE_MXFP4) return fp4_bytes((w[i][k] >> (4 * u)) & 0x0f0f0f0fu);
+    else if constexpr (QT == QTYPE_NVFP4) return fp4_bytes((w[i][k & 1] >> (k < 2 ? 0 : 4)) & 0x0f0f0f0fu);
+    else if constexpr (QT == QTYPE_Q4_K) return (w[i >> 1][k] >> (4 * (i & 1))) & 0x0f0f0f0fu;
+    else if constexpr (QT == QTYPE_Q5_K) return ((w[i >> 1][k] >> (4 * (i & 1))) & 0x0f0f0f0fu) | (((h[k] >> (4 * hb + j)) & 0x01010101u) << 4);
+    else if constexpr (QT == QTYPE_Q6_K) return ((w[i & 1][k] >> (2 * (j & 2))) & 0x0f0f0f0fu) | (((h[k] >> (2 * j)) & 0x03030303u) << 4);
+    else if constexpr (QT == QTYPE_Q2_K) return (w[0][k] >> (2 * j)) & 0x03030303u;
+    else return ((w[0][k] >> (2 * j)) & 0x03030303u) | (((h[k] >> (4 * hb + j)) & 0x01010101u) << 2);
+  }
+};
+// Four such bytes less the type's offset -> two operand pairs, exact.
+template <int QT, typename O>
+__device__ __forceinline__ void byte_pairs(uint32_t w, uint32_t& p01, uint32_t& p23) {
+  if constexpr (QT == QTYPE_Q8_0 && !std::is_same<O, __half>::value) {     // bytes above 127 do not fit the bfloat16 pattern 0x43qq
+    p01 = pack<O>(byte_to_float(w, 0) - 128.f, byte_to_float(w, 1) - 128.f);
+    p23 = pack<O>(byte_to_float(w, 2) - 128.f, byte_to_float(w, 3) - 128.f);
+  } else {
+    bytes_minus<O>(w, byte_offset<QT>(), p01, p23);
   }
 }
 
@@ -271,19 +290,24 @@ gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const 
     {
       // decode: ROWS * 8 groups of 16 weights
       const int c = h >> 1;
-#pragma unroll 1
-      for (int u = tid; u < ROWS * 8; u += kThreads) {
-        const int row = u >> 3, grp = u & 7;                     // eight threads per row
-        const uint8_t* src = w + int64_t(min(n0 + row, n - 1)) * row_bytes + int64_t(c) * sb_bytes<QT>();
+      constexpr int NJ = ROWS * 2 >= kThreads ? 4 : 2;            // ROWS * 8 / NJ units, one per thread
+      static_assert(ROWS * 8 / NJ == kThreads, "one unit per thread");
+      const int row = tid / (8 / NJ), part = tid % (8 / NJ), u = part & 1;
+      const uint8_t* src = w + int64_t(min(n0 + row, n - 1)) * row_bytes + int64_t(c) * sb_bytes<QT>();
+      Unit<QT, NJ> unit;
+      unit.load(raw + row * kRawPitch + (reinterpret_cast<uintptr_t>(src) & 15), h & 1, NJ == 4 ? 0 : part & 2, u);
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) {
+        const int grp = 2 * (unit.j0 + i) + u;
         uint32_t o[8];
-        float scale, mn;
-        group16<QT, O>(raw + row * kRawPitch + (reinterpret_cast<uintptr_t>(src) & 15), 8 * (h & 1) + grp, o, scale, mn);
-        if (h * kHalfK + 16 * grp >= k) scale = mn = 0.f;        // past the end of the row: whatever the buffer holds
+#pragma unroll
+        for (int q = 0; q < 4; ++q) byte_pairs<QT, O>(unit.bytes(i, q), o[2 * q], o[2 * q + 1]);
         uint4* dst = reinterpret_cast<uint4*>(sA + row * kPitchB + 32 * grp);
         dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
         dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
-        sS[grp * ROWS + row] = scale;
-        if constexpr (kMins) sM[grp * ROWS + row] = mn;
+        const bool in = h * kHalfK + 16 * grp < k;               // past the end of the row: whatever the buffer holds
+        sS[grp * ROWS + row] = in ? unit.scale[i] : 0.f;
+        if constexpr (kMins) sM[grp * ROWS + row] = in ? unit.mn[i] : 0.f;
       }
       if constexpr (kMins) {
         for (int u = tid; u < BT * 8; u += kThreads) {

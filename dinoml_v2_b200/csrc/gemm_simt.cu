@@ -11,6 +11,7 @@
 
 namespace b200gguf {
 
+int gemm_split(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, cudaStream_t s);
 int gemm_exact(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, cudaStream_t s);
 int gemv_planes(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, const PeerOut& peers, cudaStream_t s);
 
@@ -141,7 +142,12 @@ int gemm_rcr_simt(const void* a, const void* b, const void* bias, void* c, int q
                        m - r < 2 ? 1 : 2, n, k, no_peers(), s);
     if (rc != RC_RANGE) return rc;
   }
-  // More rows: the same exact products on the tensor cores (one or two rows of the FP4 types stay below: 16 us against 24 us).
+  // Else the same exact products by mma.sync (one or two rows of the FP4 types stay below: 16 us against 24 us).
+  // 16-bit activations on tcgen05 where the weight has enough super-block tiles for all SMs, or the rows pay for the start of that
+  // kernel (Q8_0 [4096 x 2880] float16, M = 8: 11.9 us against 14.6; MXFP4 [5760 x 2880] bfloat16, M = 24: 19.6 against 18.9, M = 200:
+  // 34.6 against 54.4; Q6_K [1024 x 2816], 88 tiles: M = 64 13.1 against 12.0, M = 200 21.8 against 27.9).
+  if (m >= 7 && (m > 128 || int64_t((n + 127) / 128) * ((k + 255) / 256) >= 256))
+    if (int rc = gemm_split(a, b, bias, c, qtype, dtype, m, n, k, s); rc != RC_RANGE) return rc;
   if (m >= 3)
     if (int rc = gemm_exact(a, b, bias, c, qtype, dtype, m, n, k, s); rc != RC_RANGE) return rc;
   switch (qtype) {

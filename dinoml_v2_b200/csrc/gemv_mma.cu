@@ -35,6 +35,7 @@ namespace b200gguf {
 
 int check_gemm_args(const void* a, const void* b, const void* c, int qtype, int dtype, int m, int n, int k);
 int gemv_planes(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, const PeerOut& peers, cudaStream_t s);
+int gemm_split(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, cudaStream_t s);
 int gemm_rcr_stream_peers(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k, int config,
                           const PeerOut* peer_out, cudaStream_t s);
 namespace stream { int sm_count(); }
@@ -361,6 +362,13 @@ int gemm_rcr_mma_peers(const void* a, const void* b, const void* bias, void* c, 
   // Q4_K, one row and more tiles than SMs: [11008 x 4096] 7.9 us on the persistent kernel with byte operands, 9.3 us here.
   if (qtype == QTYPE_Q4_K && m == 1 && (n + kGemvRows - 1) / kGemvRows > stream::sm_count())
     return gemm_rcr_stream_peers(a, b, bias, c, qtype, dtype, m, n, k, 0, &peers, s);
+  // Q6_K with ragged rows, M = 9 .. 16, on a weight large enough for tcgen05: [4096 x 11008] float16 24.5 us against 34.5 here,
+  // [8192 x 28416] M = 16 89 us against 176 (bfloat16, three weight terms: 145).
+  if (qtype == QTYPE_Q6_K && k % 2048 != 0 && m >= 9 && peers.count == 0 && peers.act == ACT_NONE &&
+      int64_t((n + 127) / 128) * (k / 256) >= (dtype == DINO_F16 ? 256 : 4096)) {
+    const int rc = gemm_split(a, b, bias, c, qtype, dtype, m, n, k, s);
+    if (rc != RC_RANGE) return rc;
+  }
   if (qtype == QTYPE_Q6_K) return gemv_q6k_mma(a, b, bias, c, dtype, m, n, k, peers, s);
   if (qtype == QTYPE_Q8_0) {
     if (peers.count > 0 || peers.act != ACT_NONE) return RC_RANGE;   // no scatter / gated epilogue for Q8_0

@@ -14,6 +14,7 @@ struct DeviceState {
   int* status = nullptr;            // [0] = status word, [1 .. kMaxCtas] = partial-tile flags
   float* workspace = nullptr;
   size_t workspace_bytes = 0;
+  std::vector<void*> outgrown;      // smaller workspaces that captured graphs may still use; given back with the set
 };
 static std::mutex g_mutex;
 // One workspace + flag set per (device, stream): launches on one stream are ordered and may share them, launches on
@@ -31,6 +32,18 @@ static std::unordered_map<StateKey, DeviceState, StateKeyHash> g_state;
 constexpr size_t kMaxSpare = 4;
 static std::unordered_map<int, std::vector<DeviceState>> g_spare;
 
+// A larger workspace, outside of stream capture only: callers warm a shape up once before capturing a graph.  At least twice the old
+// size, which stays for graphs captured with it: what a set holds is bounded by twice its largest workspace.
+static bool grow(DeviceState& st, size_t need) {
+  const size_t size = need > 2 * st.workspace_bytes ? need : 2 * st.workspace_bytes;
+  float* p = nullptr;
+  if (cudaMalloc(&p, size) != cudaSuccess) return false;
+  if (st.workspace != nullptr) st.outgrown.push_back(st.workspace);
+  st.workspace = p;
+  st.workspace_bytes = size;
+  return true;
+}
+
 static DeviceState* device_state(size_t need_workspace, cudaStream_t stream) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
@@ -46,10 +59,7 @@ static DeviceState* device_state(size_t need_workspace, cudaStream_t stream) {
     cudaMemsetAsync(st.status, 0, sizeof(int) * (1 + kMaxCtas), stream);
   }
   if (need_workspace > st.workspace_bytes) {
-    // Grown outside of stream capture only: callers warm a shape up once before capturing a graph.
-    if (st.workspace != nullptr) { cudaDeviceSynchronize(); cudaFree(st.workspace); st.workspace = nullptr; st.workspace_bytes = 0; }
-    if (cudaMalloc(&st.workspace, need_workspace) != cudaSuccess) return nullptr;
-    st.workspace_bytes = need_workspace;
+    if (!grow(st, need_workspace)) return nullptr;
   }
   return &st;
 }
@@ -66,21 +76,22 @@ static void release(cudaStream_t stream) {
       } else {
         cudaFree(it->second.status);
         if (it->second.workspace != nullptr) cudaFree(it->second.workspace);
+        for (void* p : it->second.outgrown) cudaFree(p);
       }
     }
     it = g_state.erase(it);
   }
 }
 
-static Plan make_plan(int m, int n, int k) {
+static Plan plan_for(int m, int n, int k, int bm) {
   Plan pl;
-  pl.bm = m <= 64 ? 64 : m <= 128 ? 128 : 256;
+  pl.bm = bm;
   pl.m_tiles = (m + pl.bm - 1) / pl.bm;
   // The M rows in equal tiles of a multiple of 16: M = 333 is two tiles of 176 rows, not 256 + 77 padded to 512 (the MMA time and
   // the activation bytes go with the rows of a tile).
   pl.bn = ((m + pl.m_tiles - 1) / pl.m_tiles + 15) / 16 * 16;
   const long long tiles = static_cast<long long>(pl.m_tiles) * ((n + kRowsW - 1) / kRowsW);
-  const int nsb = k / 256;
+  const int nsb = (k + 255) / 256;
   pl.units = tiles * nsb;
   int sm_count = 148;
   int dev = 0;
@@ -91,6 +102,19 @@ static Plan make_plan(int m, int n, int k) {
   pl.ctas = int(most < sm_count ? most : sm_count);
   pl.workspace_bytes = tiles % pl.ctas == 0 ? 0 : size_t(pl.ctas) * pl.bm * kRowsW * sizeof(float);
   return pl;
+}
+
+static Plan make_plan(int m, int n, int k) { return plan_for(m, n, k, m <= 64 ? 64 : m <= 128 ? 128 : 256); }
+
+// For the split-operand kernels (umma_split.cu): the same plan at their tile height, the same scratch.
+Plan split_plan(int m, int n, int k, int bm) { return plan_for(m, n, k, bm); }
+int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc) {
+  DeviceState* st = device_state(workspace_bytes, stream);
+  if (st == nullptr) return RC_LAUNCH;
+  sc->workspace = st->workspace;
+  sc->status = st->status;
+  sc->flags = st->status + 1;
+  return RC_OK;
 }
 
 // ---- allocation-free scratch -------------------------------------------------------------------

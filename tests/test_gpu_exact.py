@@ -13,6 +13,22 @@ TDT = {"float16": torch.float16, "bfloat16": torch.bfloat16, "float32": torch.fl
 BOUND = {"float16": 6e-4, "bfloat16": 4e-3, "float32": 2e-6}          # output rounding; float32: the sums
 
 
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("qtype,k", [("Q8_0", 288), ("Q6_K", 2816), ("Q4_0", 2880), ("Q2_K", 1280), ("Q3_K", 2560), ("MXFP4", 2848), ("MXFP4", 2880), ("NVFP4", 2880)])
+def test_split_operands(qtype, k, dtype):
+    """The tcgen05 kernel with split weights: full and last tiles of 128 rows, one and more activation tiles, rows of every residue."""
+    dev = torch.device("cuda:0")
+    for n, m in ((1, 129), (128, 160), (301, 257), (4099, 24)):
+        blocks = S.random_blocks(qtype, n, k, seed=n + k)
+        x = torch.from_numpy(S.random_activations(m, k, 7, "float32")).to(dev).to(TDT[dtype])
+        bias = torch.randn(n, device=dev).to(TDT[dtype])
+        ref = x.double().cpu().numpy() @ oracle.dequantize(blocks, qtype, k).astype(np.float64).T + bias.double().cpu().numpy()
+        y = kernels.gemm_rcr(x, torch.from_numpy(blocks).to(dev), qtype, bias)
+        assert kernels.device_status() == 0
+        _, _, norm = oracle.max_errors(ref, y.float().cpu().numpy())
+        assert norm <= BOUND[dtype], (n, m, norm)
+
+
 @pytest.mark.parametrize("dtype", sorted(TDT))
 @pytest.mark.parametrize("qtype", sorted(QTYPES))
 def test_edges(qtype, dtype):
