@@ -58,7 +58,7 @@ namespace umma {
 constexpr int kRowsW = 128;            // weight rows per CTA (UMMA M)
 constexpr int kBK = 64;                // K per pipeline stage (one 128-byte swizzle atom of 16-bit values)
 constexpr int kProducerThreads = 512;
-constexpr int kGroupThreads = 256;     // producers of one K stage
+constexpr int kGroupThreads = 256;     // producers of half a super-block
 constexpr int kThreads = kProducerThreads + 96;   // + activation TMA warp, MMA warp, packed-weight TMA warp
 constexpr uint32_t kSpinLimit = 1u << 24;   // try_wait polls before a wait gives up (each poll suspends ~tens of ns or more)
 
@@ -360,6 +360,10 @@ constexpr int kStagesPerSb = 4;         // 256 weights / kBK: the MMA loop relie
 constexpr int kWSlotCols = kBK / 2;     // 64 16-bit values per lane = 32 columns
 constexpr int kSmemBudget = 227 * 1024;
 template <int BM> constexpr bool coarse_handover() { return BM < 256; }
+// Q4_K, Q5_K: a producer thread takes one whole stage (64 weights = 32 bytes of nibbles, two sub-blocks) of its row instead of half of
+// two stages: two scales and mins to decode instead of four, one hand-over instead of two (350 -> 263 instructions per 64 weights;
+// [8192 x 28672] Q4_K, M = 2048: 825 -> 772 us).
+template <int QT> constexpr bool whole_stage() { return QT == QTYPE_Q4_K || QT == QTYPE_Q5_K; }
 template <int BM> constexpr int stage_units() { return BM >= 256 ? 1 : BM >= 128 ? 2 : 3; }
 template <int BM> constexpr int x_tile_bytes() { return BM * kBK * 2; }
 template <int QT> constexpr int raw_box_bytes() { return kRowsW * RawGeom<QT>::kPitch; }
@@ -434,7 +438,6 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
   constexpr int kBlockBytes = RawGeom<QT>::kSuper;
   const uint32_t idesc = (1u << 4) | (P::kFormat << 7) | (P::kFormat << 10) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kRowsW >> 4) << 24);
   const uint32_t x_bytes = uint32_t(p.bn) * (kBK * 2);        // bytes of one activation stage (its shared-memory slot holds BM rows)
-  constexpr uint32_t kWarpArrivals = kGroupThreads / 32;     // one elected arrive per producer warp of a group
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -466,7 +469,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
 
   if (tid == 0) {
     for (int s = 0; s < NB; ++s) {
-      mbar_init(full(s), (COARSE ? 2 : 1) * kWarpArrivals + 1);   // the producer warps that fill it + the TMA lane's arrive.expect_tx
+      mbar_init(full(s), (COARSE ? 16 : whole_stage<QT>() ? 4 : 8) + 1);   // the producer warps that fill it + the TMA lane's arrive.expect_tx
       mbar_init(empty(s), 1);
     }
     for (int s = 0; s < NSR; ++s) {
@@ -632,20 +635,19 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
       return true;
     };
     int pend_t = -1, pend_b = 0, pend_e = 0;                    // segment whose epilogue has not run yet
+    // packed ring and stage ring positions, counted along (a division per super-block showed in the instruction count)
+    int rslot = 0, ub = 0;
+    uint32_t rphase = 0, uphase = 1;                            // uphase: of the `empty` barrier to wait for, from the second lap on
     for (int t = tile_hi; t >= tile_lo && alive; --t, ++segi) {
       int sb_b, sb_e;
       walk.segment(t, sb_b, sb_e);
       for (int sb = sb_b; sb < sb_e && alive; ++sb, ++it) {
-        const int rslot = it % NSR;
-        {
-          int ok = 1;
-          if (lane == 0) ok = mbar_wait(rawfull(rslot), uint32_t(it / NSR) & 1u, abort_flag, p.status, ST_FULL_TIMEOUT) ? 1 : 0;
-          ok = __shfl_sync(0xffffffffu, ok, 0);
-          if (!ok) { alive = false; break; }
-        }
+        if (!warp_wait(rawfull(rslot), rphase, abort_flag, p.status, ST_FULL_TIMEOUT)) { alive = false; break; }
         const uint8_t* rowbase = raw + rslot * kRawBytes + row * kPitch;
         // ---- copy this thread's packed words to registers
-        uint32_t qw[(QT == QTYPE_Q8_0 || QT == QTYPE_Q5_K) ? 16 : 12];
+        constexpr bool kWhole = whole_stage<QT>();
+        const int my_stage = warp >> 2;       // kWhole: this warp's stage of the super-block
+        uint32_t qw[QT == QTYPE_Q5_K ? 20 : QT == QTYPE_Q8_0 ? 16 : 12];
         float dscale = 0.f, dmin = 0.f;
         float sub_scale[4];                   // Q6_K: int8 scales of quads 0..3; Q8_0: d of this thread's four blocks
         float sub_min[4] = {0.f, 0.f, 0.f, 0.f};   // Q2_K: -dmin * min of the thread's four sub-blocks
@@ -668,21 +670,26 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
           const uint4 hdr = *reinterpret_cast<const uint4*>(rowbase);
           dscale = half_bits_to_float(uint16_t(hdr.x & 0xffffu));
           dmin = half_bits_to_float(uint16_t(hdr.x >> 16));
-          // sub-blocks 4*grp .. 4*grp+3 belong to this thread's two stages
-          const uint32_t scw = grp == 0 ? (hdr.y & 0x3f3f3f3fu) : ((hdr.w & 0x0f0f0f0fu) | (((hdr.y >> 6) & 0x03030303u) << 4));
-          const uint32_t mnw = grp == 0 ? (hdr.z & 0x3f3f3f3fu) : (((hdr.w >> 4) & 0x0f0f0f0fu) | (((hdr.z >> 6) & 0x03030303u) << 4));
-          qw[8] = scw;
-          qw[9] = mnw;
+          // sub-blocks 2 * my_stage and 2 * my_stage + 1: 6-bit fields in place for the first four, split across two bytes after
+          const int sh = 16 * (my_stage & 1);
+          const uint32_t sc = my_stage < 2 ? hdr.y >> sh & 0x3f3fu : (hdr.w >> sh & 0x0f0fu) | (hdr.y >> sh >> 2 & 0x3030u);
+          const uint32_t mn = my_stage < 2 ? hdr.z >> sh & 0x3f3fu : (hdr.w >> sh >> 4 & 0x0f0fu) | (hdr.z >> sh >> 2 & 0x3030u);
+          sub_scale[0] = dscale * float(sc & 0xffu);
+          sub_scale[1] = dscale * float(sc >> 8);
+          sub_min[0] = -(dmin * float(mn & 0xffu));
+          sub_min[1] = -(dmin * float(mn >> 8));
 #pragma unroll
-          for (int ls = 0; ls < 2; ++ls) {
-            const uint4 q = *reinterpret_cast<const uint4*>(rowbase + kQsOff + 64 * grp + 32 * ls + 16 * lhalf);
-            qw[4 * ls] = q.x; qw[4 * ls + 1] = q.y; qw[4 * ls + 2] = q.z; qw[4 * ls + 3] = q.w;
+          for (int h = 0; h < 2; ++h) {
+            const uint4 q = *reinterpret_cast<const uint4*>(rowbase + kQsOff + 32 * my_stage + 16 * h);
+            qw[4 * h] = q.x; qw[4 * h + 1] = q.y; qw[4 * h + 2] = q.z; qw[4 * h + 3] = q.w;
           }
-          if constexpr (QT == QTYPE_Q5_K) {     // bit 2*(2*grp+ls) + {0, 1} of qh byte l: fifth bit of weight l in the low / high sub-block
-            const uint4 qh = *reinterpret_cast<const uint4*>(rowbase + 16 + 16 * lhalf);
-            qw[12] = qh.x; qw[13] = qh.y; qw[14] = qh.z; qw[15] = qh.w;
+          if constexpr (QT == QTYPE_Q5_K) {     // bit 2 * my_stage + {0, 1} of qh byte l: fifth bit of weight l in the low / high sub-block
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              const uint4 qh = *reinterpret_cast<const uint4*>(rowbase + 16 + 16 * h);
+              qw[12 + 4 * h] = qh.x; qw[13 + 4 * h] = qh.y; qw[14 + 4 * h] = qh.z; qw[15 + 4 * h] = qh.w;
+            }
           }
-          sub_scale[0] = sub_scale[1] = sub_scale[2] = sub_scale[3] = 0.f;
         } else if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4) {
           constexpr int BB = QT == QTYPE_Q4_0 ? 18 : 17;
           // this thread's four blocks (4*grp ..) start a0 bytes into the row's window; block b feeds half b%2 of stage 2*grp + b/2
@@ -791,20 +798,16 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
               for (int i = 0; i < 4; ++i) q8_to_pairs<T>(qw[8 * ls + 4 * h + i], d256, c, o[2 * i], o[2 * i + 1]);
             }
           } else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) {
-            // stage = 64-weight group: low nibbles -> its first sub-block (k' 0..31), high nibbles -> its second (k' 32..63)
-            const int sh = 16 * ls;
-            const float sc0 = float((qw[8] >> sh) & 0xff), sc1 = float((qw[8] >> (sh + 8)) & 0xff);
-            const float mn0 = float((qw[9] >> sh) & 0xff), mn1 = float((qw[9] >> (sh + 8)) & 0xff);
+            // 16 of the 32 bytes (ls: which): low nibbles -> the stage's first sub-block (o0), high nibbles -> its second (o1)
             const V off = P::splat(P::kMagic);
-            const V s_lo = P::splat(dscale * sc0), a_lo = P::splat(-(dmin * mn0));
-            const V s_hi = P::splat(dscale * sc1), a_hi = P::splat(-(dmin * mn1));
+            const V s_lo = P::splat(sub_scale[0]), a_lo = P::splat(sub_min[0]), s_hi = P::splat(sub_scale[1]), a_hi = P::splat(sub_min[1]);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
               uint32_t lo = qw[4 * ls + i] & 0x0f0f0f0fu, hi = (qw[4 * ls + i] >> 4) & 0x0f0f0f0fu;
               if constexpr (QT == QTYPE_Q5_K) {
-                const int j = 2 * (2 * grp + ls);
-                lo |= ((qw[12 + i] >> j) & 0x01010101u) * 16u;
-                hi |= ((qw[12 + i] >> (j + 1)) & 0x01010101u) * 16u;
+                const int j = 2 * my_stage;
+                lo |= ((qw[12 + 4 * ls + i] >> j) & 0x01010101u) * 16u;
+                hi |= ((qw[12 + 4 * ls + i] >> (j + 1)) & 0x01010101u) * 16u;
               }
               bytes_to_pairs<T>(lo, off, s_lo, a_lo, o0[2 * i], o0[2 * i + 1]);
               bytes_to_pairs<T>(hi, off, s_hi, a_hi, o1[2 * i], o1[2 * i + 1]);
@@ -893,35 +896,50 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             tmem_st8(tile + 16 + 8 * lhalf, o1);
           }
         };
-        // one lane polls the barrier, the warp follows
-        auto wait_empty = [&](int b, int trip) -> bool {
-          int ok = 1;
-          if (lane == 0) ok = mbar_wait(empty(b), uint32_t(trip - 1) & 1u, abort_flag, p.status, ST_EMPTY_TIMEOUT) ? 1 : 0;
-          ok = __shfl_sync(0xffffffffu, ok, 0);
+        // kWhole: [0 / 1][0 / 1] = first / second 16 weights of the stage's first / second sub-block
+        auto store_whole = [&](uint32_t tile, const uint32_t (&ow)[2][2][8]) {
+          tmem_st8(tile, ow[0][0]);
+          tmem_st8(tile + 8, ow[1][0]);
+          tmem_st8(tile + 16, ow[0][1]);
+          tmem_st8(tile + 24, ow[1][1]);
+        };
+        auto wait_empty = [&](int b, uint32_t parity) -> bool {
+          const bool ok = warp_wait(empty(b), parity, abort_flag, p.status, ST_EMPTY_TIMEOUT);
           if (ok) tcgen05_fence_after();
-          return ok != 0;
+          return ok;
         };
         if constexpr (COARSE) {
           // hand-over per super-block: unpack both stages (no TMEM slot needed yet), then wait for the slot, store, signal once
-          const int ub = it % U, trip = it / U;
           uint32_t ow[2][2][8];
           unpack_stage(0, ow[0][0], ow[0][1]);
           unpack_stage(1, ow[1][0], ow[1][1]);
-          if (trip > 0 && !wait_empty(ub, trip)) { alive = false; break; }
+          if (it >= U && !wait_empty(ub, uphase)) { alive = false; break; }
+          if constexpr (kWhole) {
+            store_whole(tmem_lane + uint32_t((ub * kStagesPerSb + my_stage) * kWSlotCols), ow);
+          } else {
 #pragma unroll
-          for (int ls = 0; ls < 2; ++ls) {
-            const uint32_t tile = tmem_lane + uint32_t((ub * kStagesPerSb + 2 * grp + ls) * kWSlotCols);
-            store_stage(tile, ow[ls][0], ow[ls][1]);
+            for (int ls = 0; ls < 2; ++ls)
+              store_stage(tmem_lane + uint32_t((ub * kStagesPerSb + 2 * grp + ls) * kWSlotCols), ow[ls][0], ow[ls][1]);
           }
           tmem_st_wait();
           tcgen05_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(full(ub));
+        } else if constexpr (kWhole) {
+          uint32_t ow[2][2][8];
+          unpack_stage(0, ow[0][0], ow[0][1]);
+          unpack_stage(1, ow[1][0], ow[1][1]);
+          if (it > 0 && !wait_empty(my_stage, uint32_t(it - 1) & 1u)) { alive = false; break; }
+          store_whole(tmem_lane + uint32_t(my_stage * kWSlotCols), ow);
+          tmem_st_wait();
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(full(my_stage));
         } else {
 #pragma unroll
           for (int ls = 0; ls < 2; ++ls) {
             const int slot = 2 * grp + ls;       // stage ring slot = K stage inside the super-block
-            if (it > 0 && !wait_empty(slot, it)) { alive = false; break; }
+            if (it > 0 && !wait_empty(slot, uint32_t(it - 1) & 1u)) { alive = false; break; }
             const uint32_t tile = tmem_lane + uint32_t(slot * kWSlotCols);   // column k'/2 of this slot
             uint32_t o0[8], o1[8];
             unpack_stage(ls, o0, o1);
@@ -933,6 +951,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
           }
         }
         if (!alive) break;
+        if (++rslot == NSR) { rslot = 0; rphase ^= 1u; }
+        if (++ub == U) { ub = 0; uphase ^= 1u; }
         // The previous segment's epilogue runs only now, after the first super-block of this segment has been unpacked:
         // the MMA warp finds its next weight tiles ready the moment the accumulator is handed back.
         if (sb == sb_b && pend_t >= 0) {
