@@ -17,8 +17,8 @@
 //     higher-numbered one computes (it adds the partial, empties the words and stores) - no waiting in practice, the
 //     dependency points to a lower-numbered CTA, which is dispatched first, and the summation order is fixed.  One
 //     prologue (activation sums) per CTA instead of one per tile;
-//   * one producer warp issues, per (tile, K chunk of 8 super-blocks), sixteen 1-D bulk copies (cp.async.bulk, one per
-//     weight row, 1152 B each) into a ring of D shared-memory stages; a stage is "full" when its bytes have landed
+//   * one producer warp issues, per (tile, K chunk of 8 super-blocks), one 2-D box of 16 weight rows (cp.async.bulk.tensor; ragged
+//     rows, Q8_0 and the first lap of the ring: a 1-D bulk copy per row) into a ring of D shared-memory stages; a stage is "full" when its bytes have landed
 //     (mbarrier transaction count) and "empty" when its 8 consumer warps have arrived.  The ring runs across tile
 //     boundaries.  No thread spends issue slots on per-16-byte copies and no CTA barrier sits in the loop;
 //   * NG groups of 8 consumer warps take the stages round-robin (warp w of a group unpacks super-block w of the chunk
@@ -41,6 +41,7 @@
 #include "gemv_int_planes.cuh"
 #include "gemv_q6k_common.cuh"
 #include "gemv_stream_common.cuh"
+#include "tensor_map.cuh"
 
 namespace b200gguf {
 
@@ -59,9 +60,9 @@ template <> struct Geom<QTYPE_Q6_K> { static constexpr int kSbBytes = 210, kPitc
 // Q5_K = the Q4_K block with 32 more bytes (one high bit per weight) between the scales and the nibbles: same 8-byte reads,
 // 8 x 176 + 32 = 1440 B is 32 (mod 128) like the Q4_K pitch.
 template <> struct Geom<QTYPE_Q5_K> { static constexpr int kSbBytes = 176, kPitch = kKC * 176 + 32; };
-// The further types: packed bytes per 256 weights of a row; the pitch is the stage piece rounded up to 128 B, plus 16 (4 words:
-// the 4-byte reads of 8 rows x 4 lanes hit 32 distinct banks) and every row starts 16-byte aligned (bulk-copy destination).
-template <int BYTES> struct PaddedGeom { static constexpr int kSbBytes = BYTES, kPitch = (kKC * BYTES + 127) / 128 * 128 + 16; };
+// The further types: packed bytes per 256 weights of a row; the pitch is the stage piece made an odd multiple of 16 B (the
+// 4-byte reads of 8 rows x 4 lanes then hit 32 distinct banks).
+template <int BYTES> struct PaddedGeom { static constexpr int kSbBytes = BYTES, kPitch = kKC * BYTES + ((kKC * BYTES) % 32 == 16 ? 0 : 16); };
 template <> struct Geom<QTYPE_Q4_0> : PaddedGeom<8 * 18> {};
 template <> struct Geom<QTYPE_Q2_K> : PaddedGeom<84> {};
 template <> struct Geom<QTYPE_Q3_K> : PaddedGeom<110> {};
@@ -71,6 +72,11 @@ template <> struct Geom<QTYPE_Q8_0> : PaddedGeom<8 * 34> {};
 // RAG: weight rows that are not multiples of 16 bytes.  A row's piece then starts up to 15 bytes into the 16-byte aligned window
 // that is copied, at a phase of its own.
 template <int QT, bool RAG> constexpr int stage_pitch() { return RAG ? (kKC * Geom<QT>::kSbBytes + 30 + 15) / 16 * 16 : Geom<QT>::kPitch; }
+// Whether a stage is fetched as one 2-D box over the weight (8-byte elements, at most 256 of them per row): a bulk copy per row takes 30 ns
+// on an SM's copy unit whatever its length, which capped the stream at 5.7 TB/s.  The first lap of the ring still goes row by row: the
+// rows land sooner and the map's own fetch is hidden (Q4_K, M = 1: [11008 x 4096] 8.7 us with boxes alone, 7.9 row by row; 2 x
+// [28672 x 8192] 47.2 against 55.1).
+template <int QT, bool RAG> constexpr bool tiled_copy() { return !RAG && stage_pitch<QT, RAG>() <= 256 * 8; }
 // The integer arithmetic of gemv_int_planes.cuh serves the types that have it for one and two activation rows.
 template <int QT, int MXC> constexpr bool int_path() { return MXC <= 2 && planes::has<QT>(); }
 // Q4_0 and MXFP4 (32-weight blocks: a scale and 16 bytes of nibbles), NVFP4, Q2_K and Q3_K run on tensor cores like Q4_K.
@@ -179,7 +185,8 @@ struct Place {                       // one unit of the line: (slice, tile, chun
 template <int QT, typename T, int MXC, int NG, int D, bool PROBE, bool RAG>
 __global__ void __launch_bounds__((NG * kGroupWarps + 2) * 32, NG == 1 ? 2 : 1)
 gemv_stream_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const T* __restrict__ bias, T* __restrict__ y,
-                       int m, int n, int k, int* status, uint64_t* partial, uint64_t* slice_words, const Line line, const PeerOut peers) {
+                       int m, int n, int k, int* status, uint64_t* partial, uint64_t* slice_words, const Line line, const PeerOut peers,
+                       const __grid_constant__ CUtensorMap w_map) {
   using MT = MmaType<T>;
   constexpr int NCW = NG * kGroupWarps;
   constexpr int MC = MXC == 1 ? 1 : 2;             // accumulator columns a lane keeps
@@ -259,6 +266,7 @@ gemv_stream_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const
     bool ok = true;
     int issued = 0;
     Place at = first;
+    if (tiled_copy<QT, RAG>() && lane == 0) asm volatile("prefetch.tensormap [%0];\n" ::"l"(&w_map) : "memory");
     const uint32_t sW_u32 = smem_u32(sW);
     for (int u = 0; u < nunits; ++u) {
       const int slot = u % D, it = u / D;
@@ -281,12 +289,21 @@ gemv_stream_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const
         __syncwarp();
         if (lane < rows_valid) bulk_load(sW_u32 + uint32_t(slot) * kStageBytes + uint32_t(lane) * kPitch, src - phase, bytes, full(slot));
       } else {
+       if (tiled_copy<QT, RAG>() && u >= D) {
+        // one box of 16 rows x kPitch bytes (the next chunk's first bytes pad the row; past the weight's end: zeros)
+        if (lane == 0) {
+          mbar_arrive_expect_tx(full(slot), uint32_t(kStageBytes));
+          tma_load_2d(sW_u32 + uint32_t(slot) * kStageBytes, &w_map, full(slot), chunk * (kKC * kSbBytes / 8), tile * kRows);
+        }
+        __syncwarp();
+       } else {
         const uint32_t bytes_row = uint32_t(sbs) * kSbBytes;
         if (lane == 0) mbar_arrive_expect_tx(full(slot), uint32_t(rows_valid) * bytes_row);
         __syncwarp();
         if (lane < rows_valid)
           bulk_load(sW_u32 + uint32_t(slot) * kStageBytes + uint32_t(lane) * kPitch,
                     w + int64_t(tile * kRows + lane) * row_bytes + int64_t(chunk) * (kKC * kSbBytes), bytes_row, full(slot));
+       }
       }
       issued = u + 1;
       at.back(line);
@@ -940,9 +957,20 @@ static int launch_cfg(const void* a, const void* b, const void* bias, void* c, i
   const int ctas = min(min(line.units() / line.len, sm_count() * (ctas_per_sm < 1 ? 1 : ctas_per_sm)), kMaxCtas);
   Scratch sc;
   if (int rc = stream_scratch(s, line.slices > 1, &sc)) return rc;
+  CUtensorMap w_map = {};
+  if constexpr (tiled_copy<QT, RAG>()) {
+    EncodeTiledFn enc = encode_tiled();
+    if (enc == nullptr) return RC_LAUNCH;
+    const cuuint64_t row_bytes = cuuint64_t(k / 256) * Geom<QT>::kSbBytes;
+    const cuuint64_t dims[2] = {row_bytes / 8, cuuint64_t(n)}, strides[1] = {row_bytes};
+    const cuuint32_t box[2] = {cuuint32_t(stage_pitch<QT, RAG>() / 8), cuuint32_t(kRows)}, estr[2] = {1, 1};
+    if (enc(&w_map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 2, const_cast<void*>(b), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return RC_LAUNCH;
+  }
   const cudaError_t err = gemv_launch(kern, ctas, 1, (NG * kGroupWarps + 2) * 32, smem, s, static_cast<const T*>(a),
                                       static_cast<const uint8_t*>(b), static_cast<const T*>(bias), static_cast<T*>(c), m, n, k, status,
-                                      sc.partial, sc.slice_words, line, peers);
+                                      sc.partial, sc.slice_words, line, peers, w_map);
   return err == cudaSuccess ? RC_OK : RC_LAUNCH;
 }
 
