@@ -67,6 +67,22 @@ def _tensor_struct(ptr: int, shape, dtype: str, keep: list) -> _DinoTensor:
     return _DinoTensor(ptr, arr, len(shape), DTYPE_ENUM[dtype], None, 0, numel * DTYPE_NBYTES[dtype], DEVICE_CUDA, FLAG_CONTIGUOUS, 0)
 
 
+_SMALL_RESULT_BYTES = 65536      # run_numpy: up to here a result is copied out of the plan's own arena (a copy costs less than a loan)
+_LOAN_BYTES = 64 << 20           # host memory that the loans of one set of input shapes may hold
+
+
+class _Loan:
+    """Host memory that the arrays of one result are views of.  When the last of them is dropped it goes back to its plan."""
+    __slots__ = ("arena", "pool", "__array_interface__")
+
+    def __init__(self, arena: dict[str, Any], pool: list):
+        self.arena, self.pool = arena, pool
+        self.__array_interface__ = arena["interface"]
+
+    def __del__(self):
+        self.pool.append(self.arena)
+
+
 def load(path: str | Path, *, load_constants: bool | None = None) -> "RuntimeModule":
     return RuntimeModule(Path(path), load_constants=load_constants)
 
@@ -208,7 +224,7 @@ class Session:
         self._user_stream = 0
         self._graph_replay = False
         self.numpy_graph_replay = True        # run_numpy keeps its arenas, so its launch sequences are replayed as CUDA graphs
-        self.numpy_zero_copy_bytes = 65536    # run_numpy: results up to this size are stored by the kernels into pinned host memory
+        self.numpy_zero_copy_bytes = 4 << 20  # run_numpy: results up to this size are stored by the kernels into pinned host memory
 
     def close(self) -> None:
         self._runner = None
@@ -310,6 +326,9 @@ class Session:
         """Host arrays in, host arrays out.  All inputs of a call are packed into ONE pinned arena and go to the device
         in one copy, the module runs on the same stream, all outputs come back in one copy from one device arena, and
         the host waits once.  Arenas, tensor descriptors and the stream are cached per set of input shapes.
+        Results above 64 KB are views of host memory that the plan lends (`_Loan`) and gets back once the caller has dropped
+        them: fresh arrays of that size are pages the kernel has to map and clear first, then a second pass over the data.  A
+        caller that keeps more than four results, or 64 MB of them, gets copies from there on.
         bfloat16 travels as uint16 bit patterns or as float32 arrays (rounded to nearest even), and comes back as
         float32; float16 / float32 keep their numpy dtypes."""
         meta = self.module.metadata
@@ -331,27 +350,49 @@ class Session:
         # one native call: H2D of the input arena, the launches (a replayed graph in steady state), D2H of the output arena
         # (none when the outputs are small: the kernels then store straight into the pinned arena), one wait - all on the
         # plan's stream, with graph replay on for this call unless the user switched it on for the session anyway
+        loan = self._borrow(plan) if plan["loans"] else None
+        arena = plan["arena"] if loan is None or plan["all_bf16_out"] else loan.arena
         self.module._check(lib.dino_session_run_staged_on(
             self._handle, plan["stream_ptr"], int(self.numpy_graph_replay or self._graph_replay), plan["pin_in_ptr"], plan["dev_in_ptr"],
-            plan["in_bytes"], plan["ins"], len(plan["ins"]), plan["outs"], len(plan["outs"]), plan["dev_out_ptr"], plan["pin_out_ptr"],
+            plan["in_bytes"], plan["ins"], len(plan["ins"]), arena["outs"], len(arena["outs"]), plan["dev_out_ptr"], arena["ptr"],
             plan["copy_out_bytes"]))
         out = {}
         if plan["all_bf16_out"]:
             # the whole pinned arena widens in ONE native call into one float32 buffer; the results are views of it
-            wide = np.empty(plan["out_bytes"] // 2, dtype=np.float32)
-            lib.dino_convert_bf16_to_f32(plan["pin_out_ptr"], wide.ctypes.data, wide.size)
+            wide = np.empty(plan["out_bytes"] // 2, dtype=np.float32) if loan is None else np.asarray(loan)
+            lib.dino_convert_bf16_to_f32(arena["ptr"], wide.ctypes.data if loan is None else loan.arena["ptr"], wide.size)
             for name, (first, count, shape) in plan["out_slices"].items():
                 out[name] = wide[first:first + count].reshape(shape)
             return out
-        for o in meta["outputs"]:
-            view = plan["out_views"][o["name"]]
-            if o["dtype"] == "bfloat16":
-                res = np.empty(view.shape, dtype=np.float32)      # the 16 bits become the high half of each float
-                lib.dino_convert_bf16_to_f32(plan["out_ptrs"][o["name"]], res.ctypes.data, res.size)
-                out[o["name"]] = res
+        if loan is not None:
+            lent = np.asarray(loan)
+            for name, shape, np_dtype, offset in plan["out_views"]:
+                out[name] = np.ndarray(shape, np_dtype, lent, offset)
+            return out
+        host = arena["host"]
+        for name, shape, np_dtype, offset in plan["out_views"]:
+            view = np.ndarray(shape, np_dtype, host, offset)
+            if np_dtype is np.uint16:                             # bfloat16: the 16 bits become the high half of each float
+                res = np.empty(shape, dtype=np.float32)
+                lib.dino_convert_bf16_to_f32(arena["ptr"] + offset, res.ctypes.data, res.size)
+                out[name] = res
             else:
-                out[o["name"]] = view.copy()
+                out[name] = view.copy()
         return out
+
+    def _borrow(self, plan: dict[str, Any]) -> "_Loan | None":
+        """Memory for one result: a loan that came back, or a new one while the plan may make more; else none.  The first run of a
+        plan borrows nothing (shapes that come once pay for no second arena)."""
+        pool = plan["pool"]
+        if pool:
+            try:
+                return _Loan(pool.pop(), pool)
+            except IndexError:                                    # another thread took it
+                pass
+        if plan["loans_made"] > plan["loans"]:
+            return None
+        plan["loans_made"] += 1
+        return _Loan(plan["make_arena"](), pool) if plan["loans_made"] > 1 else None
 
     def _make_numpy_plan(self, arrays: Mapping[str, np.ndarray]) -> dict[str, Any]:
         import torch
@@ -373,30 +414,40 @@ class Session:
         out_off, out_bytes = layout(out_entries)
         dev = torch.device("cuda", torch.cuda.current_device())
         plan = {"pin_in": torch.empty(in_bytes, dtype=torch.uint8).pin_memory(), "dev_in": torch.empty(in_bytes, dtype=torch.uint8, device=dev),
-                "pin_out": torch.empty(out_bytes, dtype=torch.uint8).pin_memory(), "dev_out": torch.empty(out_bytes, dtype=torch.uint8, device=dev),
-                "stream": torch.cuda.Stream(device=dev), "keep": []}
-        host_in, host_out = plan["pin_in"].numpy(), plan["pin_out"].numpy()
-
-        def views(entries, offs, host):
-            return {name: host[offs[name]:offs[name] + int(np.prod(shape)) * esize[dtype]].view(np_dt[dtype]).reshape(shape)
-                    for name, shape, dtype in entries}
-
-        plan["in_views"], plan["out_views"] = views(in_entries, in_off, host_in), views(out_entries, out_off, host_out)
-        plan.update(in_bytes=in_bytes, out_bytes=out_bytes, out_off=out_off, pin_in_ptr=plan["pin_in"].data_ptr(),
-                    dev_in_ptr=plan["dev_in"].data_ptr(), pin_out_ptr=plan["pin_out"].data_ptr(), dev_out_ptr=plan["dev_out"].data_ptr(),
-                    any_bf16=any(o["dtype"] == "bfloat16" for o in meta["outputs"]))
+                "dev_out": torch.empty(out_bytes, dtype=torch.uint8, device=dev), "stream": torch.cuda.Stream(device=dev), "keep": []}
+        host_in = plan["pin_in"].numpy()
+        plan["in_views"] = {name: host_in[in_off[name]:in_off[name] + int(np.prod(shape)) * esize[dtype]].view(np_dt[dtype]).reshape(shape)
+                            for name, shape, dtype in in_entries}
+        plan["out_views"] = [(name, shape, np_dt[dtype], out_off[name]) for name, shape, dtype in out_entries]
         plan["ins"] = (_DinoTensor * len(in_entries))(*[_tensor_struct(plan["dev_in"].data_ptr() + in_off[n], s, d, plan["keep"])
                                                         for n, s, d in in_entries])
-        # Decode-sized results (up to 64 KB in all) are written by the kernels straight into the pinned host arena (mapped into
-        # the device's address space at the same address): no device-to-host copy node, one hop less before the host may read.
-        zero_copy = out_bytes <= self.numpy_zero_copy_bytes
-        out_base = plan["pin_out"].data_ptr() if zero_copy else plan["dev_out"].data_ptr()
-        plan["outs"] = (_DinoTensor * len(out_entries))(*[_tensor_struct(out_base + out_off[n], s, d, plan["keep"]) for n, s, d in out_entries])
-        plan.update(copy_out_bytes=0 if zero_copy else out_bytes, stream_ptr=plan["stream"].cuda_stream,
-                    in_ptrs={n: plan["pin_in"].data_ptr() + in_off[n] for n, _, _ in in_entries},
-                    out_ptrs={n: plan["pin_out"].data_ptr() + out_off[n] for n, _, _ in out_entries})
-        plan["all_bf16_out"] = bool(out_entries) and all(d == "bfloat16" for _, _, d in out_entries)
-        plan["out_slices"] = {n: (out_off[n] // 2, int(np.prod(sh)), tuple(sh)) for n, sh, _ in out_entries}
+        # Results up to 4 MB are written by the kernels straight into the pinned host arena (mapped into the device's address
+        # space at the same address): no device-to-host copy node, one hop less before the host may read (seven linears, float16
+        # results: M = 4 120 -> 109 us, M = 64 453 -> 426 us).  Above 64 KB only if no node reads a result back across the bus.
+        read_back = {i for node in self._graph["nodes"] for i in node["inputs"]} & {o["name"] for o in meta["outputs"]}
+        zero_copy = out_bytes <= self.numpy_zero_copy_bytes and (out_bytes <= _SMALL_RESULT_BYTES or not read_back)
+        all_bf16 = bool(out_entries) and all(d == "bfloat16" for _, _, d in out_entries)
+        dev_out_ptr = plan["dev_out"].data_ptr()
+
+        def make_arena(pinned: bool = True) -> dict[str, Any]:
+            """Host memory for one result (pinned: the kernels or the copy engine write it; else 16-bit results are widened into it)."""
+            if not pinned:
+                host = np.empty(out_bytes // 2, dtype=np.float32)
+                return {"host": host, "ptr": host.ctypes.data, "interface": host.__array_interface__}
+            tensor = torch.empty(out_bytes, dtype=torch.uint8).pin_memory()
+            host, ptr, keep = tensor.numpy(), tensor.data_ptr(), []
+            base = ptr if zero_copy else dev_out_ptr
+            outs = (_DinoTensor * len(out_entries))(*[_tensor_struct(base + out_off[n], s, d, keep) for n, s, d in out_entries])
+            return {"host": host, "tensor": tensor, "ptr": ptr, "interface": host.__array_interface__, "outs": outs, "keep": keep}
+
+        plan.update(in_bytes=in_bytes, out_bytes=out_bytes, pin_in_ptr=plan["pin_in"].data_ptr(), dev_in_ptr=plan["dev_in"].data_ptr(),
+                    dev_out_ptr=dev_out_ptr, copy_out_bytes=0 if zero_copy else out_bytes, stream_ptr=plan["stream"].cuda_stream,
+                    in_ptrs={n: plan["pin_in"].data_ptr() + in_off[n] for n, _, _ in in_entries}, all_bf16_out=all_bf16,
+                    out_slices={n: (out_off[n] // 2, int(np.prod(sh)), tuple(sh)) for n, sh, _ in out_entries}, arena=make_arena())
+        lent_bytes = out_bytes * 2 if all_bf16 else out_bytes
+        mixed = not all_bf16 and any(d == "bfloat16" for _, _, d in out_entries)
+        plan.update(pool=[], loans_made=0, loans=0 if lent_bytes <= _SMALL_RESULT_BYTES or mixed else min(4, _LOAN_BYTES // lent_bytes),
+                    make_arena=lambda: make_arena(not all_bf16))
         return plan
 
     # -- benchmark
@@ -440,7 +491,7 @@ class Session:
         import torch
         torch.cuda.synchronize()
         ms = (ctypes.c_double * iterations)()
-        self.module._check(self._lib.dino_session_benchmark(self._handle, plan["ins"], len(plan["ins"]), plan["outs"], len(plan["outs"]),
+        self.module._check(self._lib.dino_session_benchmark(self._handle, plan["ins"], len(plan["ins"]), plan["arena"]["outs"], len(plan["arena"]["outs"]),
                                                             warmup, iterations, ms, iterations))
         return summarize_ms(list(ms), native_entrypoint="dino_session_benchmark", timing_source="cuda_events", graph_replay=True, warmup=warmup)
 
