@@ -27,7 +27,7 @@
 // (shapes, pointers) combination the second time it sees it and replay the graph from then on.
 // DINOML_PROFILE_RUN[_VERBOSE|_SECTIONS] time every launch with events, as src/dinoml/templates/gpu_module.cu.j2:785-983.
 #if defined(__SSE2__)
-#include <emmintrin.h>
+#include <immintrin.h>
 #endif
 #include <cstdio>
 #include <cstdlib>
@@ -1027,11 +1027,44 @@ int dino_session_run_staged_on(DinoSession* session, void* stream, int graph_rep
 // a NaN; widening is the 16 bits followed by 16 zeros.
 // Written on 32-bit integer views with no call in the loop body so that the host compiler vectorizes them (an 11008-element
 // result widens in 0.4 us instead of 3 us).
+// Where the processor has AVX2, whole vectors of 16: a run of M = 16 converts 0.6 M values, on the caller's thread, before and after
+// the kernels.
 typedef uint32_t __attribute__((may_alias)) aliased_u32;
+#if defined(__SSE2__)
+__attribute__((target("avx2"))) static size_t f32_to_bf16_avx2(const float* src, uint16_t* dst, size_t count) {
+  const __m256i one = _mm256_set1_epi32(1), half = _mm256_set1_epi32(0x7FFF);
+  size_t i = 0;
+  for (; i + 16 <= count; i += 16) {
+    __m256i v[2];
+    for (int h = 0; h < 2; ++h) {
+      const __m256i bits = _mm256_loadu_si256(reinterpret_cast<const __m256i*>(src + i + 8 * h));
+      const __m256i odd = _mm256_and_si256(_mm256_srli_epi32(bits, 16), one);
+      v[h] = _mm256_srli_epi32(_mm256_add_epi32(_mm256_add_epi32(bits, half), odd), 16);
+    }
+    // packs within 128-bit lanes: the middle two quarters change places
+    _mm256_storeu_si256(reinterpret_cast<__m256i*>(dst + i), _mm256_permute4x64_epi64(_mm256_packus_epi32(v[0], v[1]), 0xD8));
+  }
+  return i;
+}
+__attribute__((target("avx2"))) static size_t bf16_to_f32_avx2(const uint16_t* src, float* dst, size_t count) {
+  size_t i = 0;
+  for (; i + 16 <= count; i += 16)
+    for (int h = 0; h < 2; ++h) {
+      const __m256i v = _mm256_cvtepu16_epi32(_mm_loadu_si128(reinterpret_cast<const __m128i*>(src + i + 8 * h)));
+      _mm256_storeu_si256(reinterpret_cast<__m256i*>(dst + i + 8 * h), _mm256_slli_epi32(v, 16));
+    }
+  return i;
+}
+static const bool kHaveAvx2 = __builtin_cpu_supports("avx2");
+#endif
 void dino_convert_f32_to_bf16(const float* src, uint16_t* dst, size_t count) {
   const aliased_u32* __restrict__ in = reinterpret_cast<const aliased_u32*>(src);
   uint16_t* __restrict__ out = dst;
-  for (size_t i = 0; i < count; ++i) {
+  size_t i = 0;
+#if defined(__SSE2__)
+  if (kHaveAvx2) i = f32_to_bf16_avx2(src, dst, count);
+#endif
+  for (; i < count; ++i) {
     const uint32_t bits = in[i];
     out[i] = uint16_t((bits + 0x7FFFu + ((bits >> 16) & 1u)) >> 16);
   }
@@ -1039,6 +1072,7 @@ void dino_convert_f32_to_bf16(const float* src, uint16_t* dst, size_t count) {
 void dino_convert_bf16_to_f32(const uint16_t* src, float* dst, size_t count) {
   size_t i = 0;
 #if defined(__SSE2__)
+  if (kHaveAvx2) i = bf16_to_f32_avx2(src, dst, count);
   // 8 values per step: interleaving with zeros puts each 16-bit pattern into the high half of a 32-bit lane
   const __m128i zero = _mm_setzero_si128();
   for (; i + 8 <= count; i += 8) {
