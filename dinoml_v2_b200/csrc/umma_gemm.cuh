@@ -357,6 +357,11 @@ template <int BM> constexpr bool coarse_handover() { return BM < 256; }
 // two stages: two scales and mins to decode instead of four, one hand-over instead of two (350 -> 263 instructions per 64 weights;
 // [8192 x 28672] Q4_K, M = 2048: 825 -> 772 us).
 template <int QT> constexpr bool whole_stage() { return QT == QTYPE_Q4_K || QT == QTYPE_Q5_K; }
+// A producer warp signals a stored slot only after it has fetched the next super-block's words, so that the tcgen05.st and the fetch
+// overlap (M = 16, ncu: 21 % of the warps' time went on such waits; [8192 x 28672] Q4_K 46.3 -> 42.3 us, gated 2 x [28672 x 8192] 88.0
+// -> 82.5, Q6_K [8192 x 28672] 54.4 -> 53.3).  On the two-deep ring of BM = 128 the later signal costs more than it hides (38.0 ->
+// 39.3 us at M = 100), and so it does for the types with a longer unpack (1-3 %).
+template <int QT, int BM> constexpr bool late_signal() { return BM <= 64 && (QT == QTYPE_Q4_K || QT == QTYPE_Q6_K); }
 template <int BM> constexpr int stage_units() { return BM >= 256 ? 1 : BM >= 128 ? 2 : 3; }
 template <int BM> constexpr int x_tile_bytes() { return BM * kBK * 2; }
 template <int QT> constexpr int raw_box_bytes() { return kRowsW * RawGeom<QT>::kPitch; }
@@ -631,6 +636,17 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     // packed ring and stage ring positions, counted along (a division per super-block showed in the instruction count)
     int rslot = 0, ub = 0;
     uint32_t rphase = 0, uphase = 1;                            // uphase: of the `empty` barrier to wait for, from the second lap on
+    constexpr bool kLate = late_signal<QT, BM>();               // owed: the slot stored last, not signalled yet
+    int owed = -1;
+    auto signal_owed = [&]() {
+      if (kLate && owed >= 0) {
+        tmem_st_wait();
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(full(owed));
+        owed = -1;
+      }
+    };
     for (int t = tile_hi; t >= tile_lo && alive; --t, ++segi) {
       int sb_b, sb_e;
       walk.segment(t, sb_b, sb_e);
@@ -776,8 +792,15 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             sub_scale[i] = float(int(int8_t(wsel >> (8 * (2 * (i & 1) + lhalf)))));
           }
         }
+        if (kLate && owed >= 0) {
+          tmem_st_wait();
+          tcgen05_fence_before();
+        }
         __syncwarp();                          // every lane holds its words: the ring slot may be refilled
-        if (lane == 0) mbar_arrive(rawfree(rslot));
+        if (lane == 0) {
+          mbar_arrive(rawfree(rslot));
+          if (kLate && owed >= 0) mbar_arrive(full(owed));
+        }
         // K stage ls (0 / 1) of this thread's half of the super-block -> two groups of 8 words: 16 values each for
         // k' = 16*lhalf .. +15 and k' = 32 + 16*lhalf .. +15 of the 64-wide stage.
         auto unpack_stage = [&](int ls, uint32_t (&o0)[8], uint32_t (&o1)[8]) {
@@ -914,10 +937,14 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
             for (int ls = 0; ls < 2; ++ls)
               store_stage(tmem_lane + uint32_t((ub * kStagesPerSb + 2 * grp + ls) * kWSlotCols), ow[ls][0], ow[ls][1]);
           }
-          tmem_st_wait();
-          tcgen05_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(full(ub));
+          if constexpr (kLate) {
+            owed = ub;
+          } else {
+            tmem_st_wait();
+            tcgen05_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full(ub));
+          }
         } else if constexpr (kWhole) {
           uint32_t ow[2][2][8];
           unpack_stage(0, ow[0][0], ow[0][1]);
@@ -949,6 +976,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         // The previous segment's epilogue runs only now, after the first super-block of this segment has been unpacked:
         // the MMA warp finds its next weight tiles ready the moment the accumulator is handed back.
         if (sb == sb_b && pend_t >= 0) {
+          signal_owed();
           if (!epilogue(pend_t, pend_b, pend_e, segi - 1)) { alive = false; break; }
           pend_t = -1;
         }
@@ -956,6 +984,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
       if (!alive) break;
       pend_t = t; pend_b = sb_b; pend_e = sb_e;
     }
+    if (alive) signal_owed();
     if (alive && pend_t >= 0) epilogue(pend_t, pend_b, pend_e, segi - 1);
   } else if (warp == 16) {
     // ------------------------------------------------------------------ activation TMA
