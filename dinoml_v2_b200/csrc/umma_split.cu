@@ -9,7 +9,7 @@ int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc);
 
 template <int QT, typename T>
 static int run(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
-  const Plan pl = split_plan(m, n, k, split_bm<T>());
+  const Plan pl = split_plan(m, n, k, split_bm<QT, T>());
   Scratch sc;
   if (int rc = split_state(pl.workspace_bytes, s, &sc)) return rc;
   return launch_split<QT, T>(a, b, bias, c, m, n, k, pl, sc, s);

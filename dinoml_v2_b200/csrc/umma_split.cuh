@@ -4,16 +4,16 @@
 //
 // Same frame as umma_gemm.cuh (weights as the UMMA A operand from tensor memory, activations by TMA, stream-K, bounded waits); what differs:
 //   * no weight is cut to 16 bits: a dequantized weight (fp32) is the sum of TERMS 16-bit numbers - three bfloat16 (24 bits), or two
-//     float16 (22 bits, below the rounding of an fp32 sum over K; never finer than float16's own subnormals) - in TERMS operand slots
-//     per stage, one MMA each against the same activation tile.  (Not for float32 activations: the tensor cores' own accumulation leaves
+//     float16 (22 bits, below the rounding of an fp32 sum over K; never finer than float16's own subnormals), fewer where they hold it
+//     exactly - in TERMS operand slots per stage, one MMA each against the same activation tile.  (Not for float32 activations: the tensor cores' own accumulation leaves
 //     6e-6 on a sum, thirty times what mma.sync with fp32 scaling does.)
 //   * R = 16 / gcd(16, row bytes) consecutive rows together are a multiple of 16 bytes: the tensor map's rows are groups of R weight
 //     rows, and R boxes per super-block fetch the rows of one residue each, at that residue's 16-byte aligned window.  (One bulk
 //     copy per row was measured first: 128 copies of 224 bytes take 6.5 us, whatever the arithmetic.)  Only a last tile that is not
 //     full is copied row by row, so that nothing beyond the weight is read;
 //   * K may be any multiple of the block (the tail of the last super-block counts as zero).
-// Tensor memory holds the accumulator and TERMS slots for four stages, so a tile has up to 256 activation rows with two terms and 128
-// with three.
+// Tensor memory holds the accumulator and TERMS slots for four stages, so a tile has up to 256 activation rows with one or two terms and
+// 128 with three.
 #pragma once
 #include "gemm_exact.cuh"
 #include "gemv_stream_common.cuh"
@@ -22,18 +22,37 @@
 namespace b200gguf {
 namespace umma {
 
-template <typename T> constexpr int split_terms() { return std::is_same<T, __half>::value ? 2 : 3; }
-template <typename T> constexpr int split_bm() { return std::is_same<T, __half>::value ? 256 : 128; }
+// Terms that hold a weight exactly, or to 22 bits: an FP4 code times its scale has at most six significant bits, a Q4_0 quant times
+// its scale fifteen.
+template <int QT, typename T> constexpr int split_terms() {
+  return QT == QTYPE_MXFP4 || QT == QTYPE_NVFP4 ? 1 : QT == QTYPE_Q4_0 || std::is_same<T, __half>::value ? 2 : 3;
+}
+template <int QT, typename T> constexpr int split_bm() { return split_terms<QT, T>() < 3 ? 256 : 128; }
 template <int QT> constexpr int split_raw_slots() { return exact::sb_bytes<QT>() > 240 ? 2 : 3; }
 template <int QT, typename T> constexpr size_t split_smem() {
-  return 1024 + size_t(kStagesPerSb) * split_bm<T>() * kBK * 2 + size_t(split_raw_slots<QT>()) * kRowsW * exact::raw_pitch<QT>() + 512;
+  return 1024 + size_t(kStagesPerSb) * split_bm<QT, T>() * kBK * 2 + size_t(split_raw_slots<QT>()) * kRowsW * exact::raw_pitch<QT>() + 512;
 }
 
 // Group i of a unit -> its dequantized weights as TERMS 16-bit numbers each (term[.][q][..]).
 template <int QT, typename O, int TERMS>
 __device__ __forceinline__ void split16(const exact::Unit<QT, 4>& unit, int i, float scale, float mn, uint32_t (&term)[TERMS][2][8], int q) {
   constexpr int kOff = exact::byte_offset<QT>();
-  if constexpr (TERMS == 2 && !exact::has_mins<QT>()) {
+  if constexpr (TERMS == 1) {
+    // FP4: byte - 12 = 2 e2m1, times half the scale; both factors and the product are exact in either 16-bit type (0x43qq is 128 + q as
+    // bfloat16; as float16 0x50qq is 32 + q / 32, which leaves the scale 32 times larger, away from the subnormals)
+    using V = typename Pair<O>::V;
+    constexpr bool kHalf = std::is_same<O, __half>::value;
+    const V s1 = Pair<O>::splat(kHalf ? 32.f * scale : scale), off = Pair<O>::splat(kHalf ? 32.f + float(kOff) / 32.f : 128.f + float(kOff));
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t w = unit.bytes(i, k);
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const uint32_t magic = __byte_perm(w, kHalf ? 0x50505050u : 0x43434343u, e == 0 ? 0x4140 : 0x4342);
+        term[0][q][2 * k + e] = as_u32<V>(__hmul2(__hsub2(as_pair<V>(magic), off), s1));
+      }
+    }
+  } else if constexpr (TERMS == 2 && std::is_same<O, __half>::value && !exact::has_mins<QT>()) {
     // float16, packed: with r = (byte - offset) / 32 (0x50qq is 32 + q / 32) and 32 scale = s1 + s2, hi = fl(r s1), and
     // lo = fl(r s2 + (r s1 - hi)) with the parenthesis exact: three instructions per pair
     const float s32 = 32.f * scale;
@@ -81,7 +100,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const uint8_t* __restrict__ w, int residues,
                   const Params p) {
   using P = Pair<T>;
-  constexpr int BM = split_bm<T>(), TERMS = split_terms<T>(), NSR = split_raw_slots<QT>(), NS = kStagesPerSb;
+  constexpr int BM = split_bm<QT, T>(), TERMS = split_terms<QT, T>(), NSR = split_raw_slots<QT>(), NS = kStagesPerSb;
   constexpr int kXTile = BM * kBK * 2, kPitch = exact::raw_pitch<QT>(), kRawBytes = kRowsW * kPitch, kSbBytes = exact::sb_bytes<QT>();
   constexpr uint32_t kTmemCols = 512;
   static_assert(BM + NS * TERMS * kWSlotCols <= 512, "tensor memory");
