@@ -143,10 +143,12 @@ int gemm_rcr_simt(const void* a, const void* b, const void* bias, void* c, int q
     if (rc != RC_RANGE) return rc;
   }
   // Else the same exact products by mma.sync (one or two rows of the FP4 types stay below: 16 us against 24 us).
-  // 16-bit activations on tcgen05 where the weight has enough super-block tiles for all SMs, or the rows pay for the start of that
-  // kernel (Q8_0 [4096 x 2880] float16, M = 8: 11.9 us against 14.6; MXFP4 [5760 x 2880] bfloat16, M = 24: 19.6 against 18.9, M = 200:
-  // 34.6 against 54.4; Q6_K [1024 x 2816], 88 tiles: M = 64 13.1 against 12.0, M = 200 21.8 against 27.9).
-  if (m >= 7 && (m > 128 || int64_t((n + 127) / 128) * ((k + 255) / 256) >= 256))
+  // 16-bit activations on tcgen05 where the weight has enough super-block tiles for all SMs, or tiles and rows together pay for the
+  // start of that kernel (Q8_0 [4096 x 2880] float16, M = 8: 11.9 us against 14.6; MXFP4 [5760 x 2880] bfloat16, M = 24: 13.2 against
+  // 18.9; [2048 x 2880], 192 tiles: M = 64 MXFP4 11.8 against 14.9, Q8_0 14.5 against 15.9, M = 32 11.0 / 13.4 against 11.3 / 12.0;
+  // Q6_K [1024 x 2816], 88 tiles: M = 100 18.7 against 15.7, M = 200 21.8 against 27.9).
+  const int64_t tiles = int64_t((n + 127) / 128) * ((k + 255) / 256);
+  if (m >= 7 && (m > 128 || tiles >= 256 || tiles * m >= 12288))
     if (int rc = gemm_split(a, b, bias, c, qtype, dtype, m, n, k, s); rc != RC_RANGE) return rc;
   if (m >= 3)
     if (int rc = gemm_exact(a, b, bias, c, qtype, dtype, m, n, k, s); rc != RC_RANGE) return rc;
