@@ -9,8 +9,9 @@
 //     6e-6 on a sum, thirty times what mma.sync with fp32 scaling does.)
 //   * R = 16 / gcd(16, row bytes) consecutive rows together are a multiple of 16 bytes: the tensor map's rows are groups of R weight
 //     rows, and R boxes per super-block fetch the rows of one residue each, at that residue's 16-byte aligned window.  (One bulk
-//     copy per row was measured first: 128 copies of 224 bytes take 6.5 us, whatever the arithmetic.)  Only a last tile that is not
-//     full is copied row by row, so that nothing beyond the weight is read;
+//     copy per row was measured first: 128 copies of 224 bytes take 6.5 us, whatever the arithmetic; used for the last tile alone it
+//     still took NVFP4 [5230 x 2880], M = 24, from 14 to 21 us.)  A last group that is not full has a map of its own, as wide as the
+//     rows it has, so that nothing beyond the weight is read;
 //   * K may be any multiple of the block (the tail of the last super-block counts as zero).
 // Tensor memory holds the accumulator and TERMS slots for four stages, so a tile has up to 256 activation rows with one or two terms and
 // 128 with three.
@@ -97,8 +98,8 @@ __device__ __forceinline__ void split16(const exact::Unit<QT, 4>& unit, int i, f
 
 template <int QT, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
-gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const uint8_t* __restrict__ w, int residues,
-                  const Params p) {
+gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap w_tail_map,
+                  const uint8_t* __restrict__ w, int residues, const Params p) {
   using P = Pair<T>;
   constexpr int BM = split_bm<QT, T>(), TERMS = split_terms<QT, T>(), NSR = split_raw_slots<QT>(), NS = kStagesPerSb;
   constexpr int kXTile = BM * kBK * 2, kPitch = exact::raw_pitch<QT>(), kRawBytes = kRowsW * kPitch, kSbBytes = exact::sb_bytes<QT>();
@@ -321,30 +322,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         const int slot = it % NSR, use = it / NSR;
         if (use > 0 && !warp_wait(rawfree(slot), uint32_t(use - 1) & 1u, abort_flag, p.status, ST_EMPTY_TIMEOUT)) { ok = false; break; }
         const int64_t at = int64_t(sb) * kSbBytes;
-        if (n0 + kRowsW <= p.n) {
-          // lane r < residues: the box of the rows r, r + residues, ... (16-bit elements: Q8_0 windows are wider than 256 bytes)
-          if (lane == 0) mbar_arrive_expect_tx(rawfull(slot), uint32_t(kRawBytes));
-          __syncwarp();
-          if (lane < residues)
-            tma_load_2d(smem_u32(raw + slot * kRawBytes + lane * rows_per_box * kPitch), &w_map, rawfull(slot),
-                        int(((int64_t(lane) * row_bytes + at) & ~int64_t(15)) >> 1), n0 / residues);
-          continue;
-        }
-        const uint32_t piece = uint32_t(min(int64_t(kSbBytes), row_bytes - at));
-        uint32_t bytes[4], total = 0;
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint8_t* src = w + int64_t(min(n0 + lane + 32 * i, p.n - 1)) * row_bytes + at;
-          bytes[i] = ((uint32_t(reinterpret_cast<uintptr_t>(src)) & 15u) + piece + 15u) & ~15u;
-          total += bytes[i];
-        }
-        total = __reduce_add_sync(0xffffffffu, total);
-        if (lane == 0) mbar_arrive_expect_tx(rawfull(slot), total);
+        // lane r < residues: the box of the rows r, r + residues, ... (16-bit elements: Q8_0 windows are wider than 256 bytes).  In a tile
+        // that reaches past the full groups the residues which the last group still has take its map; what a map does not hold is zero.
+        if (lane == 0) mbar_arrive_expect_tx(rawfull(slot), uint32_t(kRawBytes));
         __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint8_t* src = w + int64_t(min(n0 + lane + 32 * i, p.n - 1)) * row_bytes + at;
-          stream::bulk_load(smem_u32(raw + slot * kRawBytes + row_offset(lane + 32 * i)), src - (reinterpret_cast<uintptr_t>(src) & 15), bytes[i], rawfull(slot));
+        if (lane < residues) {
+          const bool tail = n0 + kRowsW > p.n && (lane < p.n % residues || p.n < residues);
+          tma_load_2d(smem_u32(raw + slot * kRawBytes + lane * rows_per_box * kPitch), tail ? &w_tail_map : &w_map, rawfull(slot),
+                      int(((int64_t(lane) * row_bytes + at) & ~int64_t(15)) >> 1), n0 / residues);
         }
       }
     }
@@ -405,7 +390,7 @@ int launch_split(const void* x, const void* w, const void* bias, void* c, int m,
   EncodeTiledFn enc = encode_tiled();
   if (enc == nullptr) return RC_LAUNCH;
   const cuuint32_t estr[2] = {1, 1};
-  CUtensorMap x_map, w_map;
+  CUtensorMap x_map, w_map, w_tail_map;
   {
     const cuuint64_t dims[2] = {cuuint64_t(k), cuuint64_t(m)};
     const cuuint64_t strides[1] = {cuuint64_t(k) * 2};
@@ -414,20 +399,21 @@ int launch_split(const void* x, const void* w, const void* bias, void* c, int m,
             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return RC_LAUNCH;
   }
-  // Groups of `residues` weight rows as the map's rows.  A weight with fewer rows than a group has no full tile and no box: its map
-  // only has to be valid.
+  // Groups of `residues` weight rows as the maps' rows: the full groups, and all groups at the width of the last one (whose odd byte, if
+  // any, is rounded up to an element).  A weight with fewer rows than a group has only the second.
   const int64_t row_bytes = int64_t(k / QTraits<QT>::kBlock) * QTraits<QT>::kBytes;
   int residues = 1;
   while ((row_bytes * residues) & 15) residues *= 2;
-  {
-    const int64_t group = row_bytes * residues;
-    const cuuint64_t dims[2] = {cuuint64_t(group / 2), cuuint64_t(n / residues > 0 ? n / residues : 1)};
+  const int64_t group = row_bytes * residues, rest = n % residues ? (n % residues) * row_bytes : group;
+  auto encode_rows = [&](CUtensorMap* map, int64_t width, int64_t rows) {
+    const cuuint64_t dims[2] = {cuuint64_t((width + 1) / 2), cuuint64_t(rows)};
     const cuuint64_t strides[1] = {cuuint64_t(group)};
     const cuuint32_t box[2] = {cuuint32_t(exact::raw_pitch<QT>() / 2), cuuint32_t(kRowsW / residues)};
-    if (enc(&w_map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-      return RC_LAUNCH;
-  }
+    return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(w), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  const int64_t groups = (int64_t(n) + residues - 1) / residues;
+  if (!encode_rows(&w_tail_map, rest, groups) || !encode_rows(&w_map, n < residues ? rest : group, n < residues ? 1 : n / residues)) return RC_LAUNCH;
   auto kern = gemm_split_kernel<QT, T>;
   constexpr size_t smem = split_smem<QT, T>();
   static_assert(smem <= size_t(kSmemBudget), "shared-memory rings exceed the per-CTA limit");
@@ -444,7 +430,7 @@ int launch_split(const void* x, const void* w, const void* bias, void* c, int m,
   p.bn = pl.bn;
   p.units = pl.units;
   p.peers = no_peers();
-  return gemv_launch(kern, pl.ctas, 1, kThreads, smem, s, x_map, w_map, static_cast<const uint8_t*>(w), residues, p) == cudaSuccess ? RC_OK : RC_LAUNCH;
+  return gemv_launch(kern, pl.ctas, 1, kThreads, smem, s, x_map, w_map, w_tail_map, static_cast<const uint8_t*>(w), residues, p) == cudaSuccess ? RC_OK : RC_LAUNCH;
 }
 
 }  // namespace umma
