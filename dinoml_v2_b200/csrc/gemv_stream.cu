@@ -1,8 +1,5 @@
 // Host side of the persistent decode GEMV (kernel: gemv_stream.cuh): scratch, status word, configurations, the instantiations with
 // 16-byte weight rows and 16-bit activations.
-#include <map>
-#include <vector>
-
 #include "gemv_stream.cuh"
 
 namespace b200gguf {
@@ -24,21 +21,7 @@ int* stream_status_ptr() {
   return ptr[dev];
 }
 
-// Partial sums of cut tiles: one set per (device, stream) - launches on one stream are ordered (a launch writes its partials
-// only after the preceding kernel has completed, see griddepcontrol.wait in the kernel) and may share it, launches on different
-// streams may overlap and must not.  16 x 8 words per CTA, and (for the launches that cut K) the slice words; zeroed once; every word a launch writes is emptied again by the CTA
-// that consumes it.
-constexpr size_t kPartialBytes = size_t(kMaxCtas) * kRows * 8 * sizeof(uint64_t);
-struct ScratchKey {
-  int dev;
-  cudaStream_t stream;
-  bool operator<(const ScratchKey& o) const { return dev != o.dev ? dev < o.dev : stream < o.stream; }
-};
-static std::mutex g_scratch_mutex;
-static std::map<ScratchKey, Scratch> g_scratch;
-// Sets of streams that are gone (see stream_release), for the next new stream of their device.
-constexpr size_t kMaxSpare = 4;
-static std::map<int, std::vector<Scratch>> g_spare;
+static ScratchSets<StreamScratch> g_sets;        // zeroed once; every word a launch writes is emptied again by the CTA that consumes it
 
 int sm_count() {
   static int counts[kGemvMaxDevices] = {};      // written once per device with the same value
@@ -59,37 +42,14 @@ static int zeroed(uint64_t** p, size_t bytes, cudaStream_t stream) {
 int stream_scratch(cudaStream_t stream, bool slices, Scratch* out) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) return RC_LAUNCH;
-  std::lock_guard<std::mutex> lock(g_scratch_mutex);
-  Scratch& sc = g_scratch[ScratchKey{dev, stream}];
-  if (sc.partial == nullptr) {
-    std::vector<Scratch>& spare = g_spare[dev];
-    if (!spare.empty()) {
-      sc = spare.back();                        // empty already: every word written was consumed
-      spare.pop_back();
-    } else if (int rc = zeroed(&sc.partial, kPartialBytes, stream)) {
-      return rc;
-    }
-  }
+  std::lock_guard<std::mutex> lock(g_sets.mutex);
+  Scratch& sc = g_sets.at(dev, stream);
+  if (sc.partial == nullptr)
+    if (int rc = zeroed(&sc.partial, kStreamPartialBytes, stream)) return rc;
   if (slices && sc.slice_words == nullptr)
-    if (int rc = zeroed(&sc.slice_words, kSliceBytes, stream)) return rc;
+    if (int rc = zeroed(&sc.slice_words, kStreamSliceBytes, stream)) return rc;
   *out = sc;
   return RC_OK;
-}
-
-// `stream` is about to be destroyed and has no work left: its set is kept for a later stream (a bounded number) or freed.
-void stream_release(cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_scratch_mutex);
-  for (auto it = g_scratch.begin(); it != g_scratch.end();) {
-    if (it->first.stream != stream) { ++it; continue; }
-    std::vector<Scratch>& spare = g_spare[it->first.dev];
-    if (it->second.partial != nullptr && spare.size() < kMaxSpare) {
-      spare.push_back(it->second);
-    } else {
-      if (it->second.partial != nullptr) cudaFree(it->second.partial);
-      if (it->second.slice_words != nullptr) cudaFree(it->second.slice_words);
-    }
-    it = g_scratch.erase(it);
-  }
 }
 
 // Tuning configurations (the `config` byte of a variant code, see dinoml_b200_gguf.h).  0 = the default for the shape.
@@ -165,7 +125,10 @@ static int launch_q(const void* a, const void* b, const void* bias, void* c, int
 
 }  // namespace stream
 
-void stream_release_scratch(cudaStream_t s) { stream::stream_release(s); }
+void stream_release_scratch(cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(stream::g_sets.mutex);
+  stream::g_sets.release(s);
+}
 
 bool gemv_stream_supports(int qtype, int dtype, int m, int n, int k) {
   (void)n;
@@ -228,12 +191,9 @@ int stream_device_status() {
     cudaMemset(status, 0, sizeof(int));
     int dev = -1;
     cudaGetDevice(&dev);
-    std::lock_guard<std::mutex> lock(stream::g_scratch_mutex);
-    for (auto& entry : stream::g_scratch)
-      if (entry.first.dev == dev) {
-        if (entry.second.partial != nullptr) cudaMemset(entry.second.partial, 0, stream::kPartialBytes);
-        if (entry.second.slice_words != nullptr) cudaMemset(entry.second.slice_words, 0, stream::kSliceBytes);
-      }
+    std::lock_guard<std::mutex> lock(stream::g_sets.mutex);
+    stream::g_sets.for_each(dev, [](StreamScratch& set) { set.empty(nullptr); });
+    cudaStreamSynchronize(nullptr);             // before a launch on any stream
   }
   return value;
 }

@@ -41,6 +41,7 @@
 #include "gemv_int_planes.cuh"
 #include "gemv_q6k_common.cuh"
 #include "gemv_stream_common.cuh"
+#include "scratch_sets.h"
 #include "tensor_map.cuh"
 
 namespace b200gguf {
@@ -130,9 +131,7 @@ __device__ __forceinline__ void fp4x8_operands(uint32_t w, uint32_t& lo01, uint3
 }
 
 constexpr int kGroupWarps = kKC;
-constexpr int kMaxCtas = 320;                   // cut-tile words are laid out by CTA
 constexpr int kMaxSlices = 4;
-constexpr size_t kSliceBytes = size_t(1) << 20; // slice words of a launch: tiles x slices x 16 rows x activation rows x 8 bytes
 constexpr int kBarBytes = 256;                  // mbarrier area in front of the ring (up to 32 barriers)
 
 template <int MXC, int NCW> struct RedBuf {
@@ -923,7 +922,7 @@ gemv_stream_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const
 }
 
 // ---------------------------------------------------------------------------------------- host side
-struct Scratch { uint64_t *partial = nullptr, *slice_words = nullptr; };       // partial sums of cut tiles, of K slices
+using Scratch = StreamScratch;
 int stream_scratch(cudaStream_t stream, bool slices, Scratch* out);             // gemv_stream.cu: one set per (device, stream)
 int sm_count();                                                 // of the current device
 
@@ -954,7 +953,7 @@ static int launch_cfg(const void* a, const void* b, const void* bias, void* c, i
   static SmemOptIn granted;
   if (!smem_opt_in(kern, smem, granted)) return RC_LAUNCH;
   // a CTA owns at least as many units as a tile of the line has, so that a tile is cut between two CTAs at most
-  const int ctas = min(min(line.units() / line.len, sm_count() * (ctas_per_sm < 1 ? 1 : ctas_per_sm)), kMaxCtas);
+  const int ctas = min(min(line.units() / line.len, sm_count() * (ctas_per_sm < 1 ? 1 : ctas_per_sm)), kStreamMaxCtas);
   Scratch sc;
   if (int rc = stream_scratch(s, line.slices > 1, &sc)) return rc;
   CUtensorMap w_map = {};
@@ -991,7 +990,7 @@ static int launch_int(const void* a, const void* b, const void* bias, void* c, i
   if (nchunks >= 4 && (tiles <= sm_count() || !fits<QT, MXC, 1, 2, RAG>(nchunks, 2))) {
     const int slices = min(kMaxSlices, nchunks / 2);
     len = (nchunks + slices - 1) / slices;
-    if (size_t(tiles) * ((nchunks + len - 1) / len) * (kRows * MXC * sizeof(uint64_t)) > kSliceBytes) len = nchunks;
+    if (size_t(tiles) * ((nchunks + len - 1) / len) * (kRows * MXC * sizeof(uint64_t)) > kStreamSliceBytes) len = nchunks;
   }
   if (fits<QT, MXC, 1, D, RAG>(len, 2)) return launch_cfg<QT, T, MXC, 1, D, false, RAG>(a, b, bias, c, MXC, n, k, 2, peers, s, len);
   if constexpr (D > 3)

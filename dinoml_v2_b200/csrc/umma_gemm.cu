@@ -1,8 +1,6 @@
 // Host side of the tcgen05 prefill GEMM: per-(device, stream) scratch, the stream-K plan, the allocation-free scratch and the
 // entry that checks a problem and hands it to the weight type's translation unit.  The kernel is in umma_gemm.cuh.
 #include <mutex>
-#include <unordered_map>
-#include <vector>
 
 #include "umma_gemm.cuh"
 
@@ -10,31 +8,11 @@ namespace b200gguf {
 
 namespace umma {
 
-struct DeviceState {
-  int* status = nullptr;            // [0] = status word, [1 .. kMaxCtas] = partial-tile flags
-  float* workspace = nullptr;
-  size_t workspace_bytes = 0;
-  std::vector<void*> outgrown;      // smaller workspaces that captured graphs may still use; given back with the set
-};
-static std::mutex g_mutex;
-// One workspace + flag set per (device, stream): launches on one stream are ordered and may share them, launches on
-// different streams may overlap on the GPU and must not.
-struct StateKey {
-  int dev;
-  cudaStream_t stream;
-  bool operator==(const StateKey& o) const { return dev == o.dev && stream == o.stream; }
-};
-struct StateKeyHash {
-  size_t operator()(const StateKey& k) const { return std::hash<void*>()(static_cast<void*>(k.stream)) * 31u + size_t(k.dev); }
-};
-static std::unordered_map<StateKey, DeviceState, StateKeyHash> g_state;
-// Sets of streams that are gone (see release), for the next new stream of their device.
-constexpr size_t kMaxSpare = 4;
-static std::unordered_map<int, std::vector<DeviceState>> g_spare;
+static ScratchSets<UmmaScratch> g_sets;
 
 // A larger workspace, outside of stream capture only: callers warm a shape up once before capturing a graph.  At least twice the old
 // size, which stays for graphs captured with it: what a set holds is bounded by twice its largest workspace.
-static bool grow(DeviceState& st, size_t need) {
+static bool grow(UmmaScratch& st, size_t need) {
   const size_t size = need > 2 * st.workspace_bytes ? need : 2 * st.workspace_bytes;
   float* p = nullptr;
   if (cudaMalloc(&p, size) != cudaSuccess) return false;
@@ -44,43 +22,19 @@ static bool grow(DeviceState& st, size_t need) {
   return true;
 }
 
-static DeviceState* device_state(size_t need_workspace, cudaStream_t stream) {
+static UmmaScratch* device_state(size_t need_workspace, cudaStream_t stream) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
-  std::lock_guard<std::mutex> lock(g_mutex);
-  DeviceState& st = g_state[StateKey{dev, stream}];
-  std::vector<DeviceState>& spare = g_spare[dev];
-  if (st.status == nullptr && !spare.empty()) {
-    st = spare.back();                          // flags are down: every flag raised was lowered by its reader
-    spare.pop_back();
-  }
+  std::lock_guard<std::mutex> lock(g_sets.mutex);
+  UmmaScratch& st = g_sets.at(dev, stream);
   if (st.status == nullptr) {
     if (cudaMalloc(&st.status, sizeof(int) * (1 + kMaxCtas)) != cudaSuccess) return nullptr;
-    cudaMemsetAsync(st.status, 0, sizeof(int) * (1 + kMaxCtas), stream);
+    st.empty(stream);
   }
   if (need_workspace > st.workspace_bytes) {
     if (!grow(st, need_workspace)) return nullptr;
   }
   return &st;
-}
-
-// `stream` is about to be destroyed and has no work left: its set is kept for a later stream (a bounded number) or freed.
-static void release(cudaStream_t stream) {
-  std::lock_guard<std::mutex> lock(g_mutex);
-  for (auto it = g_state.begin(); it != g_state.end();) {
-    if (it->first.stream != stream) { ++it; continue; }
-    std::vector<DeviceState>& spare = g_spare[it->first.dev];
-    if (it->second.status != nullptr) {
-      if (spare.size() < kMaxSpare) {
-        spare.push_back(it->second);
-      } else {
-        cudaFree(it->second.status);
-        if (it->second.workspace != nullptr) cudaFree(it->second.workspace);
-        for (void* p : it->second.outgrown) cudaFree(p);
-      }
-    }
-    it = g_state.erase(it);
-  }
 }
 
 static Plan plan_for(int m, int n, int k, int bm) {
@@ -109,7 +63,7 @@ static Plan make_plan(int m, int n, int k) { return plan_for(m, n, k, m <= 64 ? 
 // For the split-operand kernels (umma_split.cu): the same plan at their tile height, the same scratch.
 Plan split_plan(int m, int n, int k, int bm) { return plan_for(m, n, k, bm); }
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc) {
-  DeviceState* st = device_state(workspace_bytes, stream);
+  UmmaScratch* st = device_state(workspace_bytes, stream);
   if (st == nullptr) return RC_LAUNCH;
   sc->workspace = st->workspace;
   sc->status = st->status;
@@ -133,7 +87,7 @@ static StaticScratch g_static[kMaxDevices];
 static int static_scratch(Scratch* out) {
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return RC_LAUNCH;
-  std::lock_guard<std::mutex> lock(g_mutex);
+  std::lock_guard<std::mutex> lock(g_sets.mutex);
   StaticScratch& st = g_static[dev];
   if (!st.ready) {
     void* ws = nullptr;
@@ -158,7 +112,7 @@ static int launch_bm(int qtype, int dtype, const void* a, const void* b, const v
     if (pl.workspace_bytes > kStaticScratchBytes) return RC_RANGE;
     if (int rc = static_scratch(&sc)) return rc;
   } else {
-    DeviceState* st = device_state(pl.workspace_bytes, s);
+    UmmaScratch* st = device_state(pl.workspace_bytes, s);
     if (st == nullptr) return RC_LAUNCH;
     sc.workspace = st->workspace;
     sc.status = st->status;
@@ -180,7 +134,10 @@ static int launch_bm(int qtype, int dtype, const void* a, const void* b, const v
 
 }  // namespace umma
 
-void umma_release_scratch(cudaStream_t s) { umma::release(s); }
+void umma_release_scratch(cudaStream_t s) {
+  std::lock_guard<std::mutex> lock(umma::g_sets.mutex);
+  umma::g_sets.release(s);
+}
 
 // Packed bytes per 256 weights of a row, 0 for a qtype this kernel does not unpack.
 static int super_block_bytes(int qtype) {
@@ -246,16 +203,17 @@ size_t gemm_umma_static_scratch_bytes() { return umma::kStaticScratchBytes; }
 int umma_device_status() {
   int dev = 0, value = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return -1;
-  std::lock_guard<std::mutex> lock(umma::g_mutex);
-  for (auto& entry : umma::g_state) {           // every stream's word on this device; the first non-zero one is reported
-    if (entry.first.dev != dev || entry.second.status == nullptr) continue;
+  std::lock_guard<std::mutex> lock(umma::g_sets.mutex);
+  value = umma::g_sets.take_kept_word(dev);
+  bool read = true;
+  umma::g_sets.for_each(dev, [&](UmmaScratch& set) {           // every stream's word on this device; the first non-zero one is reported
     int word = 0;
-    if (cudaMemcpy(&word, entry.second.status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
-    if (word != 0) {
-      cudaMemset(entry.second.status, 0, sizeof(int) * (1 + umma::kMaxCtas));
-      if (value == 0) value = word;
-    }
-  }
+    if (cudaMemcpy(&word, set.status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) { read = false; return; }
+    if (word == 0) return;
+    set.empty(nullptr);
+    if (value == 0) value = word;
+  });
+  if (!read) return -1;
   if (dev >= 0 && dev < umma::kMaxDevices && umma::g_static[dev].ready) {   // the static-scratch path's word: always read and cleared
     int word = 0;
     if (cudaMemcpy(&word, umma::g_static[dev].status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
@@ -264,6 +222,7 @@ int umma_device_status() {
       if (value == 0) value = word;
     }
   }
+  if (value != 0) cudaStreamSynchronize(nullptr);               // the flags are down before a launch on any stream
   return value;
 }
 

@@ -46,6 +46,7 @@
 #include <type_traits>
 
 #include "gemv_mma_common.cuh"
+#include "scratch_sets.h"
 #include "tensor_map.cuh"
 
 namespace b200gguf {
@@ -1121,7 +1122,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
 }
 
 // ---------------------------------------------------------------------------------------- host side
-constexpr int kMaxCtas = 1024;      // flag words per device; the grid never exceeds the SM count
+constexpr int kMaxCtas = kUmmaMaxCtas;
 
 // Tile shape and stream-K grid of one problem.
 struct Plan {
