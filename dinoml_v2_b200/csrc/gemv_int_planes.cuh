@@ -10,8 +10,9 @@
 // Precision.  A row's activations are fixed-point numbers relative to the largest of their 256-weight super-block: x =
 // xs * (d0 + 256 d1 + 256^2 d2 + 256^3 d3) with |x / xs| < 2^30, rounded once (an absolute error of 2^-31 of the largest; exact for
 // every 16-bit value down to 2^-19 of it).  Products and sums of a sub-block are exact integers; scales, super-blocks and rows
-// are added in fp32.  That is below the rounding of the fp32 accumulation it replaces, so float32 activations run here too.  A
-// super-block with an Inf or NaN gets the scale NaN: the row's results are NaN.
+// are added in fp32.  That is below the rounding of the fp32 accumulation it replaces, so float32 activations run here too.
+// A super-block with an Inf, a NaN or values whose sums or digits leave the range of fp32 has no planes: its scale is zero, and it
+// is multiplied in plain fp32 (plain()), which gives +-Inf or NaN as the products do.
 //
 // Every lane keeps two columns of two weight rows: lane t of a quad has digits 2 (t & 1) and 2 (t & 1) + 1.  One IMAD joins the two
 // digits, one I2F and one FFMA apply the sub-block scale; the factor 256^2 of the odd lanes and xs are applied per super-block.
@@ -75,7 +76,7 @@ __device__ __forceinline__ void transpose4(const uint32_t (&z)[4], uint32_t (&p)
   p[2] = __byte_perm(c, d, 0x5410); p[3] = __byte_perm(c, d, 0x7632);
 }
 
-// xp: the 1024 bytes of this super-block; xs: its scale; X: sums of its activations per sub-block (types with mins), or null.
+// xp: the 1024 bytes of this super-block; xs: its scale (zero: left to plain()); X: sums of its activations per sub-block (types with mins), or null.
 // Where a piece goes follows the order in which the lanes of the MMA take the weights:
 //   Q4_K, Q5_K, Q8_0: MMA j = weights 32j .. +31, lane t has weights 8t .. 8t+7 of it (8 bytes);
 //   Q4_0:             MMA j = block j, lane t has weights 4t .. (low nibbles) and 16 + 4t .. (high nibbles);
@@ -97,13 +98,14 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
     sum += f[i];
   }
   bits = __reduce_max_sync(0xffffffffu, bits);
-  const bool finite = bits < 0x7f800000u;
-  const uint32_t e = max(bits >> 23, 30u);                       // below 2^-97 the fixed point stays at 2^-126
+  // largest value from 2^-97 (its last digit is 2^-126, the smallest normal number) to 2^100 (sums over a super-block stay finite), or zero
+  const bool fits = bits - 0x0f000000u < 0x71800000u - 0x0f000000u || bits == 0u;
+  const uint32_t e = fits ? max(bits >> 23, 30u) : 30u;
   const float scale = __uint_as_float((283u - e) << 23);         // 2^(29 - (e - 127)): |x| * scale < 2^30
   uint32_t z[2][4], p[2][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int v = finite ? __float2int_rn(f[i] * scale) : 0;
+    const int v = fits ? __float2int_rn(f[i] * scale) : 0;
     z[i >> 2][i & 3] = (uint32_t(v) + 0x00808080u) ^ 0x00808080u;     // signed digits in [-128, 127], the top one in [-64, 64]
   }
   transpose4(z[0], p[0]);
@@ -125,8 +127,9 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
       *reinterpret_cast<uint2*>(xp + (j >> 1) * 256 + c * 64 + t * 16 + (j & 1) * 8) = make_uint2(p[0][c], p[1][c]);
     }
   }
-  if (lane == 0) *xs = finite ? __uint_as_float((e - 29u) << 23) : __uint_as_float(0x7fffffffu);
+  if (lane == 0) *xs = fits ? __uint_as_float((e - 29u) << 23) : 0.f;
   if constexpr (has_mins<QT>()) {
+    if (!fits) sum = 0.f;
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     if constexpr (sub16<QT>()) {
       if ((lane & 1) == 0) X[lane >> 1] = sum;
@@ -166,8 +169,9 @@ __device__ __forceinline__ uint2 word2(const uint8_t* p) {       // two consecut
 // xp / xs / X: digit planes, scales and sums of this super-block for activation row 0; row 1 follows at the given strides.
 // blocks: valid 32-weight blocks of this super-block (8 except at the end of a row whose K is not a multiple of 256).
 // res[0], res[1]: sums of rows lane/4 and lane/4 + 8 over this lane's two digits; xt: folded mins of row lane/2.
+// Returns the scale of this lane's activation row.
 template <int QT, int MXC, bool ODD, bool RAG>
-__device__ __forceinline__ void superblock(const uint8_t* bs, const uint8_t* b0, const uint8_t* b1, float (*sS)[sub16<QT>() ? kScalePitch : 8], const uint8_t* xp,
+__device__ __forceinline__ float superblock(const uint8_t* bs, const uint8_t* b0, const uint8_t* b1, float (*sS)[sub16<QT>() ? kScalePitch : 8], const uint8_t* xp,
                                            int xp_stride, const float* xs, int xs_stride, const float* X, int X_stride, int blocks, int lane,
                                            float (&res)[2], float (&xt)[MXC]) {
   constexpr int PH = RAG ? -1 : ODD ? 2 : 0;
@@ -257,7 +261,7 @@ __device__ __forceinline__ void superblock(const uint8_t* bs, const uint8_t* b0,
     *reinterpret_cast<float4*>(srow + 8 * shalf + 4) = make_float4(sc[1], sc[3], sc[5], sc[7]);
   }
   __syncwarp();
-  const float lane_scale = xs[MXC == 2 ? (t >> 1) * xs_stride : 0] * ((t & 1) ? 65536.f : 1.f);
+  const float row_scale = xs[MXC == 2 ? (t >> 1) * xs_stride : 0], lane_scale = row_scale * ((t & 1) ? 65536.f : 1.f);
   const uint8_t* px = xp + (MXC == 2 ? (g >> 2) * xp_stride : 0);
   float sum0 = 0.f, sum1 = 0.f;
   auto apply = [&](const int (&c)[4], float s0, float s1) {
@@ -385,6 +389,32 @@ __device__ __forceinline__ void superblock(const uint8_t* bs, const uint8_t* b0,
   }
   res[0] = fmaf(lane_scale, sum0, res[0]);
   res[1] = fmaf(lane_scale, sum1, res[1]);
+  return row_scale;
+}
+
+// The same super-block in plain fp32, one FMA per weight as the dequantizer gives it, for activations without planes: what this lane adds
+// to its two sums.  b0, b1 as above; x: the super-block of this lane's activation row, `valid` values of it; mine: whether that row
+// has no planes here.  All lanes call it.
+template <int QT, typename T, int MXC>
+__device__ __noinline__ float2 plain(const uint8_t* b0, const uint8_t* b1, const T* x, int valid, bool mine, int t) {
+  constexpr int kUnits = QTraits<QT>::kBlock / 8;                 // of eight weights, dealt to the lanes that share the row
+  float2 sum = make_float2(0.f, 0.f);
+  for (int u = MXC == 2 ? t & 1 : t; 8 * u < valid; u += MXC == 2 ? 2 : 4) {
+    float f[8], w[8];
+    load8<T>(x + 8 * u, f);
+    decode8<QT>(b0 + u / kUnits * QTraits<QT>::kBytes, 8 * (u % kUnits), w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum.x = fmaf(f[i], w[i], sum.x);
+    decode8<QT>(b1 + u / kUnits * QTraits<QT>::kBytes, 8 * (u % kUnits), w);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) sum.y = fmaf(f[i], w[i], sum.y);
+  }
+  if (MXC == 1) {                                                 // join() counts lanes t = 0, 1
+    sum.x += __shfl_xor_sync(0xffffffffu, sum.x, 2);
+    sum.y += __shfl_xor_sync(0xffffffffu, sum.y, 2);
+    mine = mine && t < 2;
+  }
+  return mine ? sum : make_float2(0.f, 0.f);
 }
 
 // Sums of rows lane/4 and lane/4 + 8 over the digit lanes: afterwards lane t = 0 holds row 0's results (and lane t = 2 row 1's).

@@ -523,12 +523,18 @@ gemv_stream_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const
           const uint8_t* xp = sPlanes + psb * planes::kSbBytes;
           const int blocks = RAG ? min(8, (k - sb * 256) / QTraits<QT>::kBlock) : 8;
           constexpr bool kTwoByteBlocks = QT == QTYPE_Q6_K || QT == QTYPE_Q3_K;      // odd super-blocks of a stage start 2 bytes off a word boundary
+          float scale;
           if (!RAG && kTwoByteBlocks && (wq & 1))
-            planes::superblock<QT, MXC, true, false>(bs, b0, b1, sS[cw], xp, plane_sbs * planes::kSbBytes, sXs + psb, plane_sbs, sX + psb * sums_per_sb,
-                                                     plane_sbs * sums_per_sb, blocks, lane, ires, xt);
+            scale = planes::superblock<QT, MXC, true, false>(bs, b0, b1, sS[cw], xp, plane_sbs * planes::kSbBytes, sXs + psb, plane_sbs, sX + psb * sums_per_sb,
+                                                             plane_sbs * sums_per_sb, blocks, lane, ires, xt);
           else
-            planes::superblock<QT, MXC, false, RAG>(bs, b0, b1, sS[cw], xp, plane_sbs * planes::kSbBytes, sXs + psb, plane_sbs, sX + psb * sums_per_sb,
-                                                    plane_sbs * sums_per_sb, blocks, lane, ires, xt);
+            scale = planes::superblock<QT, MXC, false, RAG>(bs, b0, b1, sS[cw], xp, plane_sbs * planes::kSbBytes, sXs + psb, plane_sbs, sX + psb * sums_per_sb,
+                                                            plane_sbs * sums_per_sb, blocks, lane, ires, xt);
+          if (__any_sync(0xffffffffu, scale == 0.f)) {
+            const float2 rest = planes::plain<QT, T, MXC>(b0, b1, x + int64_t(MXC == 2 ? t >> 1 : 0) * k + sb * 256, min(256, k - sb * 256), scale == 0.f, t);
+            ires[0] += rest.x;
+            ires[1] += rest.y;
+          }
         }
         __syncwarp();                            // every lane is done with the stage (and with sS)
         if (lane == 0) mbar_arrive(empty(slot));

@@ -48,3 +48,39 @@ def test_range_of_the_activations(qtype):
     x[1, 5] = float("inf")
     y = kernels.gemm_rcr(x, torch.from_numpy(S.random_blocks(qtype, n, k, seed=5)).to(dev), qtype)
     assert torch.isfinite(y[0]).all() and not torch.isfinite(y[1]).any()
+
+
+@pytest.mark.parametrize("dtype", sorted(TDT))
+@pytest.mark.parametrize("qtype", sorted(KS))
+def test_values_without_planes(qtype, dtype):
+    """Infinities, NaN and (where the type has them) values near the ends of its range: what the products give, for each row by itself."""
+    dev = torch.device("cuda:0")
+    n = 40
+    for k in KS[qtype]:
+        blocks = S.random_blocks(qtype, n, k, seed=k)
+        w = oracle.dequantize(blocks, qtype, k).astype(np.float64)
+        variants = ["simt"] + (["stream"] if dtype != "float32" and kernels.variant_supports("stream", qtype, dtype, 2, n, k) else [])
+        special = [(3, np.inf), (k - 1, -np.inf), (k // 2, np.nan)]
+        if dtype != "float16":
+            special += [(5, 1e36), (k - 2, -1e37)]                # times weights below 20: results below 3.4e38
+            assert np.abs(w).max() < 20
+        base = S.random_activations(2, k, 31, "float32")
+        for at, value in special + [(slice(None), 0.0)] + ([(slice(0, 256), 1e-34)] if dtype != "float16" else []):
+            x = base.copy()
+            x[0, at] = value
+            if value == 1e-34:
+                x[0] = 1e-34 * base[0]
+            for rows in (x[:1], x):
+                xt = torch.from_numpy(rows).to(dev).to(TDT[dtype])
+                xd = xt.double().cpu().numpy()
+                with np.errstate(all="ignore"):
+                    ref = (xd[:, None, :] * w[None]).sum(-1)
+                for variant in variants:
+                    y = kernels.gemm_rcr(xt, torch.from_numpy(blocks).to(dev), qtype, variant=variant).double().cpu().numpy()
+                    assert kernels.device_status() == 0
+                    assert np.array_equal(np.isnan(y), np.isnan(ref)), (k, at, value, variant)
+                    assert np.array_equal(np.where(np.isinf(ref), ref, 0), np.where(np.isinf(y), y, 0)), (k, at, value, variant)
+                    for r in range(len(rows)):
+                        if np.isfinite(ref[r]).all():
+                            largest = np.abs(ref[r]).max()
+                            assert np.abs(y[r] - ref[r]).max() <= BOUND[dtype] * largest, (k, at, value, variant, r)
