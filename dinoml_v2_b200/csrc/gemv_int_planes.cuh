@@ -8,15 +8,21 @@
 // activation row use four (one row) or eight (two rows) columns that were idle.
 //
 // Precision.  A row's activations are fixed-point numbers relative to the largest of their 256-weight super-block: x =
-// xs * (d0 + 256 d1 + 256^2 d2 + 256^3 d3) with |x / xs| < 2^30, rounded once (an absolute error of 2^-31 of the largest; exact for
-// every 16-bit value down to 2^-19 of it).  Products and sums of a sub-block are exact integers; scales, super-blocks and rows
-// are added in fp32.  That is below the rounding of the fp32 accumulation it replaces, so float32 activations run here too.
-// A super-block with an Inf, a NaN or values whose sums or digits leave the range of fp32 has no planes: its scale is zero, and it
-// is multiplied in plain fp32 (plain()), which gives +-Inf or NaN as the products do.
+// xs * (d0 + 256 d1 + 256^2 d2 + 256^3 d3) with |x / xs| < 2^30.  With the largest in [2^E, 2^(E+1)) a value is rounded once, by at most
+// 2^(E-30); float32 values from 2^(E-6) on, float16 from 2^(E-19) and bfloat16 from 2^(E-22) are exact.  Products and sums of a sub-block
+// are exact integers; scales, super-blocks and rows are added in fp32.
+// Where the large values of a super-block meet weights that are zero, only the small ones are left in the result, and the rounding is
+// to be measured against them.  So planes are made only where at most a quarter of the values that are not zero lie below 2^(E-8) (16-bit
+// types, whose larger values are exact: 2^(E-14)).  For the other three quarters the rounding is at most 2^-22 of the value (float32): with
+// normally distributed values 2^-24 of their deviation, no more than the fp32 sums of products that this replaces.
+// A super-block with a wider range than that, with an Inf, a NaN or values whose sums or digits leave the range of fp32 has no planes: its
+// scale is zero, and it is multiplied weight by weight (plain()), which gives +-Inf or NaN as the products do.
 //
 // Every lane keeps two columns of two weight rows: lane t of a quad has digits 2 (t & 1) and 2 (t & 1) + 1.  One IMAD joins the two
 // digits, one I2F and one FFMA apply the sub-block scale; the factor 256^2 of the odd lanes and xs are applied per super-block.
 #pragma once
+#include <type_traits>
+
 #include "gemv_mma_common.cuh"
 
 namespace b200gguf {
@@ -98,16 +104,16 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
     sum += f[i];
   }
   bits = __reduce_max_sync(0xffffffffu, bits);
-  // largest value from 2^-97 (its last digit is 2^-126, the smallest normal number) to 2^100 (sums over a super-block stay finite), or zero
-  const bool fits = bits - 0x0f000000u < 0x71800000u - 0x0f000000u || bits == 0u;
-  const uint32_t e = fits ? max(bits >> 23, 30u) : 30u;
+  const uint32_t e = max(bits >> 23, 30u);
   const float scale = __uint_as_float((283u - e) << 23);         // 2^(29 - (e - 127)): |x| * scale < 2^30
-  uint32_t z[2][4], p[2][4];
+  constexpr uint32_t kBelow = std::is_same<T, float>::value ? 8 : 14;
+  uint32_t below = 0, z[2][4], p[2][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    const int v = fits ? __float2int_rn(f[i] * scale) : 0;
-    z[i >> 2][i & 3] = (uint32_t(v) + 0x00808080u) ^ 0x00808080u;     // signed digits in [-128, 127], the top one in [-64, 64]
+    below += (__float_as_uint(f[i]) & 0x7fffffffu) < ((e - kBelow) << 23) ? 1u : 0u;
+    z[i >> 2][i & 3] = (uint32_t(__float2int_rn(f[i] * scale)) + 0x00808080u) ^ 0x00808080u;     // signed digits in [-128, 127], the top one in [-64, 64]
   }
+  below = __reduce_add_sync(0xffffffffu, below);                 // zeros among them
   transpose4(z[0], p[0]);
   transpose4(z[1], p[1]);
 #pragma unroll
@@ -126,6 +132,16 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
       const int j = lane >> 2, t = lane & 3;
       *reinterpret_cast<uint2*>(xp + (j >> 1) * 256 + c * 64 + t * 16 + (j & 1) * 8) = make_uint2(p[0][c], p[1][c]);
     }
+  }
+  // largest value from 2^-97 (its last digit is 2^-126, the smallest normal number) to 2^100 (sums over a super-block stay finite), or zero;
+  // looked at last, beside the stores: whatever planes a scale of zero has, they add nothing
+  bool fits = bits - 0x0f000000u < 0x71800000u - 0x0f000000u || bits == 0u;
+  if (4 * below > 256) {
+    uint32_t used = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) used += f[i] != 0.f ? 1u : 0u;
+    used = __reduce_add_sync(0xffffffffu, used);
+    fits = fits && 4 * (below + used - 256) <= used;
   }
   if (lane == 0) *xs = fits ? __uint_as_float((e - 29u) << 23) : 0.f;
   if constexpr (has_mins<QT>()) {
@@ -392,29 +408,30 @@ __device__ __forceinline__ float superblock(const uint8_t* bs, const uint8_t* b0
   return row_scale;
 }
 
-// The same super-block in plain fp32, one FMA per weight as the dequantizer gives it, for activations without planes: what this lane adds
-// to its two sums.  b0, b1 as above; x: the super-block of this lane's activation row, `valid` values of it; mine: whether that row
+// The same super-block weight by weight, as the dequantizer gives them, for activations without planes: what this lane adds to its two
+// sums.  Added up in fp64, so that the result is no further off than by planes.  Q4_K [11008 x 4096], M = 1: 34 us
+// with every super-block this way, 15.6 us with one of sixteen, 7.9 us with none.  b0, b1 as above; x: the super-block of this lane's activation row, `valid` values of it; mine: whether that row
 // has no planes here.  All lanes call it.
 template <int QT, typename T, int MXC>
 __device__ __noinline__ float2 plain(const uint8_t* b0, const uint8_t* b1, const T* x, int valid, bool mine, int t) {
   constexpr int kUnits = QTraits<QT>::kBlock / 8;                 // of eight weights, dealt to the lanes that share the row
-  float2 sum = make_float2(0.f, 0.f);
+  double sum[2] = {0., 0.};
   for (int u = MXC == 2 ? t & 1 : t; 8 * u < valid; u += MXC == 2 ? 2 : 4) {
     float f[8], w[8];
     load8<T>(x + 8 * u, f);
     decode8<QT>(b0 + u / kUnits * QTraits<QT>::kBytes, 8 * (u % kUnits), w);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sum.x = fmaf(f[i], w[i], sum.x);
+    for (int i = 0; i < 8; ++i) sum[0] = fma(double(f[i]), double(w[i]), sum[0]);
     decode8<QT>(b1 + u / kUnits * QTraits<QT>::kBytes, 8 * (u % kUnits), w);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) sum.y = fmaf(f[i], w[i], sum.y);
+    for (int i = 0; i < 8; ++i) sum[1] = fma(double(f[i]), double(w[i]), sum[1]);
   }
   if (MXC == 1) {                                                 // join() counts lanes t = 0, 1
-    sum.x += __shfl_xor_sync(0xffffffffu, sum.x, 2);
-    sum.y += __shfl_xor_sync(0xffffffffu, sum.y, 2);
+    sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], 2);
+    sum[1] += __shfl_xor_sync(0xffffffffu, sum[1], 2);
     mine = mine && t < 2;
   }
-  return mine ? sum : make_float2(0.f, 0.f);
+  return mine ? make_float2(float(sum[0]), float(sum[1])) : make_float2(0.f, 0.f);
 }
 
 // Sums of rows lane/4 and lane/4 + 8 over the digit lanes: afterwards lane t = 0 holds row 0's results (and lane t = 2 row 1's).

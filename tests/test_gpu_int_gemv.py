@@ -84,3 +84,54 @@ def test_values_without_planes(qtype, dtype):
                         if np.isfinite(ref[r]).all():
                             largest = np.abs(ref[r]).max()
                             assert np.abs(y[r] - ref[r]).max() <= BOUND[dtype] * largest, (k, at, value, variant, r)
+
+
+def _zero_weights(blocks, qtype, k, columns):
+    """Quants of these columns -> the value that stands for a weight of zero (types without mins)."""
+    for col in columns:
+        sb, i = col // 256, col % 256
+        half, quad, l = i // 128, i % 128 // 32, i % 32
+        if qtype == "Q8_0":
+            blocks[:, 34 * (col // 32) + 2 + col % 32] = 0
+        elif qtype == "Q4_0":
+            at, high = 18 * (col // 32) + 2 + col % 16, col % 32 >= 16
+            blocks[:, at] = (blocks[:, at] & (0x0F if high else 0xF0)) | (0x80 if high else 0x08)
+        elif qtype == "Q6_K":                             # 32 = low nibble 0, high two bits 2
+            at = 210 * sb + 64 * half + 32 * (quad & 1) + l
+            blocks[:, at] &= 0x0F if quad >= 2 else 0xF0
+            at = 210 * sb + 128 + 32 * half + l
+            blocks[:, at] = (blocks[:, at] & (0xFF ^ (3 << (2 * quad)))) | (2 << (2 * quad))
+        else:                                             # Q3_K: 4 = low bits 0, mask bit 1
+            blocks[:, 110 * sb + 32 + 32 * half + l] &= 0xFF ^ (3 << (2 * quad))
+            blocks[:, 110 * sb + l] |= 1 << (4 * half + quad)
+    return blocks
+
+
+@pytest.mark.parametrize("dtype", sorted(TDT))
+@pytest.mark.parametrize("qtype", ["Q8_0", "Q6_K", "Q4_0", "Q3_K"])
+def test_outliers_on_zero_weights(qtype, dtype):
+    """Channels whose activations are 2^s times the others' and whose weights are zero: what is left in the result keeps the accuracy that
+    it has without them.  One such channel per super-block, or every other one."""
+    dev = torch.device("cuda:0")
+    n, k = 300, 2048
+    for columns in (range(37, k, 256), range(1, k, 2)):
+        blocks = _zero_weights(S.random_blocks(qtype, n, k, seed=9), qtype, k, columns)
+        w = oracle.dequantize(blocks, qtype, k).astype(np.float64)
+        assert not w[:, list(columns)].any() and w.any()
+        for s in (4, 6, 7, 8, 10, 12, 15, 20, 26, 40):
+            x = S.random_activations(2, k, 12, "float32")
+            shrink = 2.0 ** -20 if dtype == "float16" and s > 12 else 1.0        # keeps 2^s times a value in range
+            if dtype == "float16" and s > 20:
+                continue
+            x *= shrink ** 0.5
+            x[:, list(columns)] *= 2.0 ** s
+            xt = torch.from_numpy(x).to(dev).to(TDT[dtype])
+            ref = xt.double().cpu().numpy() @ w.T
+            for m in (1, 2):
+                for variant in ["simt"] + (["stream"] if kernels.variant_supports("stream", qtype, dtype, m, n, k) else []):
+                    y = kernels.gemm_rcr(xt[:m].contiguous(), torch.from_numpy(blocks).to(dev), qtype, variant=variant)
+                    assert kernels.device_status() == 0
+                    _, _, norm = oracle.max_errors(ref[:m], y.float().cpu().numpy())
+                    # float16 results of 2^-10 and less: their spacing is 2^-24 at least
+                    floor = 2.0 ** -25 / np.abs(ref[:m]).max() if dtype == "float16" else 0.0
+                    assert norm <= BOUND[dtype] + floor, (len(columns), s, m, variant, norm)
