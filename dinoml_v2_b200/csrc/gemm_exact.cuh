@@ -14,7 +14,11 @@
 //   * warps 4 x 2 take ROWS/4 x BT/2 of the tile with ldmatrix operands;
 //   * with few tiles K is cut across a cluster of up to 8 CTAs whose sums meet through distributed shared memory.
 // Two CTAs share an SM (< 113 KB each), so that one decodes while the other keeps the tensor pipe busy.
+//
+// A result that is not finite (or, with float32 activations, smaller than 2^-100) is computed again weight by weight: an infinite
+// activation has no three parts, and a quant times an activation may leave the range of fp32 before the scale brings it back.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -408,6 +412,7 @@ gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const 
         sums[(wn * (BT / 2) + j * 8 + 2 * t + (q & 1)) * kSumPitch + wm * (ROWS / 4) + i * 16 + g + 8 * (q >> 1)] = res[i][j][q];
   const int slices = int(gridDim.z);
   if (slices > 1) cluster_barrier(); else __syncthreads();
+  bool again = false;
   for (int idx = int(blockIdx.z) * kThreads + tid; idx < ROWS * BT; idx += slices * kThreads) {
     const int r = idx % ROWS, col = idx / ROWS;
     if (n0 + r >= n || m0 + col >= m) continue;
@@ -419,7 +424,16 @@ gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const 
       v = *at;
     if (bias != nullptr) v += MmaType<T>::to_float(bias[n0 + r]);
     y[int64_t(m0 + col) * n + n0 + r] = MmaType<T>::from_float(v);
+    again = again || !(fabsf(v) < INFINITY) || (PL == 3 && v != 0.f && fabsf(v) < 0x1p-100f);
   }
+  // float32 activations beyond what three bfloat16 numbers, or their sums with quants, hold: not results of the tiles
+  if (again)
+    for (int idx = int(blockIdx.z) * kThreads + tid; idx < ROWS * BT; idx += slices * kThreads) {
+      const int r = idx % ROWS, col = idx / ROWS;
+      if (n0 + r < n && m0 + col < m)
+        redo<QT, T, PL == 3>(y + int64_t(m0 + col) * n + n0 + r, x + int64_t(m0 + col) * k, w + int64_t(n0 + r) * row_bytes,
+                             bias != nullptr ? MmaType<T>::to_float(bias[n0 + r]) : 0.f, 1, n, k);
+    }
   if (slices > 1) cluster_barrier();           // nobody leaves while its sums may still be read
 }
 

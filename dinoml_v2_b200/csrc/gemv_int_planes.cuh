@@ -58,22 +58,6 @@ __device__ __forceinline__ void mma16(int (&d)[4], uint32_t a0, uint32_t a1, uin
 }
 
 // ---- activations -> digit planes (one warp per super-block and row; lane i holds weights 8i .. 8i+7)
-template <typename T> __device__ __forceinline__ void load8(const T* p, float (&x)[8]);
-template <> __device__ __forceinline__ void load8<float>(const float* p, float (&x)[8]) {
-  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
-  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-}
-template <typename T> __device__ __forceinline__ void load8(const T* p, float (&x)[8]) {
-  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
-  const uint32_t r[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = MmaType<T>::pair_to_float2(r[i]);
-    x[2 * i] = f.x;
-    x[2 * i + 1] = f.y;
-  }
-}
-
 // Four numbers -> their digits, plane by plane: byte i of p[c] is digit c of z[i].
 __device__ __forceinline__ void transpose4(const uint32_t (&z)[4], uint32_t (&p)[4]) {
   const uint32_t a = __byte_perm(z[0], z[1], 0x5140), b = __byte_perm(z[2], z[3], 0x5140);

@@ -1,5 +1,6 @@
 // Pieces shared by the mma.sync decode GEMV kernels (Q4_K, Q6_K): operand types, cp.async helpers.
 #pragma once
+#include <cmath>
 #include <mutex>
 
 #include "gguf_common.cuh"
@@ -74,6 +75,42 @@ template <> struct MmaType<float> {                      // outputs of the integ
   static __device__ __forceinline__ float to_float(float v) { return v; }
   static __device__ __forceinline__ float from_float(float v) { return v; }
 };
+
+// Eight consecutive activations from a 16-byte aligned address.
+template <typename T> __device__ __forceinline__ void load8(const T* p, float (&x)[8]) {
+  const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
+  const uint32_t r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = MmaType<T>::pair_to_float2(r[i]);
+    x[2 * i] = f.x;
+    x[2 * i + 1] = f.y;
+  }
+}
+template <> __device__ __forceinline__ void load8<float>(const float* p, float (&x)[8]) {
+  const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w; x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
+}
+// Results of one weight row that a tensor-core kernel cannot hold (operands split into parts make Inf - Inf of an infinite or very large
+// activation), weight by weight as the dequantizer gives them, added up in fp64: those of y[0], y[n], .. y[(rows - 1) n] that this thread
+// stored and that are not finite or (TINY) smaller than 2^-100, for activation rows x, x + k, ..  Out of line: next to never called.
+template <int QT, typename T, bool TINY>
+__device__ __noinline__ void redo(T* y, const T* x, const uint8_t* wrow, float bias, int rows, int n, int k) {
+  constexpr int kUnits = QTraits<QT>::kBlock / 8;
+  for (int r = 0; r < rows; ++r, y += n, x += k) {
+    const float had = fabsf(MmaType<T>::to_float(*y));
+    if (had < INFINITY && (!TINY || had == 0.f || had >= 0x1p-100f)) continue;
+    double sum = 0.;
+    for (int u = 0; 8 * u < k; ++u) {
+      float f[8], v[8];
+      load8<T>(x + 8 * u, f);
+      decode8<QT>(wrow + int64_t(u / kUnits) * QTraits<QT>::kBytes, 8 * (u % kUnits), v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) sum = fma(double(f[i]), double(v[i]), sum);
+    }
+    *y = MmaType<T>::from_float(float(sum) + bias);
+  }
+}
 
 // Four registers holding 0.f whose contents the compiler cannot see through: a stable zero C tuple for mma_c.
 __device__ __forceinline__ void opaque_zero4(float (&z)[4]) {

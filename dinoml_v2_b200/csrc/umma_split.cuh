@@ -12,7 +12,9 @@
 //     copy per row was measured first: 128 copies of 224 bytes take 6.5 us, whatever the arithmetic; used for the last tile alone it
 //     still took NVFP4 [5230 x 2880], M = 24, from 14 to 21 us.)  A last group that is not full has a map of its own, as wide as the
 //     rows it has, so that nothing beyond the weight is read;
-//   * K may be any multiple of the block (the tail of the last super-block counts as zero).
+//   * K may be any multiple of the block (the tail of the last super-block counts as zero);
+//   * a result that is not finite is computed again weight by weight: two or three parts of a weight make Inf - Inf of an
+//     infinite activation.
 // Tensor memory holds the accumulator and TERMS slots for four stages, so a tile has up to 256 activation rows with one or two terms and
 // 128 with three.
 #pragma once
@@ -99,11 +101,12 @@ __device__ __forceinline__ void split16(const exact::Unit<QT, 4>& unit, int i, f
 template <int QT, typename T>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap w_tail_map,
-                  const uint8_t* __restrict__ w, int residues, const Params p) {
+                  const T* __restrict__ x, const uint8_t* __restrict__ w, int residues, const Params p) {
   using P = Pair<T>;
   constexpr int BM = split_bm<QT, T>(), TERMS = split_terms<QT, T>(), NSR = split_raw_slots<QT>(), NS = kStagesPerSb;
   constexpr int kXTile = BM * kBK * 2, kPitch = exact::raw_pitch<QT>(), kRawBytes = kRowsW * kPitch, kSbBytes = exact::sb_bytes<QT>();
   constexpr uint32_t kTmemCols = 512;
+  constexpr bool kRedo = TERMS > 1;
   static_assert(BM + NS * TERMS * kWSlotCols <= 512, "tensor memory");
   const uint32_t idesc = (1u << 4) | (P::kFormat << 7) | (P::kFormat << 10) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kRowsW >> 4) << 24);
   const uint32_t x_bytes = uint32_t(p.bn) * (kBK * 2);
@@ -203,6 +206,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         if (!producer_sync()) return false;
       }
       const float bias_v = (finishes && p.bias != nullptr && n_row < p.n) ? MmaType<T>::to_float(static_cast<const T*>(p.bias)[n_row]) : 0.f;
+      float check = 0.f;                            // NaN once a result is not finite
       for (int col = (warp >> 2) * 16; col < p.bn; col += 64) {
         uint32_t r[16];
         tmem_ld16(tmem_base + lanes + uint32_t(col), r);
@@ -223,11 +227,17 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
           if (n_row < p.n) {
             T* dst = static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row;
 #pragma unroll
-            for (int j = 0; j < 16; ++j)
+            for (int j = 0; j < 16; ++j) {
+              if constexpr (kRedo) check = fmaf(0.f, __uint_as_float(r[j]), check);
               if (m0 + col + j < p.m) dst[int64_t(j) * p.n] = MmaType<T>::from_float(__uint_as_float(r[j]) + bias_v);
+            }
           }
         }
       }
+      if (kRedo && check != 0.f && n_row < p.n)
+        for (int col = (warp >> 2) * 16; col < min(p.bn, p.m - m0); col += 64)
+          redo<QT, T, false>(static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row, x + int64_t(m0 + col) * p.k, w + int64_t(n_row) * row_bytes, bias_v,
+                             min(16, p.m - m0 - col), p.n, p.k);
       if (!finishes) {
         if (!producer_sync()) return false;
         if (tid == 0) { __threadfence(); st_release(p.flags + cta, 1); }
@@ -430,7 +440,8 @@ int launch_split(const void* x, const void* w, const void* bias, void* c, int m,
   p.bn = pl.bn;
   p.units = pl.units;
   p.peers = no_peers();
-  return gemv_launch(kern, pl.ctas, 1, kThreads, smem, s, x_map, w_map, w_tail_map, static_cast<const uint8_t*>(w), residues, p) == cudaSuccess ? RC_OK : RC_LAUNCH;
+  return gemv_launch(kern, pl.ctas, 1, kThreads, smem, s, x_map, w_map, w_tail_map, static_cast<const T*>(x),
+                     static_cast<const uint8_t*>(w), residues, p) == cudaSuccess ? RC_OK : RC_LAUNCH;
 }
 
 }  // namespace umma

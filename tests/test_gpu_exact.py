@@ -44,3 +44,34 @@ def test_edges(qtype, dtype):
             assert kernels.device_status() == 0
             _, _, norm = oracle.max_errors(ref, y.float().cpu().numpy())
             assert norm <= BOUND[dtype], (k, n, m, norm)
+
+
+@pytest.mark.parametrize("dtype", sorted(TDT))
+@pytest.mark.parametrize("qtype,k", [("Q8_0", 288), ("Q6_K", 2816), ("Q4_0", 2880), ("Q2_K", 1280), ("Q3_K", 2560), ("MXFP4", 2848), ("NVFP4", 2880),
+                                     ("Q4_K", 1280), ("Q5_K", 768)])
+def test_infinite_and_huge_activations(qtype, k, dtype):
+    """Rows with an Inf, a NaN or values near the end of the type's range get what the products give, the other rows what they had."""
+    dev = torch.device("cuda:0")
+    n = 40
+    blocks = S.random_blocks(qtype, n, k, seed=k)
+    w = oracle.dequantize(blocks, qtype, k).astype(np.float64)
+    largest = float(torch.finfo(TDT[dtype]).max)
+    for m in (3, 9, 40, 130):                               # 130: with 16-bit activations the tcgen05 kernel
+        base = torch.from_numpy(S.random_activations(m, k, 41, "float32")).to(dev).to(TDT[dtype])
+        x = base.clone()
+        x[0, 5], x[1, k - 1], x[2, k // 2] = float("inf"), float("-inf"), float("nan")
+        if m > 3:
+            x[m - 1, 7], x[m - 2, 9], x[m - 2, 300 % k] = largest, float("inf"), float("-inf")
+            x[3] = base[3] * 1e-36 if dtype != "float16" else 0
+        xd = x.double().cpu().numpy()
+        with np.errstate(all="ignore"):
+            ref = (xd[:, None, :] * w[None]).sum(-1)
+            ref[np.abs(ref) > largest] *= np.inf               # results beyond the type
+        y = kernels.gemm_rcr(x, torch.from_numpy(blocks).to(dev), qtype, variant="simt").double().cpu().numpy()
+        assert kernels.device_status() == 0
+        assert np.array_equal(np.isnan(y), np.isnan(ref)), m
+        assert np.array_equal(np.where(np.isinf(ref), ref, 0), np.where(np.isinf(y), y, 0)), m
+        for r in range(m):
+            fine = np.isfinite(ref[r])
+            if fine.any():
+                assert np.abs(y[r][fine] - ref[r][fine]).max() <= BOUND[dtype] * np.abs(ref[r][fine]).max(), (m, r)
