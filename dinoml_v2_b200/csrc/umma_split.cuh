@@ -14,7 +14,7 @@
 //     rows it has, so that nothing beyond the weight is read;
 //   * K may be any multiple of the block (the tail of the last super-block counts as zero);
 //   * a result that is not finite is computed again weight by weight: two or three parts of a weight make Inf - Inf of an
-//     infinite activation.
+//     infinite activation, and a weight or its scale (times 32) may be beyond float16.
 // Tensor memory holds the accumulator and TERMS slots for four stages, so a tile has up to 256 activation rows with one or two terms and
 // 128 with three.
 #pragma once
@@ -30,6 +30,8 @@ namespace umma {
 template <int QT, typename T> constexpr int split_terms() {
   return QT == QTYPE_MXFP4 || QT == QTYPE_NVFP4 ? 1 : QT == QTYPE_Q4_0 || std::is_same<T, __half>::value ? 2 : 3;
 }
+// Whether a scale may be one that the type of the operands does not hold.
+template <int QT, typename T> constexpr bool split_checks_scale() { return QT == QTYPE_MXFP4 && std::is_same<T, __half>::value; }
 template <int QT, typename T> constexpr int split_bm() { return split_terms<QT, T>() < 3 ? 256 : 128; }
 template <int QT> constexpr int split_raw_slots() { return exact::sb_bytes<QT>() > 240 ? 2 : 3; }
 template <int QT, typename T> constexpr size_t split_smem() {
@@ -41,10 +43,16 @@ template <int QT, typename O, int TERMS>
 __device__ __forceinline__ void split16(const exact::Unit<QT, 4>& unit, int i, float scale, float mn, uint32_t (&term)[TERMS][2][8], int q) {
   constexpr int kOff = exact::byte_offset<QT>();
   if constexpr (TERMS == 1) {
-    // FP4: byte - 12 = 2 e2m1, times half the scale; both factors and the product are exact in either 16-bit type (0x43qq is 128 + q as
-    // bfloat16; as float16 0x50qq is 32 + q / 32, which leaves the scale 32 times larger, away from the subnormals)
+    // FP4: byte - 12 = 2 e2m1, times half the scale; both factors and the product are exact in bfloat16, and in float16 for the scales that
+    // it holds (0x43qq is 128 + q as bfloat16; as float16 0x50qq is 32 + q / 32, which leaves the scale 32 times larger, away from the
+    // subnormals).  A ue4m3 scale is always one of them; an e8m0 scale is from 2^-23 to 2^11.  A group with another one becomes NaN,
+    // unless its weights are all zero, and the results of the row are computed again.
     using V = typename Pair<O>::V;
     constexpr bool kHalf = std::is_same<O, __half>::value;
+    if constexpr (split_checks_scale<QT, O>()) {
+      if (scale != 0.f && !(scale >= 0x1p-24f && scale <= 0x1p10f))
+        scale = ((unit.w[i][0] | unit.w[i][1] | unit.w[i][2] | unit.w[i][3]) >> (4 * unit.u)) & 0x07070707u ? NAN : 0.f;
+    }
     const V s1 = Pair<O>::splat(kHalf ? 32.f * scale : scale), off = Pair<O>::splat(kHalf ? 32.f + float(kOff) / 32.f : 128.f + float(kOff));
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -106,7 +114,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   constexpr int BM = split_bm<QT, T>(), TERMS = split_terms<QT, T>(), NSR = split_raw_slots<QT>(), NS = kStagesPerSb;
   constexpr int kXTile = BM * kBK * 2, kPitch = exact::raw_pitch<QT>(), kRawBytes = kRowsW * kPitch, kSbBytes = exact::sb_bytes<QT>();
   constexpr uint32_t kTmemCols = 512;
-  constexpr bool kRedo = TERMS > 1;
+  constexpr bool kRedo = TERMS > 1 || split_checks_scale<QT, T>();
   static_assert(BM + NS * TERMS * kWSlotCols <= 512, "tensor memory");
   const uint32_t idesc = (1u << 4) | (P::kFormat << 7) | (P::kFormat << 10) | (uint32_t(p.bn >> 3) << 17) | (uint32_t(kRowsW >> 4) << 24);
   const uint32_t x_bytes = uint32_t(p.bn) * (kBK * 2);

@@ -75,3 +75,45 @@ def test_infinite_and_huge_activations(qtype, k, dtype):
             fine = np.isfinite(ref[r])
             if fine.any():
                 assert np.abs(y[r][fine] - ref[r][fine]).max() <= BOUND[dtype] * np.abs(ref[r][fine]).max(), (m, r)
+
+
+D_AT = {"Q8_0": (34, (0,)), "Q6_K": (210, (208,)), "Q4_0": (18, (0,)), "Q2_K": (84, (80, 82)), "Q3_K": (110, (108,))}
+
+
+@pytest.mark.parametrize("qtype,k", [("Q8_0", 288), ("Q6_K", 2816), ("Q4_0", 2880), ("Q2_K", 1280), ("Q3_K", 2560), ("MXFP4", 2848)])
+def test_float16_scales_of_any_size(qtype, k):
+    """Block scales that float16 operands do not hold, beside ones that they do, in the tcgen05 kernel with split weights."""
+    dev = torch.device("cuda:0")
+    n, m = 40, 260
+    blocks = S.random_blocks(qtype, n, k, seed=k)
+    if qtype == "MXFP4":
+        e = blocks[:, ::17]                             # the exponent byte of every block of a row
+        for row, byte in enumerate((127 + 11, 127 + 12, 127 + 20, 127 - 23, 127 - 24, 127 - 30)):
+            e[row] = byte
+        e[6, 3], e[7, 5] = 127 + 14, 127 - 27           # one block of the row
+        for row, byte in ((8, 0), (9, 254)):            # blocks whose weights are zero, with any scale
+            for col in range(17 * 4, 17 * 6):
+                blocks[row, col] = 0 if col % 17 else byte
+    else:
+        size, offsets = D_AT[qtype]
+        for row, d in enumerate((2000.0, 2100.0, 30000.0, 60000.0, 6e-8, 3e-5)):
+            for at in offsets:
+                for i, byte in enumerate(np.float16(d).tobytes()):
+                    blocks[row, at + i::size] = byte
+        blocks[6, offsets[0]:offsets[0] + 2] = np.frombuffer(np.float16(50000.0).tobytes(), np.uint8)      # its first block only
+    w = oracle.dequantize(blocks, qtype, k).astype(np.float64)
+    x = torch.from_numpy(S.random_activations(m, k, 43, "float32")).to(dev)
+    x[: m // 2] *= 2.0 ** -14                           # for results of the large scales, and of the small ones
+    x[m // 2:] *= 2.0 ** 12
+    x = x.half()
+    xd = x.double().cpu().numpy()
+    ref = xd @ w.T
+    y = kernels.gemm_rcr(x, torch.from_numpy(blocks).to(dev), qtype).double().cpu().numpy()
+    assert kernels.device_status() == 0
+    # float16 rounding of the result, 1e-5 of the products' magnitudes for the sums, half the smallest float16 step
+    bound = 2.0 ** -11 * np.abs(ref) + 1e-5 * (np.abs(xd) @ np.abs(w).T) + 2.0 ** -25
+    inside = np.abs(ref) + bound < 65504
+    assert inside[:, :8].any(axis=0).all()
+    assert (np.abs(y[inside] - ref[inside]) <= bound[inside]).all()
+    beyond = np.abs(ref) - bound >= 65520
+    assert (np.isinf(y[beyond]) & (np.sign(y[beyond]) == np.sign(ref[beyond]))).all()
