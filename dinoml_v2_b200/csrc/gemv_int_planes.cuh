@@ -81,23 +81,24 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
     for (int i = 0; i < 8; ++i) f[i] = 0.f;
   }
   float sum = 0.f;
-  uint32_t bits = 0;
+  uint32_t bits = 0, least = 0xffffffffu;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    bits = max(bits, __float_as_uint(f[i]) & 0x7fffffffu);      // as integers: an Inf or NaN is larger than every finite value
+    const uint32_t magnitude = __float_as_uint(f[i]) & 0x7fffffffu;      // as integers: an Inf or NaN is larger than every finite value
+    bits = max(bits, magnitude);
+    least = min(least, magnitude);
     sum += f[i];
   }
   bits = __reduce_max_sync(0xffffffffu, bits);
   const uint32_t e = max(bits >> 23, 30u);
   const float scale = __uint_as_float((283u - e) << 23);         // 2^(29 - (e - 127)): |x| * scale < 2^30
   constexpr uint32_t kBelow = std::is_same<T, float>::value ? 8 : 14;
-  uint32_t below = 0, z[2][4], p[2][4];
+  const uint32_t low = (e - kBelow) << 23;
+  const uint32_t lanes = __ballot_sync(0xffffffffu, least < low);        // with a value below, zeros among them
+  uint32_t z[2][4], p[2][4];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    below += (__float_as_uint(f[i]) & 0x7fffffffu) < ((e - kBelow) << 23) ? 1u : 0u;
+  for (int i = 0; i < 8; ++i)
     z[i >> 2][i & 3] = (uint32_t(__float2int_rn(f[i] * scale)) + 0x00808080u) ^ 0x00808080u;     // signed digits in [-128, 127], the top one in [-64, 64]
-  }
-  below = __reduce_add_sync(0xffffffffu, below);                 // zeros among them
   transpose4(z[0], p[0]);
   transpose4(z[1], p[1]);
 #pragma unroll
@@ -120,12 +121,15 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
   // largest value from 2^-97 (its last digit is 2^-126, the smallest normal number) to 2^100 (sums over a super-block stay finite), or zero;
   // looked at last, beside the stores: whatever planes a scale of zero has, they add nothing
   bool fits = bits - 0x0f000000u < 0x71800000u - 0x0f000000u || bits == 0u;
-  if (4 * below > 256) {
-    uint32_t used = 0;
+  if (__popc(lanes) > 8) {                                       // else a quarter of the values at most
+    uint32_t count = 0;                                          // values that are not zero, and (high half) those of them that lie below
 #pragma unroll
-    for (int i = 0; i < 8; ++i) used += f[i] != 0.f ? 1u : 0u;
-    used = __reduce_add_sync(0xffffffffu, used);
-    fits = fits && 4 * (below + used - 256) <= used;
+    for (int i = 0; i < 8; ++i) {
+      const uint32_t magnitude = __float_as_uint(f[i]) & 0x7fffffffu;
+      count += magnitude == 0u ? 0u : magnitude < low ? 0x10001u : 1u;
+    }
+    count = __reduce_add_sync(0xffffffffu, count);
+    fits = fits && 4 * (count >> 16) <= (count & 0xffffu);
   }
   if (lane == 0) *xs = fits ? __uint_as_float((e - 29u) << 23) : 0.f;
   if constexpr (has_mins<QT>()) {
