@@ -26,11 +26,18 @@ def _require_cuda(t: torch.Tensor, name: str) -> None:
 _binding = None
 
 
+class _NoBinding:
+    """Stands in for a native binding that does not load: every call is left to the wrapper's own path."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
 def _native_call(name: str):
     """A function of the native binding.  The binding is loaded on the first call."""
     global _binding
     if _binding is None:
-        _binding = _native.binding()
+        _binding = _native.binding() or _NoBinding()
     return getattr(_binding, name)
 
 

@@ -282,7 +282,7 @@ class Session:
         ins, outs, keep = self._pack(inputs, outputs)
         self.module._check(self._lib.dino_session_run(self._handle, ins, len(ins), outs, len(outs)))
 
-    def _make_runner(self):
+    def _make_runner(self, native):
         """What the native run_torch needs of the graph: ports by name and tensor number, and how shapes follow from the nodes."""
         if not hasattr(self, "_graph"):
             self._graph = json.loads((self.module.path / "graph.dinoir.json").read_text())
@@ -296,16 +296,16 @@ class Session:
             rows = consts[node["inputs"][1]]["shape"][0]
             nodes.append((number[node["inputs"][0]], number[node["outputs"][0]], rows // 2 if node["op"].startswith("dual_gemm_rcr_") else rows))
         ports = lambda entries: [(e["name"], number[e["name"]], e["dtype"]) for e in entries]
-        from . import _native
         run = ctypes.cast(self._lib.dino_session_run, ctypes.c_void_p).value
-        return _native.binding().make_runner(run, self._handle.value, len(number), ports(self.module.metadata["inputs"]),
-                                             ports(self.module.metadata["outputs"]), nodes)
+        return native.make_runner(run, self._handle.value, len(number), ports(self.module.metadata["inputs"]),
+                                  ports(self.module.metadata["outputs"]), nodes)
 
     def run_torch(self, inputs: Mapping[str, Any], outputs: Mapping[str, Any] | None = None) -> dict[str, Any]:
-        if self._handle:
-            if self._runner is None:
-                from . import _native
-                self._runner, self._run_native = self._make_runner(), _native.binding().run_torch
+        if self._handle and self._runner is None:
+            from . import _native
+            native = _native.binding()
+            self._runner, self._run_native = (self._make_runner(native), native.run_torch) if native is not None else (False, None)
+        if self._handle and self._runner:
             done = self._run_native(self._runner, inputs, outputs)        # None: not the plain case, taken apart below
             if done is not None:
                 if type(done) is int:

@@ -9,7 +9,7 @@ import torch
 
 import dinoml_v2_b200 as dml
 import oracle
-from dinoml_v2_b200 import gguf_file, profiling, synthetic as S
+from dinoml_v2_b200 import gguf_file, kernels, profiling, synthetic as S
 
 pytestmark = pytest.mark.gpu
 
@@ -371,3 +371,35 @@ def test_profile_run_environment_contract(tmp_path, capfd, monkeypatch):
     with pytest.raises(RuntimeError, match="did not match"):
         sess.run_numpy({"x": S.random_activations(2, 1024, 1, "float32")})
     mod.close()
+
+
+def test_wrappers_with_and_without_the_native_binding(tmp_path, monkeypatch):
+    import sys
+    from dinoml_v2_b200 import _native
+    dev = torch.device("cuda:0")
+    n, k = 64, 512
+    blocks = S.random_blocks("Q4_K", n, k, 3)
+    w = torch.from_numpy(blocks).to(dev)
+    x = torch.randn(3, k, device=dev).to(torch.bfloat16)
+    gguf_file.write_gguf(tmp_path / "w.gguf", {"w": ("Q4_K", (n, k), blocks)})
+    spec = dml.trace(dml.nn.Linear(k, n, bias=False, dtype="bfloat16"), inputs={"x": dml.TensorSpec([dml.Dim("m", 1, 8, buckets=(1, 8)), k], "bfloat16")},
+                     constants={"weight": dml.gguf_constant(tmp_path / "w.gguf", "w")})
+    module = dml.runtime.load(dml.compile(spec, dml.Target("cuda"), tmp_path / "art").path)
+    module.load_encoded_constants()
+
+    def results():
+        session = module.create_session()
+        out = [kernels.gemm_rcr(x, w, "Q4_K"), kernels.dual_gemm_rcr(x, w, "Q4_K"), kernels.dequantize_rows(w, "Q4_K", k), session.run_torch({"x": x})["t0"]]
+        return [t.clone() for t in out]
+
+    first = results()
+    assert _native.binding() is not None
+    for owner in (_native, kernels):
+        monkeypatch.setattr(owner, "_binding", None)
+    monkeypatch.delattr(dml, "_torch_binding")
+    monkeypatch.setitem(sys.modules, "dinoml_v2_b200._torch_binding", None)
+    with pytest.warns(RuntimeWarning, match="slower host path"):
+        second = results()
+    assert kernels.device_status() == 0
+    assert all(torch.equal(a, b) for a, b in zip(first, second))
+    module.close()

@@ -339,3 +339,24 @@ def test_variant_predicate_is_the_librarys_own():
     assert not mf.variant_supports("stream:4", 9, qtype="Q4_K", dtype="float16", n=64, k=512)
     assert not mf.variant_supports("mma", 4, qtype="Q4_K", dtype="float32", n=64, k=512)
     assert mf.variant_code("stream:3") == 4 | (3 << 8) and mf.variant_code("umma") == 3
+
+
+def test_wrappers_without_the_native_binding(monkeypatch):
+    """_torch_binding.so is built against one torch: where it does not load the wrappers go on by themselves, after one warning."""
+    import sys
+    import torch
+    from dinoml_v2_b200 import _native, kernels
+    try:
+        _native.lib()
+    except _native.NativeLibraryMissing:
+        pytest.skip("the kernel library is not built")
+    for module in (_native, kernels):
+        monkeypatch.setattr(module, "_binding", None)
+    monkeypatch.delattr(dml, "_torch_binding", raising=False)
+    monkeypatch.setitem(sys.modules, "dinoml_v2_b200._torch_binding", None)
+    with pytest.warns(RuntimeWarning, match="slower host path"):
+        assert _native.binding() is None
+    a, b = torch.zeros(1, 256), torch.zeros(16, 144, dtype=torch.uint8)
+    for call in (lambda: kernels.gemm_rcr(a, b, "Q4_K"), lambda: kernels.dual_gemm_rcr(a, b, "Q4_K"), lambda: kernels.dequantize_rows(b, "Q4_K", 256)):
+        with pytest.raises(ValueError, match="must be a CUDA tensor"):
+            call()
