@@ -25,6 +25,8 @@
 #include "gemv_mma_common.cuh"
 
 namespace b200gguf {
+namespace stream { int sm_count(); }             // gemv_stream.cu
+
 namespace exact {
 
 constexpr int kThreads = 256;
@@ -448,10 +450,11 @@ int launch_tile(const void* a, const void* b, const void* bias, void* c, int m, 
   if (m_tiles > 65535) return RC_RANGE;
   // The number of K slices with the shortest walk: rounds of two CTAs per SM times super-blocks per slice (a slice costs about two
   // super-blocks more for its start and the exchange of sums).
+  const int64_t slots = 2 * stream::sm_count();
   int slices = 1;
   int64_t best = INT64_MAX;
   for (int z = 1; z <= 8 && z <= nsb; ++z) {
-    const int64_t walk = ((int64_t(tiles) * m_tiles * z + 2 * 148 - 1) / (2 * 148)) * ((nsb + z - 1) / z + 2);
+    const int64_t walk = ((int64_t(tiles) * m_tiles * z + slots - 1) / slots) * ((nsb + z - 1) / z + 2);
     if (walk < best) { best = walk; slices = z; }
   }
   cudaLaunchConfig_t cfg = {};
@@ -475,12 +478,12 @@ int launch_tile(const void* a, const void* b, const void* bias, void* c, int m, 
 template <int QT, typename T>
 int launch(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
   constexpr bool kPlanes = x_planes<T>() == 3;
-  const int64_t row_tiles = (n + 127) / 128;
+  const int64_t row_tiles = (n + 127) / 128, quarter = stream::sm_count() / 4;
   if constexpr (!kPlanes) {
-    if (m > 64 && row_tiles * ((m + 127) / 128) >= 37) return launch_tile<QT, T, 128, 128>(a, b, bias, c, m, n, k, s);
-    if (m > 32 && row_tiles * ((m + 63) / 64) >= 37) return launch_tile<QT, T, 128, 64>(a, b, bias, c, m, n, k, s);
+    if (m > 64 && row_tiles * ((m + 127) / 128) >= quarter) return launch_tile<QT, T, 128, 128>(a, b, bias, c, m, n, k, s);
+    if (m > 32 && row_tiles * ((m + 63) / 64) >= quarter) return launch_tile<QT, T, 128, 64>(a, b, bias, c, m, n, k, s);
   } else {
-    if (row_tiles * ((m + 31) / 32) >= 37) return launch_tile<QT, T, 128, 32>(a, b, bias, c, m, n, k, s);
+    if (row_tiles * ((m + 31) / 32) >= quarter) return launch_tile<QT, T, 128, 32>(a, b, bias, c, m, n, k, s);
   }
   return launch_tile<QT, T, 64, 32>(a, b, bias, c, m, n, k, s);
 }

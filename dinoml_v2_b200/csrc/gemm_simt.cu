@@ -1,12 +1,11 @@
-// Fused GGUF gemm_rcr, CUDA-core variant ("simt"): C[M,N] = A[M,K] * dequant(W[N,K])^T (+ bias).
-//
-// One warp per weight row; lanes stride over 8-wide K units, decode them exactly as the dequantizer
-// does, and accumulate in fp32 with FMA; a shuffle tree finishes the row.  Every (activation, output)
-// dtype and every M is supported, which makes this the reference-faithful fallback of the candidate
-// family (the behavioural ancestor is the reference's one-wave-per-column prototype,
-// kernels/rocm/src/ck_gguf_q8_gemm.hip:1168-1207) and the only variant that keeps fp32 activations
-// un-rounded.  It reads W once per group of MT activation rows, so it is bandwidth-efficient only
-// for M <= MT; the tensor-core variants take over elsewhere.
+// The "simt" family of the fused GGUF gemm_rcr: C[M,N] = A[M,K] * dequant(W[N,K])^T (+ bias) for every type, activation dtype, M and
+// any K that is a multiple of the block - float32 activations and weight rows that are not multiples of 16 bytes in the first place.
+// The entry at the end picks the kernel by size: the byte-operand GEMV (gemv_planes.cu), the exact tensor-core GEMM (gemm_exact.cuh), tcgen05
+// with split weights (umma_split.cuh), and for what they leave - one or two rows of the FP4 types, 16-bit activations on aligned rows when
+// this family is asked for by name - the CUDA-core kernel below: one warp per weight row; lanes stride over 8-wide K units, decode
+// them exactly as the dequantizer does, and accumulate in fp32 with FMA; a shuffle tree finishes the row.  It reads W once per group
+// of MT activation rows (behavioural ancestor: the reference's one-wave-per-column prototype,
+// kernels/rocm/src/ck_gguf_q8_gemm.hip:1168-1207).
 #include "gemv_mma_common.cuh"
 
 namespace b200gguf {
@@ -114,8 +113,12 @@ int check_gemm_args(const void* a, const void* b, const void* c, int qtype, int 
 int gemm_rcr_simt(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k,
                   cudaStream_t s) {
   if (int rc = check_gemm_args(a, b, c, qtype, dtype, m, n, k)) return rc;
-  // Up to six rows: the byte-operand GEMV, two rows at a time (the weight stays in the L2 between the passes), where the type has it
-  // ([4096 x 4096] Q8_0, float32, M = 4: two launches of 5.9 us against 23 us on the CUDA cores).
+  // Up to six rows: the byte-operand GEMV, two rows at a time, where the type has it.  It reads the weight up to three times and is
+  // still ahead of one pass of the exact GEMM, whose mma.sync work is for 32 rows whatever M is, in the L2 or out of it.  float32 Q8_0,
+  // M = 3 / 5, us: [4096 x 4096], 18 MB: 12.1 / 18.2 against 24.4; [28672 x 8192], 250 MB: 88 / 134 against 320; [128256 x 4096], 558 MB:
+  // 173 / 259 against 550; Q4_K [65536 x 8192] 113 / 172 against 646.  bfloat16 has a third of that MMA work: Q8_0 [32000 x 2880], 98 MB,
+  // 47 / 69 against 92, [128256 x 4128], 563 MB, 298 / 475 against 444; Q4_0 [5760 x 2880] 13.5 / 20.5 against 16.9, Q3_K [4096 x 2560]
+  // 10.2 / 15.8 against 13.9: at M = 5 and 6 the shortest and the longest of these would be 7 - 20 % better off there.
   if (m <= 6) {
     const size_t esz = dtype == DINO_F32 ? 4 : 2;
     int rc = RC_OK;
