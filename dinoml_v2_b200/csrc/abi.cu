@@ -80,8 +80,8 @@ int select_variant(int qtype, int dtype, int m, int n, int k) {
     return DINOML_B200_GGUF_VARIANT_UMMA;
   // M <= 8: the persistent bulk-copy GEMV (M <= 2 with byte operands), except where the tile kernel measured faster:
   //   Q4_K, M = 1 / 2, with fewer row tiles than SMs / half the SMs on K < 8192, where making the digit planes is a large part of the
-  //   launch ([1024 x 4096]: 3.2 us against 3.9, M = 2: 3.8 against 4.7), and M = 1 on the shapes whose waves fill the tile kernel's
-  //   grid (named mma; the family runs them on the persistent kernel since that takes byte operands);
+  //   launch ([1024 x 4096]: 3.2 us against 3.9, M = 2: 3.8 against 4.7).  (Q4_K, M = 1, on shapes that fill three quarters of the tile
+  //   kernel's last wave keeps the name it has had, mma, for callers that read it; that family runs them on the persistent kernel too.)
   //   Q4_K, M >= 3, with fewer row tiles than half the SMs on a long K: the tile kernel cuts K across a cluster and so uses more SMs
   //   ([256 x 14336], M = 8: 4.9 us against 9.3 us);
   //   Q6_K, M >= 3, on weights below 32 M elements ([4096 x 4096], M = 4: 6.3 us against 6.8 us), where the launch is too short
@@ -90,7 +90,7 @@ int select_variant(int qtype, int dtype, int m, int n, int k) {
     bool tile_kernel = false;
     if (qtype == QTYPE_Q4_K && m == 1) {
       const int slots = 3 * sms, waves = (tiles + slots - 1) / slots;
-      // the mma family: it keeps the shapes with fewer tiles than SMs and hands the others to the persistent kernel itself
+      // fewer tiles than SMs: the tile kernel itself; full waves: only the name, the mma family hands them to the persistent kernel
       tile_kernel = (tiles <= sms && k < 8192) || (tiles >= slots && double(tiles) / (double(waves) * slots) >= 0.75);
     } else if (qtype == QTYPE_Q4_K) {
       tile_kernel = 2 * tiles <= sms && (m == 2 ? k < 8192 : m < 4 || k >= 8192);

@@ -397,9 +397,10 @@ __device__ __forceinline__ float superblock(const uint8_t* bs, const uint8_t* b0
 }
 
 // The same super-block weight by weight, as the dequantizer gives them, for activations without planes: what this lane adds to its two
-// sums.  Added up in fp64, so that the result is no further off than by planes.  Q4_K [11008 x 4096], M = 1: 34 us
-// with every super-block this way, 15.6 us with one of sixteen, 7.9 us with none.  b0, b1 as above; x: the super-block of this lane's activation row, `valid` values of it; mine: whether that row
-// has no planes here.  All lanes call it.
+// sums.  Added up in fp64, so that the result is no further off than by planes.  Q4_K [11008 x 4096], M = 1: 34 us with every super-block
+// this way, 15.6 us with one of sixteen, 7.9 us with none.
+// b0, b1 as above; x: the super-block of this lane's activation row, `valid` values of it; mine: whether that row has no planes here.  All
+// lanes call it.
 template <int QT, typename T, int MXC>
 __device__ __noinline__ float2 plain(const uint8_t* b0, const uint8_t* b1, const T* x, int valid, bool mine, int t) {
   constexpr int kUnits = QTraits<QT>::kBlock / 8;                 // of eight weights, dealt to the lanes that share the row

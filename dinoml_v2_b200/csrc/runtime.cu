@@ -1023,8 +1023,8 @@ int dino_session_run_staged_on(DinoSession* session, void* stream, int graph_rep
 }
 
 // float32 <-> bfloat16 bit patterns on the host, for callers whose arrays are float32 (numpy has no bfloat16): round to
-// nearest even exactly as the reference's Python does (src/dinoml/ir.py:68-73: bits + 0x7FFF + lsb, high half), NaN kept
-// a NaN; widening is the 16 bits followed by 16 zeros.
+// nearest even exactly as the reference's Python does (src/dinoml/ir.py:68-73: bits + 0x7FFF + lsb, high half; like there, a NaN with
+// mantissa bits all over, 0x7fff8000 and up, comes out as a zero); widening is the 16 bits followed by 16 zeros.
 // Written on 32-bit integer views with no call in the loop body so that the host compiler vectorizes them (an 11008-element
 // result widens in 0.4 us instead of 3 us).
 // Where the processor has AVX2, whole vectors of 16: a run of M = 16 converts 0.6 M values, on the caller's thread, before and after

@@ -26,7 +26,9 @@ DUAL_OPS = ("dual_gemm_rcr_silu", "dual_gemm_rcr_fast_gelu", "dual_gemm_rcr_bias
 SUPPORTED_OPS = ("gemm_rcr", "gemm_rcr_bias") + DUAL_OPS
 VARIANT_CODES = {"simt": 1, "mma": 2, "umma": 3, "stream": 4}
 # Tuning configurations of the persistent GEMV (csrc/gemv_stream.cu): each is a candidate of its own, as the tile / stage /
-# warp entries of the reference's CUTLASS catalogue are (src/dinoml/kernels/providers/cutlass/gemm.py:19-127).
+# warp entries of the reference's CUTLASS catalogue are (src/dinoml/kernels/providers/cutlass/gemm.py:19-127).  Warps and ring slots are
+# those of the 16-bit-operand arithmetic (M = 3..8, the FP4 types at every M).  With byte operands (M = 1, 2) every configuration runs 8
+# consumer warps and the ring that fits beside the digit planes; only ctas_per_sm still tells them apart, so 1, 2 and 3 time alike there.
 STREAM_CONFIGS = {1: {"consumer_warps": 8, "ring_slots": {"Q4_K": 5, "Q6_K": 4, "Q5_K": 4, "Q4_0": 5, "MXFP4": 5, "NVFP4": 5, "Q2_K": 5, "Q3_K": 5}, "ctas_per_sm": 1},
                   2: {"consumer_warps": 16, "ring_slots": {"Q4_K": 6, "Q6_K": 4, "Q5_K": 4, "Q4_0": 6, "MXFP4": 6, "NVFP4": 6, "Q2_K": 6, "Q3_K": 6}, "ctas_per_sm": 1},
                   3: {"consumer_warps": 16, "ring_slots": {"Q4_K": 8, "Q6_K": 6, "Q5_K": 6, "Q4_0": 8, "MXFP4": 8, "NVFP4": 8, "Q2_K": 8, "Q3_K": 8}, "ctas_per_sm": 1},
@@ -35,6 +37,10 @@ STREAM_QTYPES = ("Q4_K", "Q6_K", "Q5_K", "Q4_0", "MXFP4", "NVFP4", "Q2_K", "Q3_K
 # further types the tcgen05 GEMM unpacks (besides Q4_K, Q6_K, Q8_0); MXFP4 and NVFP4 become exact 16-bit operands
 UMMA_MORE_QTYPES = ("Q5_K", "Q4_0", "MXFP4", "NVFP4", "Q2_K", "Q3_K")
 
+# What a family is made of.  A family's entry may hand a call on to the kernel that measured faster: "mma" runs Q4_K at M = 1 on more row tiles
+# than SMs, and Q8_0 and ragged Q6_K at M = 1, 2, on the persistent kernel with byte operands (mma.sync.m16n8k32), large ragged Q6_K at
+# M = 9..16 on tcgen05 with split weights; "simt" is the family of float32 activations and ragged weight rows and picks by M among the
+# byte-operand GEMV, the exact mma.sync GEMM, tcgen05 with split weights and the CUDA-core kernel described here.
 _B200_TUNING = {
     "simt": {"kind": "gemv_simt", "rows_per_warp": 1, "activation_rows_per_pass": 4, "staging": "ldg", "tensor_cores": "none"},
     "mma": {"kind": "gemv", "rows_per_cta": 16, "stage_super_blocks": 4, "stages": [3, 4, 6], "staging": "cp_async16",
