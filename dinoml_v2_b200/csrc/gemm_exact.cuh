@@ -429,13 +429,13 @@ gemm_exact_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const 
     again = again || !(fabsf(v) < INFINITY) || (PL == 3 && v != 0.f && fabsf(v) < 0x1p-100f);
   }
   // float32 activations beyond what three bfloat16 numbers, or their sums with quants, hold: not results of the tiles
-  if (again)
-    for (int idx = int(blockIdx.z) * kThreads + tid; idx < ROWS * BT; idx += slices * kThreads) {
-      const int r = idx % ROWS, col = idx / ROWS;
-      if (n0 + r < n && m0 + col < m)
-        redo<QT, T, PL == 3>(y + int64_t(m0 + col) * n + n0 + r, x + int64_t(m0 + col) * k, w + int64_t(n0 + r) * row_bytes,
-                             bias != nullptr ? MmaType<T>::to_float(bias[n0 + r]) : 0.f, 1, n, k);
-    }
+  static_assert(kThreads % ROWS == 0, "a thread's results are one weight row's");
+  if (again) {
+    const int idx = int(blockIdx.z) * kThreads + tid, r = idx % ROWS, col = idx / ROWS, step = slices * (kThreads / ROWS);
+    const int cols = min(BT, m - m0);            // of this tile; this thread stored col, col + step, ..
+    redo<QT, T, PL == 3>(y + int64_t(m0 + col) * n + n0 + r, int64_t(step) * n, x + int64_t(m0 + col) * k, int64_t(step) * k, w + int64_t(n0 + r) * row_bytes,
+                         bias != nullptr ? MmaType<T>::to_float(bias[n0 + r]) : 0.f, (cols - col + step - 1) / step, k);
+  }
   if (slices > 1) cluster_barrier();           // nobody leaves while its sums may still be read
 }
 

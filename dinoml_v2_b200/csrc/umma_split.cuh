@@ -244,8 +244,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       }
       if (kRedo && check != 0.f && n_row < p.n)
         for (int col = (warp >> 2) * 16; col < min(p.bn, p.m - m0); col += 64)
-          redo<QT, T, false>(static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row, x + int64_t(m0 + col) * p.k, w + int64_t(n_row) * row_bytes, bias_v,
-                             min(16, p.m - m0 - col), p.n, p.k);
+          redo<QT, T, false>(static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row, p.n, x + int64_t(m0 + col) * p.k, p.k, w + int64_t(n_row) * row_bytes,
+                             bias_v, min(16, p.m - m0 - col), p.k);
       if (!finishes) {
         if (!producer_sync()) return false;
         if (tid == 0) { __threadfence(); st_release(p.flags + cta, 1); }

@@ -56,12 +56,17 @@ def test_infinite_and_huge_activations(qtype, k, dtype):
     blocks = S.random_blocks(qtype, n, k, seed=k)
     w = oracle.dequantize(blocks, qtype, k).astype(np.float64)
     largest = float(torch.finfo(TDT[dtype]).max)
-    for m in (3, 9, 40, 130):                               # 130: with 16-bit activations the tcgen05 kernel
+    for m, kind in ((3, ""), (9, ""), (40, ""), (130, ""), (131, "infinite"), (132, "tiny")):        # from 130 with 16-bit activations the tcgen05 kernel
         base = torch.from_numpy(S.random_activations(m, k, 41, "float32")).to(dev).to(TDT[dtype])
+        if kind == "infinite":                              # every row at one place, beside the ones below
+            base[:, 11] = float("inf")
+        elif kind == "tiny" and dtype != "float16":
+            base *= 1e-34
         x = base.clone()
         x[0, 5], x[1, k - 1], x[2, k // 2] = float("inf"), float("-inf"), float("nan")
         if m > 3:
-            x[m - 1, 7], x[m - 2, 9], x[m - 2, 300 % k] = largest, float("inf"), float("-inf")
+            x[m - 1, 7] = 1.0 if kind == "infinite" else largest          # largest x weight + Inf x weight is Inf or NaN with the arithmetic's range
+            x[m - 2, 9], x[m - 2, 300 % k] = float("inf"), float("-inf")
             x[3] = base[3] * 1e-36 if dtype != "float16" else 0
         xd = x.double().cpu().numpy()
         with np.errstate(all="ignore"):
