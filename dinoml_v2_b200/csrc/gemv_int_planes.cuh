@@ -121,7 +121,7 @@ __device__ __forceinline__ void make(const T* x, int valid, int lane, uint8_t* x
   // largest value from 2^-97 (its last digit is 2^-126, the smallest normal number) to 2^100 (sums over a super-block stay finite), or zero;
   // looked at last, beside the stores: whatever planes a scale of zero has, they add nothing
   bool fits = bits - 0x0f000000u < 0x71800000u - 0x0f000000u || bits == 0u;
-  if (__popc(lanes) > 8) {                                       // else a quarter of the values at most
+  if (__builtin_expect(__popc(lanes) > 8, 0)) {                  // else a quarter of the values at most
     uint32_t count = 0;                                          // values that are not zero, and (high half) those of them that lie below
 #pragma unroll
     for (int i = 0; i < 8; ++i) {

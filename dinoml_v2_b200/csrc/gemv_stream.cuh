@@ -530,7 +530,7 @@ gemv_stream_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w, const
           else
             scale = planes::superblock<QT, MXC, false, RAG>(bs, b0, b1, sS[cw], xp, plane_sbs * planes::kSbBytes, sXs + psb, plane_sbs, sX + psb * sums_per_sb,
                                                             plane_sbs * sums_per_sb, blocks, lane, ires, xt);
-          if (__any_sync(0xffffffffu, scale == 0.f)) {
+          if (__builtin_expect(__any_sync(0xffffffffu, scale == 0.f), 0)) {
             const float2 rest = planes::plain<QT, T, MXC>(b0, b1, x + int64_t(MXC == 2 ? t >> 1 : 0) * k + sb * 256, min(256, k - sb * 256), scale == 0.f, t);
             ires[0] += rest.x;
             ires[1] += rest.y;

@@ -49,10 +49,6 @@ __device__ __forceinline__ void split16(const exact::Unit<QT, 4>& unit, int i, f
     // unless its weights are all zero, and the results of the row are computed again.
     using V = typename Pair<O>::V;
     constexpr bool kHalf = std::is_same<O, __half>::value;
-    if constexpr (split_checks_scale<QT, O>()) {
-      if (scale != 0.f && !(scale >= 0x1p-24f && scale <= 0x1p10f))
-        scale = ((unit.w[i][0] | unit.w[i][1] | unit.w[i][2] | unit.w[i][3]) >> (4 * unit.u)) & 0x07070707u ? NAN : 0.f;
-    }
     const V s1 = Pair<O>::splat(kHalf ? 32.f * scale : scale), off = Pair<O>::splat(kHalf ? 32.f + float(kOff) / 32.f : 128.f + float(kOff));
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
@@ -61,6 +57,13 @@ __device__ __forceinline__ void split16(const exact::Unit<QT, 4>& unit, int i, f
       for (int e = 0; e < 2; ++e) {
         const uint32_t magic = __byte_perm(w, kHalf ? 0x50505050u : 0x43434343u, e == 0 ? 0x4140 : 0x4342);
         term[0][q][2 * k + e] = as_u32<V>(__hmul2(__hsub2(as_pair<V>(magic), off), s1));
+      }
+    }
+    if constexpr (split_checks_scale<QT, O>()) {
+      if (__builtin_expect(scale != 0.f && !(scale >= 0x1p-24f && scale <= 0x1p10f), 0)) {
+        const uint32_t fill = ((unit.w[i][0] | unit.w[i][1] | unit.w[i][2] | unit.w[i][3]) >> (4 * unit.u)) & 0x07070707u ? 0x7fff7fffu : 0u;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) term[0][q][k] = fill;
       }
     }
   } else if constexpr (TERMS == 2 && std::is_same<O, __half>::value && !exact::has_mins<QT>()) {
@@ -191,6 +194,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       return warp_poll(epibar, epi_phase++ & 1u, ST_ACC_TIMEOUT);
     };
     bool dep_waited = false;
+    float check = 0.f;                              // NaN once one of this thread's results is not finite
     auto epilogue = [&](int t, int sb_b, int sb_e, int segi) -> bool {
       if (!dep_waited) {
         asm volatile("griddepcontrol.wait;\n" ::: "memory");
@@ -214,7 +218,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
         if (!producer_sync()) return false;
       }
       const float bias_v = (finishes && p.bias != nullptr && n_row < p.n) ? MmaType<T>::to_float(static_cast<const T*>(p.bias)[n_row]) : 0.f;
-      float check = 0.f;                            // NaN once a result is not finite
       for (int col = (warp >> 2) * 16; col < p.bn; col += 64) {
         uint32_t r[16];
         tmem_ld16(tmem_base + lanes + uint32_t(col), r);
@@ -242,10 +245,6 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
           }
         }
       }
-      if (kRedo && check != 0.f && n_row < p.n)
-        for (int col = (warp >> 2) * 16; col < min(p.bn, p.m - m0); col += 64)
-          redo<QT, T, false>(static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row, p.n, x + int64_t(m0 + col) * p.k, p.k, w + int64_t(n_row) * row_bytes,
-                             bias_v, min(16, p.m - m0 - col), p.k);
       if (!finishes) {
         if (!producer_sync()) return false;
         if (tid == 0) { __threadfence(); st_release(p.flags + cta, 1); }
@@ -306,6 +305,17 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       pend_t = t; pend_b = sb_b; pend_e = sb_e;
     }
     if (alive && pend_t >= 0) epilogue(pend_t, pend_b, pend_e, segi - 1);
+    if (kRedo && check != 0.f)                      // at the end, where nothing else is held: inside the epilogue it cost 2 - 5 % of a launch
+      for (int t = tile_hi; t >= tile_lo; --t) {
+        int sb_b, sb_e;
+        walk.segment(t, sb_b, sb_e);
+        const int n_row = (t / p.m_tiles) * kRowsW + row, m0 = (t % p.m_tiles) * p.bn;
+        if (sb_e != nsb || n_row >= p.n) continue;
+        const float bias_v = p.bias != nullptr ? MmaType<T>::to_float(static_cast<const T*>(p.bias)[n_row]) : 0.f;
+        for (int col = (warp >> 2) * 16; col < min(p.bn, p.m - m0); col += 64)
+          redo<QT, T, false>(static_cast<T*>(p.out) + int64_t(m0 + col) * p.n + n_row, p.n, x + int64_t(m0 + col) * p.k, p.k, w + int64_t(n_row) * row_bytes,
+                             bias_v, min(16, p.m - m0 - col), p.k);
+      }
   } else if (warp == 16) {
     // ------------------------------------------------------------------ activation TMA
     asm volatile("griddepcontrol.wait;\n" ::: "memory");
