@@ -1,5 +1,8 @@
 // Host side of the tcgen05 prefill GEMM: per-(device, stream) scratch, the stream-K plan, the allocation-free scratch and the
 // entry that checks a problem and hands it to the weight type's translation unit.  The kernel is in umma_gemm.cuh.
+#include <array>
+#include <cmath>
+#include <map>
 #include <mutex>
 
 #include "umma_gemm.cuh"
@@ -37,31 +40,119 @@ static UmmaScratch* device_state(size_t need_workspace, cudaStream_t stream) {
   return &st;
 }
 
-static Plan plan_for(int m, int n, int k, int bm) {
+static int current_sm_count() {
+  int sm_count = 148, dev = 0;
+  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+  return sm_count;
+}
+
+// Clusters of `size` CTAs that the current device runs at once, with one or two CTAs per SM: fewer than the SMs alone would give, since
+// a cluster stays within a GPC (B200, one CTA per SM: 33 clusters of four, 15 of eight).  Asked once per device.
+__global__ void __launch_bounds__(16 * 32 + 96, 1) footprint_of_one() {}
+__global__ void __launch_bounds__(8 * 32 + 96, 2) footprint_of_two() {}
+static int max_clusters(int size, int ctas_per_sm) {
+  static std::mutex mutex;
+  static std::map<int, std::array<int, 18>> table;                 // by device: [9 * (ctas_per_sm - 1) + size], -1 = not asked yet
+  int dev = 0;
+  if (size < 1 || size > 8 || cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mutex);
+  auto at = table.find(dev);
+  if (at == table.end()) {
+    at = table.emplace(dev, std::array<int, 18>()).first;
+    at->second.fill(-1);
+  }
+  int& known = at->second[9 * (ctas_per_sm - 1) + size];
+  if (known < 0) {
+    const bool two = ctas_per_sm == 2;
+    void (*kern)() = two ? footprint_of_two : footprint_of_one;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(size) * 1024);
+    cfg.blockDim = dim3(two ? 8 * 32 + 96 : 16 * 32 + 96);
+    cfg.dynamicSmemBytes = two ? kSmemHalf : kSmemBudget;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = unsigned(size);
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int clusters = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cfg.dynamicSmemBytes)) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();
+      clusters = 0;
+    }
+    known = clusters;
+  }
+  return known;
+}
+
+// ctas_per_sm: of the kernel that runs tiles of this height; pairs (bm = 256) are half as many workers.  most_slices: of K, in a cluster.
+static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slices) {
   Plan pl;
+  pl.ctas_per_sm = ctas_per_sm;
+  const int wide = bm == 256 ? 2 : 1;
   pl.bm = bm;
   pl.m_tiles = (m + pl.bm - 1) / pl.bm;
-  // The M rows in equal tiles of a multiple of 16: M = 333 is two tiles of 176 rows, not 256 + 77 padded to 512 (the MMA time and
-  // the activation bytes go with the rows of a tile).
-  pl.bn = ((m + pl.m_tiles - 1) / pl.m_tiles + 15) / 16 * 16;
-  const long long tiles = static_cast<long long>(pl.m_tiles) * ((n + kRowsW - 1) / kRowsW);
+  // The M rows in equal tiles of a multiple of 16 (pairs: 32): M = 333 is two tiles of 192 rows, not 256 + 77 padded to 512 (the MMA
+  // time and the activation bytes go with the rows of a tile).
+  pl.bn = ((m + pl.m_tiles - 1) / pl.m_tiles + 16 * wide - 1) / (16 * wide) * (16 * wide);
+  const long long tiles = static_cast<long long>(pl.m_tiles) * ((n + wide * kRowsW - 1) / (wide * kRowsW));
   const int nsb = (k + 255) / 256;
   pl.units = tiles * nsb;
-  int sm_count = 148;
-  int dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  if (sm_count > kMaxCtas) sm_count = kMaxCtas;
-  // at least four super-blocks per CTA: a small problem is not cut into more pieces than its finishers can add up quickly
+  const int sm_count = current_sm_count();
+  int slots = sm_count * ctas_per_sm / wide;
+  if (slots * wide > kMaxCtas) slots = kMaxCtas / wide;
+  if (slots < 1) slots = 1;
+  // Three ways to cut the work, compared by their time in super-blocks:
+  //   * whole tiles, one per worker, or K slices of them in clusters whose sums meet in shared memory, where all of them run at once: a CTA's own
+  //     super-blocks, more of them where another CTA shares its SM, and the join;
+  //   * stream-K: an equal share of all units, and the hand-over of cut tiles through the L2, which grows with the rows of a tile.
+  // us, [4096 x 4096] Q4_K, M = 16: slices 2 / 4 / 8 9.2 / 7.1 / 8.2, stream-K 10.6; [4096 x 14336] 26.2 / 19.4 / 15.1, stream-K 17.6;
+  // [11008 x 4096] 2 / 3 13.0 / 12.6, stream-K 14.5; M = 64, [32768 x 4096]: whole 26.8, stream-K 29.7; [20480 x 4096] 25.8 / 23.1; M = 200,
+  // [11008 x 4096]: whole 24.8, stream-K 27.8; [1024 x 4096] 2 / 3 / 4 16.0 / 13.9 / 12.4, whole 21.7, stream-K 18.9.
+  // (stream-K: at least four super-blocks per worker, a small problem is not cut into more pieces than its finishers can add up quickly.)
   const long long most = pl.units / 4 > 1 ? pl.units / 4 : 1;
-  pl.ctas = int(most < sm_count ? most : sm_count);
-  pl.workspace_bytes = tiles % pl.ctas == 0 ? 0 : size_t(pl.ctas) * pl.bm * kRowsW * sizeof(float);
+  pl.workers = int(most < slots ? most : slots);
+  const float join = wide == 2 ? 1.f : 0.f, each = wide == 2 ? 0.7f : 0.3f;
+  const float hand_over = (wide == 2 ? 9.f : ctas_per_sm == 1 ? 7.f : 3.f + float(pl.bn) / 16.f) + 0.4f * float(pl.workers) / float(tiles);
+  float best = float(pl.units * wide) / float(sm_count) + hand_over;
+  pl.slices = 0;                                                     // stream-K
+  for (int s = 1; s <= most_slices && s <= nsb && tiles <= max_clusters(s * wide, ctas_per_sm); ++s) {
+    const float load = float(tiles * s * wide) / float(sm_count), own = float(nsb) / float(s);
+    const float share = load <= 1.f ? 1.f : s == 1 ? 1.75f : fminf(1.75f, sqrtf(load * sqrtf(load)) + own / 64.f);
+    const float cost = 0.5f * (float((nsb + s - 1) / s) + own) * share + (s > 1 ? join + each * float(s) : 0.f);
+    if (cost < best) { pl.slices = s; best = cost; }
+  }
+  if (pl.slices > 0) {
+    pl.workers = int(tiles);
+    pl.shared = (nsb + pl.slices - 1) / pl.slices <= 12;
+    pl.workspace_bytes = 0;
+    return pl;
+  }
+  pl.slices = 1;
+  pl.shared = pl.units <= 12ll * pl.workers;
+  pl.workspace_bytes = tiles % pl.workers == 0 ? 0 : size_t(pl.workers) * wide * pl.bn * kRowsW * sizeof(float);
   return pl;
 }
 
-static Plan make_plan(int m, int n, int k) { return plan_for(m, n, k, m <= 64 ? 64 : m <= 128 ? 128 : 256); }
+static int tile_height(int m) { return m <= 64 ? 64 : m <= 128 ? 128 : 256; }
+static Plan make_plan(int qtype, int m, int n, int k) {
+  const int bm = tile_height(m), tiles = (n + kRowsW - 1) / kRowsW, sms = current_sm_count();
+  const bool eight = eight_fit(qtype, bm) && (bm == 64 || (2 * tiles > sms && tiles <= sms && k <= 16 * 256));
+  return plan_for(m, n, k, bm, eight ? 2 : 1, bm == 256 ? 4 : 8);
+}
+// What the built-in scratch takes is decided by this figure: a partial tile of whole height on every SM, where a tile count that the SMs do
+// not divide needs one.
+static size_t nominal_workspace(int m, int n, int k) {
+  const int bm = tile_height(m), nsb = (k + 255) / 256;
+  const long long tiles = static_cast<long long>((m + bm - 1) / bm) * ((n + kRowsW - 1) / kRowsW), most = tiles * nsb / 4;
+  const int sm_count = current_sm_count();
+  const long long ctas = most < 1 ? 1 : most < sm_count ? most : sm_count;
+  return tiles % ctas == 0 ? 0 : size_t(ctas) * bm * kRowsW * sizeof(float);
+}
 
 // For the split-operand kernels (umma_split.cu): the same plan at their tile height, the same scratch.
-Plan split_plan(int m, int n, int k, int bm) { return plan_for(m, n, k, bm); }
+Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced) { return plan_for(m, n, k, bm, ctas_per_sm, !sliced ? 1 : bm == 256 ? 4 : 8); }
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc) {
   UmmaScratch* st = device_state(workspace_bytes, stream);
   if (st == nullptr) return RC_LAUNCH;
@@ -106,10 +197,15 @@ static int static_scratch(Scratch* out) {
 
 static int launch_bm(int qtype, int dtype, const void* a, const void* b, const void* bias, void* c, int m, int n, int k, bool use_static,
                      const PeerOut& peers, cudaStream_t s) {
-  const Plan pl = make_plan(m, n, k);
+  Plan pl = make_plan(qtype, m, n, k);
   Scratch sc{nullptr, nullptr, nullptr};
   if (use_static) {
-    if (pl.workspace_bytes > kStaticScratchBytes) return RC_RANGE;
+    if (nominal_workspace(m, n, k) > kStaticScratchBytes) return RC_RANGE;
+    if (pl.workspace_bytes > kStaticScratchBytes) {       // fewer workers, so that their partial tiles fit
+      const size_t each = pl.workspace_bytes / pl.workers;
+      pl.workers = int(kStaticScratchBytes / each);
+      pl.workspace_bytes = pl.workers * each;
+    }
     if (int rc = static_scratch(&sc)) return rc;
   } else {
     UmmaScratch* st = device_state(pl.workspace_bytes, s);
@@ -162,7 +258,8 @@ bool gemm_umma_supports(int qtype, int dtype, int m, int n, int k) {
 
 size_t gemm_umma_workspace(int qtype, int dtype, int m, int n, int k) {
   if (!gemm_umma_supports(qtype, dtype, m, n, k)) return 0;
-  return umma::make_plan(m, n, k).workspace_bytes;
+  const size_t need = umma::make_plan(qtype, m, n, k).workspace_bytes, nominal = umma::nominal_workspace(m, n, k);
+  return need > nominal ? need : nominal;
 }
 
 static int gemm_rcr_umma_impl(const void* a, const void* b, const void* bias, void* c, int qtype, int dtype, int m, int n, int k,

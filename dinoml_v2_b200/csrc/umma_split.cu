@@ -4,15 +4,19 @@
 namespace b200gguf {
 namespace umma {
 
-Plan split_plan(int m, int n, int k, int bm);                                                             // umma_gemm.cu
+Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced);                                            // umma_gemm.cu
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc);
 
-template <int QT, typename T>
-static int run(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
-  const Plan pl = split_plan(m, n, k, split_bm<QT, T>());
+template <int QT, typename T, int BM>
+static int run_bm(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
+  const Plan pl = split_plan(m, n, k, BM, SplitGeo<QT, T, BM>::Of::kCtasPerSm, SplitGeo<QT, T, BM>::Of::SLICED);
   Scratch sc;
   if (int rc = split_state(pl.workspace_bytes, s, &sc)) return rc;
-  return launch_split<QT, T>(a, b, bias, c, m, n, k, pl, sc, s);
+  return launch_split<QT, T, BM>(a, b, bias, c, m, n, k, pl, sc, s);
+}
+template <int QT, typename T>
+static int run(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
+  return m <= 64 ? run_bm<QT, T, 64>(a, b, bias, c, m, n, k, s) : m <= 128 ? run_bm<QT, T, 128>(a, b, bias, c, m, n, k, s) : run_bm<QT, T, 256>(a, b, bias, c, m, n, k, s);
 }
 
 }  // namespace umma
