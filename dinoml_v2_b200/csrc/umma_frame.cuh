@@ -267,6 +267,7 @@ inline cudaError_t launch_frame(Kernel kern, int workers, int slices, cudaStream
   attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = S::PAIR || slices > 1 ? 2 : 1;
+  if ((S::PAIR ? 2 : 1) * slices > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return cudaErrorInvalidConfiguration;
   return cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
@@ -418,7 +419,7 @@ template <class S> struct Cta {
     for (int t = tile_hi; t >= tile_lo && ok; --t) {
       int sb_b, sb_e;
       walk.segment(t, sb_b, sb_e);
-      const int m0 = (t % p.m_tiles) * p.bn + (S::PAIR ? rank * (p.bn >> 1) : 0);
+      const int m0 = (t % p.m_tiles) * p.bn + (S::PAIR ? rank * (tile_rows(t) >> 1) : 0);
       for (int st = sb_b * kStagesPerSb; st < sb_e * kStagesPerSb && ok; st += S::HS) {
         if (!wait(empty(u.at), u.phase ^ 1u, ST_EMPTY_TIMEOUT)) { ok = false; break; }
         if (elect_one()) {
@@ -443,7 +444,7 @@ template <class S> struct Cta {
   __device__ __forceinline__ void issue_mmas() const {
     if (S::PAIR && rank != 0) return;
     constexpr uint32_t kFormat = Pair<T>::kFormat;
-    const uint32_t idesc = (1u << 4) | (kFormat << 7) | (kFormat << 10) | (uint32_t(p.bn >> 3) << 17) | (uint32_t((S::PAIR ? 2 : 1) * kRowsW >> 4) << 24);
+    const uint32_t idesc0 = (1u << 4) | (kFormat << 7) | (kFormat << 10) | (uint32_t((S::PAIR ? 2 : 1) * kRowsW >> 4) << 24);
     const uint64_t db0 = smem_desc_sw128(smem_u32(xtiles));
     const uint16_t both = uint16_t(3u << lead);                  // the CTAs of the pair
     Ring u{0, 0u};
@@ -458,6 +459,7 @@ template <class S> struct Cta {
         tcgen05_fence_after();
       }
       uint32_t accumulate = 0;
+      const uint32_t idesc = idesc0 | (uint32_t(tile_rows(t) >> 3) << 17);
       for (int h = (sb_e - sb_b) * S::kUnits; h > 0; --h) {       // one wait, 4 HS TERMS MMAs, one commit per unit
         ok = wait(full(u.at), u.phase, ST_FULL_TIMEOUT);
         if (!ok) break;
@@ -515,6 +517,11 @@ template <class S> struct Cta {
     if (*abort_flag) {
       for (int i = max(0, issued - S::NRAW); i < issued; ++i) mbar_wait_plain(rawfull(i % S::NRAW), uint32_t(i / S::NRAW) & 1u);
     }
+  }
+  // Activation rows of tile t that the MMAs multiply: the last tile of a panel has fewer where its rows end before it does (M = 333: 192 and 160).
+  __device__ __forceinline__ int tile_rows(int t) const {
+    if (!S::PAIR) return p.bn;
+    return min(p.bn, (p.m - (t % p.m_tiles) * p.bn + 31) & ~31);
   }
   __device__ __forceinline__ int row0(int t) const { return ((t / p.m_tiles) * (S::PAIR ? 2 : 1) + rank) * kRowsW; }      // of this CTA's part of tile t
 
@@ -648,7 +655,8 @@ template <class S> struct Cta {
     return true;
   }
   // ... and that of all threads of the cluster: four rows of a column at a time, so that few trips to the other CTAs' memory follow one
-  // another (a row at a time: [4096 x 4096], M = 64, 10.2 us instead of 9.2; several columns at a time spill registers).
+  // another (a row at a time: [4096 x 4096], M = 64, 10.2 us instead of 9.2; several columns at a time spill registers; sums pushed to the CTA that
+  // finishes them, by remote stores and a barrier or by st.async: [1024 x 4096], M = 16, 5.0 -> 5.8, [4096 x 4096], M = 512, 21.1 -> 22.7 and 24.7).
   template <bool GATED, bool SCATTER, typename Seen>
   __device__ __forceinline__ void join_slices(Seen seen_sum) {
     using P = Pair<T>;

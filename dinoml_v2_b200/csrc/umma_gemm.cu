@@ -50,18 +50,19 @@ static int current_sm_count() {
 // a cluster stays within a GPC (B200, one CTA per SM: 33 clusters of four, 15 of eight).  Asked once per device.
 __global__ void __launch_bounds__(16 * 32 + 96, 1) footprint_of_one() {}
 __global__ void __launch_bounds__(8 * 32 + 96, 2) footprint_of_two() {}
+constexpr int kMostSlices = 16;                                   // CTAs of a cluster: sixteen where the weight has so few tiles that enough clusters fit
 static int max_clusters(int size, int ctas_per_sm) {
   static std::mutex mutex;
-  static std::map<int, std::array<int, 18>> table;                 // by device: [9 * (ctas_per_sm - 1) + size], -1 = not asked yet
+  static std::map<int, std::array<int, 34>> table;                 // by device: [17 * (ctas_per_sm - 1) + size], -1 = not asked yet
   int dev = 0;
-  if (size < 1 || size > 8 || cudaGetDevice(&dev) != cudaSuccess) return 0;
+  if (size < 1 || size > 16 || cudaGetDevice(&dev) != cudaSuccess) return 0;
   std::lock_guard<std::mutex> lock(mutex);
   auto at = table.find(dev);
   if (at == table.end()) {
-    at = table.emplace(dev, std::array<int, 18>()).first;
+    at = table.emplace(dev, std::array<int, 34>()).first;
     at->second.fill(-1);
   }
-  int& known = at->second[9 * (ctas_per_sm - 1) + size];
+  int& known = at->second[17 * (ctas_per_sm - 1) + size];
   if (known < 0) {
     const bool two = ctas_per_sm == 2;
     void (*kern)() = two ? footprint_of_two : footprint_of_one;
@@ -77,6 +78,7 @@ static int max_clusters(int size, int ctas_per_sm) {
     cfg.numAttrs = 1;
     int clusters = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cfg.dynamicSmemBytes)) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
       cudaGetLastError();
       clusters = 0;
@@ -86,8 +88,9 @@ static int max_clusters(int size, int ctas_per_sm) {
   return known;
 }
 
-// ctas_per_sm: of the kernel that runs tiles of this height; pairs (bm = 256) are half as many workers.  most_slices: of K, in a cluster.
-static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slices) {
+// ctas_per_sm: of the kernel that runs tiles of this height; pairs (bm = 256) are half as many workers.  most_slices: of K, in a cluster.  terms:
+// of a weight, a super-block takes that much longer.
+static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slices, int terms) {
   Plan pl;
   pl.ctas_per_sm = ctas_per_sm;
   const int wide = bm == 256 ? 2 : 1;
@@ -113,8 +116,8 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
   // (stream-K: at least four super-blocks per worker, a small problem is not cut into more pieces than its finishers can add up quickly.)
   const long long most = pl.units / 4 > 1 ? pl.units / 4 : 1;
   pl.workers = int(most < slots ? most : slots);
-  const float join = wide == 2 ? 1.f : 0.f, each = wide == 2 ? 0.7f : 0.3f;
-  const float hand_over = (wide == 2 ? 9.f : ctas_per_sm == 1 ? 7.f : 3.f + float(pl.bn) / 16.f) + 0.4f * float(pl.workers) / float(tiles);
+  const float join = (wide == 2 ? 1.f : 0.f) / float(terms), each = (wide == 2 ? 0.7f : 0.3f) / float(terms);
+  const float hand_over = ((wide == 2 ? 9.f : ctas_per_sm == 1 ? 7.f : 3.f + float(pl.bn) / 16.f) + 0.4f * float(pl.workers) / float(tiles)) / float(terms);
   float best = float(pl.units * wide) / float(sm_count) + hand_over;
   pl.slices = 0;                                                     // stream-K
   for (int s = 1; s <= most_slices && s <= nsb && tiles <= max_clusters(s * wide, ctas_per_sm); ++s) {
@@ -139,7 +142,7 @@ static int tile_height(int m) { return m <= 64 ? 64 : m <= 128 ? 128 : 256; }
 static Plan make_plan(int qtype, int m, int n, int k) {
   const int bm = tile_height(m), tiles = (n + kRowsW - 1) / kRowsW, sms = current_sm_count();
   const bool eight = eight_fit(qtype, bm) && (bm == 64 || (2 * tiles > sms && tiles <= sms && k <= 16 * 256));
-  return plan_for(m, n, k, bm, eight ? 2 : 1, bm == 256 ? 4 : 8);
+  return plan_for(m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), 1);
 }
 // What the built-in scratch takes is decided by this figure: a partial tile of whole height on every SM, where a tile count that the SMs do
 // not divide needs one.
@@ -152,7 +155,9 @@ static size_t nominal_workspace(int m, int n, int k) {
 }
 
 // For the split-operand kernels (umma_split.cu): the same plan at their tile height, the same scratch.
-Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced) { return plan_for(m, n, k, bm, ctas_per_sm, !sliced ? 1 : bm == 256 ? 4 : 8); }
+Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms) {
+  return plan_for(m, n, k, bm, ctas_per_sm, !sliced ? 1 : kMostSlices / (bm == 256 ? 2 : 1), terms);
+}
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc) {
   UmmaScratch* st = device_state(workspace_bytes, stream);
   if (st == nullptr) return RC_LAUNCH;

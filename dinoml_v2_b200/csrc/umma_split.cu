@@ -4,12 +4,12 @@
 namespace b200gguf {
 namespace umma {
 
-Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced);                                            // umma_gemm.cu
+Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms);                                          // umma_gemm.cu
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc);
 
 template <int QT, typename T, int BM>
 static int run_bm(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
-  const Plan pl = split_plan(m, n, k, BM, SplitGeo<QT, T, BM>::Of::kCtasPerSm, SplitGeo<QT, T, BM>::Of::SLICED);
+  const Plan pl = split_plan(m, n, k, BM, SplitGeo<QT, T, BM>::Of::kCtasPerSm, SplitGeo<QT, T, BM>::Of::SLICED, SplitGeo<QT, T, BM>::kTerms);
   Scratch sc;
   if (int rc = split_state(pl.workspace_bytes, s, &sc)) return rc;
   return launch_split<QT, T, BM>(a, b, bias, c, m, n, k, pl, sc, s);

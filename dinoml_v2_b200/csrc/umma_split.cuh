@@ -32,16 +32,24 @@ template <int QT, typename T> constexpr int split_terms() {
 }
 // Whether a scale may be one that the type of the operands does not hold.
 template <int QT, typename T> constexpr bool split_checks_scale() { return QT == QTYPE_MXFP4 && std::is_same<T, __half>::value; }
-// Rings of a tile height.  A hand-over unit is half a super-block with one term, a K stage with more.
+// Types whose stages share packed bytes.
+template <int QT> constexpr bool shares_bytes() { return QT == QTYPE_Q6_K || QT == QTYPE_Q2_K || QT == QTYPE_Q3_K; }
+// Rings of a tile height.  A hand-over unit is half a super-block with one term, a K stage with more.  Two CTAs share an SM up to 64 activation
+// rows with one or two terms (128 with one); three terms would leave each of them two stages, and the words of types that share bytes between
+// stages do not fit beside two terms.  What a producer thread takes of a super-block:
+//   kHalf: eight producer warps, (row, half), the two stages of half a super-block one after the other;
+//   kRun: sixteen, types that share bytes, (row, half, run): 16 weights of every 32 of a half;
+//   kStage: sixteen, the others, (row, half, stage);
+//   else (three terms beside 256 columns of sums) the ring is shorter than a super-block: eight warps take one stage of both halves each.
 template <int QT, typename T, int BM> struct SplitGeo {
   static constexpr int kTerms = split_terms<QT, T>(), HS = kTerms == 1 ? 2 : 1;
   static constexpr bool kPair = BM == 256;
+  static constexpr int PW = !kPair && kTerms * BM <= 128 && !shares_bytes<QT>() ? 8 : 16;
   static constexpr int kPart = kRowsW * exact::raw_pitch<QT>(), kUnit = HS * (kPair ? BM / 2 : BM) * kBK * 2, kRest = 1024 + 512;
-  static constexpr int kHalfUnits = (256 - BM) / (HS * kTerms * kWSlotCols), kFullUnits = (512 - BM) / (HS * kTerms * kWSlotCols);
-  static constexpr int PW = !kPair && kHalfUnits >= 2 && kRest + kHalfUnits * kUnit + 2 * kPart <= kSmemHalf ? 8 : 16;
-  static constexpr int NB = PW == 8 ? kHalfUnits : kFullUnits < 4 ? kFullUnits : 4;
+  static constexpr int kColumns = (PW == 8 ? 256 : 512) - BM, kMost = kColumns / (HS * kTerms * kWSlotCols), NB = kMost < 6 ? kMost : 6;
   static constexpr int kFit = ((PW == 8 ? kSmemHalf : kSmemBudget) - kRest - NB * kUnit) / kPart, NRAW = kFit < 4 ? kFit : 4;
-  using Of = Shape<T, BM, PW, kPair, kTerms, HS, NB, NRAW, kPart, PW, 8, BM * kRowsW * 4 <= NB * kUnit + NRAW * kPart>;
+  static constexpr bool kHalf = PW == 8, kLong = NB >= kStagesPerSb / HS, kRun = !kHalf && kLong && shares_bytes<QT>(), kStage = !kHalf && kLong && !kRun;
+  using Of = Shape<T, BM, PW, kPair, kTerms, HS, NB, NRAW, kPart, PW, kHalf || (kStage && HS == 1) ? 4 : 8, BM * kRowsW * 4 <= NB * kUnit + NRAW * kPart>;
 };
 
 // Group i of a unit -> its dequantized weights as TERMS 16-bit numbers each (term[.][..]).
@@ -119,7 +127,8 @@ template <int QT, typename T, int BM>
 __global__ void __launch_bounds__(SplitGeo<QT, T, BM>::Of::kThreads, SplitGeo<QT, T, BM>::Of::kCtasPerSm)
 gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap w_tail_map,
                   const T* __restrict__ x, const uint8_t* __restrict__ w, int residues, const __grid_constant__ Params p) {
-  using S = typename SplitGeo<QT, T, BM>::Of;
+  using G = SplitGeo<QT, T, BM>;
+  using S = typename G::Of;
   constexpr int PW = S::PW, TERMS = S::TERMS, HS = S::HS, kPitch = exact::raw_pitch<QT>(), kSbBytes = exact::sb_bytes<QT>();
   constexpr bool kRedo = TERMS > 1 || split_checks_scale<QT, T>();
   extern __shared__ uint8_t smem_raw[];
@@ -131,77 +140,121 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   auto seen = [&](float v) { if constexpr (kRedo) check = fmaf(0.f, v, check); };
 
   if (warp < PW) {
-    // ------------------------------------------------------------------ producers (roles as in gemm_umma_kernel)
-    const int row = 32 * (warp & 3) + lane, lhalf = (warp >> 2) & 1;
+    // ------------------------------------------------------------------ producers
+    const int row = 32 * (warp & 3) + lane, sub = (warp >> 2) & 1, team = warp >> 3;
     const uint32_t tmem_a = cta.tmem_base + (uint32_t(32 * (warp & 3)) << 16) + uint32_t(BM);
     const int my_row = ((row & (residues - 1)) * rows_per_box + row / residues) * kPitch;      // in a raw slot: by residue
     bool alive = true;
     int segi = 0, pend_t = -1, pend_b = 0, pend_e = 0;
-    // Sixteen warps: the first eight take one half of the super-block and the others the other half - or, where the ring is shorter than a
-    // super-block, one stage of both halves each: a slot must belong to the same warps on every lap, or a wait for it could take the lap
-    // before for the one it means.
-    constexpr bool kStagewise = S::kJobs == 1 && S::NB < S::kUnits;
-    static_assert(!kStagewise || (HS == 1 && S::NB == 2), "two groups of warps, two slots");
-    static_assert((kStagewise || S::kJobs == 2 ? 2 / (kStagewise ? 1 : HS) : S::kUnits) <= S::NB, "the units of a round fit into the ring");
-    constexpr int kRounds = kStagewise ? 2 : S::kJobs, kGroups = kStagewise ? 2 : 4;      // halves a warp visits, 32-weight groups it takes of each
-    const int first = S::kJobs == 1 ? warp >> 3 : 0, j0 = kStagewise ? 2 * first : 0;
+    // A warp's units are at most NB apart (a wait for a slot could otherwise take the lap before for the one it means), and before the
+    // epilogue of the segment before it stores none that only the MMAs after that epilogue set free.
+    constexpr bool kHalf = G::kHalf, kStage = G::kStage, kRun = G::kRun;
+    constexpr int kStep = kRun || (kHalf && HS == 1) ? 3 : kStage ? S::kUnits : 2;      // from the warp's last unit of a super-block (else: half) to its next one
+    static_assert(kStep <= S::NB, "laps");
+    const int half = kHalf ? sub : team, stage = kHalf ? 0 : sub;
     typename Cta<S>::Ring raw{0, 0u}, unit{0, 0u};
-    unit.step(kStagewise ? first : first * (2 / HS), S::NB);
+    unit.step(kHalf || kRun ? half * (2 / HS) : kStage ? (HS == 2 ? half : 2 * half + stage) : team, S::NB);
+    static_assert(!kRun || HS == 1, "types that share bytes have two terms at least");
+    using Words = exact::Unit<QT, kRun ? 4 : 2>;                       // of a 16-weight run of the stage's two 32-weight groups, or of the half's four
+    auto epilogue_before = [&](bool first_sb) -> bool {
+      if (!first_sb || pend_t < 0) return true;
+      const int t = pend_t;
+      pend_t = -1;
+      return cta.template epilogue<false, false>(t, pend_b, pend_e, segi - 1, seen);
+    };
+    auto slot_free = [&]() -> bool {
+      if (!cta.wait(cta.empty(unit.at), unit.phase ^ 1u, ST_EMPTY_TIMEOUT)) return false;
+      tcgen05_fence_after();
+      return true;
+    };
+    auto signal = [&](int by) {
+      tmem_st_wait();
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) cta.arrive_lead(cta.full(unit.at));
+      unit.step(by, S::NB);
+    };
+    // 16 weights (run u of the 32-weight group j of half hb) to the unit's stage `st`
+    auto unpack = [&](const Words& w, int i, int at, uint32_t (&out)[TERMS][8]) {
+      const bool in = at < p.k;                                        // else past the end of the row
+      split16<QT, T, TERMS>(w, i, in ? w.scale[i] : 0.f, in ? w.mn[i] : 0.f, out);
+    };
+    auto put = [&](int st, int column, const uint32_t (&out)[TERMS][8]) {
+#pragma unroll
+      for (int tm = 0; tm < TERMS; ++tm) tmem_st8(tmem_a + uint32_t(((unit.at * HS + st) * TERMS + tm) * kWSlotCols + column), out[tm]);
+    };
     for (int t = cta.tile_hi; t >= cta.tile_lo && alive; --t, ++segi) {
       int sb_b, sb_e;
       cta.walk.segment(t, sb_b, sb_e);
       const uint8_t* wrow = w + int64_t(min(cta.row0(t) + row, p.n - 1)) * row_bytes;
       for (int sb = sb_b; sb < sb_e && alive; ++sb) {
+        if (!cta.wait(cta.rawfull(raw.at), raw.phase, ST_FULL_TIMEOUT)) { alive = false; break; }
+        const uint8_t* block = cta.raw + raw.at * S::RAW_BYTES + my_row + (reinterpret_cast<uintptr_t>(wrow + int64_t(sb) * kSbBytes) & 15);
+        auto words_read = [&]() {                                      // every lane holds its words: the ring slot may be refilled
+          __syncwarp();
+          if (lane == 0) mbar_arrive(cta.rawfree(raw.at));
+          raw.step(1, S::NRAW);
+        };
+        if constexpr (kRun) {
+          Words words;
+          words.load(block, half, 0, sub);
+          words_read();
+#pragma unroll
+          for (int st = 0; st < 2; ++st) {
+            constexpr int kEarly = TERMS == 2 ? 2 : 1;                 // groups unpacked before their slot is waited for (three terms of two spill)
+            uint32_t out[kEarly][TERMS][8];
+            auto group = [&](int i) { unpack(words, 2 * st + i, sb * 256 + 128 * half + 64 * st + 32 * i + 16 * sub, out[i % kEarly]); };
+#pragma unroll
+            for (int i = 0; i < kEarly; ++i) group(i);
+            if (!slot_free()) { alive = false; break; }
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+              if (i >= kEarly) group(i);
+              put(0, 16 * i + 8 * sub, out[i % kEarly]);
+            }
+            signal(st == 0 ? 1 : kStep);
+            if (st == 0) alive = epilogue_before(sb == sb_b);
+            if (!alive) break;
+          }
+        } else if constexpr (kHalf || kStage) {
+          Words words[2];
+#pragma unroll
+          for (int st = 0; st < (kHalf ? 2 : 1); ++st) {
+            const int mine = kHalf ? st : stage;                       // stage of the half
+            words[0].load(block, half, 2 * mine, 0);
+            words[1].load(block, half, 2 * mine, 1);
+            if (!kHalf || st == 1) words_read();
+#pragma unroll
+            for (int piece = 0; piece < 4; ++piece) {
+              const int i = piece >> 1, u = piece & 1;
+              uint32_t out[TERMS][8];
+              unpack(words[u], i, sb * 256 + 128 * half + 64 * mine + 32 * i + 16 * u, out);
+              if (piece == 0 && (HS == 1 || st == 0) && !slot_free()) { alive = false; break; }
+              put(HS == 2 ? mine : 0, 16 * i + 8 * u, out);
+            }
+            if (!alive) break;
+            if (HS == 1 || !kHalf || st == 1) {
+              signal(kHalf && HS == 1 && st == 0 ? 1 : kStep);
+              if (st == 0 || HS == 2) alive = epilogue_before(sb == sb_b);
+            }
+            if (!alive) break;
+          }
+        } else {
+          // sixteen warps, a ring of two stages: team i takes stage i of either half, thread (row, run) 32 weights of it
 #pragma unroll 1
-        for (int job = 0; job < kRounds; ++job) {
-          const int grp = kRounds == 1 ? first : job;
-          if (job == 0 && !cta.wait(cta.rawfull(raw.at), raw.phase, ST_FULL_TIMEOUT)) { alive = false; break; }
-          const uint8_t* block = cta.raw + raw.at * S::RAW_BYTES + my_row + (reinterpret_cast<uintptr_t>(wrow + int64_t(sb) * kSbBytes) & 15);
-          exact::Unit<QT, kGroups> weights;       // K values 16 lhalf .. and 32 + 16 lhalf .. of this thread's 64-wide stages
-          weights.load(block, grp, j0, lhalf);
-          if (job == kRounds - 1) {
-            __syncwarp();
-            if (lane == 0) mbar_arrive(cta.rawfree(raw.at));              // every lane holds its words: the ring slot may be refilled
-            raw.step(1, S::NRAW);
-          }
-          // One or two terms: a unit is unpacked before its slots are waited for; three would not fit into the registers.
-          constexpr bool kFirst = TERMS < 3;
+          for (int hb = 0; hb < 2 && alive; ++hb) {
+            Words words;
+            words.load(block, hb, 2 * team, sub);
+            if (hb == 1) words_read();
+            if (!slot_free()) { alive = false; break; }
 #pragma unroll
-          for (int h = 0; h < (kStagewise ? 1 : 2 / HS); ++h) {
-            uint32_t term[kFirst ? 2 * HS : 1][TERMS][8];
-            auto unpack = [&](int i, uint32_t (&out)[TERMS][8]) {
-              const bool in = sb * 256 + 128 * grp + 32 * (j0 + i) + 16 * lhalf < p.k;      // else past the end of the row
-              split16<QT, T, TERMS>(weights, i, in ? weights.scale[i] : 0.f, in ? weights.mn[i] : 0.f, out);
-            };
-            auto put = [&](int i, const uint32_t (&out)[TERMS][8]) {                 // i: 32-weight group of the unit
-#pragma unroll
-              for (int tm = 0; tm < TERMS; ++tm)
-                tmem_st8(tmem_a + uint32_t(((unit.at * HS + (i >> 1)) * TERMS + tm) * kWSlotCols + 16 * (i & 1) + 8 * lhalf), out[tm]);
-            };
-            if constexpr (kFirst) {
-#pragma unroll
-              for (int i = 0; i < 2 * HS; ++i) unpack(2 * HS * h + i, term[i]);
+            for (int i = 0; i < 2; ++i) {
+              uint32_t out[TERMS][8];
+              unpack(words, i, sb * 256 + 128 * hb + 64 * team + 32 * i + 16 * sub, out);
+              put(0, 16 * i + 8 * sub, out);
             }
-            if (!cta.wait(cta.empty(unit.at), unit.phase ^ 1u, ST_EMPTY_TIMEOUT)) { alive = false; break; }
-            tcgen05_fence_after();
-#pragma unroll
-            for (int i = 0; i < 2 * HS; ++i) {
-              if constexpr (!kFirst) unpack(2 * HS * h + i, term[0]);
-              put(i, term[kFirst ? i : 0]);
-            }
-            tmem_st_wait();
-            tcgen05_fence_before();
-            __syncwarp();
-            if (lane == 0) cta.arrive_lead(cta.full(unit.at));
-            unit.step(kStagewise ? 2 : 1, S::NB);
-          }
-          if (!alive) break;
-          if constexpr (S::kJobs == 1 && !kStagewise) unit.step(2 / HS, S::NB);        // the other half's units
-          // The previous segment's epilogue, once the stage ring holds the first units of this one: no unit may be waited for that only
-          // the MMAs after that epilogue set free.
-          if (sb == sb_b && pend_t >= 0) {
-            if (!cta.template epilogue<false, false>(pend_t, pend_b, pend_e, segi - 1, seen)) { alive = false; break; }
-            pend_t = -1;
+            signal(kStep);
+            if (hb == 0) alive = epilogue_before(sb == sb_b);
           }
         }
       }
