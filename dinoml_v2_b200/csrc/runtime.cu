@@ -24,7 +24,8 @@
 //                          its launch (the next weight is copied on a second stream while the current one computes);
 //   grouped_offload        the same at the granularity of groups of constants (one group = e.g. one layer).
 // Steady state: dino_session_set_graph_replay(session, 1) makes dino_session_run capture the launch sequence of a
-// (shapes, pointers) combination the second time it sees it and replay the graph from then on.
+// (shapes, pointers) combination the second time it sees it and replay the graph from then on.  Linears of it that do not read one another's
+// results are branches of that graph.
 // DINOML_PROFILE_RUN[_VERBOSE|_SECTIONS] time every launch with events, as src/dinoml/templates/gpu_module.cu.j2:785-983.
 #if defined(__SSE2__)
 #include <immintrin.h>
@@ -36,6 +37,7 @@
 #include <map>
 #include <sstream>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/dinoml_b200_runtime.h"
@@ -155,6 +157,10 @@ struct DinoSession {
   size_t graph_launches = 0;
   size_t graph_generation = 0;
   std::vector<int64_t> pending_key;     // combination of the run in progress; counted as seen once that run has succeeded
+  // replayed runs: linears that do not need one another's results run side by side on these (made when first needed)
+  static constexpr int kSides = 3;
+  cudaStream_t side[kSides] = {};
+  cudaEvent_t forked = nullptr, joined[kSides] = {};
 };
 
 namespace {
@@ -475,9 +481,93 @@ int parse_profile_sections(const char* env, std::vector<ProfileSection>* out) {
   return 0;
 }
 
-// One pass over the plan.  `launch == false` only validates and computes shapes.
+// Which launches of a pass may run side by side: a stream per node, 0 = the session's own.  A node follows the one whose result it reads, the
+// others go where the fewest weight bytes are.  Empty: one after another, because there is nothing to gain (one chain; above 128 rows a
+// launch fills the GPU for long), or because a result is written over another result or an input, whose order counts.
+// A launch of a few microseconds is mostly its start and its tail, and these overlap here: one layer (q, k, v, o, gated pair, down; hidden 4096,
+// 14336 between), M = 1 / 8 / 32 / 128: 50.6 / 73.4 / 69.5 / 110.9 us, one after another 57.1 / 78.8 / 76.2 / 117.
+std::vector<int> side_by_side(const DinoModule& mod, const std::vector<std::vector<int64_t>>& shapes, const std::vector<void*>& ptr) {
+  constexpr int64_t kMostRows = 128;
+  std::vector<int> branch(mod.nodes.size(), 0), writer(mod.tensors.size(), -1);
+  std::vector<int64_t> rows(mod.tensors.size(), 0);
+  std::vector<std::pair<uintptr_t, uintptr_t>> read, written;
+  auto range = [&](int t, int64_t count) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(ptr[t]);
+    return std::make_pair(at, at + size_t(count) * dtype_size(mod.tensors[t].dtype));
+  };
+  for (int t : mod.inputs) {
+    int64_t count = 1;
+    for (int64_t d : shapes[t]) count *= d;
+    rows[t] = shapes[t].empty() || shapes[t].back() == 0 ? 0 : count / shapes[t].back();
+    read.push_back(range(t, count));
+  }
+  size_t load[1 + DinoSession::kSides] = {};
+  bool several = false;
+  for (size_t i = 0; i < mod.nodes.size(); ++i) {
+    const NodeSpec& node = mod.nodes[i];
+    const ConstantSpec& w = mod.constants[node.b];
+    int at = 0;
+    if (writer[node.a] >= 0) at = branch[writer[node.a]];
+    else for (int b = 1; b <= DinoSession::kSides; ++b) if (load[b] < load[at]) at = b;
+    branch[i] = at;
+    several = several || at != 0;
+    load[at] += w.nbytes;
+    if (writer[node.out] >= 0) return {};
+    writer[node.out] = int(i);
+    rows[node.out] = rows[node.a];
+    if (rows[node.out] > kMostRows) return {};
+    written.push_back(range(node.out, rows[node.out] * (w.shape[0] / (node.activation != 0 ? 2 : 1))));
+  }
+  for (size_t i = 0; i < written.size(); ++i) {
+    auto meets = [&](const std::pair<uintptr_t, uintptr_t>& o) { return written[i].first < o.second && o.first < written[i].second; };
+    for (size_t j = 0; j < written.size(); ++j) if (j != i && meets(written[j])) return {};
+    for (const auto& o : read) if (meets(o)) return {};
+  }
+  return several ? branch : std::vector<int>();
+}
+
+bool make_sides(DinoSession* s) {
+  if (s->forked == nullptr && cudaEventCreateWithFlags(&s->forked, cudaEventDisableTiming) != cudaSuccess) return false;
+  for (int i = 0; i < DinoSession::kSides; ++i) {
+    if (s->side[i] == nullptr && cudaStreamCreateWithFlags(&s->side[i], cudaStreamNonBlocking) != cudaSuccess) return false;
+    if (s->joined[i] == nullptr && cudaEventCreateWithFlags(&s->joined[i], cudaEventDisableTiming) != cudaSuccess) return false;
+  }
+  return true;
+}
+
+// The streams of one pass: forked from the session's stream, joined to it again however the pass ends.
+struct Branches {
+  DinoSession* s;
+  std::vector<int> of;                  // per node; empty: all on the session's stream
+  bool used[DinoSession::kSides] = {};
+  int rc = 0;
+  Branches(DinoSession* session, std::vector<int> branch) : s(session), of(std::move(branch)) {
+    if (of.empty()) return;
+    if (!make_sides(s) || cudaEventRecord(s->forked, s->stream) != cudaSuccess) { cudaGetLastError(); of.clear(); return; }
+    for (int b : of)
+      if (b > 0 && !used[b - 1]) {
+        if (cudaStreamWaitEvent(s->side[b - 1], s->forked, 0) != cudaSuccess) { rc = cuda_fail("cudaStreamWaitEvent", cudaGetLastError()); return; }
+        used[b - 1] = true;
+      }
+  }
+  cudaStream_t stream(size_t node) const { return of.empty() || of[node] == 0 ? s->stream : s->side[of[node] - 1]; }
+  int join() {
+    int result = 0;
+    for (int i = 0; i < DinoSession::kSides; ++i)
+      if (used[i]) {
+        used[i] = false;
+        cudaError_t err = cudaEventRecord(s->joined[i], s->side[i]);
+        if (err == cudaSuccess) err = cudaStreamWaitEvent(s->stream, s->joined[i], 0);
+        if (err != cudaSuccess) result = cuda_fail("joining the session's streams", err);
+      }
+    return result;
+  }
+  ~Branches() { join(); }
+};
+
+// One pass over the plan.  `launch == false` only validates and computes shapes.  side: independent launches may run side by side.
 int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs,
-             bool validate) {
+             bool validate, bool side = false) {
   DinoModule& mod = *s->module;
   if (validate) {
     if (num_inputs != mod.inputs.size()) return fail("dino_session_run expected " + std::to_string(mod.inputs.size()) + " inputs");
@@ -512,6 +602,8 @@ int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTe
   for (size_t i = 0; i < num_outputs; ++i) ptr[mod.outputs[i]] = outputs[i].data ? tensor_ptr(outputs[i]) : nullptr;
   for (size_t i = 0; i < mod.tensors.size(); ++i) if (mod.tensors[i].role == 2) ptr[i] = s->temps[i];
 
+  Branches branches(s, side ? side_by_side(mod, s->shapes, ptr) : std::vector<int>());
+  if (branches.rc != 0) return branches.rc;
   for (size_t ni = 0; ni < mod.nodes.size(); ++ni) {
     const NodeSpec& node = mod.nodes[ni];
     ConstantSpec& w = mod.constants[node.b];
@@ -567,9 +659,9 @@ int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTe
     }
     const int rc = node.activation != 0
                        ? b200gguf::dual_gemm_rcr(ptr[node.a], wptr, bias, ptr[node.out], w.qtype, ospec.dtype, int(m), int(n), int(k),
-                                                 node.activation, variant, s->stream)
+                                                 node.activation, variant, branches.stream(ni))
                        : b200gguf::gemm_rcr(ptr[node.a], wptr, bias, ptr[node.out], w.qtype, ospec.dtype, int(m), int(n), int(k),
-                                            variant, s->stream);
+                                            variant, branches.stream(ni));
     if (profile_run) cudaEventRecord(ev1.back(), s->stream);
     for (ProfileSection& sec : sections)
       if (sec.end == launch_index) { cudaEventRecord(sec.e1, s->stream); sec.stopped = true; }
@@ -598,6 +690,7 @@ int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTe
                   ", variant " + std::to_string(variant) + ") failed: " + why);
     }
   }
+  if (int rc = branches.join()) return rc;
   if (profile_run || !sections.empty()) {
     if (profile_run) cudaEventRecord(total1, s->stream);
     if (cudaStreamSynchronize(s->stream) != cudaSuccess) return fail("profile run: stream synchronize failed");
@@ -831,6 +924,16 @@ int dino_session_destroy(DinoSession* session) {
     b200gguf::umma_release_scratch(session->owned_stream);
     cudaStreamDestroy(session->owned_stream);
   }
+  for (int i = 0; i < DinoSession::kSides; ++i) {
+    if (session->side[i] != nullptr) {
+      cudaStreamSynchronize(session->side[i]);
+      b200gguf::stream_release_scratch(session->side[i]);
+      b200gguf::umma_release_scratch(session->side[i]);
+      cudaStreamDestroy(session->side[i]);
+    }
+    if (session->joined[i] != nullptr) cudaEventDestroy(session->joined[i]);
+  }
+  if (session->forked != nullptr) cudaEventDestroy(session->forked);
   for (auto& entry : session->graphs)
     if (entry.second.exec != nullptr) cudaGraphExecDestroy(entry.second.exec);
   for (void* p : session->temps) if (p != nullptr) cudaFree(p);
@@ -877,6 +980,7 @@ int dino_session_get_state_pointer(DinoSession* session, size_t state_index, voi
 int dino_session_set_graph_replay(DinoSession* session, int enabled) {
   if (session == nullptr) return fail("dino_session_set_graph_replay received null pointer");
   session->graph_replay = enabled != 0;
+  if (session->graph_replay && !make_sides(session)) cudaGetLastError();      // else by the first run that needs them
   return 0;
 }
 
@@ -934,7 +1038,7 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
   // seen once, and that run succeeded (every lazily created workspace of the kernels exists): capture this one
   cudaGraph_t graph = nullptr;
   if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); cg.seen = -1; return 0; }
-  const int rc = run_plan(s, inputs, num_inputs, outputs, num_outputs, true);
+  const int rc = run_plan(s, inputs, num_inputs, outputs, num_outputs, true, true);
   const bool ended = cudaStreamEndCapture(s->stream, &graph) == cudaSuccess && graph != nullptr;
   bool ok = rc == 0 && ended && cudaGraphInstantiate(&cg.exec, graph, 0) == cudaSuccess;
   if (graph) cudaGraphDestroy(graph);
@@ -951,6 +1055,13 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
   return 1;
 }
 
+// The ordinary run that comes before a capture takes the same streams, so that the workspaces that the kernels keep for each exist by then; not
+// inside a capture of the caller's, where they could not be made.
+static bool will_be_replayed(DinoSession* s) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return !s->pending_key.empty() && cudaStreamIsCapturing(s->stream, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+}
+
 // A combination counts as seen once a run of it has succeeded the ordinary way.
 static void note_ordinary_run(DinoSession* s) {
   if (s->pending_key.empty()) return;
@@ -965,7 +1076,7 @@ int dino_session_run(DinoSession* session, const DinoTensor* inputs, size_t num_
   session->pending_key.clear();
   if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, &replay_rc)) {
     if (replay_rc != 0) return replay_rc;
-  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true)) {
+  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true, will_be_replayed(session))) {
     return rc;
   } else {
     note_ordinary_run(session);
@@ -992,7 +1103,7 @@ int dino_session_run_staged(DinoSession* session, const void* host_in, void* dev
   session->pending_key.clear();
   if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, &replay_rc)) {
     if (replay_rc != 0) return replay_rc;
-  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true)) {
+  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true, will_be_replayed(session))) {
     return rc;
   } else {
     note_ordinary_run(session);
