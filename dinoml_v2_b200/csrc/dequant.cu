@@ -4,334 +4,346 @@
 // src/dinoml/templates/gpu_module.cu.j2:35-42 and calls from src/dinoml/lowering/ops/gemm.py:745,
 // keeping its name and argument list so the generated launch text links unchanged.
 //
-// HBM-bound and write-dominated (Q4_K -> f32 writes 7.1 bytes per byte read).  Every packed byte is loaded once:
-//   Q4_K: a thread owns 8 quant bytes = the low nibbles (8 weights of sub-block 2g) and the high nibbles (8 weights
-//         of sub-block 2g+1) of one 64-weight group; 16 threads per block, the 16-byte header is one broadcast load;
-//   Q6_K: a thread owns 8 positions l of one 128-weight half: 8 ql bytes, the 8 ql bytes 32 further, 8 qh bytes ->
-//         four runs of 8 weights (one per quad); 8 threads per block;
-//   Q8_0: a thread owns 8 consecutive weights.
-//   the six further types: see dequant_items_kernel below.
-// Decoding uses explicitly rounded fp32 operations (bit-exact), and each run of 8 outputs is one 32-byte (f32) or
-// 16-byte (f16 / bf16) streaming store.  Float outputs (write bound) keep the simpler one-unit-per-thread kernel, which
-// measured faster there (Q4_K -> f32 4.77 vs 4.35 TB/s); 16-bit outputs gain 8 % (Q4_K) to 35 % (Q6_K).
+// HBM-bound and write-dominated (Q4_K -> f32 writes 7.1 bytes per byte read).  One kernel for the nine types and three outputs: an item
+// is R consecutive packed bytes and every run of R weights that they hold, so each packed byte is loaded once and each run is one
+// streaming store of whole 32-byte sectors.  What was measured, [11008 x 4096] in a graph, buffers of more than the L2 in turn, before
+// (one 8-weight unit per thread, or items with 8-weight runs, two per thread) -> now, us:
+//                f16                          f32
+//   Q4_K    20.5 -> 18.6  (6.2 TB/s)    42.7 -> 33.8  (6.1 TB/s)
+//   Q5_K    28.9 -> 19.9                52.1 -> 34.7
+//   Q6_K    25.0 -> 22.0                50.4 -> 35.9
+//   Q8_0    28.7 -> 23.0                45.2 -> 36.8
+//   Q4_0    21.3 -> 19.3                46.9 -> 33.2
+//   Q2_K    18.9 -> 17.6                38.5 -> 32.2
+//   Q3_K    23.5 -> 19.3                48.9 -> 33.3
+//   MXFP4   24.7 -> 19.2                46.2 -> 32.9
+//   NVFP4   24.8 -> 20.5                47.0 -> 32.9
+// and [512 x 2048], where the launch counts: 2.1 - 2.9 -> 1.5 - 1.9 (f16), 2.8 - 4.7 -> 2.0 - 2.5 (f32).  Where it came from:
+//   * a 256-bit store per run: as two 128-bit stores, each half fills its sectors (f32: 43 -> 34);
+//   * four quants decoded at a time: masks and shifts for four bytes at once, then one byte permute (0x4B0000qq is 2^23 + q) and one exact
+//     subtraction per weight instead of shift, mask and conversion (Q5_K 28.9 -> 20.7);
+//   * words for blocks that start at any address, shifted into place, instead of bytes or halves (MXFP4 24.7 -> 19.9);
+//   * programmatic dependent launch, 0.3 - 0.4 us per call: the next kernel's CTAs are let in once a CTA holds its packed bytes.  From the first
+//     instruction on they would fill the SMs that happen to be free, and a small grid ends up uneven (Q2_K [2048 x 4096] 4.7 -> 5.2).
+// Decoding uses explicitly rounded fp32 operations, those of decode8<QT> in its order (bit-exact).
 #include "gguf_common.cuh"
+
+#include <type_traits>
 
 namespace b200gguf {
 
-template <typename T> struct Pack8;
-template <> struct Pack8<float> {
-  static __device__ __forceinline__ void store(float* dst, const float (&w)[8]) {
-    float4* p = reinterpret_cast<float4*>(dst);
-    __stcs(p, make_float4(w[0], w[1], w[2], w[3]));
-    __stcs(p + 1, make_float4(w[4], w[5], w[6], w[7]));
-  }
-};
-template <> struct Pack8<__half> {
-  static __device__ __forceinline__ void store(__half* dst, const float (&w)[8]) {
-    uint4 v;
-    __half2 h;
-    h = __floats2half2_rn(w[0], w[1]); v.x = *reinterpret_cast<uint32_t*>(&h);
-    h = __floats2half2_rn(w[2], w[3]); v.y = *reinterpret_cast<uint32_t*>(&h);
-    h = __floats2half2_rn(w[4], w[5]); v.z = *reinterpret_cast<uint32_t*>(&h);
-    h = __floats2half2_rn(w[6], w[7]); v.w = *reinterpret_cast<uint32_t*>(&h);
-    __stcs(reinterpret_cast<uint4*>(dst), v);
-  }
-};
-template <> struct Pack8<__nv_bfloat16> {
-  static __device__ __forceinline__ void store(__nv_bfloat16* dst, const float (&w)[8]) {
-    uint4 v;
-    __nv_bfloat162 h;
-    h = __floats2bfloat162_rn(w[0], w[1]); v.x = *reinterpret_cast<uint32_t*>(&h);
-    h = __floats2bfloat162_rn(w[2], w[3]); v.y = *reinterpret_cast<uint32_t*>(&h);
-    h = __floats2bfloat162_rn(w[4], w[5]); v.z = *reinterpret_cast<uint32_t*>(&h);
-    h = __floats2bfloat162_rn(w[6], w[7]); v.w = *reinterpret_cast<uint32_t*>(&h);
-    __stcs(reinterpret_cast<uint4*>(dst), v);
-  }
-};
-
 constexpr int kDequantThreads = 256;
-constexpr int kUnitsPerThread = 4;
 
-// Q8_0 and every float output: total_units = rows * n_per_row / 8.  Units are numbered in output order, so unit u
-// covers outputs [8u, 8u+8) and lives in block u / (kBlock/8).
-template <int QT, typename T>
-__global__ void __launch_bounds__(kDequantThreads)
-dequant_rows_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t total_units) {
-  constexpr int kUnitsPerBlock = QTraits<QT>::kBlock / 8;
-  const int64_t base = (int64_t(blockIdx.x) * kUnitsPerThread) * kDequantThreads + threadIdx.x;
-#pragma unroll
-  for (int i = 0; i < kUnitsPerThread; ++i) {
-    const int64_t u = base + int64_t(i) * kDequantThreads;
-    if (u < total_units) {
-      const int64_t blk = u / kUnitsPerBlock;
-      const int kk0 = int(u - blk * kUnitsPerBlock) * 8;
-      float w[8];
-      decode8<QT>(in + blk * QTraits<QT>::kBytes, kk0, w);
-      Pack8<T>::store(out + u * 8, w);
-    }
+// 32 bytes of output of one thread, streaming: one 256-bit store where the output starts at a 32-byte boundary (every run then
+// does), else two of 128 bits.
+__device__ __forceinline__ void store32(void* p, const uint32_t (&v)[8], bool wide) {
+  if (wide) {
+    asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]),
+                 "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
+  } else {
+    __stcs(static_cast<uint4*>(p), make_uint4(v[0], v[1], v[2], v[3]));
+    __stcs(static_cast<uint4*>(p) + 1, make_uint4(v[4], v[5], v[6], v[7]));
   }
 }
 
-// Q4_K: item = (block, 64-weight group g, 8-byte piece p of the group's 32 quant bytes); 16 items per block.
-// Formula per weight: (d * sc) * q - (dmin * m), each product / difference rounded (as decode8<QTYPE_Q4_K>).
-// Bound by the memory system (writes are three quarters of the bytes).  A quant becomes a float by one byte permute (0x4B0000qq is
-// 2^23 + q) and one exact subtraction instead of shift, mask and conversion, and WIDE takes the header and the quants in one load each:
-// [11008 x 4096] -> float16 23.5 -> 22.0 us.  Four items or one per thread, or plain stores: 22.7.
-// WIDE: the packed buffer starts at a 16-byte boundary, so every block (144 B) does; else it is 4-byte aligned.
-template <typename T, bool WIDE>
-__global__ void __launch_bounds__(kDequantThreads)
-dequant_q4k_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t total_items) {
-  const int64_t base = (int64_t(blockIdx.x) * 2) * kDequantThreads + threadIdx.x;
+// N words of packed bytes from p.  A: alignment of p.  1: any address; the aligned words around p are shifted into place, except where
+// `edge` says that such a word holds bytes outside the buffer.  0: any address in shared memory (with four bytes after the last).
+template <int N, int A>
+__device__ __forceinline__ void load_words(const uint8_t* __restrict__ p, bool edge, uint32_t (&v)[N]) {
+  if constexpr (A == 16 && N == 4) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+    v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w;
+  } else if constexpr (A == 16 && N == 2) {
+    const uint2 q = __ldg(reinterpret_cast<const uint2*>(p));
+    v[0] = q.x; v[1] = q.y;
+  } else if constexpr (A == 0) {
+    const int off = int(__cvta_generic_to_shared(p)) & 3;
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - off);
+    uint32_t r[N + 1];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int64_t it = base + int64_t(i) * kDequantThreads;
-    if (it >= total_items) continue;
-    const int64_t blk = it >> 4;
-    const int g = int(it & 15) >> 2, piece = int(it & 3);
-    const uint8_t* b = in + blk * 144;
-    const uint8_t* qb = b + 16 + 32 * g + 8 * piece;
-    uint4 hdr;
-    uint2 q;
-    if constexpr (WIDE) {
-      hdr = __ldg(reinterpret_cast<const uint4*>(b));
-      q = __ldg(reinterpret_cast<const uint2*>(qb));
+    for (int i = 0; i <= N; ++i) r[i] = w[i];
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __funnelshift_r(r[i], r[i + 1], 8 * off);
+  } else if constexpr (A >= 4) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __ldg(reinterpret_cast<const uint32_t*>(p) + i);
+  } else {
+    if (edge) {
+#pragma unroll
+      for (int i = 0; i < N; ++i)
+        v[i] = uint32_t(p[4 * i]) | uint32_t(p[4 * i + 1]) << 8 | uint32_t(p[4 * i + 2]) << 16 | uint32_t(p[4 * i + 3]) << 24;
+      return;
+    }
+    const int off = int(reinterpret_cast<uintptr_t>(p) & 3);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p - off);
+    uint32_t r[N + 1];
+#pragma unroll
+    for (int i = 0; i < N; ++i) r[i] = __ldg(w + i);
+    r[N] = off ? __ldg(w + N) : 0u;
+#pragma unroll
+    for (int i = 0; i < N; ++i) v[i] = __funnelshift_r(r[i], r[i + 1], 8 * off);
+  }
+}
+__device__ __forceinline__ float half_of(uint32_t word, int hi) { return half_bits_to_float(uint16_t(hi ? word >> 16 : word & 0xffffu)); }
+// Four FP4 codes (high nibbles of the bytes zero) -> bytes 12 + twice the value: look-ups of the eight magnitudes, both signs.
+__device__ __forceinline__ uint32_t fp4_biased(uint32_t w) {
+  const uint32_t mag = w & 0x07070707u;
+  const uint32_t sel = __byte_perm(mag | (mag >> 4), 0u, 0x4420);
+  const uint32_t pos = __byte_perm(0x0F0E0D0Cu, 0x18141210u, sel), neg = __byte_perm(0x090A0B0Cu, 0x00040608u, sel);
+  const uint32_t sign = ((w >> 3) & 0x01010101u) * 0xffu;
+  return (pos & ~sign) | (neg & sign);
+}
+
+// Geometry of a type's items (R: weights per run).
+//   Q4_0 / MXFP4: R of a block's 16 bytes: low nibbles = weights 0 .. 15, high nibbles = weights 16 .. 31
+//   Q8_0:         R weights
+//   NVFP4:        one sub-block: low nibbles = its first 8 weights, high nibbles = the other 8
+//   Q4_K / Q5_K:  R of the 32 bytes of a 64-weight group: low nibbles its first half, high nibbles the other; Q5_K: and R bytes of qh
+//   Q6_K:         R of the 32 ql bytes that hold 32-weight quarters `half` and `half` + 2 of a 128-weight half, and R bytes of qh
+//   Q2_K / Q3_K:  R of the 32 bytes of a 128-weight half: bit pairs j = 0..3 are runs 32 apart; Q3_K: and R mask bytes
+template <int QT, int R> struct ItemGeom {
+  static constexpr bool k16 = QT == QTYPE_NVFP4 && R == 16;         // a sub-block's 8 bytes are its 16 weights
+  static constexpr int kRuns = QT == QTYPE_Q8_0 ? 1 : QT == QTYPE_Q6_K ? 2 : (QT == QTYPE_Q2_K || QT == QTYPE_Q3_K) ? 4
+                             : QT == QTYPE_NVFP4 ? 16 / R : 2;
+  static constexpr int kItems = QTraits<QT>::kBlock / (kRuns * R);  // per block
+  // alignment that every block has in a buffer that has it
+  static constexpr int kAlign = (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) ? 16 : (QT == QTYPE_Q2_K || QT == QTYPE_NVFP4) ? 4 : 1;
+  static constexpr int kBias = QT == QTYPE_Q8_0 ? 128 : QT == QTYPE_Q6_K ? 32 : QT == QTYPE_Q4_0 ? 8 : QT == QTYPE_Q3_K ? 4
+                             : (QT == QTYPE_MXFP4 || QT == QTYPE_NVFP4) ? 12 : 0;
+  static constexpr bool kMin = QT == QTYPE_Q4_K || QT == QTYPE_Q5_K || QT == QTYPE_Q2_K;
+};
+
+// Weights per run: 32 bytes of output.  16-bit Q2_K and Q3_K, whose items hold four runs, take 8 (16-byte stores): with 16 a matrix has too
+// few threads (Q2_K [2048 x 4096] 5.4 -> 4.7 us, Q3_K 5.1 -> 4.7; [11008 x 4096] equal).
+template <int QT, typename T> constexpr int run_of() { return sizeof(T) == 4 || QT == QTYPE_Q2_K || QT == QTYPE_Q3_K ? 8 : 16; }
+
+template <int QT, typename T, int A> struct Item {
+  static constexpr int R = run_of<QT, T>(), N = R / 4;
+  using G = ItemGeom<QT, R>;
+  static constexpr int kQ = QT == QTYPE_NVFP4 ? 2 : N;              // words of quants
+  static constexpr bool kHigh = QT == QTYPE_Q5_K || QT == QTYPE_Q6_K || QT == QTYPE_Q3_K;
+  uint32_t q[kQ], h[kHigh ? N : 1], s[4];
+
+  __device__ __forceinline__ void load(const uint8_t* __restrict__ b, int item, bool edge) {
+    if constexpr (QT == QTYPE_Q4_0) {
+      s[0] = uint32_t(b[0]) | uint32_t(b[1]) << 8;
+      load_words<N, A>(b + 2 + R * item, edge, q);
+    } else if constexpr (QT == QTYPE_Q8_0) {
+      s[0] = ld_u16(b);
+      load_words<N, A>(b + 2 + R * item, edge, q);
+    } else if constexpr (QT == QTYPE_MXFP4) {
+      s[0] = b[0];
+      load_words<N, A>(b + 1 + R * item, edge, q);
+    } else if constexpr (QT == QTYPE_NVFP4) {
+      const int sub = G::k16 ? item : item >> (G::kRuns == 2 ? 0 : 1);
+      s[0] = b[sub];
+      load_words<2, A>(b + 4 + 8 * sub, edge, q);
+    } else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) {
+      constexpr int kQs = QT == QTYPE_Q4_K ? 16 : 48, P = 32 / R;
+      load_words<4, A>(b, edge, s);
+      load_words<N, A>(b + kQs + 32 * (item / P) + R * (item % P), edge, q);
+      if constexpr (QT == QTYPE_Q5_K) load_words<N, A>(b + 16 + R * (item % P), edge, h);
     } else {
-      const uint32_t *hw = reinterpret_cast<const uint32_t*>(b), *qp = reinterpret_cast<const uint32_t*>(qb);
-      hdr = make_uint4(__ldg(hw), __ldg(hw + 1), __ldg(hw + 2), __ldg(hw + 3));
-      q = make_uint2(__ldg(qp), __ldg(qp + 1));
-    }
-    const float d = half_bits_to_float(uint16_t(hdr.x & 0xffffu)), dmin = half_bits_to_float(uint16_t(hdr.x >> 16));
-    // 6-bit (scale, min) of sub-blocks 2g (low nibbles) and 2g+1 (high nibbles): in place for the first four, split across two bytes after
-    const int sh = 16 * (g & 1);
-    const uint32_t sc2 = g < 2 ? hdr.y >> sh & 0x3f3fu : (hdr.w >> sh & 0x0f0fu) | (hdr.y >> sh >> 2 & 0x3030u);
-    const uint32_t mn2 = g < 2 ? hdr.z >> sh & 0x3f3fu : (hdr.w >> sh >> 4 & 0x0f0fu) | (hdr.z >> sh >> 2 & 0x3030u);
-    T* dst = out + blk * 256 + 64 * g + 8 * piece;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const float ds = __fmul_rn(d, float(sc2 >> (8 * h) & 0xffu)), dm = __fmul_rn(dmin, float(mn2 >> (8 * h) & 0xffu));
-      const uint32_t q0 = (q.x >> (4 * h)) & 0x0f0f0f0fu, q1 = (q.y >> (4 * h)) & 0x0f0f0f0fu;
-      auto quant = [](uint32_t v, int e) { return __fsub_rn(__uint_as_float(__byte_perm(v, 0x4B000000u, 0x7440u + e)), 8388608.f); };
-      float w[8];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        w[e] = __fsub_rn(__fmul_rn(ds, quant(q0, e)), dm);
-        w[4 + e] = __fsub_rn(__fmul_rn(ds, quant(q1, e)), dm);
+      constexpr int P = 32 / R;
+      if constexpr (QT == QTYPE_Q6_K) {
+        const int hb = item / (2 * P), half = item / P & 1, l0 = R * (item % P);
+        uint32_t sc[2];
+        load_words<2, A>(b + 192 + 8 * hb, edge, sc);
+        s[0] = sc[0]; s[1] = sc[1];
+        s[3] = ld_u16(b + 208);
+        load_words<N, A>(b + 64 * hb + 32 * half + l0, edge, q);
+        load_words<N, A>(b + 128 + 32 * hb + l0, edge, h);
+      } else if constexpr (QT == QTYPE_Q2_K) {
+        const int hb = item / P, l0 = R * (item % P);
+        uint32_t sc[2];
+        load_words<2, A>(b + 8 * hb, edge, sc);
+        s[0] = sc[0]; s[1] = sc[1];
+        uint32_t d[1];
+        load_words<1, A>(b + 80, edge, d);
+        s[3] = d[0];
+        load_words<N, A>(b + 16 + 32 * hb + l0, edge, q);
+      } else {
+        const int hb = item / P, l0 = R * (item % P);
+        uint32_t sc[3];
+        load_words<3, A>(b + 96, edge, sc);
+        s[0] = sc[0]; s[1] = sc[1]; s[2] = sc[2];
+        s[3] = uint32_t(b[108]) | uint32_t(b[109]) << 8;
+        load_words<N, A>(b + 32 + 32 * hb + l0, edge, q);
+        load_words<N, A>(b + l0, edge, h);
       }
-      Pack8<T>::store(dst + 32 * h, w);
     }
   }
-}
 
-// Q6_K: item = (block, 128-weight half hb, 8 positions l0..l0+7); 8 items per block.  Weight 128*hb + 32*quad + l is
-// (d * scale[8*hb + 2*quad + l/16]) * (q - 32) with q = nibble of ql | two bits of qh (as decode8<QTYPE_Q6_K>).
-template <typename T>
-__global__ void __launch_bounds__(kDequantThreads)
-dequant_q6k_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t total_items) {
-  const int64_t base = (int64_t(blockIdx.x) * 2) * kDequantThreads + threadIdx.x;
+  // Run j: its first output in the block, its scale and min (products rounded as decode8<QT>'s) and its weights as biased bytes.
+  __device__ __forceinline__ int first(int item, int j) const {
+    constexpr int P = 32 / R;
+    if constexpr (QT == QTYPE_Q8_0) return R * item;
+    else if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4) return R * item + 16 * j;
+    else if constexpr (QT == QTYPE_NVFP4) return 16 * item + 8 * j;
+    else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) return 64 * (item / P) + R * (item % P) + 32 * j;
+    else if constexpr (QT == QTYPE_Q6_K) return 128 * (item / (2 * P)) + 32 * (item / P & 1) + R * (item % P) + 64 * j;
+    else return 128 * (item / P) + R * (item % P) + 32 * j;
+  }
+  __device__ __forceinline__ void scale(int item, int j, float& ds, float& dm) const {
+    dm = 0.f;
+    if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_Q8_0) ds = half_of(s[0], 0);
+    else if constexpr (QT == QTYPE_MXFP4) ds = e8m0_half(s[0]);
+    else if constexpr (QT == QTYPE_NVFP4) ds = ue4m3_half(s[0]);
+    else if constexpr (QT == QTYPE_Q4_K || QT == QTYPE_Q5_K) {
+      // 6-bit (scale, min) of sub-block 2g + j: in place for the first four, split across two bytes after
+      const int g = item / (32 / R), sh = 16 * (g & 1) + 8 * j;
+      const uint32_t sc = g < 2 ? s[1] >> sh & 0x3fu : (s[3] >> sh & 0x0fu) | (s[1] >> sh >> 2 & 0x30u);
+      const uint32_t mn = g < 2 ? s[2] >> sh & 0x3fu : (s[3] >> sh >> 4 & 0x0fu) | (s[2] >> sh >> 2 & 0x30u);
+      ds = __fmul_rn(half_of(s[0], 0), float(sc));
+      dm = __fmul_rn(half_of(s[0], 1), float(mn));
+    } else {
+      const int hb = item / (32 / R), u = (R * (item % (32 / R))) >> 4, i4 = 2 * (j & 1) + u;     // sub-block 8 hb + 2 j + u
+      if constexpr (QT == QTYPE_Q6_K) {
+        ds = __fmul_rn(half_of(s[3], 0), float(int(int8_t(s[j] >> (8 * (2 * (item / (32 / R) & 1) + u))))));
+      } else if constexpr (QT == QTYPE_Q2_K) {
+        const uint32_t b = s[j >> 1] >> (8 * i4);
+        ds = __fmul_rn(half_of(s[3], 0), float(b & 0x0fu));
+        dm = __fmul_rn(half_of(s[3], 1), float(b >> 4 & 0x0fu));
+      } else {
+        // sub-block 4 qd + i4: low nibble in byte (4 qd + i4) % 8 (its high half from sub-block 8 on), two high bits in byte 8 + i4 at 2 qd
+        const uint32_t low = s[j >> 1] >> (8 * i4 + 4 * hb) & 0x0fu, high = s[2] >> (8 * i4 + 2 * (2 * hb + (j >> 1))) & 0x03u;
+        ds = __fmul_rn(half_of(s[3], 0), float(int(low | high << 4) - 32));
+      }
+    }
+  }
+  __device__ __forceinline__ uint32_t bytes(int item, int j, int k) const {
+    if constexpr (QT == QTYPE_Q8_0) return q[k] ^ 0x80808080u;
+    else if constexpr (QT == QTYPE_Q4_0) return q[k] >> (4 * j) & 0x0f0f0f0fu;
+    else if constexpr (QT == QTYPE_MXFP4) return fp4_biased(q[k] >> (4 * j) & 0x0f0f0f0fu);
+    else if constexpr (QT == QTYPE_NVFP4) return fp4_biased((G::k16 ? q[k & 1] >> (2 * (k & 2)) : q[k & 1] >> (4 * j)) & 0x0f0f0f0fu);
+    else if constexpr (QT == QTYPE_Q4_K) return q[k] >> (4 * j) & 0x0f0f0f0fu;
+    else if constexpr (QT == QTYPE_Q5_K) return (q[k] >> (4 * j) & 0x0f0f0f0fu) | (h[k] >> (2 * (item / (32 / R)) + j) & 0x01010101u) << 4;
+    else if constexpr (QT == QTYPE_Q6_K) return (q[k] >> (4 * j) & 0x0f0f0f0fu) | (h[k] >> (4 * j + 2 * (item / (32 / R) & 1)) & 0x03030303u) << 4;
+    else if constexpr (QT == QTYPE_Q2_K) return q[k] >> (2 * j) & 0x03030303u;
+    else return (q[k] >> (2 * j) & 0x03030303u) | (h[k] >> (4 * (item / (32 / R)) + j) & 0x01010101u) << 2;
+  }
+  __device__ __forceinline__ void emit(T* dst, int item, bool wide) const {
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int64_t it = base + int64_t(i) * kDequantThreads;
-    if (it >= total_items) continue;
-    const int64_t blk = it >> 3;
-    const int hb = int(it & 7) >> 2, l0 = 8 * int(it & 3);
-    const uint8_t* b = in + blk * 210;                     // 2-byte aligned
-    const float d = half_bits_to_float(uint16_t(ld_u16(b + 208)));
-    const uint32_t la[2] = {ld_u32_a2(b + 64 * hb + l0), ld_u32_a2(b + 64 * hb + l0 + 4)};
-    const uint32_t lb[2] = {ld_u32_a2(b + 64 * hb + 32 + l0), ld_u32_a2(b + 64 * hb + 32 + l0 + 4)};
-    const uint32_t hh[2] = {ld_u32_a2(b + 128 + 32 * hb + l0), ld_u32_a2(b + 128 + 32 * hb + l0 + 4)};
-    const int8_t* scales = reinterpret_cast<const int8_t*>(b + 192) + 8 * hb + (l0 >> 4);
-    T* dst = out + blk * 256 + 128 * hb + l0;
+    for (int j = 0; j < G::kRuns; ++j) {
+      float ds, dm;
+      scale(item, j, ds, dm);
+      uint32_t v[R * int(sizeof(T)) / 4];
 #pragma unroll
-    for (int quad = 0; quad < 4; ++quad) {
-      const float ds = __fmul_rn(d, float(int(scales[2 * quad])));
-      float w[8];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const uint32_t l4 = ((quad & 1) ? lb[h] : la[h]) >> ((quad & 2) ? 4 : 0);
-        const uint32_t h4 = hh[h] >> (2 * quad);
+      for (int k = 0; k < N; ++k) {
+        const uint32_t by = bytes(item, j, k);
+        float w[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          const int qv = int(((l4 >> (8 * e)) & 0x0f) | (((h4 >> (8 * e)) & 0x03) << 4)) - 32;
-          w[4 * h + e] = __fmul_rn(ds, float(qv));
+          // byte q as a float: 0x4B0000qq is 2^23 + q, and the difference is exact
+          const float x = __fsub_rn(__uint_as_float(__byte_perm(by, 0x4B000000u, 0x7440u + e)), float(8388608 + G::kBias));
+          w[e] = G::kMin ? __fsub_rn(__fmul_rn(ds, x), dm) : __fmul_rn(ds, x);
+        }
+        if constexpr (sizeof(T) == 4) {
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[4 * k + e] = __float_as_uint(w[e]);
+        } else if constexpr (std::is_same<T, __half>::value) {
+          const __half2 a = __floats2half2_rn(w[0], w[1]), c = __floats2half2_rn(w[2], w[3]);
+          v[2 * k] = *reinterpret_cast<const uint32_t*>(&a); v[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&c);
+        } else {
+          const __nv_bfloat162 a = __floats2bfloat162_rn(w[0], w[1]), c = __floats2bfloat162_rn(w[2], w[3]);
+          v[2 * k] = *reinterpret_cast<const uint32_t*>(&a); v[2 * k + 1] = *reinterpret_cast<const uint32_t*>(&c);
         }
       }
-      Pack8<T>::store(dst + 32 * quad, w);
+      if constexpr (R * sizeof(T) == 32) store32(dst + first(item, j), v, wide);
+      else __stcs(reinterpret_cast<uint4*>(dst + first(item, j)), make_uint4(v[0], v[1], v[2], v[3]));
     }
   }
-}
+};
 
-// The six further types, 16-bit outputs: item = 8 consecutive packed bytes and every run of 8 weights they hold, so that each
-// packed byte is loaded once (the one-unit-per-thread kernel loads a nibble byte twice, a Q2_K byte four times and a Q3_K
-// mask byte eight times).  Arithmetic is decode8<QT>'s, operation for operation.
-//   Q4_0 / MXFP4: item = (block, half p of its 16 bytes): low nibbles = weights 8p .., high nibbles = weights 16 + 8p ..
-//   NVFP4:        item = (block, sub-block s): low nibbles = its first 8 weights, high nibbles = the other 8
-//   Q5_K:         item = (block, 64-weight group g, piece of 8 bytes): as Q4_K, plus bits 2g, 2g+1 of 8 bytes of qh
-//   Q2_K / Q3_K:  item = (block, half hb, 8 positions l0 ..): four runs (bit pairs j = 0..3) of 8 weights 32 apart
-// A: alignment the launcher found for the packed buffer (blocks of these types are only 1-, 2- or 4-byte multiples).
-template <int QT> struct ItemGeom;
-template <> struct ItemGeom<QTYPE_Q4_0> { static constexpr int kItems = 2, kAlign = 2; };
-template <> struct ItemGeom<QTYPE_MXFP4> { static constexpr int kItems = 2, kAlign = 1; };
-template <> struct ItemGeom<QTYPE_NVFP4> { static constexpr int kItems = 4, kAlign = 4; };
-template <> struct ItemGeom<QTYPE_Q5_K> { static constexpr int kItems = 16, kAlign = 4; };
-template <> struct ItemGeom<QTYPE_Q2_K> { static constexpr int kItems = 8, kAlign = 4; };
-template <> struct ItemGeom<QTYPE_Q3_K> { static constexpr int kItems = 8, kAlign = 2; };
-template <int QT> constexpr bool has_item_kernel() {
-  return QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4 || QT == QTYPE_NVFP4 || QT == QTYPE_Q5_K || QT == QTYPE_Q2_K || QT == QTYPE_Q3_K;
-}
+// Items per thread.  Two for 16-bit NVFP4, whose item is a single store of few instructions: [28672 x 8192] 96 us, 105 with one ([2048 x 4096]
+// 5.1 / 5.0).  One elsewhere: Q8_0 [2048 x 4096] 5.8 -> 5.7 (f16), 8.8 -> 8.2 (f32), Q4_K 4.6 -> 5.2 with two.
+template <int QT, typename T> constexpr int items_per_thread() { return QT == QTYPE_NVFP4 && sizeof(T) == 2 ? 2 : 1; }
 
-template <int A>
-__device__ __forceinline__ uint2 ld8(const uint8_t* p) {      // 8 bytes at an A-byte aligned address
-  if (A >= 4) {
-    const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
-    return make_uint2(__ldg(w), __ldg(w + 1));
-  }
-  if (A == 2) return make_uint2(ld_u32_a2(p), ld_u32_a2(p + 4));
-  uint32_t lo = 0, hi = 0;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { lo |= uint32_t(p[i]) << (8 * i); hi |= uint32_t(p[4 + i]) << (8 * i); }
-  return make_uint2(lo, hi);
-}
-__device__ __forceinline__ uint32_t byte_of(const uint2& q, int e) { return ((e < 4 ? q.x : q.y) >> (8 * (e & 3))) & 0xffu; }
-
+// A: alignment of the packed buffer where all its blocks keep it (16: Q4_K and Q5_K; 4: also Q2_K and NVFP4), 1: any start and block size,
+// 0: Q6_K from a 16-byte boundary, through shared memory.  An item of Q6_K is 3 misaligned pieces of its block; a CTA's 32 or 16 blocks
+// in 16-byte loads first cost a barrier and save the rest: [11008 x 4096] f16 25.0 -> 22.0 us, f32 37.0 -> 35.9, [512 x 2048] f32 3.1 -> 2.4.
+// The other types with odd blocks have shorter pieces and lose by it: Q8_0 f16 23.4 -> 24.5, Q3_K 19.3 -> 20.7, MXFP4 19.2 -> 20.9, Q4_0 equal.
 template <int QT, typename T, int A>
 __global__ void __launch_bounds__(kDequantThreads)
-dequant_items_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t total_items) {
-  constexpr int kBytes = QTraits<QT>::kBytes, kBlock = QTraits<QT>::kBlock;
-  const int64_t base = (int64_t(blockIdx.x) * 2) * kDequantThreads + threadIdx.x;
+dequant_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t total_items, int64_t first_edge, int64_t last_edge, bool wide) {
+  using G = ItemGeom<QT, run_of<QT, T>()>;
+  constexpr int kPer = items_per_thread<QT, T>();
+  const int64_t base = int64_t(blockIdx.x) * (kPer * kDequantThreads) + threadIdx.x;
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");          // the packed bytes may be the preceding kernel's output
+  Item<QT, T, A> it[kPer];
+  if constexpr (A == 0) {
+    constexpr int kBlocks = kDequantThreads / G::kItems, kBytes = kBlocks * QTraits<QT>::kBytes, kVec = kBytes / 16;
+    static_assert(kPer == 1 && kBytes % 16 == 0, "");
+    __shared__ __align__(16) uint8_t stage[kBytes + 16];
+    const int64_t blk0 = int64_t(blockIdx.x) * kBlocks, blocks = total_items / G::kItems;
+    const uint8_t* src = in + blk0 * QTraits<QT>::kBytes;
+    const int bytes = blocks - blk0 >= kBlocks ? kBytes : int(blocks - blk0) * QTraits<QT>::kBytes, vecs = bytes / 16;
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    const int64_t it = base + int64_t(i) * kDequantThreads;
-    if (it >= total_items) continue;
-    const int64_t blk = it / ItemGeom<QT>::kItems;
-    const int item = int(it - blk * ItemGeom<QT>::kItems);
-    const uint8_t* b = in + blk * kBytes;
-    T* dst = out + blk * kBlock;
-    float w[8];
-    if constexpr (QT == QTYPE_Q4_0 || QT == QTYPE_MXFP4) {
-      const float d = QT == QTYPE_Q4_0 ? half_at(b) : e8m0_half(b[0]);
-      const uint2 q = ld8<A>(b + (kBytes - 16) + 8 * item);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const uint32_t nib = (byte_of(q, e) >> (4 * h)) & 0x0fu;
-          w[e] = QT == QTYPE_Q4_0 ? __fmul_rn(d, float(int(nib) - 8)) : __fmul_rn(d, float(fp4_code_value(nib)));
-        }
-        Pack8<T>::store(dst + 8 * item + 16 * h, w);
-      }
-    } else if constexpr (QT == QTYPE_NVFP4) {
-      const float d = ue4m3_half(b[item]);
-      const uint2 q = ld8<A>(b + 4 + 8 * item);
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-#pragma unroll
-        for (int e = 0; e < 8; ++e) w[e] = __fmul_rn(d, float(fp4_code_value((byte_of(q, e) >> (4 * h)) & 0x0fu)));
-        Pack8<T>::store(dst + 16 * item + 8 * h, w);
-      }
-    } else if constexpr (QT == QTYPE_Q5_K) {
-      const int g = item >> 2, piece = item & 3;
-      const uint2 q = ld8<A>(b + 48 + 32 * g + 8 * piece), qh = ld8<A>(b + 16 + 8 * piece);
-      // the 16-byte header (d, dmin, 12 bytes of 6-bit scales and mins) as four words where the buffer is word aligned
-      const uint2 h01 = ld8<A>(b), h23 = ld8<A>(b + 8);
-      const float d = half_bits_to_float(uint16_t(h01.x & 0xffffu)), dmin = half_bits_to_float(uint16_t(h01.x >> 16));
-      const uint32_t s0 = h01.y, s1 = h23.x, s2 = h23.y;
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = 2 * g + h;
-        int sc, mn;
-        if (j < 4) {
-          sc = int(s0 >> (8 * j)) & 63;
-          mn = int(s1 >> (8 * j)) & 63;
-        } else {
-          sc = (int(s2 >> (8 * (j - 4))) & 0x0f) | ((int(s0 >> (8 * (j - 4))) >> 6 & 3) << 4);
-          mn = (int(s2 >> (8 * (j - 4))) >> 4 & 0x0f) | ((int(s1 >> (8 * (j - 4))) >> 6 & 3) << 4);
-        }
-        const float ds = __fmul_rn(d, float(sc)), dm = __fmul_rn(dmin, float(mn));
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          const int qv = int((byte_of(q, e) >> (4 * h)) & 0x0fu) + (((byte_of(qh, e) >> (2 * g + h)) & 1u) ? 16 : 0);
-          w[e] = __fsub_rn(__fmul_rn(ds, float(qv)), dm);
-        }
-        Pack8<T>::store(dst + 64 * g + 32 * h + 8 * piece, w);
-      }
-    } else {
-      const int hb = item >> 2, l0 = 8 * (item & 3);
-      constexpr int kQs = QT == QTYPE_Q2_K ? 16 : 32;
-      const uint2 q = ld8<A>(b + kQs + 32 * hb + l0);
-      uint2 hm = make_uint2(0u, 0u);
-      if constexpr (QT == QTYPE_Q3_K) hm = ld8<A>(b + l0);
-      const float d = half_at(b + (QT == QTYPE_Q2_K ? 80 : 108));
-      const float dmin = QT == QTYPE_Q2_K ? half_at(b + 82) : 0.f;
-      uint2 s01 = make_uint2(0u, 0u);          // Q3_K: the 12 scale bytes in three words (the third in s2)
-      uint32_t s2 = 0u;
-      if constexpr (QT == QTYPE_Q3_K) {
-        s01 = ld8<A>(b + 96);
-        s2 = A >= 2 ? ld_u32_a2(b + 104) : (uint32_t(b[104]) | (uint32_t(b[105]) << 8) | (uint32_t(b[106]) << 16) | (uint32_t(b[107]) << 24));
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int is = 8 * hb + 2 * j + (l0 >= 16 ? 1 : 0);
-        if constexpr (QT == QTYPE_Q2_K) {
-          const uint32_t scale = b[is];
-          const float ds = __fmul_rn(d, float(scale & 0x0fu)), dm = __fmul_rn(dmin, float(scale >> 4));
-#pragma unroll
-          for (int e = 0; e < 8; ++e) w[e] = __fsub_rn(__fmul_rn(ds, float(int(byte_of(q, e) >> (2 * j)) & 3)), dm);
-        } else {
-          // 6-bit scale `is` = 4*qd + i4: low nibble in byte is % 8 (its high half for is >= 8), two high bits in byte 8 + i4 at bit 2*qd
-          const int i4 = is & 3, qd = is >> 2;
-          const uint32_t low = (((qd & 1) ? s01.y : s01.x) >> (8 * i4 + 4 * (qd >> 1))) & 0x0fu;
-          const uint32_t high = (s2 >> (8 * i4 + 2 * qd)) & 0x03u;
-          const float ds = __fmul_rn(d, float(int(low | (high << 4)) - 32));
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
-            const int low = int(byte_of(q, e) >> (2 * j)) & 3;
-            w[e] = __fmul_rn(ds, float(low - (((byte_of(hm, e) >> (4 * hb + j)) & 1u) ? 0 : 4)));
-          }
-        }
-        Pack8<T>::store(dst + 128 * hb + 32 * j + l0, w);
-      }
+    for (int i = 0; i < (kVec + kDequantThreads - 1) / kDequantThreads; ++i) {
+      const int at = i * kDequantThreads + threadIdx.x;
+      if (at < vecs) *reinterpret_cast<uint4*>(stage + 16 * at) = __ldg(reinterpret_cast<const uint4*>(src) + at);
     }
+    for (int at = 16 * vecs + threadIdx.x; at < bytes; at += kDequantThreads) stage[at] = src[at];
+    __syncthreads();
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    const int blk = threadIdx.x / G::kItems, item = threadIdx.x % G::kItems;
+    if (blk0 + blk < blocks) {
+      it[0].load(stage + blk * QTraits<QT>::kBytes, item, false);
+      it[0].emit(out + (blk0 + blk) * QTraits<QT>::kBlock, item, wide);
+    }
+    return;
   }
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int64_t at = base + i * kDequantThreads, blk = at / G::kItems;
+    if (at < total_items) it[i].load(in + blk * QTraits<QT>::kBytes, int(at % G::kItems), blk == first_edge || blk == last_edge);
+  }
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < kPer; ++i) {
+    const int64_t at = base + i * kDequantThreads, blk = at / G::kItems;
+    if (at < total_items) it[i].emit(out + blk * QTraits<QT>::kBlock, int(at % G::kItems), wide);
+  }
+}
+
+template <int QT, typename T, int A>
+static int launch_items(const void* in, void* out, int64_t weights, cudaStream_t stream) {
+  using G = ItemGeom<QT, run_of<QT, T>()>;
+  constexpr int kPer = items_per_thread<QT, T>();
+  const int64_t items = weights / QTraits<QT>::kBlock * G::kItems, per_cta = int64_t(kDequantThreads) * kPer;
+  const int64_t grid = (items + per_cta - 1) / per_cta;
+  if (grid > 0x7fffffffLL) return RC_RANGE;
+  // blocks whose first or last aligned word holds bytes outside the buffer (only A == 1 looks)
+  const uintptr_t begin = reinterpret_cast<uintptr_t>(in);
+  const int64_t blocks = weights / QTraits<QT>::kBlock, first_edge = begin & 3 ? 0 : -1;
+  const int64_t last_edge = (begin + uintptr_t(blocks) * QTraits<QT>::kBytes) & 3 ? blocks - 1 : -1;
+  const bool wide = (reinterpret_cast<uintptr_t>(out) & 31) == 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(grid));
+  cfg.blockDim = dim3(kDequantThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, dequant_kernel<QT, T, A>, static_cast<const uint8_t*>(in), static_cast<T*>(out), items, first_edge,
+                                           last_edge, wide);
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess ? RC_OK : RC_LAUNCH;
 }
 
 template <int QT, typename T>
 static int launch_dequant(const void* in, void* out, int64_t rows, int64_t n_per_row, cudaStream_t stream) {
-  const int64_t weights = rows * n_per_row;
-  // 16-bit outputs: the every-byte-once kernels; float outputs are write bound and measured faster with one 8-output
-  // unit per thread (a warp then writes 1 KiB contiguous per pair of store instructions)
-  if ((QT == QTYPE_Q4_K || QT == QTYPE_Q6_K) && sizeof(T) == 2) {
-    const int64_t items = QT == QTYPE_Q4_K ? weights / 16 : weights / 32;
-    const int64_t per_cta = int64_t(kDequantThreads) * 2;
-    const int64_t grid = (items + per_cta - 1) / per_cta;
-    if (grid > 0x7fffffffLL) return RC_RANGE;
-    if (QT == QTYPE_Q4_K && (reinterpret_cast<uintptr_t>(in) & 15) == 0)
-      dequant_q4k_kernel<T, true><<<dim3(unsigned(grid)), kDequantThreads, 0, stream>>>(static_cast<const uint8_t*>(in), static_cast<T*>(out), items);
-    else if (QT == QTYPE_Q4_K)
-      dequant_q4k_kernel<T, false><<<dim3(unsigned(grid)), kDequantThreads, 0, stream>>>(static_cast<const uint8_t*>(in), static_cast<T*>(out), items);
-    else
-      dequant_q6k_kernel<T><<<dim3(unsigned(grid)), kDequantThreads, 0, stream>>>(static_cast<const uint8_t*>(in), static_cast<T*>(out), items);
-    return cudaGetLastError() == cudaSuccess ? RC_OK : RC_LAUNCH;
-  }
-  if constexpr (has_item_kernel<QT>() && sizeof(T) == 2) {
-    const int64_t items = weights / QTraits<QT>::kBlock * ItemGeom<QT>::kItems;
-    const int64_t per_cta = int64_t(kDequantThreads) * 2;
-    const int64_t grid = (items + per_cta - 1) / per_cta;
-    if (grid > 0x7fffffffLL) return RC_RANGE;
-    const uint8_t* src = static_cast<const uint8_t*>(in);
-    // word loads where the packed buffer allows them (these types accept any byte address), byte loads otherwise
-    if (ItemGeom<QT>::kAlign > 1 && reinterpret_cast<uintptr_t>(in) % ItemGeom<QT>::kAlign == 0)
-      dequant_items_kernel<QT, T, ItemGeom<QT>::kAlign><<<dim3(unsigned(grid)), kDequantThreads, 0, stream>>>(src, static_cast<T*>(out), items);
-    else
-      dequant_items_kernel<QT, T, 1><<<dim3(unsigned(grid)), kDequantThreads, 0, stream>>>(src, static_cast<T*>(out), items);
-    return cudaGetLastError() == cudaSuccess ? RC_OK : RC_LAUNCH;
-  }
-  const int64_t total_units = weights / 8;
-  const int64_t per_cta = int64_t(kDequantThreads) * kUnitsPerThread;
-  const int64_t grid = (total_units + per_cta - 1) / per_cta;
-  if (grid > 0x7fffffffLL) return RC_RANGE;
-  dequant_rows_kernel<QT, T><<<dim3(unsigned(grid)), kDequantThreads, 0, stream>>>(
-      static_cast<const uint8_t*>(in), static_cast<T*>(out), total_units);
-  return cudaGetLastError() == cudaSuccess ? RC_OK : RC_LAUNCH;
+  using G = ItemGeom<QT, run_of<QT, T>()>;
+  const uintptr_t at = reinterpret_cast<uintptr_t>(in);
+  if constexpr (G::kAlign == 16)
+    if ((at & 15) == 0) return launch_items<QT, T, 16>(in, out, rows * n_per_row, stream);
+  if constexpr (G::kAlign >= 4)
+    if ((at & 3) == 0) return launch_items<QT, T, 4>(in, out, rows * n_per_row, stream);
+  if constexpr (QT == QTYPE_Q6_K)
+    if ((at & 15) == 0) return launch_items<QT, T, 0>(in, out, rows * n_per_row, stream);
+  if constexpr (QT == QTYPE_Q4_K) return RC_ALIGN;                  // the entry has refused these
+  else return launch_items<QT, T, 1>(in, out, rows * n_per_row, stream);
 }
 
 template <int QT>
