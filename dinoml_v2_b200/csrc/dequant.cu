@@ -268,9 +268,7 @@ __global__ void __launch_bounds__(kDequantThreads)
 dequant_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t total_items, int64_t first_edge, int64_t last_edge, bool wide) {
   using G = ItemGeom<QT, run_of<QT, T>()>;
   constexpr int kPer = items_per_thread<QT, T>();
-  const int64_t base = int64_t(blockIdx.x) * (kPer * kDequantThreads) + threadIdx.x;
   asm volatile("griddepcontrol.wait;\n" ::: "memory");          // the packed bytes may be the preceding kernel's output
-  Item<QT, T, A> it[kPer];
   if constexpr (A == 0) {
     constexpr int kBlocks = kDequantThreads / G::kItems, kBytes = kBlocks * QTraits<QT>::kBytes, kVec = kBytes / 16;
     static_assert(kPer == 1 && kBytes % 16 == 0, "");
@@ -288,21 +286,24 @@ dequant_kernel(const uint8_t* __restrict__ in, T* __restrict__ out, int64_t tota
     asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
     const int blk = threadIdx.x / G::kItems, item = threadIdx.x % G::kItems;
     if (blk0 + blk < blocks) {
-      it[0].load(stage + blk * QTraits<QT>::kBytes, item, false);
-      it[0].emit(out + (blk0 + blk) * QTraits<QT>::kBlock, item, wide);
+      Item<QT, T, A> one;
+      one.load(stage + blk * QTraits<QT>::kBytes, item, false);
+      one.emit(out + (blk0 + blk) * QTraits<QT>::kBlock, item, wide);
     }
-    return;
-  }
+  } else {
+    const int64_t base = int64_t(blockIdx.x) * (kPer * kDequantThreads) + threadIdx.x;
+    Item<QT, T, A> it[kPer];
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int64_t at = base + i * kDequantThreads, blk = at / G::kItems;
-    if (at < total_items) it[i].load(in + blk * QTraits<QT>::kBytes, int(at % G::kItems), blk == first_edge || blk == last_edge);
-  }
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+    for (int i = 0; i < kPer; ++i) {
+      const int64_t at = base + i * kDequantThreads, blk = at / G::kItems;
+      if (at < total_items) it[i].load(in + blk * QTraits<QT>::kBytes, int(at % G::kItems), blk == first_edge || blk == last_edge);
+    }
+    asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
 #pragma unroll
-  for (int i = 0; i < kPer; ++i) {
-    const int64_t at = base + i * kDequantThreads, blk = at / G::kItems;
-    if (at < total_items) it[i].emit(out + blk * QTraits<QT>::kBlock, int(at % G::kItems), wide);
+    for (int i = 0; i < kPer; ++i) {
+      const int64_t at = base + i * kDequantThreads, blk = at / G::kItems;
+      if (at < total_items) it[i].emit(out + blk * QTraits<QT>::kBlock, int(at % G::kItems), wide);
+    }
   }
 }
 

@@ -129,9 +129,10 @@ int gemm_rcr_simt(const void* a, const void* b, const void* bias, void* c, int q
   }
   // Else the same exact products by mma.sync (one or two rows of the FP4 types stay below: 16 us against 24 us).
   // 16-bit activations on tcgen05 where the weight has enough super-block tiles for all SMs, or tiles and rows together pay for the
-  // start of that kernel (Q8_0 [4096 x 2880] float16, M = 8: 11.9 us against 14.6; MXFP4 [5760 x 2880] bfloat16, M = 24: 13.2 against
-  // 18.9; [2048 x 2880], 192 tiles: M = 64 MXFP4 11.8 against 14.9, Q8_0 14.5 against 15.9, M = 32 11.0 / 13.4 against 11.3 / 12.0;
-  // Q6_K [1024 x 2816], 88 tiles: M = 100 18.7 against 15.7, M = 200 21.8 against 27.9).
+  // start of that kernel (us, there / here: Q8_0 [4096 x 2880] float16, M = 8: 10.4 / 14.2; MXFP4 [5760 x 2880] bfloat16, M = 24: 11.0 / 18.9;
+  // [2048 x 2880], 192 tiles, M = 64: MXFP4 8.4 / 15.3, Q8_0 10.9 / 16.1; Q6_K [1024 x 2816], 88 tiles, M = 200: 16.8 / 27.9).  Since that kernel
+  // cuts K across clusters it is ahead below this line too (M = 32: MXFP4 7.2 / 12.0, Q8_0 10.1 / 12.5; Q6_K M = 100 11.5 / 16.0), but its sums
+  // are 6e-6 off where these are 2e-7: what was summed here stays here.
   const int64_t tiles = int64_t((n + 127) / 128) * ((k + 255) / 256);
   if (m >= 7 && (m > 128 || tiles >= 256 || tiles * m >= 12288))
     if (int rc = gemm_split(a, b, bias, c, qtype, dtype, m, n, k, s); rc != RC_RANGE) return rc;

@@ -485,7 +485,8 @@ int parse_profile_sections(const char* env, std::vector<ProfileSection>* out) {
 // others go where the fewest weight bytes are.  Empty: one after another, because there is nothing to gain (one chain; above 128 rows a
 // launch fills the GPU for long), or because a result is written over another result or an input, whose order counts.
 // A launch of a few microseconds is mostly its start and its tail, and these overlap here: one layer (q, k, v, o, gated pair, down; hidden 4096,
-// 14336 between), M = 1 / 8 / 32 / 128: 50.6 / 73.4 / 69.5 / 110.9 us, one after another 57.1 / 78.8 / 76.2 / 117.
+// 14336 between), M = 1 / 8 / 32 / 128: one after another 57.0 / 77.6 / 84.1 / 113.2 us, side by side 50.2 / 73.6 / 70.9 / 108.2; hidden 2048,
+// 5632 between: 29.8 / 40.7 / 46.2 / 66.7 and 22.9 / 35.1 / 33.8 / 51.5.
 std::vector<int> side_by_side(const DinoModule& mod, const std::vector<std::vector<int64_t>>& shapes, const std::vector<void*>& ptr) {
   constexpr int64_t kMostRows = 128;
   std::vector<int> branch(mod.nodes.size(), 0), writer(mod.tensors.size(), -1);

@@ -44,7 +44,7 @@ constexpr int kSmemBudget = 227 * 1024, kSmemHalf = 113 * 1024;      // of a CTA
 constexpr uint32_t kSpinLimit = 1u << 22;   // try_wait polls before a wait gives up: some fifteen seconds (a launch may stand behind a long one)
 
 enum : int { ST_OK = 0, ST_EMPTY_TIMEOUT = 1, ST_FULL_TIMEOUT = 2, ST_ACC_TIMEOUT = 3, ST_PEER_TIMEOUT = 4 };
-constexpr uint32_t kFlagSpinLimit = 1u << 22;   // polls (200 ns apart) of another CTA's partial-tile flag
+constexpr uint32_t kFlagSpinLimit = 1u << 22;   // polls (100 ns apart) of another CTA's partial-tile flag
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
@@ -161,9 +161,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
                "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]),
                "r"(r[14]), "r"(r[15])
                : "memory");
-}
-__device__ __forceinline__ void tmem_st4(uint32_t taddr, const uint32_t* r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1,%2,%3,%4};\n" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 // A operand from tensor memory, B from shared memory.
@@ -518,7 +515,7 @@ template <class S> struct Cta {
       for (int i = max(0, issued - S::NRAW); i < issued; ++i) mbar_wait_plain(rawfull(i % S::NRAW), uint32_t(i / S::NRAW) & 1u);
     }
   }
-  // Activation rows of tile t that the MMAs multiply: the last tile of a panel has fewer where its rows end before it does (M = 333: 192 and 160).
+  // Activation rows of tile t that the MMAs multiply: the last tile of a panel has fewer where its rows end before it does (M = 333: 192 and 160 rows).
   __device__ __forceinline__ int tile_rows(int t) const {
     if (!S::PAIR) return p.bn;
     return min(p.bn, (p.m - (t % p.m_tiles) * p.bn + 31) & ~31);

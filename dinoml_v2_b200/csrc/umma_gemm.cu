@@ -96,7 +96,7 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
   const int wide = bm == 256 ? 2 : 1;
   pl.bm = bm;
   pl.m_tiles = (m + pl.bm - 1) / pl.bm;
-  // The M rows in equal tiles of a multiple of 16 (pairs: 32): M = 333 is two tiles of 192 rows, not 256 + 77 padded to 512 (the MMA
+  // The M rows in equal tiles of a multiple of 16 (pairs: 32): M = 333 is tiles of 192 and 160 rows, not 256 + 77 padded to 512 (the MMA
   // time and the activation bytes go with the rows of a tile).
   pl.bn = ((m + pl.m_tiles - 1) / pl.m_tiles + 16 * wide - 1) / (16 * wide) * (16 * wide);
   const long long tiles = static_cast<long long>(pl.m_tiles) * ((n + wide * kRowsW - 1) / (wide * kRowsW));
