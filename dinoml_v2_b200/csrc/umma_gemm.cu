@@ -113,6 +113,8 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
   // us, [4096 x 4096] Q4_K, M = 16: slices 2 / 4 / 8 9.2 / 7.1 / 8.2, stream-K 10.6; [4096 x 14336] 26.2 / 19.4 / 15.1, stream-K 17.6;
   // [11008 x 4096] 2 / 3 13.0 / 12.6, stream-K 14.5; M = 64, [32768 x 4096]: whole 26.8, stream-K 29.7; [20480 x 4096] 25.8 / 23.1; M = 200,
   // [11008 x 4096]: whole 24.8, stream-K 27.8; [1024 x 4096] 2 / 3 / 4 16.0 / 13.9 / 12.4, whole 21.7, stream-K 18.9.
+  // Two CTAs per SM: clusters that would not all fit with one per SM share some, which costs more the longer K is.  37 clusters of four where 33 fit,
+  // M = 12, [4696 x 8960]: 14.9, of seven 12.5; Q6_K [4736 x 14336], M = 16: 26.9 / 20.9; [4608 x 4096]: 7.9 / 9.2.
   // (stream-K: at least four super-blocks per worker, a small problem is not cut into more pieces than its finishers can add up quickly.)
   const long long most = pl.units / 4 > 1 ? pl.units / 4 : 1;
   pl.workers = int(most < slots ? most : slots);
@@ -122,7 +124,8 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
   pl.slices = 0;                                                     // stream-K
   for (int s = 1; s <= most_slices && s <= nsb && tiles <= max_clusters(s * wide, ctas_per_sm); ++s) {
     const float load = float(tiles * s * wide) / float(sm_count), own = float(nsb) / float(s);
-    const float share = load <= 1.f ? 1.f : s == 1 ? 1.75f : fminf(1.75f, sqrtf(load * sqrtf(load)) + own / 64.f);
+    const bool alone = load <= 1.f && tiles <= max_clusters(s * wide, 1);
+    const float more = fmaxf(load, 1.f), share = alone ? 1.f : s == 1 ? 1.75f : fminf(1.75f, sqrtf(more * sqrtf(more)) + own / 64.f);
     const float cost = 0.5f * (float((nsb + s - 1) / s) + own) * share + (s > 1 ? join + each * float(s) : 0.f);
     if (cost < best) { pl.slices = s; best = cost; }
   }
