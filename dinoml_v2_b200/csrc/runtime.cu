@@ -24,8 +24,8 @@
 //                          its launch (the next weight is copied on a second stream while the current one computes);
 //   grouped_offload        the same at the granularity of groups of constants (one group = e.g. one layer).
 // Steady state: dino_session_set_graph_replay(session, 1) makes dino_session_run capture the launch sequence of a
-// (shapes, pointers) combination the second time it sees it and replay the graph from then on.  Linears of it that do not read one another's
-// results are branches of that graph.
+// (shapes, pointers, stream) combination the second time it sees it and replay the graph from then on.  Linears of it that do not read one
+// another's results are branches of that graph.
 // DINOML_PROFILE_RUN[_VERBOSE|_SECTIONS] time every launch with events, as src/dinoml/templates/gpu_module.cu.j2:785-983.
 #if defined(__SSE2__)
 #include <immintrin.h>
@@ -41,6 +41,7 @@
 #include <vector>
 
 #include "../../include/dinoml_b200_runtime.h"
+#include "side_streams.h"
 #include "gguf_common.cuh"
 
 namespace b200gguf {
@@ -150,17 +151,15 @@ struct DinoSession {
   std::vector<void*> temps;                         // per tensor index (temp role only)
   std::vector<std::vector<int64_t>> shapes;         // per tensor index, as of the last run
   std::vector<bool> output_shape_valid;
-  // steady-state replay: one captured graph per (input shapes, input / output pointers) seen at least twice
+  // steady-state replay: one captured graph per (stream, input shapes, input / output pointers) seen at least twice.  A graph uses the
+  // workspaces of the stream it was captured on, so it is launched on no other.
   bool graph_replay = false;
-  struct CachedGraph { cudaGraphExec_t exec = nullptr; int seen = 0; std::vector<std::vector<int64_t>> out_shapes; };
+  struct CachedGraph { cudaGraphExec_t exec = nullptr; int seen = 0; bool branches = false; std::vector<std::vector<int64_t>> out_shapes; };
   std::map<std::vector<int64_t>, CachedGraph> graphs;
   size_t graph_launches = 0;
   size_t graph_generation = 0;
   std::vector<int64_t> pending_key;     // combination of the run in progress; counted as seen once that run has succeeded
-  // replayed runs: linears that do not need one another's results run side by side on these (made when first needed)
-  static constexpr int kSides = 3;
-  cudaStream_t side[kSides] = {};
-  cudaEvent_t forked = nullptr, joined[kSides] = {};
+  b200gguf::SideStreams sides;          // replayed runs: linears that do not need one another's results run side by side on these
 };
 
 namespace {
@@ -502,14 +501,14 @@ std::vector<int> side_by_side(const DinoModule& mod, const std::vector<std::vect
     rows[t] = shapes[t].empty() || shapes[t].back() == 0 ? 0 : count / shapes[t].back();
     read.push_back(range(t, count));
   }
-  size_t load[1 + DinoSession::kSides] = {};
+  size_t load[1 + b200gguf::SideStreams::kSides] = {};
   bool several = false;
   for (size_t i = 0; i < mod.nodes.size(); ++i) {
     const NodeSpec& node = mod.nodes[i];
     const ConstantSpec& w = mod.constants[node.b];
     int at = 0;
     if (writer[node.a] >= 0) at = branch[writer[node.a]];
-    else for (int b = 1; b <= DinoSession::kSides; ++b) if (load[b] < load[at]) at = b;
+    else for (int b = 1; b <= b200gguf::SideStreams::kSides; ++b) if (load[b] < load[at]) at = b;
     branch[i] = at;
     several = several || at != 0;
     load[at] += w.nbytes;
@@ -527,38 +526,31 @@ std::vector<int> side_by_side(const DinoModule& mod, const std::vector<std::vect
   return several ? branch : std::vector<int>();
 }
 
-bool make_sides(DinoSession* s) {
-  if (s->forked == nullptr && cudaEventCreateWithFlags(&s->forked, cudaEventDisableTiming) != cudaSuccess) return false;
-  for (int i = 0; i < DinoSession::kSides; ++i) {
-    if (s->side[i] == nullptr && cudaStreamCreateWithFlags(&s->side[i], cudaStreamNonBlocking) != cudaSuccess) return false;
-    if (s->joined[i] == nullptr && cudaEventCreateWithFlags(&s->joined[i], cudaEventDisableTiming) != cudaSuccess) return false;
-  }
-  return true;
-}
-
 // The streams of one pass: forked from the session's stream, joined to it again however the pass ends.
 struct Branches {
   DinoSession* s;
   std::vector<int> of;                  // per node; empty: all on the session's stream
-  bool used[DinoSession::kSides] = {};
+  b200gguf::SideStreams::Set* set = nullptr;
+  bool used[b200gguf::SideStreams::kSides] = {};
   int rc = 0;
   Branches(DinoSession* session, std::vector<int> branch) : s(session), of(std::move(branch)) {
     if (of.empty()) return;
-    if (!make_sides(s) || cudaEventRecord(s->forked, s->stream) != cudaSuccess) { cudaGetLastError(); of.clear(); return; }
+    set = s->sides.at(s->stream);
+    if (set == nullptr || cudaEventRecord(set->forked, s->stream) != cudaSuccess) { cudaGetLastError(); of.clear(); return; }
     for (int b : of)
       if (b > 0 && !used[b - 1]) {
-        if (cudaStreamWaitEvent(s->side[b - 1], s->forked, 0) != cudaSuccess) { rc = cuda_fail("cudaStreamWaitEvent", cudaGetLastError()); return; }
+        if (cudaStreamWaitEvent(set->side[b - 1], set->forked, 0) != cudaSuccess) { rc = cuda_fail("cudaStreamWaitEvent", cudaGetLastError()); return; }
         used[b - 1] = true;
       }
   }
-  cudaStream_t stream(size_t node) const { return of.empty() || of[node] == 0 ? s->stream : s->side[of[node] - 1]; }
+  cudaStream_t stream(size_t node) const { return of.empty() || of[node] == 0 ? s->stream : set->side[of[node] - 1]; }
   int join() {
     int result = 0;
-    for (int i = 0; i < DinoSession::kSides; ++i)
+    for (int i = 0; i < b200gguf::SideStreams::kSides; ++i)
       if (used[i]) {
         used[i] = false;
-        cudaError_t err = cudaEventRecord(s->joined[i], s->side[i]);
-        if (err == cudaSuccess) err = cudaStreamWaitEvent(s->stream, s->joined[i], 0);
+        cudaError_t err = cudaEventRecord(set->joined[i], set->side[i]);
+        if (err == cudaSuccess) err = cudaStreamWaitEvent(s->stream, set->joined[i], 0);
         if (err != cudaSuccess) result = cuda_fail("joining the session's streams", err);
       }
     return result;
@@ -566,9 +558,10 @@ struct Branches {
   ~Branches() { join(); }
 };
 
-// One pass over the plan.  `launch == false` only validates and computes shapes.  side: independent launches may run side by side.
+// One pass over the plan.  `validate == false` takes the shapes of the pass before.  side: independent launches may run side by side;
+// *branched then says whether any do.
 int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs,
-             bool validate, bool side = false) {
+             bool validate, bool side = false, bool* branched = nullptr) {
   DinoModule& mod = *s->module;
   if (validate) {
     if (num_inputs != mod.inputs.size()) return fail("dino_session_run expected " + std::to_string(mod.inputs.size()) + " inputs");
@@ -605,6 +598,7 @@ int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTe
 
   Branches branches(s, side ? side_by_side(mod, s->shapes, ptr) : std::vector<int>());
   if (branches.rc != 0) return branches.rc;
+  if (branched != nullptr) *branched = !branches.of.empty();
   for (size_t ni = 0; ni < mod.nodes.size(); ++ni) {
     const NodeSpec& node = mod.nodes[ni];
     ConstantSpec& w = mod.constants[node.b];
@@ -917,26 +911,27 @@ int dino_session_create(DinoModule* module, DinoSession** out) {
   return 0;
 }
 
+static void release_workspaces(cudaStream_t stream) {
+  b200gguf::stream_release_scratch(stream);
+  b200gguf::umma_release_scratch(stream);
+}
+
+// All captured graphs, and the side streams that no later run of this session uses without asking for them again: those of every
+// stream but *keep (null: of every stream).  Waits for the graphs that still run on those.
+static void drop_graphs(DinoSession* s, const cudaStream_t* keep) {
+  s->sides.release(keep, release_workspaces);
+  for (auto& entry : s->graphs) if (entry.second.exec != nullptr) cudaGraphExecDestroy(entry.second.exec);
+  s->graphs.clear();
+}
+
 int dino_session_destroy(DinoSession* session) {
   if (session == nullptr) return 0;
+  if (session->owned_stream != nullptr) cudaStreamSynchronize(session->owned_stream);
+  drop_graphs(session, nullptr);
   if (session->owned_stream != nullptr) {
-    cudaStreamSynchronize(session->owned_stream);
-    b200gguf::stream_release_scratch(session->owned_stream);
-    b200gguf::umma_release_scratch(session->owned_stream);
+    release_workspaces(session->owned_stream);
     cudaStreamDestroy(session->owned_stream);
   }
-  for (int i = 0; i < DinoSession::kSides; ++i) {
-    if (session->side[i] != nullptr) {
-      cudaStreamSynchronize(session->side[i]);
-      b200gguf::stream_release_scratch(session->side[i]);
-      b200gguf::umma_release_scratch(session->side[i]);
-      cudaStreamDestroy(session->side[i]);
-    }
-    if (session->joined[i] != nullptr) cudaEventDestroy(session->joined[i]);
-  }
-  if (session->forked != nullptr) cudaEventDestroy(session->forked);
-  for (auto& entry : session->graphs)
-    if (entry.second.exec != nullptr) cudaGraphExecDestroy(entry.second.exec);
   for (void* p : session->temps) if (p != nullptr) cudaFree(p);
   delete session;
   return 0;
@@ -981,7 +976,7 @@ int dino_session_get_state_pointer(DinoSession* session, size_t state_index, voi
 int dino_session_set_graph_replay(DinoSession* session, int enabled) {
   if (session == nullptr) return fail("dino_session_set_graph_replay received null pointer");
   session->graph_replay = enabled != 0;
-  if (session->graph_replay && !make_sides(session)) cudaGetLastError();      // else by the first run that needs them
+  if (session->graph_replay) session->sides.at(session->stream);       // else by the first run that needs them
   return 0;
 }
 
@@ -994,7 +989,15 @@ int dino_session_get_graph_stats(DinoSession* session, size_t* cached_graphs, si
   return 0;
 }
 
-// Steady-state path of dino_session_run: the launch sequence of one (input shapes, input / output pointers) combination is
+static int launch_graph(DinoSession* s, DinoSession::CachedGraph& cg) {
+  cudaError_t err = cudaGraphLaunch(cg.exec, s->stream);
+  ++s->graph_launches;
+  // on its own stream a session waits for every run
+  if (err == cudaSuccess && cg.branches && s->external_stream) err = s->sides.launched(s->stream);
+  return err == cudaSuccess ? 0 : cuda_fail("cudaGraphLaunch", err);
+}
+
+// Steady-state path of dino_session_run: the launch sequence of one (stream, input shapes, input / output pointers) combination is
 // captured the second time it is seen and replayed afterwards; validation ran when it was captured.  Returns 1 if the
 // call was served (rc in *rc_out), 0 if the caller should run the plan the ordinary way.
 static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs, int* rc_out) {
@@ -1004,11 +1007,10 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
     return 0;
   if (num_inputs != mod.inputs.size() || num_outputs != mod.outputs.size() || (num_inputs && !inputs) || (num_outputs && !outputs)) return 0;
   if (s->graph_generation != mod.generation) {             // constant buffers were released since: every captured pointer is stale
-    for (auto& entry : s->graphs) if (entry.second.exec != nullptr) cudaGraphExecDestroy(entry.second.exec);
-    s->graphs.clear();
+    drop_graphs(s, &s->stream);
     s->graph_generation = mod.generation;
   }
-  std::vector<int64_t> key;
+  std::vector<int64_t> key{int64_t(reinterpret_cast<intptr_t>(s->stream))};
   for (size_t i = 0; i < num_inputs; ++i) {
     if (inputs[i].shape == nullptr || inputs[i].data == nullptr) return 0;
     key.push_back(int64_t(reinterpret_cast<intptr_t>(tensor_ptr(inputs[i]))));
@@ -1019,17 +1021,12 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
     if (outputs[i].data == nullptr) return 0;
     key.push_back(int64_t(reinterpret_cast<intptr_t>(tensor_ptr(outputs[i]))));
   }
-  if (s->graphs.size() > 64 && s->graphs.find(key) == s->graphs.end()) {     // callers that pass ever-changing buffers: start over
-    for (auto& entry : s->graphs) if (entry.second.exec != nullptr) cudaGraphExecDestroy(entry.second.exec);
-    s->graphs.clear();
-  }
+  if (s->graphs.size() > 64 && s->graphs.find(key) == s->graphs.end()) drop_graphs(s, &s->stream);     // callers that pass ever-changing buffers: start over
   DinoSession::CachedGraph& cg = s->graphs[key];
   if (cg.exec != nullptr) {
     s->shapes = cg.out_shapes;
     std::fill(s->output_shape_valid.begin(), s->output_shape_valid.end(), true);
-    const cudaError_t err = cudaGraphLaunch(cg.exec, s->stream);
-    ++s->graph_launches;
-    *rc_out = err == cudaSuccess ? 0 : cuda_fail("cudaGraphLaunch", err);
+    *rc_out = launch_graph(s, cg);
     return 1;
   }
   if (cg.seen < 1) {                 // not yet run successfully the ordinary way (or a capture failed before): ordinary run
@@ -1039,7 +1036,7 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
   // seen once, and that run succeeded (every lazily created workspace of the kernels exists): capture this one
   cudaGraph_t graph = nullptr;
   if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); cg.seen = -1; return 0; }
-  const int rc = run_plan(s, inputs, num_inputs, outputs, num_outputs, true, true);
+  const int rc = run_plan(s, inputs, num_inputs, outputs, num_outputs, true, true, &cg.branches);
   const bool ended = cudaStreamEndCapture(s->stream, &graph) == cudaSuccess && graph != nullptr;
   bool ok = rc == 0 && ended && cudaGraphInstantiate(&cg.exec, graph, 0) == cudaSuccess;
   if (graph) cudaGraphDestroy(graph);
@@ -1050,9 +1047,7 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
     return 0;
   }
   cg.out_shapes = s->shapes;
-  const cudaError_t err = cudaGraphLaunch(cg.exec, s->stream);
-  ++s->graph_launches;
-  *rc_out = err == cudaSuccess ? 0 : cuda_fail("cudaGraphLaunch", err);
+  *rc_out = launch_graph(s, cg);
   return 1;
 }
 
