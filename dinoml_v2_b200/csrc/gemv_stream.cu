@@ -125,6 +125,18 @@ static int launch_q(const void* a, const void* b, const void* bias, void* c, int
 
 }  // namespace stream
 
+bool stream_reserve_scratch(cudaStream_t s, cudaStream_t like) {
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  bool made = false, slices = false;
+  {
+    std::lock_guard<std::mutex> lock(stream::g_sets.mutex);
+    if (const StreamScratch* set = stream::g_sets.find(dev, like)) { made = true; slices = set->slice_words != nullptr; }
+  }
+  stream::Scratch unused;
+  return !made || stream::stream_scratch(s, slices, &unused) == RC_OK;
+}
+
 void stream_release_scratch(cudaStream_t s) {
   std::lock_guard<std::mutex> lock(stream::g_sets.mutex);
   stream::g_sets.release(s);

@@ -53,6 +53,8 @@ int gemm_rcr(const void* a, const void* b, const void* bias, void* c, int qtype,
              int variant, cudaStream_t s);
 void stream_release_scratch(cudaStream_t s);      // workspaces the kernels keep for a stream
 void umma_release_scratch(cudaStream_t s);
+bool stream_reserve_scratch(cudaStream_t s, cudaStream_t like);      // the workspaces of `s`, with room for what `like` has had room for
+bool umma_reserve_scratch(cudaStream_t s, cudaStream_t like);
 }  // namespace b200gguf
 
 using b200gguf::set_error_message;
@@ -535,7 +537,7 @@ struct Branches {
   int rc = 0;
   Branches(DinoSession* session, std::vector<int> branch) : s(session), of(std::move(branch)) {
     if (of.empty()) return;
-    set = s->sides.at(s->stream);
+    set = s->sides.at(s->stream);       // there already: reserve_sides()
     if (set == nullptr || cudaEventRecord(set->forked, s->stream) != cudaSuccess) { cudaGetLastError(); of.clear(); return; }
     for (int b : of)
       if (b > 0 && !used[b - 1]) {
@@ -558,10 +560,19 @@ struct Branches {
   ~Branches() { join(); }
 };
 
-// One pass over the plan.  `validate == false` takes the shapes of the pass before.  side: independent launches may run side by side;
-// *branched then says whether any do.
+std::vector<void*> tensor_pointers(const DinoSession* s, const DinoTensor* inputs, size_t num_inputs, const DinoTensor* outputs, size_t num_outputs) {
+  const DinoModule& mod = *s->module;
+  std::vector<void*> ptr(mod.tensors.size(), nullptr);
+  for (size_t i = 0; i < num_inputs; ++i) ptr[mod.inputs[i]] = tensor_ptr(inputs[i]);
+  for (size_t i = 0; i < num_outputs; ++i) ptr[mod.outputs[i]] = outputs[i].data ? tensor_ptr(outputs[i]) : nullptr;
+  for (size_t i = 0; i < mod.tensors.size(); ++i) if (mod.tensors[i].role == 2) ptr[i] = s->temps[i];
+  return ptr;
+}
+
+// One pass over the plan.  `validate == false` takes the shapes of the pass before.  branch: a stream per node (side_by_side()), empty = one
+// after another.
 int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs,
-             bool validate, bool side = false, bool* branched = nullptr) {
+             bool validate, std::vector<int> branch = {}) {
   DinoModule& mod = *s->module;
   if (validate) {
     if (num_inputs != mod.inputs.size()) return fail("dino_session_run expected " + std::to_string(mod.inputs.size()) + " inputs");
@@ -591,14 +602,9 @@ int run_plan(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTe
     cudaEventRecord(total0, s->stream);
   }
   int launch_index = 0, busy_slot = -1;
-  std::vector<void*> ptr(mod.tensors.size(), nullptr);
-  for (size_t i = 0; i < num_inputs; ++i) ptr[mod.inputs[i]] = tensor_ptr(inputs[i]);
-  for (size_t i = 0; i < num_outputs; ++i) ptr[mod.outputs[i]] = outputs[i].data ? tensor_ptr(outputs[i]) : nullptr;
-  for (size_t i = 0; i < mod.tensors.size(); ++i) if (mod.tensors[i].role == 2) ptr[i] = s->temps[i];
-
-  Branches branches(s, side ? side_by_side(mod, s->shapes, ptr) : std::vector<int>());
+  const std::vector<void*> ptr = tensor_pointers(s, inputs, num_inputs, outputs, num_outputs);
+  Branches branches(s, std::move(branch));
   if (branches.rc != 0) return branches.rc;
-  if (branched != nullptr) *branched = !branches.of.empty();
   for (size_t ni = 0; ni < mod.nodes.size(); ++ni) {
     const NodeSpec& node = mod.nodes[ni];
     ConstantSpec& w = mod.constants[node.b];
@@ -976,7 +982,6 @@ int dino_session_get_state_pointer(DinoSession* session, size_t state_index, voi
 int dino_session_set_graph_replay(DinoSession* session, int enabled) {
   if (session == nullptr) return fail("dino_session_set_graph_replay received null pointer");
   session->graph_replay = enabled != 0;
-  if (session->graph_replay) session->sides.at(session->stream);       // else by the first run that needs them
   return 0;
 }
 
@@ -997,10 +1002,29 @@ static int launch_graph(DinoSession* s, DinoSession::CachedGraph& cg) {
   return err == cudaSuccess ? 0 : cuda_fail("cudaGraphLaunch", err);
 }
 
+// Before a capture with branches: the streams, and for those that launches go to the workspaces that the ordinary run of the combination
+// has found on the session's stream, which a capture could not make.  That run itself takes the launches one after another: a pass over new buffers pays
+// neither for streams and workspaces nor for a dozen event calls that it gains nothing by.  The sides have no work but the clearing of new workspaces, which
+// is waited for here, as the graph runs on another stream.
+static bool reserve_sides(DinoSession* s, const std::vector<int>& branch) {
+  if (branch.empty()) return true;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) return false;
+  b200gguf::SideStreams::Set* set = s->sides.at(s->stream);
+  bool used[b200gguf::SideStreams::kSides] = {};
+  for (int b : branch) if (b > 0) used[b - 1] = true;
+  for (int i = 0; i < b200gguf::SideStreams::kSides && set != nullptr; ++i)
+    if (used[i] && (!b200gguf::stream_reserve_scratch(set->side[i], s->stream) || !b200gguf::umma_reserve_scratch(set->side[i], s->stream) ||
+                    cudaStreamSynchronize(set->side[i]) != cudaSuccess))
+      set = nullptr;
+  if (set == nullptr) cudaGetLastError();
+  return set != nullptr;
+}
+
 // Steady-state path of dino_session_run: the launch sequence of one (stream, input shapes, input / output pointers) combination is
 // captured the second time it is seen and replayed afterwards; validation ran when it was captured.  Returns 1 if the
-// call was served (rc in *rc_out), 0 if the caller should run the plan the ordinary way.
-static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs, int* rc_out) {
+// call was served (rc in *rc_out), 0 if the caller should run the plan the ordinary way.  side: with branches in the graph.
+static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs, bool side, int* rc_out) {
   DinoModule& mod = *s->module;
   if (!s->graph_replay || module_streams_constants(mod) || std::getenv("DINOML_PROFILE_RUN") != nullptr ||
       std::getenv("DINOML_PROFILE_RUN_SECTIONS") != nullptr)
@@ -1034,9 +1058,17 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
     return 0;
   }
   // seen once, and that run succeeded (every lazily created workspace of the kernels exists): capture this one
+  std::vector<int> branch;
+  if (side) {
+    std::vector<std::vector<int64_t>> shapes(mod.tensors.size());
+    for (size_t i = 0; i < num_inputs; ++i) shapes[mod.inputs[i]].assign(inputs[i].shape, inputs[i].shape + inputs[i].ndim);
+    branch = side_by_side(mod, shapes, tensor_pointers(s, inputs, num_inputs, outputs, num_outputs));
+    if (!reserve_sides(s, branch)) branch.clear();
+  }
+  cg.branches = !branch.empty();
   cudaGraph_t graph = nullptr;
   if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); cg.seen = -1; return 0; }
-  const int rc = run_plan(s, inputs, num_inputs, outputs, num_outputs, true, true, &cg.branches);
+  const int rc = run_plan(s, inputs, num_inputs, outputs, num_outputs, true, std::move(branch));
   const bool ended = cudaStreamEndCapture(s->stream, &graph) == cudaSuccess && graph != nullptr;
   bool ok = rc == 0 && ended && cudaGraphInstantiate(&cg.exec, graph, 0) == cudaSuccess;
   if (graph) cudaGraphDestroy(graph);
@@ -1051,13 +1083,6 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
   return 1;
 }
 
-// The ordinary run that comes before a capture takes the same streams, so that the workspaces that the kernels keep for each exist by then; not
-// inside a capture of the caller's, where they could not be made.
-static bool will_be_replayed(DinoSession* s) {
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  return !s->pending_key.empty() && cudaStreamIsCapturing(s->stream, &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
-}
-
 // A combination counts as seen once a run of it has succeeded the ordinary way.
 static void note_ordinary_run(DinoSession* s) {
   if (s->pending_key.empty()) return;
@@ -1070,9 +1095,9 @@ int dino_session_run(DinoSession* session, const DinoTensor* inputs, size_t num_
   if (session == nullptr) return fail("dino_session_run received null session");
   int replay_rc = 0;
   session->pending_key.clear();
-  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, &replay_rc)) {
+  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, true, &replay_rc)) {
     if (replay_rc != 0) return replay_rc;
-  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true, will_be_replayed(session))) {
+  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true)) {
     return rc;
   } else {
     note_ordinary_run(session);
@@ -1097,9 +1122,9 @@ int dino_session_run_staged(DinoSession* session, const void* host_in, void* dev
   }
   int replay_rc = 0;
   session->pending_key.clear();
-  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, &replay_rc)) {
+  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, false, &replay_rc)) {
     if (replay_rc != 0) return replay_rc;
-  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true, will_be_replayed(session))) {
+  } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true)) {
     return rc;
   } else {
     note_ordinary_run(session);

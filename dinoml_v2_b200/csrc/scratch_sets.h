@@ -75,6 +75,11 @@ class ScratchSets {
     }
     return set;
   }
+  // The set that a stream has, null if it has none.
+  const Set* find(int dev, cudaStream_t stream) const {
+    const auto it = sets_.find(std::make_pair(dev, stream));
+    return it != sets_.end() && it->second.made() ? &it->second : nullptr;
+  }
   // `stream` is about to be destroyed and has no work left: its set is emptied and kept for a later stream (a bounded number) or freed.
   void release(cudaStream_t stream) {
     for (auto it = sets_.begin(); it != sets_.end();) {

@@ -238,6 +238,18 @@ static int launch_bm(int qtype, int dtype, const void* a, const void* b, const v
 
 }  // namespace umma
 
+bool umma_reserve_scratch(cudaStream_t s, cudaStream_t like) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  bool made = false;
+  size_t bytes = 0;
+  {
+    std::lock_guard<std::mutex> lock(umma::g_sets.mutex);
+    if (const UmmaScratch* set = umma::g_sets.find(dev, like)) { made = true; bytes = set->workspace_bytes; }
+  }
+  return !made || umma::device_state(bytes, s) != nullptr;
+}
+
 void umma_release_scratch(cudaStream_t s) {
   std::lock_guard<std::mutex> lock(umma::g_sets.mutex);
   umma::g_sets.release(s);

@@ -91,3 +91,22 @@ def test_session_dropped_behind_its_last_run(module, m):
         del session                                             # the next one gets its workspaces
     torch.cuda.synchronize()
     assert all(_same(want, got) for got in results) and kernels.device_status() == 0
+
+
+def test_first_pass_makes_no_side_workspaces(module):
+    """A pass over new buffers is launched in order: sessions that never replay hold no more memory with replay switched on than without."""
+    x, want, got = _buffers(module, 1, 60)
+
+    def taken(replay):
+        sessions = [module.create_session() for _ in range(12)]         # more than the sets that the library keeps for new streams
+        torch.cuda.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        for session in sessions:
+            session.set_graph_replay(replay)
+            session.run_torch(x, got)
+            assert _same(want, got)
+        torch.cuda.synchronize()
+        return before - torch.cuda.mem_get_info()[0]
+
+    plain = taken(False)
+    assert taken(True) <= plain + (2 << 20)                             # the driver's granularity; three workspaces a session would be 12 MB
