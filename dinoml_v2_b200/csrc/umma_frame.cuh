@@ -544,10 +544,10 @@ template <class S> struct Cta {
     int peer0 = worker;                           // first worker with a piece of this tile; peers are peer0 .. worker-1
     if (finishes && !whole) {
       peer0 = unit_owner(static_cast<long long>(t) * nsb, p.units, workers);
-      if (tid < worker - peer0) {
+      for (int peer = peer0 + tid; peer < worker; peer += S::PW * 32) {      // one tile of a very long K has more pieces than eight warps have threads
         bool seen = false;
         for (uint32_t i = 0; i < kFlagSpinLimit && !seen; ++i) {
-          seen = ld_acquire(p.flags + (peer0 + tid) * kWide + rank) != 0;
+          seen = ld_acquire(p.flags + peer * kWide + rank) != 0;
           if (!seen) __nanosleep(100);
         }
         if (!seen) { *abort_flag = 1; atomicCAS(p.status, 0, ST_PEER_TIMEOUT); }
@@ -614,7 +614,7 @@ template <class S> struct Cta {
       if (tid == 0) { __threadfence(); st_release(p.flags + worker * kWide + rank, 1); }
     } else if (!whole) {
       if (!producer_sync()) return false;    // every thread has read the peers' tiles
-      if (tid < worker - peer0) p.flags[(peer0 + tid) * kWide + rank] = 0;   // leave the flags clear for the next launch
+      for (int peer = peer0 + tid; peer < worker; peer += S::PW * 32) p.flags[peer * kWide + rank] = 0;   // leave the flags clear for the next launch
     }
     tcgen05_fence_before();
     __syncwarp();

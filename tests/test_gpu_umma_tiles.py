@@ -62,3 +62,16 @@ def test_split_cuts(qtype, k, dtype):
     for m, n in ((24, 5000), (64, 2100), (100, 5000), (128, 19500), (129, 1000), (257, 5003), (300, 19000)):
         x, w, wd = _case(qtype, dtype, m, n, k)
         _close(kernels.gemm_rcr(x, w, qtype), x.double() @ wd.T, dtype, 2)
+
+
+@pytest.mark.parametrize("qtype,m,n,k", [("Q4_K", 16, 100, 256 * 2400), ("Q4_0", 24, 100, 256 * 1200 + 32)])
+def test_a_tile_in_more_pieces_than_producer_threads(qtype, m, n, k):
+    """One tile of a very long K over all SMs, two CTAs each: 296 pieces, and 256 threads that look after them.  (Ordinary and split operands.)"""
+    x, w, wd = _case(qtype, "bfloat16", m, n, k)
+    ref = x.double() @ wd.T
+    del wd
+    variant = "umma" if k % 256 == 0 else "auto"
+    results = [kernels.gemm_rcr(x, w, qtype, variant=variant) for _ in range(4)]          # a flag that stayed up would reach the next launch
+    for y in results:
+        _close(y, ref, "bfloat16", 8)
+        assert torch.equal(y.view(torch.int16), results[0].view(torch.int16))
