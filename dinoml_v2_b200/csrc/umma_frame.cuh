@@ -41,10 +41,10 @@ constexpr int kBK = 64;                // K per pipeline stage (one 128-byte swi
 constexpr int kStagesPerSb = 4;         // 256 weights / kBK
 constexpr int kWSlotCols = kBK / 2;     // 64 16-bit values per lane = 32 columns
 constexpr int kSmemBudget = 227 * 1024, kSmemHalf = 113 * 1024;      // of a CTA alone on its SM, of two
-constexpr uint32_t kSpinLimit = 1u << 22;   // try_wait polls before a wait gives up: some fifteen seconds (a launch may stand behind a long one)
+constexpr uint32_t kSpinLimit = 1u << 24;   // try_wait polls before a wait gives up (a launch may stand behind a long one)
 
 enum : int { ST_OK = 0, ST_EMPTY_TIMEOUT = 1, ST_FULL_TIMEOUT = 2, ST_ACC_TIMEOUT = 3, ST_PEER_TIMEOUT = 4 };
-constexpr uint32_t kFlagSpinLimit = 1u << 22;   // polls (100 ns apart) of another CTA's partial-tile flag
+constexpr uint32_t kFlagSpinLimit = 1u << 23;   // polls (100 ns apart) of another CTA's partial-tile flag
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
