@@ -1,8 +1,7 @@
 // Host side of the tcgen05 prefill GEMM: per-(device, stream) scratch, the stream-K plan, the allocation-free scratch and the
 // entry that checks a problem and hands it to the weight type's translation unit.  The kernel is in umma_gemm.cuh.
-#include <array>
+#include <atomic>
 #include <cmath>
-#include <map>
 #include <mutex>
 
 #include "umma_gemm.cuh"
@@ -40,57 +39,57 @@ static UmmaScratch* device_state(size_t need_workspace, cudaStream_t stream) {
   return &st;
 }
 
-static int current_sm_count() {
-  int sm_count = 148, dev = 0;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  return sm_count;
-}
-
 // Clusters of `size` CTAs that the current device runs at once, with one or two CTAs per SM: fewer than the SMs alone would give, since
-// a cluster stays within a GPC (B200, one CTA per SM: 33 clusters of four, 15 of eight).  Asked once per device.
+// a cluster stays within a GPC (B200, one CTA per SM: 33 clusters of four, 15 of eight).
 __global__ void __launch_bounds__(16 * 32 + 96, 1) footprint_of_one() {}
 __global__ void __launch_bounds__(8 * 32 + 96, 2) footprint_of_two() {}
 constexpr int kMostSlices = 16;                                   // CTAs of a cluster: sixteen where the weight has so few tiles that enough clusters fit
-static int max_clusters(int size, int ctas_per_sm) {
-  static std::mutex mutex;
-  static std::map<int, std::array<int, 34>> table;                 // by device: [17 * (ctas_per_sm - 1) + size], -1 = not asked yet
-  int dev = 0;
-  if (size < 1 || size > 16 || cudaGetDevice(&dev) != cudaSuccess) return 0;
-  std::lock_guard<std::mutex> lock(mutex);
-  auto at = table.find(dev);
-  if (at == table.end()) {
-    at = table.emplace(dev, std::array<int, 34>()).first;
-    at->second.fill(-1);
+static int ask_clusters(int size, int ctas_per_sm) {
+  const bool two = ctas_per_sm == 2;
+  void (*kern)() = two ? footprint_of_two : footprint_of_one;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(unsigned(size) * 1024);
+  cfg.blockDim = dim3(two ? 8 * 32 + 96 : 16 * 32 + 96);
+  cfg.dynamicSmemBytes = two ? kSmemHalf : kSmemBudget;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(size);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cfg.dynamicSmemBytes)) != cudaSuccess ||
+      cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    clusters = 0;
   }
-  int& known = at->second[17 * (ctas_per_sm - 1) + size];
-  if (known < 0) {
-    const bool two = ctas_per_sm == 2;
-    void (*kern)() = two ? footprint_of_two : footprint_of_one;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(size) * 1024);
-    cfg.blockDim = dim3(two ? 8 * 32 + 96 : 16 * 32 + 96);
-    cfg.dynamicSmemBytes = two ? kSmemHalf : kSmemBudget;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = unsigned(size);
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int clusters = 0;
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(cfg.dynamicSmemBytes)) != cudaSuccess ||
-        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      clusters = 0;
-    }
-    known = clusters;
-  }
-  return known;
+  return clusters;
 }
+
+// What a plan asks about the current device, looked up once per plan; the counts themselves once per device and size (a plan looks at up to 32 of
+// them, in calls whose kernel takes 5 us).
+struct Device {
+  int dev = 0, sm_count = 148;
+  Device() {
+    if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+    else cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+  }
+  int max_clusters(int size, int ctas_per_sm) const {
+    constexpr int kKept = 64;
+    static std::atomic<int> kept[kKept][2][kMostSlices + 1];         // 1 + the count, 0: not asked yet
+    if (size < 1 || size > kMostSlices || dev < 0) return 0;
+    if (dev >= kKept) return ask_clusters(size, ctas_per_sm);
+    std::atomic<int>& known = kept[dev][ctas_per_sm - 1][size];
+    int value = known.load(std::memory_order_relaxed);
+    if (value == 0) known.store(value = 1 + ask_clusters(size, ctas_per_sm), std::memory_order_relaxed);
+    return value - 1;
+  }
+};
 
 // ctas_per_sm: of the kernel that runs tiles of this height; pairs (bm = 256) are half as many workers.  most_slices: of K, in a cluster.  terms:
 // of a weight, a super-block takes that much longer.
-static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slices, int terms) {
+static Plan plan_for(const Device& device, int m, int n, int k, int bm, int ctas_per_sm, int most_slices, int terms) {
   Plan pl;
   pl.ctas_per_sm = ctas_per_sm;
   const int wide = bm == 256 ? 2 : 1;
@@ -102,7 +101,7 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
   const long long tiles = static_cast<long long>(pl.m_tiles) * ((n + wide * kRowsW - 1) / (wide * kRowsW));
   const int nsb = (k + 255) / 256;
   pl.units = tiles * nsb;
-  const int sm_count = current_sm_count();
+  const int sm_count = device.sm_count;
   int slots = sm_count * ctas_per_sm / wide;
   if (slots * wide > kMaxCtas) slots = kMaxCtas / wide;
   if (slots < 1) slots = 1;
@@ -122,9 +121,9 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
   const float hand_over = ((wide == 2 ? 9.f : ctas_per_sm == 1 ? 7.f : 3.f + float(pl.bn) / 16.f) + 0.4f * float(pl.workers) / float(tiles)) / float(terms);
   float best = float(pl.units * wide) / float(sm_count) + hand_over;
   pl.slices = 0;                                                     // stream-K
-  for (int s = 1; s <= most_slices && s <= nsb && tiles <= max_clusters(s * wide, ctas_per_sm); ++s) {
+  for (int s = 1; s <= most_slices && s <= nsb && tiles <= device.max_clusters(s * wide, ctas_per_sm); ++s) {
     const float load = float(tiles * s * wide) / float(sm_count), own = float(nsb) / float(s);
-    const bool alone = load <= 1.f && tiles <= max_clusters(s * wide, 1);
+    const bool alone = load <= 1.f && tiles <= device.max_clusters(s * wide, 1);
     const float more = fmaxf(load, 1.f), share = alone ? 1.f : s == 1 ? 1.75f : fminf(1.75f, sqrtf(more * sqrtf(more)) + own / 64.f);
     const float cost = 0.5f * (float((nsb + s - 1) / s) + own) * share + (s > 1 ? join + each * float(s) : 0.f);
     if (cost < best) { pl.slices = s; best = cost; }
@@ -143,23 +142,24 @@ static Plan plan_for(int m, int n, int k, int bm, int ctas_per_sm, int most_slic
 
 static int tile_height(int m) { return m <= 64 ? 64 : m <= 128 ? 128 : 256; }
 static Plan make_plan(int qtype, int m, int n, int k) {
-  const int bm = tile_height(m), tiles = (n + kRowsW - 1) / kRowsW, sms = current_sm_count();
+  const Device device;
+  const int bm = tile_height(m), tiles = (n + kRowsW - 1) / kRowsW, sms = device.sm_count;
   const bool eight = eight_fit(qtype, bm) && (bm == 64 || (2 * tiles > sms && tiles <= sms && k <= 16 * 256));
-  return plan_for(m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), 1);
+  return plan_for(device, m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), 1);
 }
 // What the built-in scratch takes is decided by this figure: a partial tile of whole height on every SM, where a tile count that the SMs do
 // not divide needs one.
 static size_t nominal_workspace(int m, int n, int k) {
   const int bm = tile_height(m), nsb = (k + 255) / 256;
   const long long tiles = static_cast<long long>((m + bm - 1) / bm) * ((n + kRowsW - 1) / kRowsW), most = tiles * nsb / 4;
-  const int sm_count = current_sm_count();
+  const int sm_count = Device().sm_count;
   const long long ctas = most < 1 ? 1 : most < sm_count ? most : sm_count;
   return tiles % ctas == 0 ? 0 : size_t(ctas) * bm * kRowsW * sizeof(float);
 }
 
 // For the split-operand kernels (umma_split.cu): the same plan at their tile height, the same scratch.
 Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms) {
-  return plan_for(m, n, k, bm, ctas_per_sm, !sliced ? 1 : kMostSlices / (bm == 256 ? 2 : 1), terms);
+  return plan_for(Device(), m, n, k, bm, ctas_per_sm, !sliced ? 1 : kMostSlices / (bm == 256 ? 2 : 1), terms);
 }
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc) {
   UmmaScratch* st = device_state(workspace_bytes, stream);
