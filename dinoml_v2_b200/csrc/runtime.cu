@@ -993,6 +993,12 @@ int dino_session_get_graph_stats(DinoSession* session, size_t* cached_graphs, si
   if (graph_launches) *graph_launches = session->graph_launches;
   return 0;
 }
+int dino_session_get_branched_graphs(DinoSession* session, size_t* branched_graphs) {
+  if (session == nullptr || branched_graphs == nullptr) return fail("dino_session_get_branched_graphs received null pointer");
+  *branched_graphs = 0;
+  for (const auto& entry : session->graphs) *branched_graphs += entry.second.exec != nullptr && entry.second.branches ? 1 : 0;
+  return 0;
+}
 
 static int launch_graph(DinoSession* s, DinoSession::CachedGraph& cg) {
   cudaError_t err = cudaGraphLaunch(cg.exec, s->stream);

@@ -49,6 +49,7 @@ def _configure(lib: ctypes.CDLL) -> None:
         "dino_session_run_staged": [vp, vp, vp, sz, T, sz, T, sz, vp, vp, sz],
         "dino_session_run_staged_on": [vp, vp, ci, vp, vp, sz, T, sz, T, sz, vp, vp, sz],
         "dino_session_set_graph_replay": [vp, ci], "dino_session_get_graph_stats": [vp, ctypes.POINTER(sz), ctypes.POINTER(sz)],
+        "dino_session_get_branched_graphs": [vp, ctypes.POINTER(sz)],
     }.items():
         fn = getattr(lib, name)
         fn.argtypes, fn.restype = args, ci

@@ -107,6 +107,8 @@ DINOML_B200_API int dino_session_release_temp_arena(struct DinoSession* session)
 DINOML_B200_API int dino_session_get_state_pointer(struct DinoSession* session, size_t state_index, void** out_data);
 DINOML_B200_API int dino_session_set_graph_replay(struct DinoSession* session, int enabled);
 DINOML_B200_API int dino_session_get_graph_stats(struct DinoSession* session, size_t* cached_graphs, size_t* graph_launches);
+/* How many of the cached graphs run linears that do not read one another's results side by side. */
+DINOML_B200_API int dino_session_get_branched_graphs(struct DinoSession* session, size_t* branched_graphs);
 /* :995 / :706-993 - validates every tensor, then launches the plan on the session stream.  With DINOML_PROFILE_RUN set every
  * launch is bracketed by events and "[dinoml_profile] ..." lines go to stderr (DINOML_PROFILE_RUN_VERBOSE: one line per launch;
  * DINOML_PROFILE_RUN_SECTIONS=name:first:last,...: elapsed time of launch ranges), as gpu_module.cu.j2:785-983. */
