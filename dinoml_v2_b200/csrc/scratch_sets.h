@@ -38,7 +38,7 @@ struct StreamScratch {
 };
 
 // tcgen05 GEMMs: partial tiles, and the status word followed by a flag per CTA.
-constexpr int kUmmaMaxCtas = 1024;    // flag words per set; the grid never exceeds the SM count
+constexpr int kUmmaMaxCtas = 1024;    // flag words per set: a stream-K launch has at most so many CTAs (up to two per SM), and only those use flags
 struct UmmaScratch {
   int* status = nullptr;            // [0] = status word, [1 .. kUmmaMaxCtas] = partial-tile flags
   float* workspace = nullptr;

@@ -304,7 +304,7 @@ template <class S> struct Cta {
   uint32_t epi_phase = 0;
 
   // Barriers: full[NB], empty[NB], rawfull[NRAW], rawfree[NRAW], accumulator full, accumulator free, drain, epilogue.  A unit is "full"
-  // when its 8 producer warps have written the weight tiles AND the activation tiles' bytes have landed (one barrier, one
+  // when its producer warps (FILL, 8 if teams share) have written the weight tiles AND the activation tiles' bytes have landed (one barrier, one
   // wait for the MMA warp); it is "empty" when the MMAs that read it have completed (one tcgen05.commit, watched by
   // producers and TMA).  In a pair the even CTA's `full` and `accumulator free` count both CTAs.
   __device__ __forceinline__ uint32_t full(int u) const { return bar0 + 8u * u; }

@@ -7,8 +7,9 @@
 // The frame is umma_frame.cuh's.  Packed bytes: a 2-D byte tensor map over the weight, one box (Q8_0: two) of 128 rows x the 16-byte aligned
 // window around a 256-weight super-block; no thread spends issue slots on the copy.  The producers copy their own words to registers,
 // release the ring slot, then unpack with 32-bit logic + packed bf16x2/f16x2 math: thread (row = 32*(warp%4)+lane, half = (warp%8)/4)
-// unpacks 64 weights of one half of the super-block (PW = 8: of both, one after the other) and writes them to its TMEM lane; then
-// tcgen05.wait::st + mbarrier arrive.  The warps only meet at mbarriers, never at a CTA barrier.
+// unpacks the 128 weights of its half of the super-block, one K stage after the other, and writes them to its TMEM lane; then
+// tcgen05.wait::st + mbarrier arrive.  Sixteen warps are two teams of eight that take turns, or, where a worker has few super-blocks, share each: team
+// = half, and a thread unpacks one K stage.  The warps only meet at mbarriers, never at a CTA barrier.
 // The packed-weight tensor map needs weight rows that are multiples of 16 bytes: any K % 256 == 0 for the types whose 256
 // weights take a multiple of 16 bytes, K % 512 == 0 for MXFP4 (136 bytes), K % 1024 == 0 for Q2_K (84), K % 2048 == 0 for
 // Q6_K (210) and Q3_K (110).  Other

@@ -15,8 +15,8 @@
 //   * K may be any multiple of the block (the tail of the last super-block counts as zero);
 //   * a result that is not finite is computed again weight by weight: two or three parts of a weight make Inf - Inf of an
 //     infinite activation, and a weight or its scale (times 32) may be beyond float16.
-// Tensor memory holds the accumulator and TERMS slots for four stages, so a tile has up to 256 activation rows with one or two terms and
-// 128 with three.
+// Tensor memory holds the accumulator and a ring of stages, TERMS slots each: up to 256 activation rows (in pairs) with a ring of at least a
+// super-block for one or two terms, of two stages for three.
 #pragma once
 #include "gemm_exact.cuh"
 #include "gemv_stream_common.cuh"
