@@ -491,8 +491,8 @@ template <class S> struct Cta {
   }
 
   // ------------------------------------------------------------------ packed weights
-  // load(slot address, barrier, super-block, part, weight row): called by the converged warp once the slot is free.
-  template <int PARTS, typename Load>
+  // load(slot address, barrier, super-block, weight row): called by the converged warp once the slot is free.
+  template <typename Load>
   __device__ __forceinline__ void load_weights(Load load) const {
     Ring r{0, 0u};
     int issued = 0;
@@ -501,15 +501,13 @@ template <class S> struct Cta {
       int sb_b, sb_e;
       walk.segment(t, sb_b, sb_e);
       const int n0 = row0(t);
-      for (int sb = sb_b; sb < sb_e && ok; ++sb)
-#pragma unroll
-        for (int part = 0; part < PARTS; ++part) {
-          if (!wait(rawfree(r.at), r.phase ^ 1u, ST_EMPTY_TIMEOUT)) { ok = false; break; }
-          load(smem_u32(raw) + uint32_t(r.at * S::RAW_BYTES), rawfull(r.at), sb, part, n0);
-          __syncwarp();
-          ++issued;
-          r.step(1, S::NRAW);
-        }
+      for (int sb = sb_b; sb < sb_e && ok; ++sb) {
+        if (!wait(rawfree(r.at), r.phase ^ 1u, ST_EMPTY_TIMEOUT)) { ok = false; break; }
+        load(smem_u32(raw) + uint32_t(r.at * S::RAW_BYTES), rawfull(r.at), sb, n0);
+        __syncwarp();
+        ++issued;
+        r.step(1, S::NRAW);
+      }
     }
     if (*abort_flag) {
       for (int i = max(0, issued - S::NRAW); i < issued; ++i) mbar_wait_plain(rawfull(i % S::NRAW), uint32_t(i / S::NRAW) & 1u);

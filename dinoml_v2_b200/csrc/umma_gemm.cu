@@ -145,7 +145,16 @@ static Plan make_plan(int qtype, int m, int n, int k) {
   const Device device;
   const int bm = tile_height(m), tiles = (n + kRowsW - 1) / kRowsW, sms = device.sm_count;
   const bool eight = eight_fit(qtype, bm) && (bm == 64 || (2 * tiles > sms && tiles <= sms && k <= 16 * 256));
-  return plan_for(device, m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), 1);
+  Plan pl = plan_for(device, m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), 1);
+  if (qtype == QTYPE_Q8_0) {
+    // A Q8_0 row has a scale per 32 weights and nothing that two threads would both unpack, but twice the bytes: up to 64 rows its teams take turns, so
+    // that the ring holds two super-blocks for each (us, shared / turns: [6144 x 4096], M = 16 13.5 / 12.5, [28672 x 4096] 38.0 / 35.3); above, the ring is two
+    // in all, and where workers cut tiles both teams take every one ([28672 x 4096], M = 100 42.8 / 44.1, M = 129 47.6 / 48.9, [3000 x 7168], M = 700 35.2 / 35.9).
+    const bool stream_k = pl.slices == 1 && pl.workers != pl.units / ((k + 255) / 256);
+    const long long each = stream_k ? pl.units / pl.workers : ((k + 255) / 256 + pl.slices - 1) / pl.slices;
+    pl.shared = each <= (bm == 64 ? 1 : bm == 128 || stream_k ? 32 : 12);
+  }
+  return pl;
 }
 // What the built-in scratch takes is decided by this figure: a partial tile of whole height on every SM, where a tile count that the SMs do
 // not divide needs one.

@@ -26,20 +26,21 @@ namespace b200gguf {
 namespace umma {
 
 // Rings of a tile height: a hand-over unit is half a super-block, two stages.  kFits: whether they fit, with two CTAs on an SM (PW = 8) a ring of
-// two packed slots beside the stage ring that half of the tensor memory holds.
+// two packed super-blocks beside the stage ring that half of the tensor memory holds.  Q8_0 (272 bytes) has no room for them there.
 template <int QT, int BM, int PW> struct Geo {
   static constexpr bool kPair = BM == 256;
-  static constexpr int kBoxes = RawGeom<QT>::kBoxes, kPart = kRowsW * RawGeom<QT>::kPitch;
-  static constexpr int NB = PW == 8 ? (256 - BM) / (2 * kWSlotCols) : BM == 64 ? 6 : 4;
+  static constexpr int kPart = kRowsW * RawGeom<QT>::kPitch * RawGeom<QT>::kBoxes;
+  static constexpr int NB = PW == 8 ? (256 - BM) / (2 * kWSlotCols) : 4;
   static constexpr int kUnit = 2 * (kPair ? BM / 2 : BM) * kBK * 2, kRest = 1024 + 512;
   static constexpr int kFit = ((PW == 8 ? kSmemHalf : kSmemBudget) - kRest - NB * kUnit) / kPart;
   static constexpr bool kFits = kFit >= 2 && !(kPair && PW == 8);
-  static constexpr int kEach = PW / 8 * kBoxes;             // slots of a lap's turn: a slot belongs to the same team on every lap
+  static constexpr int kEach = PW / 8;                      // slots of a lap's turn: a slot belongs to the same team on every lap
   static constexpr int kSlots = kFit < 6 ? kFit : 6, NRAW = !kFits ? 2 : PW == 8 ? kSlots : kSlots / kEach * kEach;
   template <typename T> using Of = Shape<T, BM, PW, kPair, 1, 2, NB, NRAW, kPart, 8, 4>;
 };
 // Producer warps of a launch.  Up to 64 activation rows the producers are the bound, and two CTAs of eight on an SM pay ([28672 x 8192]
-// Q4_K, M = 16: 39 us against 43).  Above that the stage ring of half an SM is short, and they pay only for weights of more than half as many
+// Q4_K, M = 16: 39 us against 43), but for Q8_0: with one and a half super-blocks in the ring of half an SM it was 5 - 17 % slower than sixteen warps with
+// four in theirs ([28672 x 4096], M = 16: 40.7 us against 35.3; [8192 x 28672] 70.1 against 55.8; [14336 x 4096], M = 128 31.0 against 24.9).  Above that the stage ring of half an SM is short, and they pay only for weights of more than half as many
 // tiles as SMs, which K slices of whole SMs cannot serve, and a short K ([11008 x 4096], M = 100: 17.1 us against 19.0; [5760 x 4096] 13.2
 // against 13.0).
 template <int QT> constexpr bool eight_fit(int bm) { return bm == 64 ? Geo<QT, 64, 8>::kFits : bm == 128 && Geo<QT, 128, 8>::kFits; }
@@ -49,7 +50,7 @@ template <int QT, typename T, int BM, bool SCATTER, int PW>
 __global__ void __launch_bounds__(Geo<QT, BM, PW>::template Of<T>::kThreads, Geo<QT, BM, PW>::template Of<T>::kCtasPerSm)
 gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap w_map, const __grid_constant__ Params p) {
   using S = typename Geo<QT, BM, PW>::template Of<T>;
-  constexpr int kPitch = RawGeom<QT>::kPitch, kBoxes = RawGeom<QT>::kBoxes, kBlockBytes = RawGeom<QT>::kSuper;
+  constexpr int kPitch = RawGeom<QT>::kPitch, kBoxes = RawGeom<QT>::kBoxes, kBlockBytes = RawGeom<QT>::kSuper, kBox = kRowsW * kPitch;
   extern __shared__ uint8_t smem_raw[];
   Cta<S> cta(p, smem_raw);
   const int warp = cta.warp, lane = cta.lane;
@@ -68,7 +69,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
     const int stride = shared ? 1 : S::kTeams;                  // this warp's super-blocks: every stride-th
     int turn = shared ? 0 : team;                               // super-blocks until its next one
     typename Cta<S>::Ring raw{0, 0u}, unit{0, 0u};
-    raw.step(turn * kBoxes, S::NRAW);
+    raw.step(turn, S::NRAW);
     unit.step(turn * 2 + half, S::NB);
     for (int t = cta.tile_hi; t >= cta.tile_lo && alive; --t, ++segi) {
       int sb_b, sb_e;
@@ -77,14 +78,8 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         if (S::kTeams > 1 && turn-- > 0) continue;
         turn = stride - 1;
         if (!cta.wait(cta.rawfull(raw.at), raw.phase, ST_FULL_TIMEOUT)) { alive = false; break; }
-        const int slot0 = raw.at;
-        if (kBoxes == 2) {                                      // Q8_0: a warp waits for both boxes and frees both, so that it misses no lap of a slot
-          raw.step(1, S::NRAW);
-          if (!cta.wait(cta.rawfull(raw.at), raw.phase, ST_FULL_TIMEOUT)) { alive = false; break; }
-          if (lane == 0) mbar_arrive(cta.rawfree(half == 0 ? raw.at : slot0));      // the other half's box: seen, not read
-        }
-        const int slot = kBoxes == 2 && half == 0 ? slot0 : raw.at;
-        const uint8_t* rowbase = cta.raw + slot * S::RAW_BYTES + row * kPitch;
+        const int slot = raw.at;
+        const uint8_t* rowbase = cta.raw + slot * S::RAW_BYTES + (kBoxes == 2 ? half * kBox : 0) + row * kPitch;
         using H = Half<QT, T>;
         H w;
         auto words_read = [&]() {                               // every lane holds its words: the ring slot may be refilled
@@ -126,7 +121,7 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         tcgen05_fence_before();
         __syncwarp();
         if (lane == 0) cta.arrive_lead(cta.full(unit.at));
-        raw.step((stride - 1) * kBoxes + 1, S::NRAW);
+        raw.step(stride, S::NRAW);
         unit.step(2 * stride, S::NB);
         // The previous segment's epilogue runs only now, after the first super-block of this segment has been unpacked (the ring holds it):
         // the MMA warp finds its next weight tiles ready the moment the accumulator is handed back.
@@ -150,12 +145,13 @@ gemm_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
   } else if (warp == PW + 1) {
     cta.issue_mmas();
   } else {
-    cta.template load_weights<kBoxes>([&](uint32_t slot, uint32_t bar, int sb, int part, int n0) {
+    cta.load_weights([&](uint32_t slot, uint32_t bar, int sb, int n0) {
       if (elect_one()) {
         mbar_arrive_expect_tx(bar, uint32_t(S::RAW_BYTES));
         // x coordinate = block start rounded down to 16 bytes; rows past N and bytes past the row end read as zero.  The second box of Q8_0:
         // blocks 4..7 start 8 bytes in
-        tma_load_2d(slot, &w_map, bar, kBoxes == 2 ? sb * kBlockBytes + 128 * part : (sb * kBlockBytes) & ~15, n0);
+        tma_load_2d(slot, &w_map, bar, (sb * kBlockBytes) & ~15, n0);
+        if (kBoxes == 2) tma_load_2d(slot + uint32_t(kBox), &w_map, bar, sb * kBlockBytes + 128, n0);
       }
     });
   }
@@ -245,8 +241,7 @@ constexpr bool eight_fit(int qtype, int bm) {
 template <int QT, typename T>
 int launch_dtype(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, const Plan& pl, Scratch sc, const PeerOut& peers,
                  cudaStream_t s) {
-  static_assert(Geo<QT, 64, 8>::kFits, "two CTAs per SM");
-  if (pl.bm == 64) return launch<QT, T, 64, 8>(a, b, bias, c, m, n, k, pl, sc, peers, s);
+  if (pl.bm == 64) return launch<QT, T, 64, Geo<QT, 64, 8>::kFits ? 8 : 16>(a, b, bias, c, m, n, k, pl, sc, peers, s);
   if (pl.bm == 256) return launch<QT, T, 256, 16>(a, b, bias, c, m, n, k, pl, sc, peers, s);
   if constexpr (Geo<QT, 128, 8>::kFits)
     if (pl.ctas_per_sm == 2) return launch<QT, T, 128, 8>(a, b, bias, c, m, n, k, pl, sc, peers, s);

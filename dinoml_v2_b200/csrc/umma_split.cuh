@@ -270,7 +270,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
   } else if (warp == PW + 1) {
     cta.issue_mmas();
   } else {
-    cta.template load_weights<1>([&](uint32_t slot, uint32_t bar, int sb, int, int n0) {
+    cta.load_weights([&](uint32_t slot, uint32_t bar, int sb, int n0) {
       // lane r < residues: the box of the rows r, r + residues, ... (16-bit elements: Q8_0 windows are wider than 256 bytes).  In a tile
       // that reaches past the full groups the residues which the last group still has take its map; what a map does not hold is zero.
       if (lane == 0) mbar_arrive_expect_tx(bar, uint32_t(S::RAW_BYTES));

@@ -38,7 +38,7 @@ __device__ __forceinline__ void fetch(const uint8_t* aligned, uint32_t* out) {
 // 16-byte aligned) are wider than a TMA box may be (256 elements), so they travel as two boxes of 144 B: blocks 0..3
 // start at byte 0 of the first, blocks 4..7 at byte 8 of the second (which starts at byte 128 of the 272).  Every pitch
 // is an odd number of 16-byte chunks, so 16-byte reads of 8 consecutive rows hit all 32 banks.
-//   kSuper: packed bytes per 256 weights of a row; kBoxes: TMA boxes per super-block, each in a ring slot of its own.
+//   kSuper: packed bytes per 256 weights of a row; kBoxes: TMA boxes per super-block, one behind the other in its ring slot.
 template <int QT> struct RawGeom;
 template <> struct RawGeom<QTYPE_Q4_K> { static constexpr int kPitch = 144, kSuper = 144, kBoxes = 1; };
 template <> struct RawGeom<QTYPE_Q5_K> { static constexpr int kPitch = 176, kSuper = 176, kBoxes = 1; };   // Q4_K + 32 bytes of fifth bits
