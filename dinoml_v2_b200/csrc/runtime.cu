@@ -162,6 +162,9 @@ struct DinoSession {
   size_t graph_generation = 0;
   std::vector<int64_t> pending_key;     // combination of the run in progress; counted as seen once that run has succeeded
   b200gguf::SideStreams sides;          // replayed runs: linears that do not need one another's results run side by side on these
+  bool staged = false;                  // the run in progress is a staged one, which is waited for on whatever stream it is
+  // The issuing stream that a run's side streams go by: runs that are waited for never overlap, and share a set whatever their streams.
+  cudaStream_t issuing() const { return external_stream && !staged ? stream : owned_stream; }
 };
 
 namespace {
@@ -537,7 +540,7 @@ struct Branches {
   int rc = 0;
   Branches(DinoSession* session, std::vector<int> branch) : s(session), of(std::move(branch)) {
     if (of.empty()) return;
-    set = s->sides.at(s->stream);       // there already: reserve_sides()
+    set = s->sides.at(s->issuing());    // there already: reserve_sides()
     if (set == nullptr || cudaEventRecord(set->forked, s->stream) != cudaSuccess) { cudaGetLastError(); of.clear(); return; }
     for (int b : of)
       if (b > 0 && !used[b - 1]) {
@@ -1003,20 +1006,19 @@ int dino_session_get_branched_graphs(DinoSession* session, size_t* branched_grap
 static int launch_graph(DinoSession* s, DinoSession::CachedGraph& cg) {
   cudaError_t err = cudaGraphLaunch(cg.exec, s->stream);
   ++s->graph_launches;
-  // on its own stream a session waits for every run
-  if (err == cudaSuccess && cg.branches && s->external_stream) err = s->sides.launched(s->stream);
+  if (err == cudaSuccess && cg.branches && s->issuing() == s->stream && s->external_stream) err = s->sides.launched(s->stream);      // else the run is waited for
   return err == cudaSuccess ? 0 : cuda_fail("cudaGraphLaunch", err);
 }
 
 // Before a capture with branches: the streams, and for those that launches go to the workspaces that the ordinary run of the combination
-// has found on the session's stream, which a capture could not make.  That run itself takes the launches one after another: a pass over new buffers pays
+// has found on the run's stream, which a capture could not make.  That run itself takes the launches one after another: a pass over new buffers pays
 // neither for streams and workspaces nor for a dozen event calls that it gains nothing by.  The sides have no work but the clearing of new workspaces, which
 // is waited for here, as the graph runs on another stream.
 static bool reserve_sides(DinoSession* s, const std::vector<int>& branch) {
   if (branch.empty()) return true;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(s->stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) return false;
-  b200gguf::SideStreams::Set* set = s->sides.at(s->stream);
+  b200gguf::SideStreams::Set* set = s->sides.at(s->issuing());
   bool used[b200gguf::SideStreams::kSides] = {};
   for (int b : branch) if (b > 0) used[b - 1] = true;
   for (int i = 0; i < b200gguf::SideStreams::kSides && set != nullptr; ++i)
@@ -1029,18 +1031,19 @@ static bool reserve_sides(DinoSession* s, const std::vector<int>& branch) {
 
 // Steady-state path of dino_session_run: the launch sequence of one (stream, input shapes, input / output pointers) combination is
 // captured the second time it is seen and replayed afterwards; validation ran when it was captured.  Returns 1 if the
-// call was served (rc in *rc_out), 0 if the caller should run the plan the ordinary way.  side: with branches in the graph.
-static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs, bool side, int* rc_out) {
+// call was served (rc in *rc_out), 0 if the caller should run the plan the ordinary way.
+static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inputs, DinoTensor* outputs, size_t num_outputs, int* rc_out) {
   DinoModule& mod = *s->module;
   if (!s->graph_replay || module_streams_constants(mod) || std::getenv("DINOML_PROFILE_RUN") != nullptr ||
       std::getenv("DINOML_PROFILE_RUN_SECTIONS") != nullptr)
     return 0;
   if (num_inputs != mod.inputs.size() || num_outputs != mod.outputs.size() || (num_inputs && !inputs) || (num_outputs && !outputs)) return 0;
   if (s->graph_generation != mod.generation) {             // constant buffers were released since: every captured pointer is stale
-    drop_graphs(s, &s->stream);
+    const cudaStream_t keep = s->issuing();
+    drop_graphs(s, &keep);
     s->graph_generation = mod.generation;
   }
-  std::vector<int64_t> key{int64_t(reinterpret_cast<intptr_t>(s->stream))};
+  std::vector<int64_t> key{int64_t(reinterpret_cast<intptr_t>(s->stream)), int64_t(s->staged)};
   for (size_t i = 0; i < num_inputs; ++i) {
     if (inputs[i].shape == nullptr || inputs[i].data == nullptr) return 0;
     key.push_back(int64_t(reinterpret_cast<intptr_t>(tensor_ptr(inputs[i]))));
@@ -1051,7 +1054,10 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
     if (outputs[i].data == nullptr) return 0;
     key.push_back(int64_t(reinterpret_cast<intptr_t>(tensor_ptr(outputs[i]))));
   }
-  if (s->graphs.size() > 64 && s->graphs.find(key) == s->graphs.end()) drop_graphs(s, &s->stream);     // callers that pass ever-changing buffers: start over
+  if (s->graphs.size() > 64 && s->graphs.find(key) == s->graphs.end()) {     // callers that pass ever-changing buffers: start over
+    const cudaStream_t keep = s->issuing();
+    drop_graphs(s, &keep);
+  }
   DinoSession::CachedGraph& cg = s->graphs[key];
   if (cg.exec != nullptr) {
     s->shapes = cg.out_shapes;
@@ -1064,13 +1070,10 @@ static int run_replayed(DinoSession* s, const DinoTensor* inputs, size_t num_inp
     return 0;
   }
   // seen once, and that run succeeded (every lazily created workspace of the kernels exists): capture this one
-  std::vector<int> branch;
-  if (side) {
-    std::vector<std::vector<int64_t>> shapes(mod.tensors.size());
-    for (size_t i = 0; i < num_inputs; ++i) shapes[mod.inputs[i]].assign(inputs[i].shape, inputs[i].shape + inputs[i].ndim);
-    branch = side_by_side(mod, shapes, tensor_pointers(s, inputs, num_inputs, outputs, num_outputs));
-    if (!reserve_sides(s, branch)) branch.clear();
-  }
+  std::vector<std::vector<int64_t>> shapes(mod.tensors.size());
+  for (size_t i = 0; i < num_inputs; ++i) shapes[mod.inputs[i]].assign(inputs[i].shape, inputs[i].shape + inputs[i].ndim);
+  std::vector<int> branch = side_by_side(mod, shapes, tensor_pointers(s, inputs, num_inputs, outputs, num_outputs));
+  if (!reserve_sides(s, branch)) branch.clear();
   cg.branches = !branch.empty();
   cudaGraph_t graph = nullptr;
   if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { cudaGetLastError(); cg.seen = -1; return 0; }
@@ -1101,7 +1104,7 @@ int dino_session_run(DinoSession* session, const DinoTensor* inputs, size_t num_
   if (session == nullptr) return fail("dino_session_run received null session");
   int replay_rc = 0;
   session->pending_key.clear();
-  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, true, &replay_rc)) {
+  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, &replay_rc)) {
     if (replay_rc != 0) return replay_rc;
   } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true)) {
     return rc;
@@ -1121,6 +1124,11 @@ int dino_session_run_staged(DinoSession* session, const void* host_in, void* dev
   if (session == nullptr) return fail("dino_session_run_staged received null session");
   if ((in_bytes && (host_in == nullptr || device_in == nullptr)) || (out_bytes && (host_out == nullptr || device_out == nullptr)))
     return fail("dino_session_run_staged received a null staging buffer");
+  struct Staged {
+    DinoSession* s;
+    explicit Staged(DinoSession* session) : s(session) { s->staged = true; }
+    ~Staged() { s->staged = false; }
+  } staged(session);
   cudaStream_t stream = session->stream;
   if (in_bytes) {
     const cudaError_t err = cudaMemcpyAsync(device_in, host_in, in_bytes, cudaMemcpyHostToDevice, stream);
@@ -1128,7 +1136,7 @@ int dino_session_run_staged(DinoSession* session, const void* host_in, void* dev
   }
   int replay_rc = 0;
   session->pending_key.clear();
-  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, false, &replay_rc)) {
+  if (run_replayed(session, inputs, num_inputs, outputs, num_outputs, &replay_rc)) {
     if (replay_rc != 0) return replay_rc;
   } else if (int rc = run_plan(session, inputs, num_inputs, outputs, num_outputs, true)) {
     return rc;

@@ -2,7 +2,7 @@
 //
 // Kernels keep workspaces per (device, stream), so whoever launches on these streams, or captures on them, uses the workspaces of these
 // streams.  There is a set of them per issuing stream: launches and captured graphs of one issuing stream are ordered and may share it, those of two
-// streams may overlap and must not.  The work of a captured graph runs on the stream that the graph is launched on, where the side
+// streams may overlap and must not (unless the caller orders them: runs that are waited for).  The work of a captured graph runs on the stream that the graph is launched on, where the side
 // streams' own order says nothing about it; so an event is recorded behind every such launch, and a set is given back only after it.
 #pragma once
 #include <cuda_runtime_api.h>

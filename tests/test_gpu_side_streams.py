@@ -1,5 +1,7 @@
 """Graphs with branches on streams of the caller: runs on two streams that nothing orders, and sessions that are dropped right behind their last run,
 give the bits of launches one after another."""
+import ctypes
+
 import pytest
 import torch
 
@@ -110,3 +112,21 @@ def test_first_pass_makes_no_side_workspaces(module):
 
     plain = taken(False)
     assert taken(True) <= plain + (2 << 20)                             # the driver's granularity; three workspaces a session would be 12 MB
+
+
+def test_host_runs_of_several_shapes_share_their_sides(module):
+    """Host runs have a stream per set of input shapes, and are waited for: their graphs have branches, and one set of side workspaces serves them all."""
+    names = [o["name"] for o in module.metadata["outputs"]]
+    cases = []
+    for m in (1, 5, 17, 64):
+        x, want, _ = _buffers(module, m, 70 + m)
+        torch.cuda.synchronize()
+        cases.append((x["x"].float().cpu().numpy(), {name: want[name].float().cpu() for name in names}))
+    session = module.create_session()
+    for _ in range(4):
+        for x, want in cases:
+            got = session.run_numpy({"x": x})
+            assert all(torch.equal(torch.from_numpy(got[name]), want[name]) for name in names)
+    count = ctypes.c_size_t()
+    module._check(session._lib.dino_session_get_branched_graphs(session._handle, ctypes.byref(count)))
+    assert count.value == len(cases) and session.graph_stats()["graph_launches"] == 3 * len(cases) and kernels.device_status() == 0
