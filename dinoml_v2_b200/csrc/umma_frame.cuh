@@ -457,13 +457,12 @@ template <class S> struct Cta {
       }
       uint32_t accumulate = 0;
       const uint32_t idesc = idesc0 | (uint32_t(tile_rows(t) >> 3) << 17);
-      for (int h = (sb_e - sb_b) * S::kUnits; h > 0; --h) {       // one wait, 4 HS TERMS MMAs, one commit per unit
-        ok = wait(full(u.at), u.phase, ST_FULL_TIMEOUT);
-        if (!ok) break;
+      auto unit = [&](int at) -> bool {                           // one wait, 4 HS TERMS MMAs, one commit per unit
+        if (!wait(full(at), u.phase, ST_FULL_TIMEOUT)) return false;
         tcgen05_fence_after();
         if (elect_one()) {
-          const uint32_t a0 = tmem_base + uint32_t(S::BM + u.at * (S::HS * S::TERMS * kWSlotCols));
-          const uint64_t d0 = db0 + uint64_t(uint32_t(u.at * (S::HS * S::kXTile)) >> 4);
+          const uint32_t a0 = tmem_base + uint32_t(S::BM + at * (S::HS * S::TERMS * kWSlotCols));
+          const uint64_t d0 = db0 + uint64_t(uint32_t(at * (S::HS * S::kXTile)) >> 4);
 #pragma unroll
           for (int i = 0; i < S::HS; ++i)
 #pragma unroll
@@ -474,11 +473,24 @@ template <class S> struct Cta {
                                      idesc, accumulate);
                 accumulate = 1;
               }
-          umma_commit<S::PAIR>(empty(u.at), both);
+          umma_commit<S::PAIR>(empty(at), both);
         }
         accumulate = 1;
         __syncwarp();
-        u.step(1, S::NB);
+        return true;
+      };
+      if constexpr (S::NB == S::kUnits) {                         // a ring of one super-block: every address is a constant
+        for (int sb = sb_b; sb < sb_e && ok; ++sb) {
+#pragma unroll
+          for (int i = 0; i < S::kUnits; ++i)
+            if (ok) ok = unit(i);
+          u.phase ^= 1u;
+        }
+      } else {
+        for (int h = (sb_e - sb_b) * S::kUnits; h > 0 && ok; --h) {
+          ok = unit(u.at);
+          u.step(1, S::NB);
+        }
       }
       if (ok && elect_one()) umma_commit<S::PAIR>(accbar(), both);
       __syncwarp();

@@ -46,7 +46,7 @@ template <int QT, typename T, int BM> struct SplitGeo {
   static constexpr bool kPair = BM == 256;
   static constexpr int PW = !kPair && kTerms * BM <= 128 && !shares_bytes<QT>() ? 8 : 16;
   static constexpr int kPart = kRowsW * exact::raw_pitch<QT>(), kUnit = HS * (kPair ? BM / 2 : BM) * kBK * 2, kRest = 1024 + 512;
-  static constexpr int kColumns = (PW == 8 ? 256 : 512) - BM, kMost = kColumns / (HS * kTerms * kWSlotCols), NB = kMost < 6 ? kMost : 6;
+  static constexpr int kColumns = (PW == 8 ? 256 : 512) - BM, kMost = kColumns / (HS * kTerms * kWSlotCols), kDeep = HS == 1 && PW == 16 ? 4 : 6, NB = kMost < kDeep ? kMost : kDeep;
   static constexpr int kFit = ((PW == 8 ? kSmemHalf : kSmemBudget) - kRest - NB * kUnit) / kPart, NRAW = kFit < 4 ? kFit : 4;
   static constexpr bool kHalf = PW == 8, kLong = NB >= kStagesPerSb / HS, kRun = !kHalf && kLong && shares_bytes<QT>(), kStage = !kHalf && kLong && !kRun;
   using Of = Shape<T, BM, PW, kPair, kTerms, HS, NB, NRAW, kPart, PW, kHalf || (kStage && HS == 1) ? 4 : 8, BM * kRowsW * 4 <= NB * kUnit + NRAW * kPart>;
@@ -162,26 +162,30 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
       pend_t = -1;
       return cta.template epilogue<false, false>(t, pend_b, pend_e, segi - 1, seen);
     };
-    auto slot_free = [&]() -> bool {
-      if (!cta.wait(cta.empty(unit.at), unit.phase ^ 1u, ST_EMPTY_TIMEOUT)) return false;
+    // A ring of one super-block, which a warp's next lap of is its next super-block: its slots are the same in all of them.
+    constexpr bool kFixed = S::NB == kStagesPerSb && HS == 1 && (kRun || kStage);
+    auto slot = [&](int st) { return !kFixed ? unit.at : kRun ? 2 * half + st : 2 * half + stage; };
+    auto slot_free = [&](int st) -> bool {
+      if (!cta.wait(cta.empty(slot(st)), unit.phase ^ 1u, ST_EMPTY_TIMEOUT)) return false;
       tcgen05_fence_after();
       return true;
     };
-    auto signal = [&](int by) {
+    auto signal = [&](int st, int by) {
       tmem_st_wait();
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) cta.arrive_lead(cta.full(unit.at));
-      unit.step(by, S::NB);
+      if (lane == 0) cta.arrive_lead(cta.full(slot(st)));
+      if (!kFixed) unit.step(by, S::NB);
+      else if (!kRun || st == 1) unit.phase ^= 1u;
     };
     // 16 weights (run u of the 32-weight group j of half hb) to the unit's stage `st`
     auto unpack = [&](const Words& w, int i, int at, uint32_t (&out)[TERMS][8]) {
       const bool in = at < p.k;                                        // else past the end of the row
       split16<QT, T, TERMS>(w, i, in ? w.scale[i] : 0.f, in ? w.mn[i] : 0.f, out);
     };
-    auto put = [&](int st, int column, const uint32_t (&out)[TERMS][8]) {
+    auto put = [&](int at, int st, int column, const uint32_t (&out)[TERMS][8]) {       // stage st of the unit in slot `at`
 #pragma unroll
-      for (int tm = 0; tm < TERMS; ++tm) tmem_st8(tmem_a + uint32_t(((unit.at * HS + st) * TERMS + tm) * kWSlotCols + column), out[tm]);
+      for (int tm = 0; tm < TERMS; ++tm) tmem_st8(tmem_a + uint32_t(((at * HS + st) * TERMS + tm) * kWSlotCols + column), out[tm]);
     };
     for (int t = cta.tile_hi; t >= cta.tile_lo && alive; --t, ++segi) {
       int sb_b, sb_e;
@@ -206,16 +210,16 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
             auto group = [&](int i) { unpack(words, 2 * st + i, sb * 256 + 128 * half + 64 * st + 32 * i + 16 * sub, out[i % kEarly]); };
 #pragma unroll
             for (int i = 0; i < kEarly; ++i) group(i);
-            if (!slot_free()) { alive = false; break; }
+            if (!slot_free(st)) { alive = false; break; }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
               if (i >= kEarly) group(i);
-              put(0, 16 * i + 8 * sub, out[i % kEarly]);
+              put(slot(st), 0, 16 * i + 8 * sub, out[i % kEarly]);
             }
-            signal(st == 0 ? 1 : kStep);
-            if (st == 0) alive = epilogue_before(sb == sb_b);
-            if (!alive) break;
+            signal(st, st == 0 ? 1 : kStep);
           }
+          // not between the stages, where the words would have to outlive it; the ring holds a whole super-block
+          if (alive) alive = epilogue_before(sb == sb_b);
         } else if constexpr (kHalf || kStage) {
           Words words[2];
 #pragma unroll
@@ -229,12 +233,12 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
               const int i = piece >> 1, u = piece & 1;
               uint32_t out[TERMS][8];
               unpack(words[u], i, sb * 256 + 128 * half + 64 * mine + 32 * i + 16 * u, out);
-              if (piece == 0 && (HS == 1 || st == 0) && !slot_free()) { alive = false; break; }
-              put(HS == 2 ? mine : 0, 16 * i + 8 * u, out);
+              if (piece == 0 && (HS == 1 || st == 0) && !slot_free(st)) { alive = false; break; }
+              put(slot(st), HS == 2 ? mine : 0, 16 * i + 8 * u, out);
             }
             if (!alive) break;
             if (HS == 1 || !kHalf || st == 1) {
-              signal(kHalf && HS == 1 && st == 0 ? 1 : kStep);
+              signal(st, kHalf && HS == 1 && st == 0 ? 1 : kStep);
               if (st == 0 || HS == 2) alive = epilogue_before(sb == sb_b);
             }
             if (!alive) break;
@@ -246,14 +250,14 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_consta
             Words words;
             words.load(block, hb, 2 * team, sub);
             if (hb == 1) words_read();
-            if (!slot_free()) { alive = false; break; }
+            if (!slot_free(hb)) { alive = false; break; }
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
               uint32_t out[TERMS][8];
               unpack(words, i, sb * 256 + 128 * hb + 64 * team + 32 * i + 16 * sub, out);
-              put(0, 16 * i + 8 * sub, out);
+              put(slot(hb), 0, 16 * i + 8 * sub, out);
             }
-            signal(kStep);
+            signal(hb, kStep);
             if (hb == 0) alive = epilogue_before(sb == sb_b);
           }
         }
