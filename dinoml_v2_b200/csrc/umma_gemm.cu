@@ -88,8 +88,8 @@ struct Device {
 };
 
 // ctas_per_sm: of the kernel that runs tiles of this height; pairs (bm = 256) are half as many workers.  most_slices: of K, in a cluster.  terms:
-// of a weight, a super-block takes that much longer.
-static Plan plan_for(const Device& device, int m, int n, int k, int bm, int ctas_per_sm, int most_slices, int terms) {
+// of a weight, a super-block takes that much longer.  *cost: super-blocks that the plan takes the time of.
+static Plan plan_for(const Device& device, int m, int n, int k, int bm, int ctas_per_sm, int most_slices, float terms, float* cost_of_plan = nullptr) {
   Plan pl;
   pl.ctas_per_sm = ctas_per_sm;
   const int wide = bm == 256 ? 2 : 1;
@@ -117,8 +117,8 @@ static Plan plan_for(const Device& device, int m, int n, int k, int bm, int ctas
   // (stream-K: at least four super-blocks per worker, a small problem is not cut into more pieces than its finishers can add up quickly.)
   const long long most = pl.units / 4 > 1 ? pl.units / 4 : 1;
   pl.workers = int(most < slots ? most : slots);
-  const float join = (wide == 2 ? 1.f : 0.f) / float(terms), each = (wide == 2 ? 0.7f : 0.3f) / float(terms);
-  const float hand_over = ((wide == 2 ? 9.f : ctas_per_sm == 1 ? 7.f : 3.f + float(pl.bn) / 16.f) + 0.4f * float(pl.workers) / float(tiles)) / float(terms);
+  const float join = (wide == 2 ? 1.f : 0.f) / terms, each = (wide == 2 ? 0.7f : 0.3f) / terms, pieces = float(pl.workers) / float(tiles);
+  const float hand_over = ((wide == 2 ? 9.f : ctas_per_sm == 1 ? 7.f : 3.f + float(pl.bn) / 16.f) + 0.4f * pieces) / terms;
   float best = float(pl.units * wide) / float(sm_count) + hand_over;
   pl.slices = 0;                                                     // stream-K
   for (int s = 1; s <= most_slices && s <= nsb && tiles <= device.max_clusters(s * wide, ctas_per_sm); ++s) {
@@ -128,6 +128,7 @@ static Plan plan_for(const Device& device, int m, int n, int k, int bm, int ctas
     const float cost = 0.5f * (float((nsb + s - 1) / s) + own) * share + (s > 1 ? join + each * float(s) : 0.f);
     if (cost < best) { pl.slices = s; best = cost; }
   }
+  if (cost_of_plan != nullptr) *cost_of_plan = best;
   if (pl.slices > 0) {
     pl.workers = int(tiles);
     pl.shared = (nsb + pl.slices - 1) / pl.slices <= 12;
@@ -145,7 +146,8 @@ static Plan make_plan(int qtype, int m, int n, int k) {
   const Device device;
   const int bm = tile_height(m), tiles = (n + kRowsW - 1) / kRowsW, sms = device.sm_count;
   const bool eight = eight_fit(qtype, bm) && (bm == 64 || (2 * tiles > sms && tiles <= sms && k <= 16 * 256));
-  Plan pl = plan_for(device, m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), 1);
+  // (a Q8_0 super-block takes a quarter longer than the others where the activations are not the bound: [11008 x 4096], M = 65: whole 22.8 us, stream-K 22.4)
+  Plan pl = plan_for(device, m, n, k, bm, eight ? 2 : 1, kMostSlices / (bm == 256 ? 2 : 1), qtype == QTYPE_Q8_0 && bm == 128 ? 1.25f : 1.f);
   if (qtype == QTYPE_Q8_0) {
     // A Q8_0 row has a scale per 32 weights and nothing that two threads would both unpack, but twice the bytes: up to 64 rows its teams take turns, so
     // that the ring holds two super-blocks for each (us, shared / turns: [6144 x 4096], M = 16 13.5 / 12.5, [28672 x 4096] 38.0 / 35.3); above, the ring is two
@@ -167,8 +169,8 @@ static size_t nominal_workspace(int m, int n, int k) {
 }
 
 // For the split-operand kernels (umma_split.cu): the same plan at their tile height, the same scratch.
-Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms) {
-  return plan_for(Device(), m, n, k, bm, ctas_per_sm, !sliced ? 1 : kMostSlices / (bm == 256 ? 2 : 1), terms);
+Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms, float* cost) {
+  return plan_for(Device(), m, n, k, bm, ctas_per_sm, !sliced ? 1 : kMostSlices / (bm == 256 ? 2 : 1), float(terms), cost);
 }
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc) {
   UmmaScratch* st = device_state(workspace_bytes, stream);

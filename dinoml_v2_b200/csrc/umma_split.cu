@@ -4,19 +4,37 @@
 namespace b200gguf {
 namespace umma {
 
-Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms);                                          // umma_gemm.cu
+Plan split_plan(int m, int n, int k, int bm, int ctas_per_sm, bool sliced, int terms, float* cost);                             // umma_gemm.cu
 int split_state(size_t workspace_bytes, cudaStream_t stream, Scratch* sc);
 
 template <int QT, typename T, int BM>
+static Plan plan_bm(int m, int n, int k, float* cost = nullptr) {
+  using G = SplitGeo<QT, T, BM>;
+  return split_plan(m, n, k, BM, G::Of::kCtasPerSm, G::Of::SLICED, G::kTerms, cost);
+}
+template <int QT, typename T, int BM>
 static int run_bm(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
-  const Plan pl = split_plan(m, n, k, BM, SplitGeo<QT, T, BM>::Of::kCtasPerSm, SplitGeo<QT, T, BM>::Of::SLICED, SplitGeo<QT, T, BM>::kTerms);
+  const Plan pl = plan_bm<QT, T, BM>(m, n, k);
   Scratch sc;
   if (int rc = split_state(pl.workspace_bytes, s, &sc)) return rc;
   return launch_split<QT, T, BM>(a, b, bias, c, m, n, k, pl, sc, s);
 }
+// More than 128 rows go to pairs, unless there are so few weight tiles that tiles of half as many rows, which unpack a weight twice, fill the SMs
+// better: a super-block takes 1.2 - 1.4 times as long in a pair as in a CTA of 128 rows, and the rings of two and three terms of Q2_K and Q3_K are too short for K
+// slices of pairs.  us, pairs / 128 rows: Q2_K bfloat16 [300 x 2816], M = 200 29.4 / 10.5, [1024 x 2816] 28.1 / 12.4, Q6_K 17.0 / 13.3; the other way round Q3_K
+// [5120 x 5376] 40.6 / 45.2, [8192 x 11008], M = 256 90 / 119.  Where the pairs can be sliced, or with two terms, their estimate is high, and the line lower.
+template <int QT, typename T> static bool halves(int m, int n, int k) {
+  if constexpr (split_terms<QT, T>() == 1) return false;
+  float pairs = 0.f, ctas = 0.f;
+  const Plan pl = plan_bm<QT, T, 256>(m, n, k, &pairs);
+  plan_bm<QT, T, 128>(m, n, k, &ctas);
+  constexpr float kLine = split_terms<QT, T>() == 3 && !SplitGeo<QT, T, 256>::Of::SLICED ? 0.97f : 0.8f;
+  return ctas < kLine * pairs * (1.f + float(pl.bn) / 640.f);
+}
 template <int QT, typename T>
 static int run(const void* a, const void* b, const void* bias, void* c, int m, int n, int k, cudaStream_t s) {
-  return m <= 64 ? run_bm<QT, T, 64>(a, b, bias, c, m, n, k, s) : m <= 128 ? run_bm<QT, T, 128>(a, b, bias, c, m, n, k, s) : run_bm<QT, T, 256>(a, b, bias, c, m, n, k, s);
+  if (m <= 64) return run_bm<QT, T, 64>(a, b, bias, c, m, n, k, s);
+  return m <= 128 || halves<QT, T>(m, n, k) ? run_bm<QT, T, 128>(a, b, bias, c, m, n, k, s) : run_bm<QT, T, 256>(a, b, bias, c, m, n, k, s);
 }
 
 }  // namespace umma

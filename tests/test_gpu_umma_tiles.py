@@ -75,3 +75,12 @@ def test_a_tile_in_more_pieces_than_producer_threads(qtype, m, n, k):
     for y in results:
         _close(y, ref, "bfloat16", 8)
         assert torch.equal(y.view(torch.int16), results[0].view(torch.int16))
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("qtype,k", [("Q6_K", 2816), ("Q2_K", 2816), ("Q3_K", 2560), ("Q8_0", 2080)])
+def test_split_few_weight_tiles_of_many_rows(qtype, k, dtype):
+    """More than 128 rows against one to a few weight tiles: several tiles of at most 128 rows instead of pairs, the last of them ragged."""
+    for m, n in ((129, 1), (200, 300), (257, 130), (700, 1000), (1025, 512)):
+        x, w, wd = _case(qtype, dtype, m, n, k)
+        _close(kernels.gemm_rcr(x, w, qtype), x.double() @ wd.T, dtype, 2)
