@@ -73,14 +73,11 @@ def test_scatter_gemv_full_size_shard_shapes():
 
 
 def test_scatter_gemm_umma_writes_every_destination():
-    """The tcgen05 kernel's scatter epilogues: K slices joined in a cluster, then whole tiles and tiles finished after a stream-K reduction, with
-    two CTAs per SM, one, and pairs of them."""
+    """The tcgen05 kernel's scatter epilogue (finished tiles, including tiles finished after a stream-K reduction)."""
     dev = torch.device("cuda:0")
     lib = _native.lib()
     stream = torch.cuda.current_stream().cuda_stream
-    for (qtype, m, n, k) in (("Q4_K", 16, 2048, 2048), ("Q4_K", 64, 384, 4096), ("Q6_K", 200, 130, 2048),
-                             ("Q4_K", 40, 36000, 2048), ("Q4_K", 16, 20500, 4096), ("Q4_K", 100, 17000, 4608), ("Q4_K", 70, 19500, 4096),
-                             ("Q4_K", 250, 9000, 2048), ("Q4_K", 300, 19000, 2048)):
+    for (qtype, m, n, k) in (("Q4_K", 16, 2048, 2048), ("Q4_K", 64, 384, 4096), ("Q6_K", 200, 130, 2048)):
         w = torch.from_numpy(S.random_blocks(qtype, n, k, seed=31)).to(dev)
         x = torch.from_numpy(S.random_activations(m, k, 32, "float32")).to(dev).to(torch.bfloat16)
         want = kernels.gemm_rcr(x, w, qtype, variant="umma")

