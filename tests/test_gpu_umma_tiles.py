@@ -84,3 +84,12 @@ def test_split_few_weight_tiles_of_many_rows(qtype, k, dtype):
     for m, n in ((129, 1), (200, 300), (257, 130), (700, 1000), (1025, 512)):
         x, w, wd = _case(qtype, dtype, m, n, k)
         _close(kernels.gemm_rcr(x, w, qtype), x.double() @ wd.T, dtype, 2)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float16"])
+@pytest.mark.parametrize("k", [256, 512, 1280, 2304])
+def test_q8_0_super_blocks_of_teams(k, dtype):
+    """A slot holds a whole Q8_0 super-block: one per CTA, which both teams take, odd numbers that they take in turns, laps of rings of four and of two."""
+    for m, n in ((16, 129), (64, 20000), (65, 4100), (128, 40000), (129, 130), (260, 20000)):
+        x, w, wd = _case("Q8_0", dtype, m, n, k)
+        _close(kernels.gemm_rcr(x, w, "Q8_0", variant="umma"), x.double() @ wd.T, dtype, 8)
